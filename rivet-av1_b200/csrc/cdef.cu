@@ -413,7 +413,7 @@ __device__ __forceinline__ void cdef_wait_lf(const FrameDesc& f, const uint32_t*
 template <int R, bool LFH>
 __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* __restrict__ frames,
                                                            const Item* __restrict__ items, int n_items, int wrows,
-                                                           uint32_t* __restrict__ flags) {
+                                                           int min_bd, uint32_t* __restrict__ flags) {
   AV1PF_TRACE_BEGIN();
   extern __shared__ __align__(16) int16_t cdef_smem_base[];  // [R][kDS] direction copy, then [3][wrows * kS]
   int16_t* const dwin = cdef_smem_base;
@@ -465,6 +465,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* _
       cdef_wait_lf<R>(f, flags, sc, y0, tid);
     } else {
       pdl_wait();  // the loop filter's output is complete past this point
+      if (f.bd < min_bd) continue;
     }
     __syncthreads();  // the previous item is done with the windows and block states
     if (tid < R) bstate[tid] = st;
@@ -1026,25 +1027,37 @@ cudaError_t cdef_init() {
     e = cudaFuncSetAttribute(cdef_search_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSearchSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(cdef_search_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSearchSmem);
+  if (e == cudaSuccess) e = cdef_packed_init();
   return e;
 }
 
-void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, bool lfh, bool half, uint32_t* flags,
+void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, const CdefShape& c, uint32_t* flags,
                  cudaStream_t s) {
   if (n_items <= 0) return;
+  // Frames of up to 10 bits take the packed kernel, whose half precision holds
+  // their samples exactly (1080p 10-bit: 25.5 against 36.0 us); 12-bit frames,
+  // and launches with the fused horizontal pass, this file's. A launch of both kinds runs both kernels
+  // over the whole list, each leaving the other's frames alone.
+  const bool packed = c.shallow && !c.lfh;
+  if (packed) launch_cdef_packed(frames, items, n_items, c.half, c.tall, flags, s);
+  if (packed && !c.deep) return;
+  const int min_bd = packed ? 11 : 0;
   // without the fused horizontal pass the windows hold 2 border rows each
   // side: smaller windows, more CTAs per SM
-  const int R = half ? 32 : 64;
-  const int wrows = R + 2 * (lfh ? kTopLfh : 2);
+  const int R = c.half ? 32 : 64;
+  const int wrows = R + 2 * (c.lfh ? kTopLfh : 2);
   const int grid = min(n_items, kItemGrid);
-  if (half && lfh)
-    launch_pdl(cdef_kernel<32, true>, grid, 128, size_t(cdef_smem(32, true)), s, frames, items, n_items, wrows, flags);
-  else if (half)
-    launch_pdl(cdef_kernel<32, false>, grid, 128, size_t(cdef_smem(32, false)), s, frames, items, n_items, wrows, flags);
-  else if (lfh)
-    launch_pdl(cdef_kernel<64, true>, grid, 256, size_t(cdef_smem(64, true)), s, frames, items, n_items, wrows, flags);
+  auto go = [&](auto kernel) {
+    launch_pdl(kernel, grid, 4 * R, size_t(cdef_smem(R, c.lfh)), s, frames, items, n_items, wrows, min_bd, flags);
+  };
+  if (c.half && c.lfh)
+    go(cdef_kernel<32, true>);
+  else if (c.half)
+    go(cdef_kernel<32, false>);
+  else if (c.lfh)
+    go(cdef_kernel<64, true>);
   else
-    launch_pdl(cdef_kernel<64, false>, grid, 256, size_t(cdef_smem(64, false)), s, frames, items, n_items, wrows, flags);
+    go(cdef_kernel<64, false>);
 }
 
 void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, cudaStream_t s) {

@@ -1,0 +1,503 @@
+// cdef_packed.cu — the constrained directional enhancement filter (7.15) for
+// bit depths up to 10, two samples per lane in half precision
+// (cdef_packed.cuh shows why that is exact). 12-bit frames, and launches with
+// the horizontal loop-filter pass fused in, take cdef_kernel (cdef.cu).
+//
+// Reference: rivet-av1 src/decoder/postfilter.rs:266-513, src/dsp/cdef.rs:13-90.
+//
+// What bounds it: instruction issue. The constrained taps of the 32-bit
+// kernel were 70% of its 16.2 M warp instructions per 1080p frame, on the
+// integer ALU pipe (one instruction per two clocks). Here a tap is about 10
+// instructions for two samples instead of 12 for one, half of them on the
+// multiply-add pipe, which issues every clock. 1080p 10-bit 4:2:0 against the
+// 32-bit kernel: 36.0 -> 25.5 us (cold, under ncu), 16.2 M -> 10.0 M warp
+// instructions; the chain call 70.4 -> 64.1 us, a 4K 10-bit superres chain
+// 274 -> 243 us, a batch of 16 mixed frames 831 -> 706 us. What is left is
+// latency: loads at a CTA's start and barriers between its phases.
+//
+// Which samples share a word: in luma, rows r and r + 4 of an 8x8 block; in
+// chroma, the U and V samples of a position (one block's chroma planes take
+// the same strengths and direction). Every word column exists, so a tap at
+// any offset is one aligned 32-bit load. Word rows are kPS = 74 words apart
+// and a lane takes every second column: 74 = 10 mod 32, so the 4 rows x 8
+// columns (or, for 4-wide blocks, 2 rows x 8 blocks x 2 columns) of a warp's
+// load fall in 32 different banks. Row strides of 8 columns a lane would put
+// blocks 32 columns apart in one bank.
+#include "cdef_packed.cuh"
+#include "kernels.h"
+
+namespace av1pf {
+
+namespace {
+
+constexpr int kPS = 74;  // words between word rows
+constexpr int kDS = 72;  // direction-search copy: u16 between rows (16-byte aligned)
+
+constexpr int packed_smem(int R, bool tall) { return R * kDS * 2 + R * kPS * 4 + ((tall ? R : R / 2) + 4) * kPS * 4; }
+
+// The taps of one block (postfilter.rs:489-511), 48 bytes.
+struct alignas(16) PackedTaps {
+  PStrength pri;
+  uint32_t w0, w1;  // primary weights, in both halves
+  PStrength sec;
+  int16_t off[6];  // bytes: primary k0, k1, secondary lo k0, hi k0, lo k1, hi k1
+  int32_t mode;    // 0 both kinds, 1 primary only, 2 secondary only, 3 copy
+};
+static_assert(sizeof(PackedTaps) == 48, "three 16-byte loads");
+
+__device__ __forceinline__ PackedTaps make_packed_taps(int pri, int sec, int damping, int dir, int cs,
+                                                       const int16_t (*doff)[2]) {
+  PackedTaps t;
+  t.pri = packed_strength(pri, pri ? max(damping - floor_log2(uint32_t(pri)), 0) : 0);
+  t.sec = packed_strength(sec, sec ? max(damping - floor_log2(uint32_t(sec)), 0) : 0);
+  const bool odd = (pri >> cs) & 1;  // CDEF_PRI_TAPS: [4, 2] / [3, 3]
+  t.w0 = odd ? 0x42004200u : 0x44004400u;
+  t.w1 = odd ? 0x42004200u : 0x40004000u;
+  const int dlo = (dir + 6) & 7, dhi = (dir + 2) & 7;
+  t.off[0] = doff[dir][0];
+  t.off[1] = doff[dir][1];
+  t.off[2] = doff[dlo][0];
+  t.off[3] = doff[dhi][0];
+  t.off[4] = doff[dlo][1];
+  t.off[5] = doff[dhi][1];
+  t.mode = pri ? (sec ? 0 : 1) : (sec ? 2 : 3);
+  return t;
+}
+
+// Two filtered words (1024 + sample in each half) at c and two columns on; the
+// taps' addresses serve both. MODE as in PackedTaps; with one kind of tap the
+// weights sum to 12 < 16, so the result lies within the taps' range and needs
+// no clamp.
+template <int MODE>
+__device__ __forceinline__ void packed_px2(const uint32_t* c, const PackedTaps& t, uint32_t& o0, uint32_t& o1) {
+  const uint32_t xw[2] = {c[0], c[2]};
+  __half2 sum[2], mx[2], nx[2];
+  uint32_t mn[2];
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    sum[e] = as_h2(0u);
+    mx[e] = as_h2(xw[e]);
+    nx[e] = as_h2(xw[e] ^ 0x80008000u);
+    mn[e] = xw[e];
+  }
+#pragma unroll
+  for (int k = MODE == 2 ? 2 : 0; k < (MODE == 1 ? 2 : 6); k++) {
+    const __half2 w = as_h2(k == 0 ? t.w0 : k == 1 ? t.w1 : k < 4 ? 0x40004000u : 0x3c003c00u);  // CDEF_SEC_TAPS [2, 1]
+    const int off = t.off[k];
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(c) + (side ? -off : off));
+#pragma unroll
+      for (int e = 0; e < 2; e++) packed_tap<MODE == 0>(p[2 * e], nx[e], k < 2 ? t.pri : t.sec, w, sum[e], mx[e], mn[e]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    __half2 v = packed_round(sum[e], as_h2(xw[e]));
+    if (MODE == 0) v = __hmax2(__hmin2(v, mx[e]), as_h2(mn[e]));
+    (e ? o1 : o0) = as_u32(v);
+  }
+}
+
+// Costs of directions P and P + 4 of the 8x8 block at `s` (rows kDS apart,
+// samples >> (bitdepth - 8), 0 .. 255), less a constant that all directions
+// share. The reference sums squares of partial sums of (sample - 128), each
+// over n samples weighed by 840 / n (postfilter.rs:345-401). With S the
+// partial sum of the samples themselves, (S - 128 n)^2 * 840 / n =
+// S^2 * 840 / n - 256 * 840 * S + 128^2 * 840 * n, and the last two terms add
+// up to the same over every direction's bins: comparisons and the difference
+// of two costs need only the first. It is below 255^2 * 840 * 64 < 2^32.
+// Two neighbouring samples are added at once: a bin's 16-bit halves hold sums
+// of at most 8 * 255.
+template <int P>
+__device__ __forceinline__ void packed_cost_pair(const uint16_t* s, uint32_t& c1, uint32_t& c2) {
+  constexpr int NA = P == 0 ? 14 : (P == 2 ? 8 : 11);  // words of bins of direction P
+  constexpr int NB = P == 0 ? 14 : (P == 2 ? 4 : 10);  // and of P + 4
+  uint32_t a[NA], b[NB];
+#pragma unroll
+  for (int k = 0; k < NA; k++) a[k] = 0;
+#pragma unroll
+  for (int k = 0; k < NB; k++) b[k] = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const uint4 v = *reinterpret_cast<const uint4*>(s + i * kDS);
+    const uint32_t row[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {  // columns 2q (low half) and 2q + 1
+      // direction 0: bins i + j; 1: i + j/2; 2: i; 3: 3 + i - j/2
+      a[P == 0 ? i + 2 * q : P == 1 ? i + q : P == 2 ? i : 3 + i - q] += row[q];
+      // direction 4: 7 + i - j; 5: 3 - i/2 + j; 6: j; 7: i/2 + j
+      b[P == 0 ? i - 2 * q + 6 : P == 1 ? 3 - i / 2 + 2 * q : P == 2 ? q : i / 2 + 2 * q] += row[q];
+    }
+  }
+  auto lo = [](uint32_t w) { return w & 0xffffu; };
+  auto hi = [](uint32_t w) { return w >> 16; };
+  // 840 / n of bins of n = 1 .. 8 samples
+  constexpr uint32_t dv[9] = {0, 840, 420, 280, 210, 168, 140, 120, 105};
+  // bins of 1, 2 .. 8 .. 2, 1 samples
+  auto diag = [&](auto bin) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < 15; k++) {
+      const uint32_t v = bin(k);
+      c += v * v * dv[k < 8 ? k + 1 : 15 - k];
+    }
+    return c;
+  };
+  // bins of 2, 4, 6, 8, 8, 8, 8, 8, 6, 4, 2 samples
+  auto steep = [&](auto bin) {
+    uint32_t c = 0, full = 0;
+#pragma unroll
+    for (int k = 0; k < 11; k++) {
+      const uint32_t v = bin(k);
+      if (k >= 3 && k <= 7)
+        full += v * v;
+      else
+        c += v * v * dv[k < 3 ? 2 * k + 2 : 2 * (10 - k) + 2];
+    }
+    return c + full * dv[8];
+  };
+  if (P == 0) {
+    // a word's halves are bins k and k + 1 of direction 0, k + 1 and k of 4
+    c1 = diag([&](int k) { return (k < 14 ? lo(a[k < 14 ? k : 0]) : 0u) + (k > 0 ? hi(a[k > 0 ? k - 1 : 0]) : 0u); });
+    c2 = diag([&](int k) { return (k < 14 ? hi(b[k < 14 ? k : 0]) : 0u) + (k > 0 ? lo(b[k > 0 ? k - 1 : 0]) : 0u); });
+  } else if (P == 2) {
+    uint32_t f1 = 0, f2 = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const uint32_t v = lo(a[k]) + hi(a[k]), u = (k & 1) ? hi(b[k >> 1 & 3]) : lo(b[k >> 1 & 3]);
+      f1 += v * v;
+      f2 += u * u;
+    }
+    c1 = f1 * dv[8];
+    c2 = f2 * dv[8];
+  } else {
+    c1 = steep([&](int k) { return lo(a[k < NA ? k : 0]) + hi(a[k < NA ? k : 0]); });
+    c2 = steep([&](int k) { return (k < 10 ? lo(b[k < 10 ? k : 0]) : 0u) + (k > 0 ? hi(b[k > 0 ? k - 1 : 0]) : 0u); });
+  }
+}
+
+// Eight samples of a row: as loaded, and biased two to a word. INSIDE: the
+// caller's whole window lies in the mode-info area; otherwise samples outside
+// it are unavailable (gx is a multiple of 8, so no chunk straddles column 0).
+template <bool INSIDE>
+__device__ __forceinline__ uint4 load_chunk(const uint8_t* at, int sb, int gx, int gy, int xlim, int ylim) {
+  if (!INSIDE && (gy < 0 || gy >= ylim || gx < 0 || gx + 8 > xlim)) return make_uint4(0u, 0u, 0u, 0u);
+  if (sb == 2) return *reinterpret_cast<const uint4*>(at);
+  const uint2 h = *reinterpret_cast<const uint2*>(at);
+  return make_uint4(h.x, h.y, 0u, 0u);
+}
+template <bool INSIDE>
+__device__ __forceinline__ uint4 bias_chunk(const uint4& q, const uint8_t* at, int sb, int gx, int gy, int xlim, int ylim) {
+  if (!INSIDE && (gy < 0 || gy >= ylim || gx < 0 || gx + 8 > xlim)) {
+    uint32_t o[4] = {kPNA, kPNA, kPNA, kPNA};
+    if (gy >= 0 && gy < ylim && gx >= 0)
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        if (gx + e < xlim) {
+          const uint32_t v = 0x6400u | uint32_t(sb == 1 ? at[e] : reinterpret_cast<const uint16_t*>(at)[e]);
+          o[e >> 1] = (e & 1) ? ((o[e >> 1] & 0xffffu) | (v << 16)) : ((o[e >> 1] & 0xffff0000u) | v);
+        }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  if (sb == 2) return make_uint4(q.x | kPBias, q.y | kPBias, q.z | kPBias, q.w | kPBias);
+  return make_uint4(__byte_perm(q.x, 0x64646464u, 0x4140), __byte_perm(q.x, 0x64646464u, 0x4342),
+                    __byte_perm(q.y, 0x64646464u, 0x4140), __byte_perm(q.y, 0x64646464u, 0x4342));
+}
+
+// Eight words of low halves `a` and high halves `b` at window chunk ch of nch
+// (of the first and the last only the two columns next to the superblock).
+__device__ __forceinline__ void put_words(uint32_t* row, int ch, int nch, const uint4& a, const uint4& b) {
+  uint32_t* dst = row + ch * 8 - 6;
+  const bool first = ch == 0, last = ch == nch - 1;
+  if (!first)
+    *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(a.x, b.x, 0x5410), __byte_perm(a.x, b.x, 0x7632));
+  if (!first && !last) {
+    *reinterpret_cast<uint2*>(dst + 2) = make_uint2(__byte_perm(a.y, b.y, 0x5410), __byte_perm(a.y, b.y, 0x7632));
+    *reinterpret_cast<uint2*>(dst + 4) = make_uint2(__byte_perm(a.z, b.z, 0x5410), __byte_perm(a.z, b.z, 0x7632));
+  }
+  if (!last)
+    *reinterpret_cast<uint2*>(dst + 6) = make_uint2(__byte_perm(a.w, b.w, 0x5410), __byte_perm(a.w, b.w, 0x7632));
+}
+
+// Stages the windows (postfilter.rs:464-488) in 8-sample chunks. Luma: a
+// thread takes one chunk of rows i, i + 4, i + 8 and i + 12, which are the low
+// and high halves of three word rows, so a row is loaded once and (but for the
+// thread's first and last) used twice. Chroma: one chunk of a U and of a V
+// row. All of a thread's first loads are in flight together.
+template <int R, bool INSIDE>
+__device__ __forceinline__ void stage_windows(const FrameDesc& f, int sc, int y0, uint32_t* lw, uint32_t* cw,
+                                              uint16_t* dwin, int tid) {
+  constexpr int NT = 4 * R;
+  constexpr int kSeg = (R / 4 + 2) / 3;  // threads down a chunk column and row class
+  static_assert(40 * kSeg <= NT, "one luma task a thread");
+  const int sb = f.sb, cs = f.bd - 8, sx = f.ssx, sy = f.ssy;
+  const int lxl = f.mi_cols * 4, lyl = f.mi_rows * 4, cxl = lxl >> sx, cyl = lyl >> sy;
+  const int cch = sx ? 6 : 10, cinv = sx ? 10923 : 6554;  // chroma chunks per row; ceil(2^16 / cch)
+  const int nc = f.np > 1 ? ((R >> sy) + 4) * cch : 0;
+  const int rest = (tid * 6554) >> 16, lch = tid - rest * 10;
+  const int li = (rest & 3) + 12 * (rest >> 2);  // first word row
+  const int lgx = sc * 64 - 8 + lch * 8, lgy = y0 + li - 2;
+  const bool ltask = tid < 40 * kSeg;
+  const int64_t pitch4 = f.cur[0].stride * 4 * sb;
+  const uint8_t* lat = f.cur[0].p + (int64_t(lgy) * f.cur[0].stride + lgx) * sb;
+  uint4 l[4], u, v;
+#pragma unroll
+  for (int e = 0; e < 4; e++)
+    if (ltask && li + 4 * e < R + 4) l[e] = load_chunk<INSIDE>(lat + e * pitch4, sb, lgx, lgy + 4 * e, lxl, lyl);
+  int ci, cc, gx, gy;
+  const uint8_t *uat, *vat;
+  auto load_chroma = [&](int k) {
+    ci = (k * cinv) >> 16;
+    cc = k - ci * cch;
+    gx = ((sc * 64) >> sx) - 8 + cc * 8;
+    gy = (y0 >> sy) + ci - 2;
+    uat = f.cur[1].p + (int64_t(gy) * f.cur[1].stride + gx) * sb;
+    vat = f.cur[2].p + (int64_t(gy) * f.cur[2].stride + gx) * sb;
+    u = load_chunk<INSIDE>(uat, sb, gx, gy, cxl, cyl);
+    v = load_chunk<INSIDE>(vat, sb, gx, gy, cxl, cyl);
+  };
+  if (tid < nc) load_chroma(tid);
+  if (ltask) {
+    uint4 a = bias_chunk<INSIDE>(l[0], lat, sb, lgx, lgy, lxl, lyl);
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      const int i = li + 4 * e;
+      if (i >= R) break;
+      const uint4 b = bias_chunk<INSIDE>(l[e + 1], lat + (e + 1) * pitch4, sb, lgx, lgy + 4 * (e + 1), lxl, lyl);
+      put_words(lw + i * kPS, lch, 10, a, b);
+      if (lch != 0 && lch != 9) {
+        // the superblock's own rows, at 8 bits, for the direction search: the
+        // low halves' row of each word row, and the last two of the high halves'
+        auto to8 = [&](const uint4& q) {
+          return make_uint4((q.x >> cs) & 0xff00ffu, (q.y >> cs) & 0xff00ffu, (q.z >> cs) & 0xff00ffu,
+                            (q.w >> cs) & 0xff00ffu);
+        };
+        uint16_t* dd = dwin + (i - 2) * kDS + (lch - 1) * 8;
+        if (i >= 2) *reinterpret_cast<uint4*>(dd) = to8(a);
+        if (i >= R - 4 && i < R - 2) *reinterpret_cast<uint4*>(dd + 4 * kDS) = to8(b);
+      }
+      a = b;
+    }
+  }
+  for (int k = tid; k < nc;) {
+    put_words(cw + ci * kPS, cc, cch, bias_chunk<INSIDE>(u, uat, sb, gx, gy, cxl, cyl),
+              bias_chunk<INSIDE>(v, vat, sb, gx, gy, cxl, cyl));
+    k += NT;  // more chunks than threads: chroma without vertical subsampling
+    if (k < nc) load_chroma(k);
+  }
+}
+
+// With readiness flags: waits (threads 0..47, one flag each) for the
+// loop-filter tiles under the CTA's windows: plane rows (y0 >> sy) - 2 ..
+// ((y0 + R) >> sy) + 1 and 8 columns past the superblock on either side.
+template <int R>
+__device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const uint32_t* flags, int sc, int y0, int tid) {
+  if (tid >= 48) return;
+  const int p = tid >> 4, dy = (tid >> 2) & 3, dx = tid & 3;
+  if (p >= f.np || f.lf_tiles_x[p] == 0) return;
+  const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
+  const int W = f.cur[p].w, H = f.cur[p].h;
+  const int r0 = max((y0 >> sy) - 2, 0), r1 = min(((y0 + R) >> sy) + 1, H - 1);
+  const int c0 = max(((sc * 64) >> sx) - 8, 0), c1 = min(((sc * 64 + 64) >> sx) + 7, W - 1);
+  const int ty = (r0 >> 6) + dy, tx = (c0 >> 6) + dx;
+  if (r0 > r1 || c0 > c1 || ty > (r1 >> 6) || tx > (c1 >> 6)) return;
+  flag_wait(flags + f.lf_flag_base[p] + ty * f.lf_tiles_x[p] + tx);
+}
+
+}  // namespace
+
+// Item: R luma rows of a superblock (x0 = SB column, y0 = SB row, a = which R
+// rows). 4R threads, one warp per row of 8x8 blocks. Frames above 10 bits are
+// left to cdef_kernel. The chroma window has room for `R` rows and 4 more
+// when the launch was sized for frames without vertical subsampling.
+template <int R>
+__global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const FrameDesc* __restrict__ frames,
+                                                                  const Item* __restrict__ items, int n_items,
+                                                                  uint32_t* __restrict__ flags) {
+  AV1PF_TRACE_BEGIN();
+  constexpr int NT = 4 * R;
+  extern __shared__ __align__(16) uint8_t packed_base[];
+  uint16_t* const dwin = reinterpret_cast<uint16_t*>(packed_base);                 // [R][kDS]
+  uint32_t* const lw = reinterpret_cast<uint32_t*>(packed_base + R * kDS * 2);     // [R][kPS]: rows i - 2 and i + 2
+  uint32_t* const cw = lw + R * kPS;                                               // chroma: U and V, 2 rows above
+  __shared__ uint32_t cost[8][R];
+  __shared__ PackedTaps taps[2][R];  // luma, chroma
+  __shared__ uint8_t bstate[R];      // 0 = outside the MI area, 1 = copy, 2 = filter
+  __shared__ int16_t doff[8][2];     // CDEF_DIRECTIONS in bytes of the windows
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  if (tid < 16) doff[tid >> 1][tid & 1] = int16_t((c_cdef_dirs[tid >> 1][tid & 1][0] * kPS + c_cdef_dirs[tid >> 1][tid & 1][1]) * 4);
+  FOR_EACH_ITEM(it, n_items) {
+    const Item item = items[it];
+    const FrameDesc& f = frames[item.frame];
+    const int sc = item.x0, sr = item.y0;
+    const int y0 = sr * 64 + item.a * R;  // luma row of the CTA's first row
+    const int np = f.np, sb = f.sb;
+    const int cs = f.bd - 8;
+    const int idx = f.cdef_idx[int64_t(sr) * f.cdef_stride + sc];  // postfilter.rs:285
+    // --- per 8x8: inside the MI area? skipped? (postfilter.rs:281-287, 306-310);
+    // the maps are inputs of the chain: read before waiting for the loop filter ---
+    uint8_t st = 0;
+    if (tid < R) {
+      const int r = (y0 >> 2) + 2 * (tid >> 3), c = sc * 16 + 2 * (tid & 7);
+      if (r < f.mi_rows && c < f.mi_cols) {
+        st = 1;
+        if (idx >= 0) {
+          const av1pf_mi* m = f.mi + int64_t(r) * f.mi_stride + c;
+          const int ms = f.mi_stride;
+          if (!(m[0].skip_segment & m[ms].skip_segment & m[1].skip_segment & m[ms + 1].skip_segment & AV1PF_MI_SKIP))
+            st = 2;
+        }
+      }
+    }
+    if (flags) {
+      pdl_trigger();
+      packed_wait_lf<R>(f, flags, sc, y0, tid);  // only the loop-filter tiles this CTA reads
+    } else {
+      pdl_wait();  // the loop filter's output is complete past this point
+      if (f.bd > 10) continue;
+    }
+    __syncthreads();  // the previous item is done with the windows and block states
+    if (tid < R) bstate[tid] = st;
+    const int csx = f.ssx, csy = f.ssy;
+    // the chunks reach 8 columns past the superblock, 16 luma columns in subsampled chroma
+    if (sc > 0 && sc * 64 + 80 <= f.mi_cols * 4 && y0 >= 4 && y0 + R + 4 <= f.mi_rows * 4)
+      stage_windows<R, true>(f, sc, y0, lw, cw, dwin, tid);
+    else
+      stage_windows<R, false>(f, sc, y0, lw, cw, dwin, tid);
+    __syncthreads();
+    // --- direction search (postfilter.rs:345-401): each thread two directions of one block ---
+    {
+      const int pair = warp & 3;
+      const int b = (warp >> 2) * 32 + lane;
+      if (bstate[b] == 2) {
+        const uint16_t* s = &dwin[(b >> 3) * 8 * kDS + (b & 7) * 8];
+        uint32_t c1, c2;
+        switch (pair) {
+          case 0: packed_cost_pair<0>(s, c1, c2); break;
+          case 1: packed_cost_pair<1>(s, c1, c2); break;
+          case 2: packed_cost_pair<2>(s, c1, c2); break;
+          default: packed_cost_pair<3>(s, c1, c2); break;
+        }
+        cost[pair][b] = c1;
+        cost[pair + 4][b] = c2;
+      }
+    }
+    __syncthreads();
+    // --- per-block strengths and taps (postfilter.rs:311-341): luma in threads 0 .. R - 1, chroma in the next R ---
+    if (tid < 2 * R) {
+      const int b = tid & (R - 1), uv = tid >= R ? 1 : 0;
+      int pri = 0, sec = 0, dir = 0;
+      if (bstate[b] == 2) {
+        uint32_t best = cost[0][b];
+        int y_dir = 0;
+#pragma unroll
+        for (int d = 1; d < 8; d++) {
+          const uint32_t cd = cost[d][b];
+          if (cd > best) {
+            best = cd;
+            y_dir = d;
+          }
+        }
+        if (uv) {
+          pri = f.cdef_uv_pri[idx] << cs;
+          sec = f.cdef_uv_sec[idx] << cs;
+          dir = pri == 0 ? 0 : c_cdef_uv_dir[csx][csy][y_dir];
+        } else {
+          const int32_t var = int32_t(best - cost[(y_dir + 4) & 7][b]) >> 10;
+          const int p0 = f.cdef_y_pri[idx] << cs;
+          sec = f.cdef_y_sec[idx] << cs;
+          dir = p0 == 0 ? 0 : y_dir;
+          const int var_str = (var >> 6) != 0 ? min(floor_log2(uint32_t(var >> 6)), 12) : 0;
+          pri = var != 0 ? (p0 * (4 + var_str) + 8) >> 4 : 0;
+        }
+      }
+      taps[uv][b] = make_packed_taps(pri, sec, f.cdef_damping + cs - uv, dir, cs, doff);
+    }
+    __syncthreads();
+    // --- filter + write (postfilter.rs:405-442): a warp per block row. Luma
+    // and 8-wide chroma: 4 blocks x 4 rows x 2 columns of lanes, then 4 columns
+    // on; 4-wide chroma: 8 blocks x 2 rows x 2. A lane's two words are 2
+    // columns apart; lane pairs then exchange them, so that the even lane
+    // stores 4 samples of the low halves' row (or plane) and the odd lane 4 of
+    // the high halves' ---
+    {
+      const int h = lane & 1, sel = h ? 0x7632 : 0x5410;
+      const int cbh = 8 >> csy;
+      const int npass = 2 + (np > 1 ? cbh / 2 : 0);
+      for (int pass = 0; pass < npass; pass++) {
+        const bool luma = pass < 2, wide = luma || !csx;
+        const int q = luma ? pass : pass - 2;
+        const int bx = wide ? (q & 1) * 4 + (lane >> 3) : lane >> 2;
+        const int row = wide ? ((lane >> 1) & 3) + (luma ? 0 : (q >> 1) * 4) : ((lane >> 1) & 1) + q * 2;
+        const int b = warp * 8 + bx;
+        const int lx = bx * (wide ? 8 : 4), ly = warp * (luma ? 8 : cbh) + row;
+        const uint32_t* c = (luma ? lw : cw) + (ly + 2) * kPS + 2 + lx + h;
+        const PackedTaps t = taps[luma ? 0 : 1][b];
+        const DPlane& dst = f.cdef[luma ? 0 : 1 + h];
+        const int gx = ((sc * 64) >> (luma ? 0 : csx)) + lx, gy = (y0 >> (luma ? 0 : csy)) + ly + (luma ? 4 * h : 0);
+        uint8_t* at = dst.p + (int64_t(gy) * dst.stride + gx) * sb;
+        const bool live = bstate[b] != 0;
+        for (int cols = wide ? 2 : 1; cols > 0; cols--) {
+          uint32_t o0, o1;
+          if (t.mode == 0) {
+            packed_px2<0>(c, t, o0, o1);
+          } else if (t.mode == 1) {
+            packed_px2<1>(c, t, o0, o1);
+          } else if (t.mode == 2) {
+            packed_px2<2>(c, t, o0, o1);
+          } else {
+            o0 = c[0];
+            o1 = c[2];
+          }
+          o0 ^= kPBias;  // 0x6400 | v in each half, v < 1024
+          o1 ^= kPBias;
+          const uint32_t p0 = __shfl_xor_sync(0xffffffffu, o0, 1), p1 = __shfl_xor_sync(0xffffffffu, o1, 1);
+          const uint32_t w0 = __byte_perm(h ? p0 : o0, h ? o0 : p0, sel), w1 = __byte_perm(h ? p1 : o1, h ? o1 : p1, sel);
+          if (live) {
+            if (sb == 2)
+              *reinterpret_cast<uint2*>(at) = make_uint2(w0, w1);
+            else
+              *reinterpret_cast<uint32_t*>(at) = __byte_perm(w0, w1, 0x6420);
+          }
+          c += 4;
+          at += 4 * sb;
+        }
+      }
+    }
+    __syncthreads();
+    if (flags && tid == 0) {
+      // the rows are in the CDEF planes: the half superblocks' flags
+      uint32_t* fl = flags + f.cdef_flag_base + 2 * sr * f.cdef_sbc + sc;
+      if (R == 64) {
+        flag_set(fl);
+        flag_set(fl + f.cdef_sbc);
+      } else {
+        flag_set(fl + item.a * f.cdef_sbc);
+      }
+    }
+  }
+  AV1PF_TRACE_END(2);
+}
+
+cudaError_t cdef_packed_init() {
+  cudaError_t e = cudaFuncSetAttribute(cdef_packed_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       packed_smem(64, true));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(cdef_packed_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             packed_smem(32, true));
+  return e;
+}
+
+void launch_cdef_packed(const FrameDesc* frames, const Item* items, int n_items, bool half, bool tall, uint32_t* flags,
+                        cudaStream_t s) {
+  if (n_items <= 0) return;
+  const int grid = min(n_items, kItemGrid);
+  if (half)
+    launch_pdl(cdef_packed_kernel<32>, grid, 128, size_t(packed_smem(32, tall)), s, frames, items, n_items, flags);
+  else
+    launch_pdl(cdef_packed_kernel<64>, grid, 256, size_t(packed_smem(64, tall)), s, frames, items, n_items, flags);
+}
+
+}  // namespace av1pf

@@ -61,11 +61,23 @@ void launch_lf_edges(int pass, const FrameDesc* frames, const uint64_t* list, co
 void launch_dsp_lf(int32_t* edges, const av1pf_lf_edge_params* prm, int n, cudaStream_t s);
 
 // CDEF (cdef.cu)
-// `lfh`: some item has the horizontal loop-filter pass fused (item kind 1).
-// `half`: the items are half superblocks (Item::a = 0 top, 1 bottom).
-// `flags`: the readiness flags the kernel waits for and sets, or null.
-void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, bool lfh, bool half, uint32_t* flags,
+// What a launch's frames are, as far as the choice of kernel and its shared
+// memory go.
+struct CdefShape {
+  bool lfh = false;      // some item has the horizontal loop-filter pass fused (item kind 1)
+  bool half = false;     // the items are half superblocks (Item::a = 0 top, 1 bottom)
+  bool shallow = false;  // some frame has at most 10 bits
+  bool deep = false;     // some frame has 12 bits
+  bool tall = false;     // some frame's chroma is not vertically subsampled
+};
+// `flags`: the readiness flags the kernel waits for and sets, or null (as it
+// must be for a launch with both shallow and deep frames).
+void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, const CdefShape& c, uint32_t* flags,
                  cudaStream_t s);
+// The part of it for frames of up to 10 bits (cdef_packed.cu).
+void launch_cdef_packed(const FrameDesc* frames, const Item* items, int n_items, bool half, bool tall, uint32_t* flags,
+                        cudaStream_t s);
+cudaError_t cdef_packed_init();
 // Sets cdef_kernel's dynamic shared-memory limit on the current device.
 cudaError_t cdef_init();
 void launch_dsp_cdef(const int32_t* win, const av1pf_cdef_taps* taps, uint16_t* res, int n, cudaStream_t s);

@@ -179,8 +179,7 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
       v->clear();
     plan.edge_cap = 0;
     plan.any_hlist = false;
-    plan.any_lfh = false;
-    plan.cdef_half = false;
+    plan.cdef = CdefShape{};
     plan.sr_row_max = 0;
     plan.any_lf = plan.any_cdef = plan.any_sr = plan.any_lr = plan.any_grain = plan.any_out = false;
     plan.off_frames = plan.off_lf = plan.off_lft = plan.off_lff = plan.off_cdef = plan.off_sr = plan.off_lr = plan.off_grain =
@@ -359,7 +358,9 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
     if (cdef_on) {
       plan.any_cdef = true;
       const int sbr = (i->mi_rows + 15) / 16, sbc = (i->mi_cols + 15) / 16;
-      if (d.lfh_mask) plan.any_lfh = true;
+      if (d.lfh_mask) plan.cdef.lfh = true;
+      (i->bit_depth > 10 ? plan.cdef.deep : plan.cdef.shallow) = true;
+      if (np > 1 && !i->subsampling_y) plan.cdef.tall = true;
       // one flag per half superblock
       d.cdef_flag_base = int32_t(nflags);
       d.cdef_sbc = sbc;
@@ -494,12 +495,13 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
   plan.scratch_bytes = align_up(bump.used, 256);
   if (!items) return AV1PF_OK;  // the lists and their layout are the previous call's
   plan.flag_sync = flags_fit && plan.any_lf && plan.any_cdef && plan.any_lr && !plan.any_sr && !plan.any_hlist &&
-                   plan.lf_items.empty() && plan.lft_items.empty() && plan.copy_items.empty();
+                   plan.lf_items.empty() && plan.lft_items.empty() && plan.copy_items.empty() &&
+                   !(plan.cdef.deep && plan.cdef.shallow);
   plan.n_flags = plan.flag_sync ? nflags : 0;
   // At most one wave of superblocks (4 CTAs on each SM): CDEF runs a CTA per
   // half superblock instead, so the SMs end up with equal shares.
-  plan.cdef_half = !plan.cdef_items.empty() && plan.cdef_items.size() <= size_t(kNumSMs) * 4;
-  if (plan.cdef_half) {
+  plan.cdef.half = !plan.cdef_items.empty() && plan.cdef_items.size() <= size_t(kNumSMs) * 4;
+  if (plan.cdef.half) {
     std::vector<Item> halves;
     halves.reserve(plan.cdef_items.size() * 2);
     for (const Item& it : plan.cdef_items) {
@@ -641,7 +643,7 @@ void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t s
     launch_lf_fused(frames, items(plan.off_lff), int(plan.lff_items.size()), sync, s);
   mark(1);
   if (plan.any_cdef)
-    launch_cdef(frames, items(plan.off_cdef), int(plan.cdef_items.size()), plan.any_lfh, plan.cdef_half, sync, s);
+    launch_cdef(frames, items(plan.off_cdef), int(plan.cdef_items.size()), plan.cdef, sync, s);
   mark(2);
   if (plan.any_sr) launch_superres(frames, items(plan.off_sr), int(plan.sr_items.size()), plan.sr_row_max, s);
   mark(3);

@@ -13,6 +13,7 @@
 
 #include "av1pf.h"
 #include "desc.h"
+#include "kernels.h"
 
 namespace av1pf {
 
@@ -52,8 +53,7 @@ struct Plan {
   uint32_t edge_cap = 0;
   size_t scratch_bytes = 0;   // bytes of per-frame scratch (planes, grain)
   bool any_hlist = false;  // some plane's horizontal loop-filter edges run as their own pass
-  bool any_lfh = false;    // some frame's horizontal loop-filter edges run inside the CDEF kernel
-  bool cdef_half = false;  // CDEF items are half superblocks (Item::a: 0 top, 1 bottom)
+  CdefShape cdef;          // the CDEF launch (lfh: some frame's horizontal loop-filter edges run inside it)
   // the stages can wait on readiness flags (FrameDesc::lf_flag_base ...)
   // instead of on the whole previous stage: every frame runs the fused loop filter,
   // CDEF and loop restoration, without superres or the horizontal
