@@ -301,10 +301,12 @@ int av1pf_output_noalloc(const av1pf_frame_info* info, const av1pf_params* param
  * the LR frame (the reference frame, RefData.frame) into `ref_out` over the
  * visible area, and — when `frame_out` is not NULL — the packed output frame
  * as av1pf_output does. Scratch comes from the context. The kernels are
- * queued on `stream`; the call returns once the frame's descriptors are on
- * the device. The context keeps two descriptor buffers in turn, so the call
- * may first wait on the host for the chain it queued two calls earlier:
- * a caller runs at most about two calls ahead of the GPU per context. */
+ * queued on `stream` and the call returns: the frame's descriptor travels
+ * with the launches. Only a call whose structure (geometry, stages, planes
+ * filtered) differs from that of the calls before it first uploads its work
+ * lists, and may wait on the host for the chain queued two calls earlier.
+ * The parameters are read before the call returns; the planes and maps when
+ * the kernels run. */
 int av1pf_chain(av1pf_ctx* ctx, const av1pf_frame_info* info,
                 const av1pf_params* params, const av1pf_maps* maps,
                 const av1pf_plane* in, av1pf_plane* ref_out,

@@ -167,9 +167,10 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     host_key = key_scratch;
     host_ready = true;
   }
-  // Two descriptor buffers in turn: call k's upload runs on its own stream
-  // while call k-1's kernels read the other buffer, and a buffer is
-  // rewritten only after the launches that read it are done.
+  // Two descriptor buffers in turn, each with the work lists of the structure
+  // it was last used for, readiness flags and film-grain scratch. A call whose
+  // kernels take the descriptor as a parameter and whose buffer holds its lists
+  // uploads nothing: it only launches.
   cudaError_t e = cudaSuccess;
   if (!upload) {
     e = cudaStreamCreateWithFlags(&upload, cudaStreamNonBlocking);
@@ -178,6 +179,17 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     if (e != cudaSuccess) return cuda_status(e, "descriptor stream");
   }
+  // A capture replays its launches with the epoch they were captured with, so
+  // its stages wait for one another whole; its templates join the capture.
+  cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap_status) != cudaSuccess) cudaGetLastError();
+  const bool capturing = cap_status != cudaStreamCaptureStatusNone;
+  if (epoch >= kEpochMax) {
+    // flags are compared with the epoch: before it could wrap, both buffers'
+    // are cleared by a fresh upload
+    for (MetaSlot& q : metas) q.ready = false;
+    epoch = 0;
+  }
   MetaSlot& m = metas[meta_next];
   meta_next ^= 1;
   if (m.dev.size < plan.meta_bytes + 256) {
@@ -185,15 +197,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     m.ready = false;
     if ((rc = ensure(m.dev, plan.meta_bytes + 256)) != AV1PF_OK) return rc;
   }
-  // the pinned staging buffer: its last upload must be done before it is
-  // overwritten
-  if (m.used && (e = cudaEventSynchronize(m.uploaded)) != cudaSuccess) return cuda_status(e, "staging wait");
-  if ((rc = ensure_host(m.host, plan.upload_bytes + 256)) != AV1PF_OK) return rc;
-  cudaStream_t ups = upload_override ? upload_override : upload;
-  if (m.used) cudaStreamWaitEvent(ups, m.done, 0);
-  pipe_trace::mark(6, ups);
   uint8_t* dmeta = static_cast<uint8_t*>(m.dev.ptr);
-  uint8_t* hmeta = static_cast<uint8_t*>(m.host.ptr);
   // film grain: this buffer's own scratch (the previous call's output kernel
   // reads the other buffer's), so the template kernel can start at once
   for (size_t fi = 0; fi < plan.frames.size() && fi < plan.grain_meta.size(); fi++) {
@@ -201,37 +205,54 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     plan.frames[fi].grain = reinterpret_cast<GrainScratch*>(dmeta + plan.off_grain_meta + plan.grain_meta[fi].first);
     plan.frames[fi].grain_off = dmeta + plan.off_grain_meta + plan.grain_meta[fi].second;
   }
-  if (m.ready && m.key == key_scratch) {
-    const size_t fbytes = plan.frames.size() * sizeof(FrameDesc);
-    std::memcpy(hmeta + plan.off_frames, plan.frames.data(), fbytes);
-    e = cudaMemcpyAsync(dmeta + plan.off_frames, hmeta + plan.off_frames, fbytes, cudaMemcpyHostToDevice, ups);
+  const bool resident = m.ready && m.key == key_scratch;
+  if (plan.by_value && resident) {
+    // the scratch's last readers are the launches that used this buffer before
+    if (plan.any_grain && m.used && !capturing) e = cudaStreamWaitEvent(side, m.done, 0);
   } else {
-    m.ready = false;
-    pack_meta(plan, hmeta);
-    e = cudaMemcpyAsync(dmeta, hmeta, plan.upload_bytes, cudaMemcpyHostToDevice, ups);
-    if (e == cudaSuccess) {
+    // the pinned staging buffer: its last upload must be done before it is
+    // overwritten; the device buffer: its last readers
+    if (m.used && (e = cudaEventSynchronize(m.uploaded)) != cudaSuccess) return cuda_status(e, "staging wait");
+    if ((rc = ensure_host(m.host, plan.upload_bytes + 256)) != AV1PF_OK) return rc;
+    uint8_t* hmeta = static_cast<uint8_t*>(m.host.ptr);
+    cudaStream_t ups = upload_override ? upload_override : upload;
+    if (m.used) cudaStreamWaitEvent(ups, m.done, 0);
+    pipe_trace::mark(6, ups);
+    if (resident) {
+      const size_t fbytes = plan.frames.size() * sizeof(FrameDesc);
+      std::memcpy(hmeta + plan.off_frames, plan.frames.data(), fbytes);
+      e = cudaMemcpyAsync(dmeta + plan.off_frames, hmeta + plan.off_frames, fbytes, cudaMemcpyHostToDevice, ups);
+    } else {
+      m.ready = false;
+      pack_meta(plan, hmeta);
+      e = cudaMemcpyAsync(dmeta, hmeta, plan.upload_bytes, cudaMemcpyHostToDevice, ups);
+    }
+    // the loop filter's edge-list counters start at zero: cleared here, in the
+    // upload's stream order, so the chain's stream holds kernels only
+    if (e == cudaSuccess) e = cudaMemsetAsync(dmeta + plan.off_counts, 0, 16, ups);
+    // and so do the readiness flags of a new layout, below any epoch
+    if (e == cudaSuccess && plan.n_flags && !resident)
+      e = cudaMemsetAsync(dmeta + plan.off_flags, 0, plan.n_flags * 4, ups);
+    if (e == cudaSuccess && !resident) {
       m.key = key_scratch;
       m.ready = true;
     }
+    if (e == cudaSuccess) e = cudaEventRecord(m.uploaded, ups);
+    pipe_trace::mark(7, ups);
+    // The kernels read the upload: the host waits for it rather than the
+    // chain's stream. It waited only for the chain that used this buffer two
+    // calls ago, so it has usually landed already; and with nothing between
+    // the previous call's last kernel and this call's first on the stream,
+    // programmatic dependent launch chains them (a stream-side wait here made
+    // every call boundary a full one: 9 us per 1080p frame).
+    if (e == cudaSuccess) e = stream_upload_wait ? cudaStreamWaitEvent(s, m.uploaded, 0) : cudaEventSynchronize(m.uploaded);
+    if (e == cudaSuccess && stream_upload_wait && plan.any_grain) e = cudaStreamWaitEvent(side, m.uploaded, 0);
   }
-  // the loop filter's edge-list counters start at zero: cleared here, in the
-  // upload's stream order, so the chain's stream holds kernels only
-  if (e == cudaSuccess) e = cudaMemsetAsync(dmeta + plan.off_counts, 0, 16, ups);
-  // and the stages' readiness flags start cleared
-  if (e == cudaSuccess && plan.n_flags) e = cudaMemsetAsync(dmeta + plan.off_flags, 0, plan.n_flags * 4, ups);
-  if (e == cudaSuccess) e = cudaEventRecord(m.uploaded, ups);
-  pipe_trace::mark(7, ups);
-  // The kernels read the upload: the host waits for it rather than the
-  // chain's stream. It waited only for the chain that used this buffer two
-  // calls ago, so it has usually landed already; and with nothing between
-  // the previous call's last kernel and this call's first on the stream,
-  // programmatic dependent launch chains them (a stream-side wait here made
-  // every call boundary a full one: 9 us per 1080p frame).
-  if (e == cudaSuccess) e = stream_upload_wait ? cudaStreamWaitEvent(s, m.uploaded, 0) : cudaEventSynchronize(m.uploaded);
   if (e != cudaSuccess) return cuda_status(e, "descriptor upload");
   m.used = true;
-  rc = launch_on(dmeta, s);
-  cudaEventRecord(m.done, s);
+  epoch++;
+  rc = launch_on(dmeta, s, capturing);
+  if (!capturing) cudaEventRecord(m.done, s);
   return rc;
 }
 
@@ -240,7 +261,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
 // chain without a gap at the call boundary (the first loop-filter kernel of
 // a call starts its launch while the previous call's last kernel drains);
 // profiled calls record stage events between the stages.
-int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s) {
+int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing) {
   const cudaEvent_t* ev = nullptr;
   if (prof) {
     const int slot = prof_next;
@@ -251,7 +272,7 @@ int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s) {
     prof_used[slot] = true;
     ev = prof_ev[slot];
   }
-  launch_plan(plan, dmeta, s, side, fork, join, ev, true, true, true);
+  launch_plan(plan, dmeta, s, side, fork, join, ev, true, !capturing, !capturing, plan.by_value, epoch);
   return cuda_status(cudaGetLastError(), "kernel launch");
 }
 

@@ -397,7 +397,7 @@ __device__ __forceinline__ void write_prelf(const FrameDesc& f, int p, int sc, i
 // stage_plane reads: plane rows (y0 >> sy) - 2 .. ((y0 + R) >> sy) + 1 and
 // 8 columns past the superblock on either side, within the plane.
 template <int R>
-__device__ __forceinline__ void cdef_wait_lf(const FrameDesc& f, const uint32_t* flags, int sc, int y0, int tid) {
+__device__ __forceinline__ void cdef_wait_lf(const FrameDesc& f, const SyncFlags& flags, int sc, int y0, int tid) {
   if (tid >= 48) return;
   const int p = tid >> 4, dy = (tid >> 2) & 3, dx = tid & 3;
   if (p >= f.np || f.lf_tiles_x[p] == 0) return;
@@ -407,13 +407,13 @@ __device__ __forceinline__ void cdef_wait_lf(const FrameDesc& f, const uint32_t*
   const int c0 = max(((sc * 64) >> sx) - 8, 0), c1 = min(((sc * 64 + 64) >> sx) + 7, W - 1);
   const int ty = (r0 >> 6) + dy, tx = (c0 >> 6) + dx;
   if (r0 > r1 || c0 > c1 || ty > (r1 >> 6) || tx > (c1 >> 6)) return;
-  flag_wait(flags + f.lf_flag_base[p] + ty * f.lf_tiles_x[p] + tx);
+  flag_wait(flags.p + f.lf_flag_base[p] + ty * f.lf_tiles_x[p] + tx, flags.epoch);
 }
 
-template <int R, bool LFH>
-__global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* __restrict__ frames,
-                                                           const Item* __restrict__ items, int n_items, int wrows,
-                                                           int min_bd, uint32_t* __restrict__ flags) {
+template <class F, int R, bool LFH>
+__global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items, int wrows,
+                                                           int min_bd, SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
   extern __shared__ __align__(16) int16_t cdef_smem_base[];  // [R][kDS] direction copy, then [3][wrows * kS]
   int16_t* const dwin = cdef_smem_base;
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* _
   if (tid == 0) s_one = 1;
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
-    const FrameDesc& f = frames[item.frame];
+    const FrameDesc& f = frame_of(one, frames, item.frame);
     const int sc = item.x0, sr = item.y0;
     const int y0 = sr * 64 + item.a * R;  // luma row of the CTA's first row
     const int np = f.np, sb = f.sb;
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* _
         }
       }
     }
-    if (flags) {
+    if (flags.p) {
       // only the loop-filter tiles this CTA reads
       pdl_trigger();
       cdef_wait_lf<R>(f, flags, sc, y0, tid);
@@ -593,14 +593,14 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* _
       }
     }
     __syncthreads();
-    if (flags && tid == 0) {
+    if (flags.p && tid == 0) {
       // the rows are in the CDEF planes: the half superblocks' flags
-      uint32_t* fl = flags + f.cdef_flag_base + 2 * sr * f.cdef_sbc + sc;
+      uint32_t* fl = flags.p + f.cdef_flag_base + 2 * sr * f.cdef_sbc + sc;
       if (R == 64) {
-        flag_set(fl);
-        flag_set(fl + f.cdef_sbc);
+        flag_set(fl, flags.epoch);
+        flag_set(fl + f.cdef_sbc, flags.epoch);
       } else {
-        flag_set(fl + item.a * f.cdef_sbc);
+        flag_set(fl + item.a * f.cdef_sbc, flags.epoch);
       }
     }
   }
@@ -1012,17 +1012,16 @@ __global__ void dsp_cdef_kernel(const int32_t* __restrict__ win, const av1pf_cde
 }
 
 cudaError_t cdef_init() {
-  cudaError_t e = cudaFuncSetAttribute(cdef_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       cdef_smem(64, true));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(cdef_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             cdef_smem(32, true));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(cdef_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             cdef_smem(64, false));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(cdef_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             cdef_smem(32, false));
+  cudaError_t e = cudaSuccess;
+  auto opt_in = [&](auto kernel, int bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
+  opt_in(cdef_kernel<NoFrame, 64, true>, cdef_smem(64, true));
+  opt_in(cdef_kernel<NoFrame, 32, true>, cdef_smem(32, true));
+  opt_in(cdef_kernel<NoFrame, 64, false>, cdef_smem(64, false));
+  opt_in(cdef_kernel<NoFrame, 32, false>, cdef_smem(32, false));
+  opt_in(cdef_kernel<OneFrame, 64, false>, cdef_smem(64, false));
+  opt_in(cdef_kernel<OneFrame, 32, false>, cdef_smem(32, false));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(cdef_search_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSearchSmem);
   if (e == cudaSuccess)
@@ -1031,7 +1030,7 @@ cudaError_t cdef_init() {
   return e;
 }
 
-void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, const CdefShape& c, uint32_t* flags,
+void launch_cdef(const FrameSet& frames, const Item* items, int n_items, const CdefShape& c, SyncFlags flags,
                  cudaStream_t s) {
   if (n_items <= 0) return;
   // Frames of up to 10 bits take the packed kernel, whose half precision holds
@@ -1047,17 +1046,18 @@ void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, const 
   const int R = c.half ? 32 : 64;
   const int wrows = R + 2 * (c.lfh ? kTopLfh : 2);
   const int grid = min(n_items, kItemGrid);
-  auto go = [&](auto kernel) {
-    launch_pdl(kernel, grid, 4 * R, size_t(cdef_smem(R, c.lfh)), s, frames, items, n_items, wrows, min_bd, flags);
+  const size_t smem = size_t(cdef_smem(R, c.lfh));
+  auto by_ptr = [&](auto kernel) {
+    launch_pdl(kernel, grid, 4 * R, smem, s, NoFrame{}, frames.dev, items, n_items, wrows, min_bd, flags);
   };
-  if (c.half && c.lfh)
-    go(cdef_kernel<32, true>);
+  if (c.lfh)
+    c.half ? by_ptr(cdef_kernel<NoFrame, 32, true>) : by_ptr(cdef_kernel<NoFrame, 64, true>);
   else if (c.half)
-    go(cdef_kernel<32, false>);
-  else if (c.lfh)
-    go(cdef_kernel<64, true>);
+    launch_frames(frames, cdef_kernel<NoFrame, 32, false>, cdef_kernel<OneFrame, 32, false>, grid, 4 * R, smem, s,
+                  items, n_items, wrows, min_bd, flags);
   else
-    go(cdef_kernel<64, false>);
+    launch_frames(frames, cdef_kernel<NoFrame, 64, false>, cdef_kernel<OneFrame, 64, false>, grid, 4 * R, smem, s,
+                  items, n_items, wrows, min_bd, flags);
 }
 
 void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, cudaStream_t s) {

@@ -292,7 +292,7 @@ __device__ __forceinline__ void stage_windows(const FrameDesc& f, int sc, int y0
 // loop-filter tiles under the CTA's windows: plane rows (y0 >> sy) - 2 ..
 // ((y0 + R) >> sy) + 1 and 8 columns past the superblock on either side.
 template <int R>
-__device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const uint32_t* flags, int sc, int y0, int tid) {
+__device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const SyncFlags& flags, int sc, int y0, int tid) {
   if (tid >= 48) return;
   const int p = tid >> 4, dy = (tid >> 2) & 3, dx = tid & 3;
   if (p >= f.np || f.lf_tiles_x[p] == 0) return;
@@ -302,7 +302,7 @@ __device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const uint32_
   const int c0 = max(((sc * 64) >> sx) - 8, 0), c1 = min(((sc * 64 + 64) >> sx) + 7, W - 1);
   const int ty = (r0 >> 6) + dy, tx = (c0 >> 6) + dx;
   if (r0 > r1 || c0 > c1 || ty > (r1 >> 6) || tx > (c1 >> 6)) return;
-  flag_wait(flags + f.lf_flag_base[p] + ty * f.lf_tiles_x[p] + tx);
+  flag_wait(flags.p + f.lf_flag_base[p] + ty * f.lf_tiles_x[p] + tx, flags.epoch);
 }
 
 }  // namespace
@@ -311,10 +311,10 @@ __device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const uint32_
 // rows). 4R threads, one warp per row of 8x8 blocks. Frames above 10 bits are
 // left to cdef_kernel. The chroma window has room for `R` rows and 4 more
 // when the launch was sized for frames without vertical subsampling.
-template <int R>
-__global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const FrameDesc* __restrict__ frames,
-                                                                  const Item* __restrict__ items, int n_items,
-                                                                  uint32_t* __restrict__ flags) {
+template <class F, int R>
+__global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items,
+                                                                  SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
   constexpr int NT = 4 * R;
   extern __shared__ __align__(16) uint8_t packed_base[];
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const Frame
   if (tid < 16) doff[tid >> 1][tid & 1] = int16_t((c_cdef_dirs[tid >> 1][tid & 1][0] * kPS + c_cdef_dirs[tid >> 1][tid & 1][1]) * 4);
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
-    const FrameDesc& f = frames[item.frame];
+    const FrameDesc& f = frame_of(one, frames, item.frame);
     const int sc = item.x0, sr = item.y0;
     const int y0 = sr * 64 + item.a * R;  // luma row of the CTA's first row
     const int np = f.np, sb = f.sb;
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const Frame
         }
       }
     }
-    if (flags) {
+    if (flags.p) {
       pdl_trigger();
       packed_wait_lf<R>(f, flags, sc, y0, tid);  // only the loop-filter tiles this CTA reads
     } else {
@@ -467,14 +467,14 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const Frame
       }
     }
     __syncthreads();
-    if (flags && tid == 0) {
+    if (flags.p && tid == 0) {
       // the rows are in the CDEF planes: the half superblocks' flags
-      uint32_t* fl = flags + f.cdef_flag_base + 2 * sr * f.cdef_sbc + sc;
+      uint32_t* fl = flags.p + f.cdef_flag_base + 2 * sr * f.cdef_sbc + sc;
       if (R == 64) {
-        flag_set(fl);
-        flag_set(fl + f.cdef_sbc);
+        flag_set(fl, flags.epoch);
+        flag_set(fl + f.cdef_sbc, flags.epoch);
       } else {
-        flag_set(fl + item.a * f.cdef_sbc);
+        flag_set(fl + item.a * f.cdef_sbc, flags.epoch);
       }
     }
   }
@@ -482,22 +482,27 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const Frame
 }
 
 cudaError_t cdef_packed_init() {
-  cudaError_t e = cudaFuncSetAttribute(cdef_packed_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       packed_smem(64, true));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(cdef_packed_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             packed_smem(32, true));
+  cudaError_t e = cudaSuccess;
+  auto opt_in = [&](auto kernel, int bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
+  opt_in(cdef_packed_kernel<NoFrame, 64>, packed_smem(64, true));
+  opt_in(cdef_packed_kernel<OneFrame, 64>, packed_smem(64, true));
+  opt_in(cdef_packed_kernel<NoFrame, 32>, packed_smem(32, true));
+  opt_in(cdef_packed_kernel<OneFrame, 32>, packed_smem(32, true));
   return e;
 }
 
-void launch_cdef_packed(const FrameDesc* frames, const Item* items, int n_items, bool half, bool tall, uint32_t* flags,
+void launch_cdef_packed(const FrameSet& frames, const Item* items, int n_items, bool half, bool tall, SyncFlags flags,
                         cudaStream_t s) {
   if (n_items <= 0) return;
   const int grid = min(n_items, kItemGrid);
   if (half)
-    launch_pdl(cdef_packed_kernel<32>, grid, 128, size_t(packed_smem(32, tall)), s, frames, items, n_items, flags);
+    launch_frames(frames, cdef_packed_kernel<NoFrame, 32>, cdef_packed_kernel<OneFrame, 32>, grid, 128,
+                  size_t(packed_smem(32, tall)), s, items, n_items, flags);
   else
-    launch_pdl(cdef_packed_kernel<64>, grid, 256, size_t(packed_smem(64, tall)), s, frames, items, n_items, flags);
+    launch_frames(frames, cdef_packed_kernel<NoFrame, 64>, cdef_packed_kernel<OneFrame, 64>, grid, 256,
+                  size_t(packed_smem(64, tall)), s, items, n_items, flags);
 }
 
 }  // namespace av1pf

@@ -169,19 +169,20 @@ __device__ __forceinline__ void trace_end(int kid, unsigned long long t0) {
   } while (0)
 #endif
 
-// A readiness flag: set with release semantics at GPU scope after the CTA's
+// A readiness flag, set for a launch once it holds the launch's epoch (SyncFlags):
+// set with release semantics at GPU scope after the CTA's
 // barrier (so every thread's writes before the barrier are visible to a
 // thread that sees the flag), waited for with acquire semantics. The wait is
 // bounded: after kFlagSpins polls it flags ERRF_STALL and returns.
 constexpr int kFlagSpins = 1 << 21;
-__device__ __forceinline__ void flag_set(uint32_t* p) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(1u) : "memory");
+__device__ __forceinline__ void flag_set(uint32_t* p, uint32_t epoch) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(epoch) : "memory");
 }
-__device__ __forceinline__ void flag_wait(const uint32_t* p) {
+__device__ __forceinline__ void flag_wait(const uint32_t* p, uint32_t epoch) {
   for (int k = 0; k < kFlagSpins; k++) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    if (v) return;
+    if (v >= epoch) return;
     __nanosleep(100);
   }
   atomicOr(&g_error_flags, ERRF_STALL);

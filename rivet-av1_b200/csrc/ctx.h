@@ -82,7 +82,7 @@ struct Ctx {
   bool host_ready = false;
   // descriptor buffers used in turn: device copy, pinned staging, the
   // upload's and the reading launches' events, and the structure whose work
-  // lists the device copy holds
+  // lists (and readiness flags, none above the epoch) the device copy holds
   struct MetaSlot {
     DevBuf dev;
     HostBuf host;
@@ -92,6 +92,9 @@ struct Ctx {
   };
   MetaSlot metas[2];
   int meta_next = 0;
+  // counts the calls that launch: the value their readiness flags are set to
+  static constexpr uint32_t kEpochMax = 1u << 30;
+  uint32_t epoch = 0;
   cudaStream_t upload = nullptr;  // descriptor uploads
   // the chain's stream, not the host, waits for the descriptor upload: set
   // by callers whose chains begin with a stream wait anyway (the host-buffer
@@ -124,7 +127,7 @@ struct Ctx {
   int ensure_host(HostBuf& b, size_t bytes);
   void release(DevBuf& b);
   int run(const FrameJob* jobs, int n, cudaStream_t s);
-  int launch_on(uint8_t* dmeta, cudaStream_t s);
+  int launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing);
 };
 
 void set_error(const std::string& s);

@@ -262,8 +262,9 @@ __device__ __forceinline__ void ar_plane(int lag, int16_t (*T)[kTW], const int16
 // luma, Cb and Cr auto-regressions side by side, chroma trailing luma,
 // while warps 3-7 build the scaling tables (one entry per thread) and the
 // per-stripe block offsets (one stripe per thread).
-__global__ void __launch_bounds__(256) grain_prep_kernel(const FrameDesc* __restrict__ frames,
-                                                         const Item* __restrict__ items, int n_items) {
+template <class F>
+__global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items) {
   AV1PF_TRACE_BEGIN();
   __shared__ __align__(16) int16_t T[3][kTH][kTW];
   __shared__ int32_t coef[3][25];
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(256) grain_prep_kernel(const FrameDesc* __rest
   pdl_wait();  // the previous stage's output is complete past this point
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
-    const FrameDesc& f = frames[item.frame];
+    const FrameDesc& f = frame_of(one, frames, item.frame);
     const av1pf_film_grain& g = f.g;
     const int bd = f.bd;
     const bool mono = f.np == 1;
@@ -648,7 +649,8 @@ constexpr int kOutWaitLimit = 1 << 16;  // bulk-copy waits of about 1 us each be
 // a new plane's template and scaling table as two more), all completing on
 // one barrier, while 18 threads fetch the stripe's block offsets; then 256
 // threads take 8 consecutive samples (one grain block) each per row.
-__global__ void __launch_bounds__(256, 2) output_kernel(const FrameDesc* __restrict__ frames,
+template <class F>
+__global__ void __launch_bounds__(256, 2) output_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
                                                      const Item* __restrict__ items, int n_items) {
   AV1PF_TRACE_BEGIN();
   extern __shared__ __align__(16) uint8_t out_smem[];
@@ -661,20 +663,22 @@ __global__ void __launch_bounds__(256, 2) output_kernel(const FrameDesc* __restr
   if (tid == 0) mbar_init(&sm.bar, 1);
   uint32_t phase = 0;     // parity of the barrier's current phase
   int loaded = -1;        // frame * 4 + plane whose template is in T
-  int loaded_frame = -1;  // the frame whose descriptor is in sm.fd
+  constexpr bool kOne = sizeof(F) == sizeof(OneFrame);  // the descriptor is a parameter
+  int loaded_frame = -1;  // the frame whose descriptor is in sm.fd (unused with kOne: there is one)
   // a CTA takes a contiguous run of items, the runs split as evenly as the
   // count allows: the items of a plane are consecutive, so a CTA stages that
   // plane's template once for its whole run
   const int it_begin = int(int64_t(blockIdx.x) * n_items / gridDim.x);
   const int it_end = int(int64_t(blockIdx.x + 1) * n_items / gridDim.x);
   if (it_begin < it_end) {
-    // the first item's descriptor: copied from the host before any kernel
+    // the first item's descriptor: a parameter of the launch, or copied from the host before any kernel
     // of the call ran, so it is fetched before waiting for the previous
     // stage (whose output, and the film-grain tables, are read only after)
     const Item first = items[it_begin];
-    const uint2* fs = reinterpret_cast<const uint2*>(&frames[first.frame]);
+    const uint2* fs = reinterpret_cast<const uint2*>(&frame_of(one, frames, first.frame));
     uint2* fdst = reinterpret_cast<uint2*>(&sm.fd);
-    for (int k = tid; k < int(sizeof(FrameDesc) / 8); k += 256) fdst[k] = fs[k];
+    if (!kOne)
+      for (int k = tid; k < int(sizeof(FrameDesc) / 8); k += 256) fdst[k] = fs[k];
     loaded_frame = first.frame;
   }
   __syncthreads();  // (also publishes the barrier's initialisation)
@@ -684,7 +688,7 @@ __global__ void __launch_bounds__(256, 2) output_kernel(const FrameDesc* __restr
     if (int(item.frame) != loaded_frame) {
       // the descriptor's fields are read by every thread: from shared memory
       // (the previous stripe ended with a barrier, so no thread reads it now)
-      const uint2* fs = reinterpret_cast<const uint2*>(&frames[item.frame]);
+      const uint2* fs = reinterpret_cast<const uint2*>(&frame_of(one, frames, item.frame));
       uint2* fdst = reinterpret_cast<uint2*>(&sm.fd);
       for (int k = tid; k < int(sizeof(FrameDesc) / 8); k += 256) fdst[k] = fs[k];
       __syncthreads();
@@ -692,7 +696,7 @@ __global__ void __launch_bounds__(256, 2) output_kernel(const FrameDesc* __restr
     }
     OutParams P;
     bool new_tables = false;  // the plane's template and table to fetch with the first stripe
-    const FrameDesc& f = sm.fd;
+    const FrameDesc& f = kOne ? frame_of(one, frames, 0) : sm.fd;
     const int p = item.plane;
     {
       P.bd = f.bd;
@@ -815,18 +819,22 @@ __global__ void __launch_bounds__(256, 2) output_kernel(const FrameDesc* __restr
 }
 
 cudaError_t output_init() {
-  return cudaFuncSetAttribute(output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutSmem);
+  cudaError_t e = cudaFuncSetAttribute(output_kernel<NoFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(output_kernel<OneFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutSmem);
+  return e;
 }
 
-void launch_grain_prep(const FrameDesc* frames, const Item* items, int n_items, cudaStream_t s) {
+void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s) {
   if (n_items <= 0) return;
-  launch_pdl(grain_prep_kernel, n_items, 256, 0, s, frames, items, n_items);
+  launch_frames(frames, grain_prep_kernel<NoFrame>, grain_prep_kernel<OneFrame>, n_items, 256, 0, s, items, n_items);
 }
 
-void launch_output(const FrameDesc* frames, const Item* items, int n_items, cudaStream_t s) {
+void launch_output(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s) {
   if (n_items <= 0) return;
   // one resident wave (2 CTAs per SM), each CTA a contiguous run of items
-  launch_pdl(output_kernel, min(n_items, kNumSMs * 2), 256, size_t(kOutSmem), s, frames, items, n_items);
+  launch_frames(frames, output_kernel<NoFrame>, output_kernel<OneFrame>, min(n_items, kNumSMs * 2), 256,
+                size_t(kOutSmem), s, items, n_items);
 }
 
 }  // namespace av1pf

@@ -7,10 +7,10 @@
 #include <cstdint>
 
 #include "av1pf.h"
+#include "desc.h"
 
 namespace av1pf {
 
-struct FrameDesc;
 struct Item;
 struct CdefSearchDesc;
 struct CdefGreedy;
@@ -46,6 +46,45 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t sme
   note_launch();
 }
 
+// The frames of a launch, as the stage kernels' first two parameters:
+// descriptors in device memory (after a NoFrame), or the descriptor of a
+// launch's only frame in the parameter itself (OneFrame, and null). A
+// parameter lives in the constant bank and travels with the launch: a single
+// call uploads nothing, its host thread waits for nothing, and the kernels
+// read the fields without the two dependent global loads (item, then
+// descriptor) that began every CTA.
+struct NoFrame {};
+struct OneFrame {
+  FrameDesc d;
+};
+static_assert(sizeof(OneFrame) <= 3584, "fits the 4 KB of kernel parameters with the others");
+#ifdef __CUDACC__
+__device__ __forceinline__ const FrameDesc& frame_of(const NoFrame&, const FrameDesc* p, int i) { return p[i]; }
+__device__ __forceinline__ const FrameDesc& frame_of(const OneFrame& f, const FrameDesc*, int) { return f.d; }
+#endif
+
+// What the launchers take: `one` (host memory) when not null, else `dev`.
+struct FrameSet {
+  const FrameDesc* dev = nullptr;
+  const FrameDesc* one = nullptr;
+};
+// The readiness flags of a launch: a flag is set once it holds `epoch` or a
+// later value, so calls with rising epochs share flags without clearing them.
+// p is null for launches that wait for whole stages.
+struct SyncFlags {
+  uint32_t* p = nullptr;
+  uint32_t epoch = 1;
+};
+
+template <typename... PArgs, typename... OArgs, typename... Args>
+inline void launch_frames(const FrameSet& fs, void (*by_ptr)(NoFrame, PArgs...), void (*by_value)(OneFrame, OArgs...),
+                          int grid, int block, size_t smem, cudaStream_t s, Args... args) {
+  if (fs.one)
+    launch_pdl(by_value, grid, block, smem, s, OneFrame{*fs.one}, static_cast<const FrameDesc*>(nullptr), args...);
+  else
+    launch_pdl(by_ptr, grid, block, smem, s, NoFrame{}, fs.dev, args...);
+}
+
 // Loop filter (lf.cu)
 void launch_lf_prep(const FrameDesc* frames, const Item* items, int n_items, uint64_t* list_v, uint64_t* list_h,
                     uint32_t* counts, uint32_t cap, cudaStream_t s);
@@ -54,8 +93,8 @@ void launch_lf_prep(const FrameDesc* frames, const Item* items, int n_items, uin
 void launch_lf_tiles(const FrameDesc* frames, const Item* items, int n_items, uint64_t* list_h, uint32_t* counts,
                      uint32_t cap, cudaStream_t s);
 // Both directions per 64x64 tile in shared memory (copy in -> cur included).
-// `flags`: the readiness flags the kernel sets (see FrameDesc), or null.
-void launch_lf_fused(const FrameDesc* frames, const Item* items, int n_items, uint32_t* flags, cudaStream_t s);
+// `flags`: the readiness flags the kernel sets (see FrameDesc).
+void launch_lf_fused(const FrameSet& frames, const Item* items, int n_items, SyncFlags flags, cudaStream_t s);
 void launch_lf_edges(int pass, const FrameDesc* frames, const uint64_t* list, const uint32_t* count, uint32_t cap,
                      cudaStream_t s);
 void launch_dsp_lf(int32_t* edges, const av1pf_lf_edge_params* prm, int n, cudaStream_t s);
@@ -70,12 +109,13 @@ struct CdefShape {
   bool deep = false;     // some frame has 12 bits
   bool tall = false;     // some frame's chroma is not vertically subsampled
 };
-// `flags`: the readiness flags the kernel waits for and sets, or null (as it
-// must be for a launch with both shallow and deep frames).
-void launch_cdef(const FrameDesc* frames, const Item* items, int n_items, const CdefShape& c, uint32_t* flags,
+// `flags`: the readiness flags the kernel waits for and sets (null for a launch
+// with both shallow and deep frames, or with the fused horizontal pass; the
+// latter needs the descriptors in device memory).
+void launch_cdef(const FrameSet& frames, const Item* items, int n_items, const CdefShape& c, SyncFlags flags,
                  cudaStream_t s);
 // The part of it for frames of up to 10 bits (cdef_packed.cu).
-void launch_cdef_packed(const FrameDesc* frames, const Item* items, int n_items, bool half, bool tall, uint32_t* flags,
+void launch_cdef_packed(const FrameSet& frames, const Item* items, int n_items, bool half, bool tall, SyncFlags flags,
                         cudaStream_t s);
 cudaError_t cdef_packed_init();
 // Sets cdef_kernel's dynamic shared-memory limit on the current device.
@@ -122,21 +162,21 @@ void launch_plane_sse(const SsePlane* jobs, int n, int rows_max, uint64_t* sse, 
 
 // Super-resolution (superres.cu)
 // `row_max`: the most source samples in a row among the launch's frames.
-void launch_superres(const FrameDesc* frames, const Item* items, int n_items, int row_max, cudaStream_t s);
+void launch_superres(const FrameSet& frames, const Item* items, int n_items, int row_max, cudaStream_t s);
 // Sets superres_kernel's dynamic shared-memory limit on the current device.
 cudaError_t superres_init();
 
 // Loop restoration (lr.cu)
-// `flags`: the readiness flags the kernel waits for, or null.
-void launch_lr(const FrameDesc* frames, const Item* items, int n_items, uint32_t* flags, cudaStream_t s);
+// `flags`: the readiness flags the kernel waits for.
+void launch_lr(const FrameSet& frames, const Item* items, int n_items, SyncFlags flags, cudaStream_t s);
 // Sets lr_kernel's dynamic shared-memory limit on the current device.
 cudaError_t lr_init();
 // Opts the output kernel into its dynamic shared memory (once per device).
 cudaError_t output_init();
 
 // Film grain + output packing (grain.cu)
-void launch_grain_prep(const FrameDesc* frames, const Item* items, int n_items, cudaStream_t s);
-void launch_output(const FrameDesc* frames, const Item* items, int n_items, cudaStream_t s);
+void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s);
+void launch_output(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s);
 // Uploads the LFSR jump-ahead tables (once per device).
 cudaError_t upload_grain_tables();
 

@@ -415,9 +415,9 @@ constexpr int kFChunks = kFW / 8 * kFW;  // 8-sample chunks of the window (800)
 // pass reads a sample another edge of that pass changes. The active edges of
 // each pass are listed in shared memory grouped by filter size, so a warp's
 // lanes mostly take one filter path. 256 threads.
-__global__ void __launch_bounds__(256, 4) lf_fused_kernel(const FrameDesc* __restrict__ frames,
-                                                       const Item* __restrict__ items, int n_items,
-                                                       uint32_t* __restrict__ flags) {
+template <class F>
+__global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items, SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
   const LfTables& tb = g_lf_tables;
   __shared__ __align__(16) uint16_t W[kFW * kFS];
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const FrameDesc* __res
   const int tid = threadIdx.x;
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
-    const FrameDesc& f = frames[item.frame];
+    const FrameDesc& f = frame_of(one, frames, item.frame);
     const int plane = item.plane;
     const DPlane src = f.in[plane], dst = f.cur[plane];
     const int sb = f.sb;
@@ -587,11 +587,11 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const FrameDesc* __res
         }
       }
     }
-    if (flags) {
+    if (flags.p) {
       // the tile is in cur: its readiness flag (the barrier orders every
       // thread's stores before the release)
       __syncthreads();
-      if (tid == 0) flag_set(flags + f.lf_flag_base[plane] + (y0 / kFT) * f.lf_tiles_x[plane] + x0 / kFT);
+      if (tid == 0) flag_set(flags.p + f.lf_flag_base[plane] + (y0 / kFT) * f.lf_tiles_x[plane] + x0 / kFT, flags.epoch);
     }
   }
   AV1PF_TRACE_END(1);
@@ -629,9 +629,10 @@ void launch_lf_tiles(const FrameDesc* frames, const Item* items, int n_items, ui
   launch_pdl(lf_tile_kernel, min(n_items, kItemGrid), 256, 0, s, frames, items, n_items, list_h, counts, cap);
 }
 
-void launch_lf_fused(const FrameDesc* frames, const Item* items, int n_items, uint32_t* flags, cudaStream_t s) {
+void launch_lf_fused(const FrameSet& frames, const Item* items, int n_items, SyncFlags flags, cudaStream_t s) {
   if (n_items <= 0) return;
-  launch_pdl(lf_fused_kernel, min(n_items, kItemGrid), 256, 0, s, frames, items, n_items, flags);
+  launch_frames(frames, lf_fused_kernel<NoFrame>, lf_fused_kernel<OneFrame>, min(n_items, kItemGrid), 256, 0, s,
+                items, n_items, flags);
 }
 
 void launch_lf_edges(int pass, const FrameDesc* frames, const uint64_t* list, const uint32_t* count, uint32_t cap,

@@ -296,7 +296,7 @@ __device__ __forceinline__ void sgr_flt_col(const int32_t* A, const int32_t* B, 
 // go straight to the reference frame and (frames without film grain) the
 // packed frame, 8 samples per thread and step, with no shared-memory round
 // trip and no barrier.
-__device__ __noinline__ void pass_through(const FrameDesc& f, int p, int x0, int y0, int w, int h, int tid) {
+__device__ __forceinline__ void pass_through(const FrameDesc& f, int p, int x0, int y0, int w, int h, int tid) {
   const int sb = f.sb, bps = f.bd > 8 ? 2 : 1;
   const DPlane src = f.up[p], dst = f.ref[p];
   const int pw = ((f.uw + plane_ssx(f, p)) >> plane_ssx(f, p));
@@ -559,7 +559,7 @@ __device__ __forceinline__ void restore_rect(const FrameDesc& f, const LrSmem& s
 // rows past the stripe come from the loop filter's output: the half
 // superblocks at the stripe's first and last rows waited for the tiles
 // under their windows, which reach 2 rows further.)
-__device__ __forceinline__ void lr_wait_cdef(const FrameDesc& f, const uint32_t* flags, int p, const LrGeom& geo, int x0,
+__device__ __forceinline__ void lr_wait_cdef(const FrameDesc& f, const SyncFlags& flags, int p, const LrGeom& geo, int x0,
                                              int w, int tid) {
   if (tid >= 16) return;
   const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
@@ -568,12 +568,12 @@ __device__ __forceinline__ void lr_wait_cdef(const FrameDesc& f, const uint32_t*
   const int c0 = (xa << sx) >> 6, c1 = min(((xb << sx) + sx) >> 6, f.cdef_sbc - 1);
   const int hr = h0 + (tid >> 2), c = c0 + (tid & 3);
   if (hr > h1 || c > c1) return;
-  flag_wait(flags + f.cdef_flag_base + hr * f.cdef_sbc + c);
+  flag_wait(flags.p + f.cdef_flag_base + hr * f.cdef_sbc + c, flags.epoch);
 }
 
-__global__ void __launch_bounds__(kThreads, 3) lr_kernel(const FrameDesc* __restrict__ frames,
-                                                         const Item* __restrict__ items, int n_items,
-                                                         const uint32_t* __restrict__ flags) {
+template <class F>
+__global__ void __launch_bounds__(kThreads, 3) lr_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items, SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ av1pf_lr_unit s_unit;
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const FrameDesc* __rest
 
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
-    const FrameDesc& f = frames[item.frame];
+    const FrameDesc& f = frame_of(one, frames, item.frame);
     const int p = item.plane;
     const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
     // lr_stripe (postfilter.rs:640-661)
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const FrameDesc* __rest
     if (h <= 0 || w <= 0) {
       // without flags every CTA waits, so the kernel never completes before
       // its predecessor
-      if (flags)
+      if (flags.p)
         pdl_trigger();
       else
         pdl_wait();
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const FrameDesc* __rest
     // the descriptor and the unit are inputs of the chain; the planes below
     // are the previous stage's output: all of it, or with readiness flags
     // the half superblocks under the rectangle
-    if (flags) {
+    if (flags.p) {
       pdl_trigger();
       lr_wait_cdef(f, flags, p, geo, x0, w, tid);
       __syncthreads();
@@ -667,15 +667,18 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const FrameDesc* __rest
 }
 
 cudaError_t lr_init() {
-  return cudaFuncSetAttribute(lr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  cudaError_t e = cudaFuncSetAttribute(lr_kernel<NoFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(lr_kernel<OneFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  return e;
 }
 
-void launch_lr(const FrameDesc* frames, const Item* items, int n_items, uint32_t* flags, cudaStream_t s) {
+void launch_lr(const FrameSet& frames, const Item* items, int n_items, SyncFlags flags, cudaStream_t s) {
   if (n_items <= 0) return;
   // one CTA per rectangle: the block scheduler hands rectangles of uneven
   // cost (copy, Wiener, self-guided) to SMs as they free up
-  launch_pdl(lr_kernel, min(n_items, kItemGrid), kThreads, size_t(kSmemBytes), s, frames, items, n_items,
-             static_cast<const uint32_t*>(flags));
+  launch_frames(frames, lr_kernel<NoFrame>, lr_kernel<OneFrame>, min(n_items, kItemGrid), kThreads,
+                size_t(kSmemBytes), s, items, n_items, flags);
 }
 
 }  // namespace av1pf

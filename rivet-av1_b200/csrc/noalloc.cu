@@ -215,7 +215,8 @@ extern "C" int av1pf_output_noalloc(const av1pf_frame_info* info, const av1pf_pa
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   e = cudaMemcpyAsync(d_desc, g_staging.bytes, kDescBytes + size_t(n) * sizeof(Item), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return cuda_status(e, "av1pf_output_noalloc: descriptor upload");
-  const FrameDesc* frames = reinterpret_cast<const FrameDesc*>(d_desc);
+  FrameSet frames;
+  frames.dev = reinterpret_cast<const FrameDesc*>(d_desc);
   const Item* d_list = reinterpret_cast<const Item*>(d_items);
   if (grain) launch_grain_prep(frames, d_list, 1, s);
   launch_output(frames, d_list + first_out, n - first_out, s);

@@ -498,6 +498,8 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
                    plan.lf_items.empty() && plan.lft_items.empty() && plan.copy_items.empty() &&
                    !(plan.cdef.deep && plan.cdef.shallow);
   plan.n_flags = plan.flag_sync ? nflags : 0;
+  plan.by_value = n == 1 && plan.lf_items.empty() && plan.lft_items.empty() && plan.copy_items.empty() &&
+                  !plan.any_hlist && !plan.cdef.lfh;
   // At most one wave of superblocks (4 CTAs on each SM): CDEF runs a CTA per
   // half superblock instead, so the SMs end up with equal shares.
   plan.cdef.half = !plan.cdef_items.empty() && plan.cdef_items.size() <= size_t(kNumSMs) * 4;
@@ -597,12 +599,17 @@ void pack_meta(const Plan& plan, uint8_t* host) {
 
 void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                  cudaEvent_t join, const cudaEvent_t* stage_ev, bool counts_zeroed, bool flags,
-                 bool grain_private) {
-  uint32_t* sync = flags && plan.flag_sync ? reinterpret_cast<uint32_t*>(meta + plan.off_flags) : nullptr;
+                 bool grain_private, bool by_value, uint32_t epoch) {
+  SyncFlags sync;
+  sync.p = flags && plan.flag_sync ? reinterpret_cast<uint32_t*>(meta + plan.off_flags) : nullptr;
+  sync.epoch = epoch;
   auto mark = [&](int k) {
     if (stage_ev) cudaEventRecord(stage_ev[k], s);
   };
   const FrameDesc* frames = reinterpret_cast<const FrameDesc*>(meta + plan.off_frames);
+  FrameSet fset;
+  fset.dev = frames;
+  fset.one = by_value ? plan.frames.data() : nullptr;
   auto items = [&](size_t off) { return reinterpret_cast<const Item*>(meta + off); };
   uint64_t* ev = reinterpret_cast<uint64_t*>(meta + plan.off_edges_v);
   uint64_t* eh = reinterpret_cast<uint64_t*>(meta + plan.off_edges_h);
@@ -615,7 +622,7 @@ void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t s
       cudaEventRecord(fork, s);
       cudaStreamWaitEvent(side, fork, 0);
     }
-    launch_grain_prep(frames, items(plan.off_grain), int(plan.grain_items.size()), side);
+    launch_grain_prep(fset, items(plan.off_grain), int(plan.grain_items.size()), side);
     cudaEventRecord(join, side);
   }
   mark(0);
@@ -640,18 +647,18 @@ void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t s
     if (plan.any_hlist) launch_lf_edges(1, frames, eh, counts + 1, plan.edge_cap, s);
   }
   if (plan.any_lf && !plan.lff_items.empty())
-    launch_lf_fused(frames, items(plan.off_lff), int(plan.lff_items.size()), sync, s);
+    launch_lf_fused(fset, items(plan.off_lff), int(plan.lff_items.size()), sync, s);
   mark(1);
   if (plan.any_cdef)
-    launch_cdef(frames, items(plan.off_cdef), int(plan.cdef_items.size()), plan.cdef, sync, s);
+    launch_cdef(fset, items(plan.off_cdef), int(plan.cdef_items.size()), plan.cdef, sync, s);
   mark(2);
-  if (plan.any_sr) launch_superres(frames, items(plan.off_sr), int(plan.sr_items.size()), plan.sr_row_max, s);
+  if (plan.any_sr) launch_superres(fset, items(plan.off_sr), int(plan.sr_items.size()), plan.sr_row_max, s);
   mark(3);
-  if (plan.any_lr) launch_lr(frames, items(plan.off_lr), int(plan.lr_items.size()), sync, s);
+  if (plan.any_lr) launch_lr(fset, items(plan.off_lr), int(plan.lr_items.size()), sync, s);
   mark(4);
   if (plan.any_out) {
     if (plan.any_grain) cudaStreamWaitEvent(s, join, 0);
-    launch_output(frames, items(plan.off_out), int(plan.out_items.size()), s);
+    launch_output(fset, items(plan.off_out), int(plan.out_items.size()), s);
   }
   mark(5);
 }

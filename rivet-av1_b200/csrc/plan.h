@@ -69,6 +69,8 @@ struct Plan {
   // previous call's output kernel reads.
   size_t off_grain_meta = 0;
   std::vector<std::pair<size_t, size_t>> grain_meta;
+  // one frame, all of whose kernels take its descriptor as a parameter
+  bool by_value = false;
   int sr_row_max = 0;      // superres: the most source samples in a row (sr_maxx + 1)
   bool any_lf = false, any_cdef = false, any_sr = false, any_lr = false, any_grain = false, any_out = false;
   // byte offsets of each list in the device meta buffer
@@ -107,10 +109,12 @@ void pack_meta(const Plan& plan, uint8_t* host);
 // stream order) instead of on the whole previous stage. `grain_private`:
 // the frames' film-grain scratch is this call's own (plan.grain_meta, no
 // earlier kernel still reads it), so the template kernel starts on the side
-// stream without waiting for `s`.
+// stream without waiting for `s`. `by_value` (plan.by_value): the frame's
+// descriptor travels as the kernels' parameter (plan.frames) instead of being
+// read from `meta`. `epoch`: the value that sets a readiness flag.
 void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                  cudaEvent_t join, const cudaEvent_t* stage_ev = nullptr, bool counts_zeroed = false,
-                 bool flags = false, bool grain_private = false);
+                 bool flags = false, bool grain_private = false, bool by_value = false, uint32_t epoch = 1);
 
 // Plane helpers.
 inline int plane_w(const av1pf_frame_info* i, int p, int width) {

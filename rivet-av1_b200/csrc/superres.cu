@@ -29,8 +29,9 @@ constexpr int kRows = 4;             // rows per item
 __host__ __device__ constexpr int sr_stride(int n) { return (n + 7) & ~7; }
 }  // namespace
 
-__global__ void __launch_bounds__(256) superres_kernel(const FrameDesc* __restrict__ frames,
-                                                       const Item* __restrict__ items, int n_items, int rs) {
+template <class F>
+__global__ void __launch_bounds__(256) superres_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items, int rs) {
   AV1PF_TRACE_BEGIN();
   extern __shared__ __align__(16) uint8_t sr_smem[];
   uint16_t* rows = reinterpret_cast<uint16_t*>(sr_smem);  // kRows staged source rows, rs apart
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(256) superres_kernel(const FrameDesc* __restri
     bool prelf;
     DPlane src, dst;
     {
-      const FrameDesc& f = frames[item.frame];
+      const FrameDesc& f = frame_of(one, frames, item.frame);
       p = item.plane;
       kind = item.kind;
       sy = plane_ssy(f, p);
@@ -135,14 +136,18 @@ __global__ void __launch_bounds__(256) superres_kernel(const FrameDesc* __restri
 }
 
 cudaError_t superres_init() {
-  return cudaFuncSetAttribute(superres_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kRows * sr_stride(kMaxRow) * 2);
+  const int bytes = kRows * sr_stride(kMaxRow) * 2;
+  cudaError_t e = cudaFuncSetAttribute(superres_kernel<NoFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(superres_kernel<OneFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e;
 }
 
-void launch_superres(const FrameDesc* frames, const Item* items, int n_items, int row_max, cudaStream_t s) {
+void launch_superres(const FrameSet& frames, const Item* items, int n_items, int row_max, cudaStream_t s) {
   if (n_items <= 0) return;
   const int rs = sr_stride(min(max(row_max, 8), kMaxRow));
-  launch_pdl(superres_kernel, min(n_items, kItemGrid), 256, size_t(kRows * rs * 2), s, frames, items, n_items, rs);
+  launch_frames(frames, superres_kernel<NoFrame>, superres_kernel<OneFrame>, min(n_items, kItemGrid), 256,
+                size_t(kRows * rs * 2), s, items, n_items, rs);
 }
 
 }  // namespace av1pf
