@@ -153,16 +153,30 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   // descriptors are rebuilt, and uploaded where the buffer already holds
   // the lists. Anything else is planned in full.
   structure_key(jobs, n, key_scratch);
+  auto scratch_base = [&] { return static_cast<uint8_t*>(scratch.ptr) + (scratch_turns ? meta_next * scratch_half : 0); };
   if (host_ready && key_scratch == host_key) {
-    rc = build_plan(jobs, n, static_cast<uint8_t*>(scratch.ptr), plan, &why, false);
+    rc = build_plan(jobs, n, scratch_base(), plan, &why, false);
     if (rc != AV1PF_OK) return set_error(why), rc;
   } else {
     host_ready = false;
     rc = build_plan(jobs, n, nullptr, plan, &why);
     if (rc != AV1PF_OK) return set_error(why), rc;
-    if ((rc = ensure(scratch, plan.scratch_bytes + 256)) != AV1PF_OK) return rc;
+    // Calls of small frames overlap, on two scratches in turn: where the loop
+    // filter's tiles take at most one wave (4 a SM) the GPU would be mostly
+    // idle between one call's stages (us a call, against one scratch: 352x288
+    // 20.2 / 26.7, 640x360 23.0 / 28.9, 960x540 31.4 / 38.1, 1280x720 37.2 /
+    // 36.9, 1600x900 46.8 / 49.0). Larger frames fill it, and a second scratch
+    // only takes L2 (1920x1080 57.8 / 56.6, 3840x2160 201 / 200). Under a
+    // memory cap the second scratch could take what another call needs.
+    scratch_half = (plan.scratch_bytes + 511) / 256 * 256;
+    scratch_turns = plan.flag_sync && plan.by_value && cap == 0 && plan.lff_items.size() <= size_t(kNumSMs) * 4;
+    if (scratch_turns && (rc = ensure(scratch, 2 * scratch_half)) != AV1PF_OK) {
+      cudaGetLastError();
+      scratch_turns = false;
+    }
+    if (!scratch_turns && (rc = ensure(scratch, plan.scratch_bytes + 256)) != AV1PF_OK) return rc;
     // the lists are built; with the scratch in place only the descriptors change
-    rc = build_plan(jobs, n, static_cast<uint8_t*>(scratch.ptr), plan, &why, false);
+    rc = build_plan(jobs, n, scratch_base(), plan, &why, false);
     if (rc != AV1PF_OK) return set_error(why), rc;
     host_key = key_scratch;
     host_ready = true;
@@ -191,6 +205,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     epoch = 0;
   }
   MetaSlot& m = metas[meta_next];
+  MetaSlot& other = metas[meta_next ^ 1];
   meta_next ^= 1;
   if (m.dev.size < plan.meta_bytes + 256) {
     if (m.used && (e = cudaEventSynchronize(m.done)) != cudaSuccess) return cuda_status(e, "descriptor wait");
@@ -232,10 +247,11 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     if (e == cudaSuccess) e = cudaMemsetAsync(dmeta + plan.off_counts, 0, 16, ups);
     // and so do the readiness flags of a new layout, below any epoch
     if (e == cudaSuccess && plan.n_flags && !resident)
-      e = cudaMemsetAsync(dmeta + plan.off_flags, 0, plan.n_flags * 4, ups);
+      e = cudaMemsetAsync(dmeta + plan.off_flags, 0, (plan.n_flags + 1) * 4, ups);
     if (e == cudaSuccess && !resident) {
       m.key = key_scratch;
       m.ready = true;
+      m.flagged = m.marked = 0;
     }
     if (e == cudaSuccess) e = cudaEventRecord(m.uploaded, ups);
     pipe_trace::mark(7, ups);
@@ -250,8 +266,29 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   }
   if (e != cudaSuccess) return cuda_status(e, "descriptor upload");
   m.used = true;
-  epoch++;
-  rc = launch_on(dmeta, s, capturing);
+  // How this call overlaps the previous ones (SyncFlags): it runs ahead of the
+  // previous call's end if that call and the one before it, which used this
+  // call's buffer and scratch, were flagged calls of the same structure on
+  // this stream.
+  SyncFlags call;
+  call.epoch = ++epoch;
+  const bool flagged = plan.flag_sync && !capturing;
+  if (flagged && scratch_turns && plan.by_value && last_stream == s && other.ready && other.key == key_scratch && other.flagged == epoch - 1) {
+    auto complete_word = [&](const MetaSlot& q) {
+      return reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(q.dev.ptr) + plan.off_flags) + plan.n_flags;
+    };
+    call.prev = complete_word(other);
+    call.prev_epoch = other.flagged;
+    other.marked = other.flagged;
+    if (m.flagged && m.flagged == epoch - 2 && m.marked == m.flagged) {
+      call.war = complete_word(m);
+      call.war_epoch = m.flagged;
+      call.prev_wait = true;
+    }
+  }
+  m.flagged = flagged ? epoch : 0;
+  last_stream = s;
+  rc = launch_on(dmeta, s, capturing, call);
   if (!capturing) cudaEventRecord(m.done, s);
   return rc;
 }
@@ -261,7 +298,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
 // chain without a gap at the call boundary (the first loop-filter kernel of
 // a call starts its launch while the previous call's last kernel drains);
 // profiled calls record stage events between the stages.
-int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing) {
+int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing, const SyncFlags& call) {
   const cudaEvent_t* ev = nullptr;
   if (prof) {
     const int slot = prof_next;
@@ -272,7 +309,7 @@ int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing) {
     prof_used[slot] = true;
     ev = prof_ev[slot];
   }
-  launch_plan(plan, dmeta, s, side, fork, join, ev, true, !capturing, !capturing, plan.by_value, epoch);
+  launch_plan(plan, dmeta, s, side, fork, join, ev, true, !capturing, !capturing, plan.by_value, call);
   return cuda_status(cudaGetLastError(), "kernel launch");
 }
 

@@ -88,6 +88,8 @@ struct Ctx {
     HostBuf host;
     cudaEvent_t uploaded = nullptr, done = nullptr;
     bool used = false, ready = false;
+    uint32_t flagged = 0;  // epoch of its last call, if that ran on the readiness flags
+    uint32_t marked = 0;   // the epoch that the call after it publishes once it is complete
     std::vector<int64_t> key;
   };
   MetaSlot metas[2];
@@ -95,6 +97,11 @@ struct Ctx {
   // counts the calls that launch: the value their readiness flags are set to
   static constexpr uint32_t kEpochMax = 1u << 30;
   uint32_t epoch = 0;
+  cudaStream_t last_stream = nullptr;  // of the previous call
+  // `scratch` holds two scratches, scratch_half bytes apart, used in turn with
+  // the descriptor buffers
+  bool scratch_turns = false;
+  size_t scratch_half = 0;
   cudaStream_t upload = nullptr;  // descriptor uploads
   // the chain's stream, not the host, waits for the descriptor upload: set
   // by callers whose chains begin with a stream wait anyway (the host-buffer
@@ -127,7 +134,7 @@ struct Ctx {
   int ensure_host(HostBuf& b, size_t bytes);
   void release(DevBuf& b);
   int run(const FrameJob* jobs, int n, cudaStream_t s);
-  int launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing);
+  int launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing, const SyncFlags& call);
 };
 
 void set_error(const std::string& s);

@@ -71,9 +71,24 @@ struct FrameSet {
 // The readiness flags of a launch: a flag is set once it holds `epoch` or a
 // later value, so calls with rising epochs share flags without clearing them.
 // p is null for launches that wait for whole stages.
+//
+// Consecutive calls overlap through two more words, each holding the epoch of
+// the last call of one of the context's two buffers that is known to be
+// complete. The loop filter's first CTA, once done with its own tile, waits
+// for the kernel before it on the stream, the previous call's last, and sets
+// *prev. A call whose `war` is not null runs on the scratch of the call before
+// the previous one: its loop filter writes once *war says that call is
+// complete, instead of once the previous call is, and lets CDEF launch at its
+// start; its loop restoration, which writes the caller's planes, waits until
+// *prev says the previous call is complete too (prev_wait).
 struct SyncFlags {
   uint32_t* p = nullptr;
   uint32_t epoch = 1;
+  const uint32_t* war = nullptr;
+  uint32_t war_epoch = 0;
+  uint32_t* prev = nullptr;
+  uint32_t prev_epoch = 0;
+  bool prev_wait = false;
 };
 
 template <typename... PArgs, typename... OArgs, typename... Args>

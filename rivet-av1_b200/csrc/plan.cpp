@@ -540,7 +540,7 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
   plan.off_edges_v = place(size_t(cap) * 8);
   plan.off_edges_h = place(size_t(cap) * 8);
   plan.off_counts = place(16);
-  plan.off_flags = place(plan.n_flags * 4);
+  plan.off_flags = place(plan.flag_sync ? (plan.n_flags + 1) * 4 : 0);
   {
     plan.grain_meta.assign(plan.frames.size(), {SIZE_MAX, SIZE_MAX});
     size_t g = 0;
@@ -599,10 +599,12 @@ void pack_meta(const Plan& plan, uint8_t* host) {
 
 void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                  cudaEvent_t join, const cudaEvent_t* stage_ev, bool counts_zeroed, bool flags,
-                 bool grain_private, bool by_value, uint32_t epoch) {
+                 bool grain_private, bool by_value, const SyncFlags& call) {
   SyncFlags sync;
-  sync.p = flags && plan.flag_sync ? reinterpret_cast<uint32_t*>(meta + plan.off_flags) : nullptr;
-  sync.epoch = epoch;
+  if (flags && plan.flag_sync) {
+    sync = call;
+    sync.p = reinterpret_cast<uint32_t*>(meta + plan.off_flags);
+  }
   auto mark = [&](int k) {
     if (stage_ev) cudaEventRecord(stage_ev[k], s);
   };
