@@ -153,8 +153,9 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   // descriptors are rebuilt, and uploaded where the buffer already holds
   // the lists. Anything else is planned in full.
   structure_key(jobs, n, key_scratch);
+  const bool same_structure = host_ready && key_scratch == host_key;
   auto scratch_base = [&] { return static_cast<uint8_t*>(scratch.ptr) + (scratch_turns ? meta_next * scratch_half : 0); };
-  if (host_ready && key_scratch == host_key) {
+  if (same_structure) {
     rc = build_plan(jobs, n, scratch_base(), plan, &why, false);
     if (rc != AV1PF_OK) return set_error(why), rc;
   } else {
@@ -199,13 +200,17 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   if (cudaStreamIsCapturing(s, &cap_status) != cudaSuccess) cudaGetLastError();
   const bool capturing = cap_status != cudaStreamCaptureStatusNone;
   if (epoch >= kEpochMax) {
-    // flags are compared with the epoch: before it could wrap, both buffers'
-    // are cleared by a fresh upload
-    for (MetaSlot& q : metas) q.ready = false;
+    // flags and words are compared with the epoch: before it could wrap, every
+    // call is done and all of them start over
+    for (MetaSlot& q : metas) {
+      if (q.used && (e = cudaEventSynchronize(q.done)) != cudaSuccess) return cuda_status(e, "epoch wait");
+      q.ready = false;
+    }
+    if ((e = cudaMemset(words, 0, kWords * 4)) != cudaSuccess) return cuda_status(e, "epoch words");
     epoch = 0;
   }
-  MetaSlot& m = metas[meta_next];
-  MetaSlot& other = metas[meta_next ^ 1];
+    const int turn = meta_next;
+  MetaSlot& m = metas[turn];
   meta_next ^= 1;
   if (m.dev.size < plan.meta_bytes + 256) {
     if (m.used && (e = cudaEventSynchronize(m.done)) != cudaSuccess) return cuda_status(e, "descriptor wait");
@@ -221,9 +226,17 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     plan.frames[fi].grain_off = dmeta + plan.off_grain_meta + plan.grain_meta[fi].second;
   }
   const bool resident = m.ready && m.key == key_scratch;
+  // Calls of small frames wait for the calls before them by words (SyncFlags).
+  // With film grain the template kernel then runs first on the call's stream
+  // and the output kernel starts early and waits on the SMs; its CTAs take half
+  // a SM's registers each, so only where at most one lands on a SM (us a call,
+  // against templates on the side stream and no overlap: 640x360 27.8 / 44.7,
+  // 1280x720 53.9 / 52.1, 1920x1080 70.8 / 72.4, 3840x2160 235 / 233).
+  const bool chained = scratch_turns && plan.by_value && !plan.lff_items.empty() && !capturing && !prof &&
+                       (!plan.any_grain || plan.out_items.size() <= size_t(kNumSMs));
   if (plan.by_value && resident) {
     // the scratch's last readers are the launches that used this buffer before
-    if (plan.any_grain && m.used && !capturing) e = cudaStreamWaitEvent(side, m.done, 0);
+    if (plan.any_grain && !chained && m.used && !capturing) e = cudaStreamWaitEvent(side, m.done, 0);
   } else {
     // the pinned staging buffer: its last upload must be done before it is
     // overwritten; the device buffer: its last readers
@@ -247,11 +260,10 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     if (e == cudaSuccess) e = cudaMemsetAsync(dmeta + plan.off_counts, 0, 16, ups);
     // and so do the readiness flags of a new layout, below any epoch
     if (e == cudaSuccess && plan.n_flags && !resident)
-      e = cudaMemsetAsync(dmeta + plan.off_flags, 0, (plan.n_flags + 1) * 4, ups);
+      e = cudaMemsetAsync(dmeta + plan.off_flags, 0, plan.n_flags * 4, ups);
     if (e == cudaSuccess && !resident) {
       m.key = key_scratch;
       m.ready = true;
-      m.flagged = m.marked = 0;
     }
     if (e == cudaSuccess) e = cudaEventRecord(m.uploaded, ups);
     pipe_trace::mark(7, ups);
@@ -262,31 +274,26 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     // programmatic dependent launch chains them (a stream-side wait here made
     // every call boundary a full one: 9 us per 1080p frame).
     if (e == cudaSuccess) e = stream_upload_wait ? cudaStreamWaitEvent(s, m.uploaded, 0) : cudaEventSynchronize(m.uploaded);
-    if (e == cudaSuccess && stream_upload_wait && plan.any_grain) e = cudaStreamWaitEvent(side, m.uploaded, 0);
+    if (e == cudaSuccess && stream_upload_wait && plan.any_grain && !chained) e = cudaStreamWaitEvent(side, m.uploaded, 0);
   }
   if (e != cudaSuccess) return cuda_status(e, "descriptor upload");
   m.used = true;
-  // How this call overlaps the previous ones (SyncFlags): it runs ahead of the
-  // previous call's end if that call and the one before it, which used this
-  // call's buffer and scratch, were flagged calls of the same structure on
-  // this stream.
   SyncFlags call;
   call.epoch = ++epoch;
-  const bool flagged = plan.flag_sync && !capturing;
-  if (flagged && scratch_turns && plan.by_value && last_stream == s && other.ready && other.key == key_scratch && other.flagged == epoch - 1) {
-    auto complete_word = [&](const MetaSlot& q) {
-      return reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(q.dev.ptr) + plan.off_flags) + plan.n_flags;
-    };
-    call.prev = complete_word(other);
-    call.prev_epoch = other.flagged;
-    other.marked = other.flagged;
-    if (m.flagged && m.flagged == epoch - 2 && m.marked == m.flagged) {
-      call.war = complete_word(m);
-      call.war_epoch = m.flagged;
-      call.prev_wait = true;
+  // calls right before this one, on its stream, chained and of its structure
+  const int before = same_structure && last_stream == s && resident ? chain_run : 0;
+  if (chained) {
+    call.complete = words;
+    if (plan.any_grain) {
+      call.grain = words + 1 + turn;
+      call.lf_wait = epoch - 1;
+    }
+    if (before >= 2) {
+      call.ahead = true;
+      call.lf_wait = epoch - 2;
     }
   }
-  m.flagged = flagged ? epoch : 0;
+  chain_run = chained ? before + 1 : 0;
   last_stream = s;
   rc = launch_on(dmeta, s, capturing, call);
   if (!capturing) cudaEventRecord(m.done, s);
@@ -408,6 +415,8 @@ int av1pf_ctx_create(int device, uint64_t hbm_cap_bytes, av1pf_ctx** out) {
   c->device = device;
   c->cap = hbm_cap_bytes;
   if ((e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaMalloc(&c->words, Ctx::kWords * 4)) != cudaSuccess ||
+      (e = cudaMemset(c->words, 0, Ctx::kWords * 4)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming)) != cudaSuccess) {
@@ -443,6 +452,7 @@ int av1pf_ctx_destroy(av1pf_ctx* ctx) {
   if (ctx->pipe_up) cudaStreamDestroy(ctx->pipe_up);
   if (ctx->pipe_down) cudaStreamDestroy(ctx->pipe_down);
   cudaStreamDestroy(ctx->side);
+  cudaFree(ctx->words);
   cudaStreamDestroy(ctx->own);
   cudaEventDestroy(ctx->fork);
   cudaEventDestroy(ctx->join);

@@ -188,6 +188,14 @@ __device__ __forceinline__ void flag_wait(const uint32_t* p, uint32_t epoch) {
   atomicOr(&g_error_flags, ERRF_STALL);
 }
 
+// A call's first kernel, one thread: once the kernel before it on the stream
+// is complete, so are the calls before this one. (A maximum, since nothing
+// orders this store against the next call's.)
+__device__ __forceinline__ void publish_complete(uint32_t* complete, uint32_t epoch) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("red.release.gpu.global.max.u32 [%0], %1;" ::"l"(complete), "r"(epoch - 1) : "memory");
+}
+
 // Grid-stride loop over the items of a launch.
 #define FOR_EACH_ITEM(it, n)                                   \
   for (int it = blockIdx.x; it < (n); it += gridDim.x)

@@ -54,7 +54,7 @@ struct Ctx {
   uint64_t cap = 0;   // 0 = no cap
   uint64_t held = 0;  // device bytes held by this context
   int threads = 3;  // av1pf_set_threads: device frame slots of av1pf_chain_host_many
-  cudaStream_t side = nullptr;  // grain templates beside the chain
+  cudaStream_t side = nullptr;  // grain templates beside the chain, where they are not ahead of it on its stream
   cudaStream_t own = nullptr;   // the host-buffer entry points
   cudaEvent_t fork = nullptr, join = nullptr;
   DevBuf scratch;
@@ -88,8 +88,6 @@ struct Ctx {
     HostBuf host;
     cudaEvent_t uploaded = nullptr, done = nullptr;
     bool used = false, ready = false;
-    uint32_t flagged = 0;  // epoch of its last call, if that ran on the readiness flags
-    uint32_t marked = 0;   // the epoch that the call after it publishes once it is complete
     std::vector<int64_t> key;
   };
   MetaSlot metas[2];
@@ -98,6 +96,11 @@ struct Ctx {
   static constexpr uint32_t kEpochMax = 1u << 30;
   uint32_t epoch = 0;
   cudaStream_t last_stream = nullptr;  // of the previous call
+  int chain_run = 0;                   // chained calls of one structure and stream up to the previous one
+  // device words (SyncFlags): [0] the last call known to be complete, [1 + turn]
+  // the last call whose film-grain templates are ready in that buffer
+  static constexpr int kWords = 64;
+  uint32_t* words = nullptr;
   // `scratch` holds two scratches, scratch_half bytes apart, used in turn with
   // the descriptor buffers
   bool scratch_turns = false;

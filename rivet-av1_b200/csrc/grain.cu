@@ -77,18 +77,25 @@ constexpr int kStageSrc = 512, kStageLuma = 1024;
 //
 // At every step every lane emits the value of its cell: the filtered value,
 // or the Gaussian value for the unfiltered border columns and the three top
-// rows (rows -3 .. -1 of the wavefront, walked by lanes 29 .. 31). The lane
-// k rows below receives the emission one step later by a warp shuffle: the
-// emission of lane (l - k) at step t - 1 is the cell (y - k, x + kS - 1) of
-// lane l at step t. Each lane keeps what it received from the lanes 1 .. LAG
-// above in register rings (slot t % 16; the oldest value read is 3S + LAG - 1
-// <= 14 steps old) and its own last LAG emissions: the filter reads no
-// shared memory except the cell's own Gaussian value, and the warp needs no
-// barrier between steps. The steps run in groups of 8 without branches
-// (cells outside the filter compute and store their own value back), so the
-// scheduler overlaps each step's sums over older values with the step
-// before; the step-to-step chain is the shuffle, one multiply-add, the
-// rounding and the clip.
+// rows (rows -3 .. -1 of the wavefront, walked by lanes 29 .. 31); what a lane
+// between rows emits is read by no filtered cell. Emissions travel in pairs,
+// (step t - 1, step t) in the halves of a word: the lane k rows below receives
+// a pair one step later by a warp shuffle, so that at step t it holds the
+// cells x + kS - 2 and x + kS - 1 of the row k above. Each lane keeps the
+// pairs it received from the lanes 1 .. LAG above, and its own, in register
+// registers, and two neighbouring taps are one 16-bit by 8-bit dot product. The filter reads
+// no shared memory except the cell's own Gaussian value (and a chroma cell's
+// luma), and the warp needs no barrier between steps. The steps run in groups
+// of 8 without branches; the step-to-step chain is the shuffle, two dot
+// products, the shift and the clip.
+//
+// What bounds it: one warp's serial chain of (W - 7) + S (H - 4) + 17 steps
+// (368 for luma at lag 3), which the chroma warps follow. With one multiply-add
+// a tap, cells worked out step by step and 16 steps unrolled, a luma step took
+// 217 cycles (80 instructions, fetched from a loop body beyond the instruction
+// cache) and the kernel 57 us; now 100 cycles and 27 us. Chroma's luma mean
+// without branches on the subsampling keeps its steps behind luma's (342 to
+// 200 cycles each; there are half as many).
 //
 // The luma warp publishes its completed step count in `progress` after every
 // group of 8 steps (past a warp barrier that orders its lanes' template
@@ -116,26 +123,38 @@ __device__ __forceinline__ void st_release_cta(uint32_t* p, uint32_t v) {
                : "memory");
 }
 
-// The cell lane `lane` holds at step t: row y, column x, whether the filter
-// runs there, and a template offset that is always inside the template —
-// the cell itself, or for a cell outside the template, a border cell (row 0,
-// or the first or last column) that no step filters.
-struct ArCell {
-  int y, x, off;
-  bool ar;
+// The cells lane `lane` holds at steps t0 .. t0 + 7 (t0 a multiple of 8): row
+// y, columns x .. x + 7 (from below 0 where the lane's next row begins inside
+// the group: a row is at most 82 columns and a lane's turn 32 S >= 96 steps,
+// so no group holds cells of two rows). Bit j of `in` says that column x + j
+// is inside the template, of `ar` that it is filtered.
+struct ArCells {
+  int y, x;
+  uint32_t in, ar;
 };
+__device__ __forceinline__ uint32_t bits_between(int lo, int hi) {  // bits max(lo, 0) .. min(hi, 8) - 1
+  return ((1u << min(max(hi, 0), 8)) - 1u) & ~((1u << min(max(lo, 0), 8)) - 1u);
+}
 template <int S>
-__device__ __forceinline__ ArCell ar_cell(int t, int lane, int H, int W) {
-  const int q = (t + 3 + 16 * S) / S - 16;  // floor((t + 3) / S): rows change lanes at column 0
-  const int rr = q - ((q - lane) & 31);
-  ArCell c;
+__device__ __forceinline__ ArCells ar_cells(int t0, int lane, int H, int W) {
+  const int q = (t0 + 3 + 16 * S) / S - 16;  // floor((t0 + 3) / S): rows change lanes at column 0
+  int rr = q - ((q - lane) & 31);
+  ArCells c;
+  c.x = 3 + t0 - S * rr;
+  if (c.x > 32 * S - 8) {
+    c.x -= 32 * S;
+    rr += 32;
+  }
   c.y = 3 + rr;
-  c.x = 3 + t - S * rr;
-  c.ar = rr >= 0 && c.y < H && c.x >= 3 && c.x < W - 3;
-  const int yc = c.y >= 0 && c.y < H ? c.y : 0;
-  const int xc = min(max(c.x, 0), W - 1);
-  c.off = yc * kTW + xc;
+  c.in = c.y >= 0 && c.y < H ? bits_between(-c.x, W - c.x) : 0u;
+  c.ar = rr >= 0 ? c.in & bits_between(3 - c.x, W - 3 - c.x) : 0u;
   return c;
+}
+
+// The dot product of the pairs in `a` with two of the 8-bit coefficients in `c`.
+template <bool HIGH>
+__device__ __forceinline__ int dot2(uint32_t a, uint32_t c, int acc) {
+  return HIGH ? __dp2a_hi(int(a), int(c), acc) : __dp2a_lo(int(a), int(c), acc);
 }
 
 template <int LAG, bool CHROMA>
@@ -145,39 +164,63 @@ __device__ __forceinline__ void ar_warp(int16_t (*T)[kTW], const int16_t (*Y)[kT
   constexpr int S = ar_slope<LAG>();
   constexpr int NC = 2 * LAG * (LAG + 1);
   constexpr int RW = 2 * LAG + 1;  // coefficients per row above
-  int c[NC + 1];
+  constexpr int L1 = LAG > 0 ? LAG : 1;
+  // bytes 0 .. 3 of up[k - 1][0]: the taps -LAG .. -LAG + 3 of row y - k, of [1]
+  // the next; the last tap, LAG, sits in the upper byte of its pair (its pair is
+  // the taps LAG - 1 and LAG, the former counted in the pair before)
+  uint32_t up[L1][2];
+  uint32_t left = 0;  // the row's own taps: -LAG, -LAG + 1 in bytes 0, 1 where LAG = 3, and the last pair's in bytes 2, 3
+  auto byte_of = [&](int k, int at) { return (uint32_t(coef_s[k]) & 255u) << (8 * at); };
 #pragma unroll
-  for (int k = 0; k <= NC; k++) c[k] = coef_s[k];
+  for (int k = 1; k <= LAG; k++) {
+    up[k - 1][0] = up[k - 1][1] = 0;
+#pragma unroll
+    for (int i = 0; i < RW; i++) {
+      const int at = i == RW - 1 ? i + 1 : i;  // byte position: an even number of taps, then (0, last)
+      up[k - 1][at >> 2] |= byte_of((LAG - k) * RW + i, at & 3);
+    }
+  }
+  if (LAG == 3) left = byte_of(NC - 3, 0) | byte_of(NC - 2, 1) | byte_of(NC - 1, 3);
+  if (LAG == 2) left = byte_of(NC - 2, 2) | byte_of(NC - 1, 3);
+  if (LAG == 1) left = byte_of(NC - 1, 3);
+  const int luma_coef = coef_s[NC];
   const int lane = threadIdx.x & 31;
   const int rows = H - 3;
   const int t_last = (W - 7) + S * (rows - 1);  // the last row's last filtered cell
   const bool luma_term = CHROMA && luma_on;
+  const int rnd = (1 << ar_shift) >> 1;
   int16_t* Tf = &T[0][0];
   const int16_t* Yf = &Y[0][0];
-  int own[16];                   // the lane's emission of step t in slot t % 16
-  int w[LAG > 0 ? LAG : 1][16];  // w[k - 1]: emissions of the lane k rows above, one step late
+  // Pairs of the steps before the group and, from kPast on, of the group's 8
+  // steps: own[kPast + j] the lane's (emissions of steps t0 + j - 1 and t0 + j),
+  // w[k - 1][kPast + j] those of the lane k rows above, one step late. The
+  // oldest pair the filter reads is kS + LAG - 2 <= 13 steps old. (Rings of 16
+  // slots, with 16 steps unrolled so that their slots are constants, need no
+  // moves but made a loop body that the warp waited for at every step.)
+  constexpr int kPast = 13;
+  uint32_t own[kPast + 8], w[L1][kPast + 8];
 #pragma unroll
-  for (int u = 0; u < 16; u++) {
+  for (int u = 0; u < kPast + 8; u++) {
     own[u] = 0;
 #pragma unroll
-    for (int k = 0; k < (LAG > 0 ? LAG : 1); k++) w[k][u] = 0;
+    for (int k = 0; k < L1; k++) w[k][u] = 0;
   }
   uint32_t seen = 0;  // the luma progress last read
-  // steps from -16 (the top row -3 starts at -S * 3 - 3 >= -15), in blocks of
-  // 16 so that every ring slot is a constant, and groups of 8 whose steps
-  // have no branches
-  for (int tb = -16; tb <= t_last; tb += 16) {
+  // steps from -16 (the top row -3 starts at -S * 3 - 3 >= -15), in groups of 8
+  // whose steps have no branches
+  for (int t0 = -16; t0 <= t_last; t0 += 8) {
+    {
 #pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int t0 = tb + 8 * half;
+      for (int u = 0; u < kPast; u++) {
+        own[u] = own[u + 8];
+#pragma unroll
+        for (int k = 0; k < L1; k++) w[k][u] = w[k][u + 8];
+      }
+      const ArCells e = ar_cells<S>(t0, lane, H, W);
       if (luma_term) {
         // the last luma step whose cell the group's luma terms read
-        int need = -(1 << 20);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const ArCell e = ar_cell<S>(t0 + j, lane, H, W);
-          if (e.ar) need = max(need, ((e.x - 3) << sub_x) + sub_x + S * (((e.y - 3) << sub_y) + sub_y));
-        }
+        const int x = e.x + 31 - __clz(e.ar | 1u);
+        const int need = e.ar ? ((x - 3) << sub_x) + sub_x + S * (((e.y - 3) << sub_y) + sub_y) : -(1 << 20);
         const int wneed = __reduce_max_sync(0xffffffffu, need) + kProgressBias;
         if (wneed >= int(seen)) {
           int spins = 0;
@@ -190,51 +233,70 @@ __device__ __forceinline__ void ar_warp(int16_t (*T)[kTW], const int16_t (*Y)[kT
           }
         }
       }
-      // the group's cells, their Gaussian values and luma terms, loaded
-      // ahead: a cell is written by its own lane only
-      int off[8], g[8], lum[8];
-      uint32_t arm = 0;
+      // the group's Gaussian values and luma terms, loaded ahead: a cell is
+      // written by its own lane only. g is kept scaled with the rounding
+      // constant: the filtered value is (g + sum) >> ar_shift before the clip.
+      // (What a lane loads for columns outside the template, up to 8 on either
+      // side, is never used; the templates are padded by as much.)
+      int16_t* cell = Tf + (e.in ? e.y * kTW + e.x : 0);
+      int g[8], lum[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const ArCell e = ar_cell<S>(t0 + j, lane, H, W);
-        off[j] = e.off;
-        arm |= uint32_t(e.ar) << j;
-        g[j] = Tf[e.off];
-        lum[j] = 0;
-        if (luma_term) {
-          const int lo = e.ar ? (((e.y - 3) << sub_y) + 3) * kTW + ((e.x - 3) << sub_x) + 3 : 3 * kTW + 3;
-          int l = Yf[lo];
-          if (sub_x) l += Yf[lo + 1];
-          if (sub_y) l += Yf[lo + kTW];
-          if (sub_x && sub_y) l += Yf[lo + kTW + 1];
-          lum[j] = round2(l, sub_x + sub_y) * c[NC];
+      for (int j = 0; j < 8; j++) g[j] = cell[j];
+      if (luma_term) {
+        // the mean of the luma cells under a chroma cell: of 1, 2 or 4, each
+        // counted 4, 2 or 1 times (round2 of 4 a by 2 is a, and of 2 (a + b) by
+        // 2 that of a + b by 1)
+        const int16_t* yl = Yf + (e.ar ? (((e.y - 3) << sub_y) + 3) * kTW + (e.x - 3) * (1 << sub_x) + 3 : 3 * kTW);
+        const int right = sub_x, down = sub_y ? kTW : 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const int16_t* at = yl + (j << sub_x);
+          lum[j] = ((at[0] + at[right] + at[down] + at[down + right] + 2) >> 2) * luma_coef;
         }
       }
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        const int u = 8 * half + j;
-        const int vprev = own[(u + 15) & 15];
+        const int u = kPast + j;
+        const uint32_t prev = own[u - 1];
 #pragma unroll
-        for (int k = 1; k <= LAG; k++) w[k - 1][u] = __shfl_sync(0xffffffffu, vprev, (lane - k) & 31);
-        // four partial sums over the values from earlier steps; (y - k, x +
-        // dc) came at step t + dc - kS + 1, and (y, x + dc) is the lane's
-        // own emission of step t + dc
-        int acc[4] = {lum[j], 0, 0, 0};
+        for (int k = 1; k <= LAG; k++) w[k - 1][u] = __shfl_sync(0xffffffffu, prev, (lane - k) & 31);
+        // partial sums over the pairs from earlier steps; (y - k, x + dc) came
+        // at step t + dc - kS + 1, and (y, x + dc) is the lane's own emission
+        // of step t + dc
+        int acc[3] = {(g[j] << ar_shift) + rnd + (luma_term ? lum[j] : 0), 0, 0};
         int n = 0;
+        auto at_slot = [&](int k, int dc) { return w[k - 1][u + dc - k * S + 1]; };
 #pragma unroll
-        for (int k = LAG; k >= 1; k--)
+        for (int k = LAG; k >= 1; k--) {
 #pragma unroll
-          for (int dc = -LAG; dc <= LAG; dc++)
-            if (!(k == 1 && dc == LAG)) acc[n++ & 3] += w[k - 1][(u + dc - k * S + 1 + 32) & 15] * c[(LAG - k) * RW + dc + LAG];
-#pragma unroll
-        for (int dc = -LAG; dc <= -2; dc++) acc[n++ & 3] += own[(u + dc + 16) & 15] * c[LAG * RW + LAG + dc];
-        int sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-        // the two values of the step before: the cell up and LAG to the
-        // right (just received) and the cell to the left
-        if (LAG > 0) sum += w[0][u] * c[(LAG - 1) * RW + 2 * LAG] + vprev * c[LAG * RW + LAG - 1];
-        const int v = (arm >> j) & 1u ? clip3(gmin, gmax, g[j] + round2(sum, ar_shift)) : g[j];
-        Tf[off[j]] = int16_t(v);  // a cell outside the filter gets its own value back
-        own[u] = v;
+          for (int i = 0; i + 1 < RW; i += 2) {  // taps i - LAG and i + 1 - LAG
+            const uint32_t c = up[k - 1][i >> 2];
+            acc[n % 3] = (i & 2) ? dot2<true>(at_slot(k, i + 1 - LAG), c, acc[n % 3])
+                                 : dot2<false>(at_slot(k, i + 1 - LAG), c, acc[n % 3]);
+            n++;
+          }
+          if (k > 1) {
+            constexpr int at = RW - 1;
+            acc[n % 3] = (at & 2) ? dot2<true>(at_slot(k, LAG), up[k - 1][at >> 2], acc[n % 3])
+                                  : dot2<false>(at_slot(k, LAG), up[k - 1][at >> 2], acc[n % 3]);
+            n++;
+          }
+        }
+        if (LAG == 3) acc[n % 3] = dot2<false>(own[u - 2], left, acc[n % 3]);
+        int sum = acc[0] + acc[1] + acc[2];
+        // the two values of the step before: the cell up and LAG to the right
+        // (just received at S = LAG + 1, a step earlier at lag 1) and the cell
+        // to the left
+        if (LAG > 0) {
+          constexpr int at = RW - 1;
+          sum = dot2<true>(prev, left, sum);
+          sum = (at & 2) ? dot2<true>(at_slot(1, LAG), up[0][at >> 2], sum)
+                         : dot2<false>(at_slot(1, LAG), up[0][at >> 2], sum);
+        }
+        const bool ar = (e.ar >> j) & 1u;
+        const int v = ar ? clip3(gmin, gmax, sum >> ar_shift) : g[j];
+        if (ar) cell[j] = int16_t(v);
+        own[u] = __byte_perm(prev, uint32_t(v), 0x5432);
       }
       if (!CHROMA) {
         // the warp barrier orders every lane's stores before the releases
@@ -264,17 +326,30 @@ __device__ __forceinline__ void ar_plane(int lag, int16_t (*T)[kTW], const int16
 // per-stripe block offsets (one stripe per thread).
 template <class F>
 __global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
-                                                     const Item* __restrict__ items, int n_items) {
+                                                     const Item* __restrict__ items, int n_items, SyncFlags sync) {
   AV1PF_TRACE_BEGIN();
-  __shared__ __align__(16) int16_t T[3][kTH][kTW];
+  // the templates, with room for the auto-regression's unused loads around them
+  constexpr int kPad = 128;
+  __shared__ __align__(16) int16_t T_padded[kPad + 3 * kTH * kTW + kPad];
+  int16_t(*const T)[kTH][kTW] = reinterpret_cast<int16_t(*)[kTH][kTW]>(T_padded + kPad);
   __shared__ int32_t coef[3][25];
   __shared__ uint8_t lut[3][256];
   __shared__ int16_t gauss[2048];
   __shared__ uint32_t progress;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
+  if (sync.grain) {
+    // first on the call's stream: the chain starts beside this kernel. Nothing
+    // written before the call is read; the CTA past the items publishes the
+    // previous calls' completion.
+    pdl_trigger();
+    if (int(blockIdx.x) >= n_items) {
+      if (tid == 0) publish_complete(sync.complete, sync.epoch);
+      return;
+    }
+  }
   for (int k = tid; k < 2048; k += 256) gauss[k] = g_gaussian[k];
-  pdl_wait();  // the previous stage's output is complete past this point
+  if (!sync.grain) pdl_wait();  // the previous stage's output is complete past this point
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
     const FrameDesc& f = frame_of(one, frames, item.frame);
@@ -365,6 +440,17 @@ __global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__
         }
         lut[plane][x] = uint8_t(v);
       }
+      // The scratch is written from here on: the output kernel that last read it
+      // is done, that of the call before the previous one.
+      if (sync.grain) {
+        if ((tid & 31) == 0) {
+          if (sync.ahead)
+            flag_wait(sync.complete, sync.lf_wait);
+          else
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        __syncwarp();
+      }
       // --- per-stripe block offsets (grain.rs:192-199) ---
       for (int s = tid - 96; s < f.grain_ns; s += 160) {
         uint32_t r = seed;
@@ -407,7 +493,9 @@ __global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__
         reinterpret_cast<uint32_t*>(&gs->scale[plane][0])[k - (plane << wshift)] = word;
       }
     }
+    if (sync.grain) asm volatile("fence.proxy.async;" ::: "memory");  // the output kernel reads by bulk copies
     __syncthreads();
+    if (sync.grain && tid == 0) flag_set(sync.grain, sync.epoch);
   }
   AV1PF_TRACE_END(6);
 }
@@ -651,8 +739,9 @@ constexpr int kOutWaitLimit = 1 << 16;  // bulk-copy waits of about 1 us each be
 // threads take 8 consecutive samples (one grain block) each per row.
 template <class F>
 __global__ void __launch_bounds__(256, 2) output_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
-                                                     const Item* __restrict__ items, int n_items) {
+                                                     const Item* __restrict__ items, int n_items, SyncFlags sync) {
   AV1PF_TRACE_BEGIN();
+  if (sync.ahead) pdl_trigger();
   extern __shared__ __align__(16) uint8_t out_smem[];
   OutSmem& sm = *reinterpret_cast<OutSmem*>(out_smem);
   int16_t* T = sm.T;
@@ -680,6 +769,10 @@ __global__ void __launch_bounds__(256, 2) output_kernel(const __grid_constant__ 
     if (!kOne)
       for (int k = tid; k < int(sizeof(FrameDesc) / 8); k += 256) fdst[k] = fs[k];
     loaded_frame = first.frame;
+  }
+  if (sync.grain && tid == 0) {
+    flag_wait(sync.grain, sync.epoch);
+    asm volatile("fence.proxy.async;" ::: "memory");  // the templates are read by bulk copies
   }
   __syncthreads();  // (also publishes the barrier's initialisation)
   pdl_wait();  // the previous stage's output is complete past this point
@@ -825,16 +918,17 @@ cudaError_t output_init() {
   return e;
 }
 
-void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s) {
+void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, const SyncFlags& sync, cudaStream_t s) {
   if (n_items <= 0) return;
-  launch_frames(frames, grain_prep_kernel<NoFrame>, grain_prep_kernel<OneFrame>, n_items, 256, 0, s, items, n_items);
+  launch_frames(frames, grain_prep_kernel<NoFrame>, grain_prep_kernel<OneFrame>, n_items + (sync.grain ? 1 : 0), 256, 0, s, items,
+                n_items, sync);
 }
 
-void launch_output(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s) {
+void launch_output(const FrameSet& frames, const Item* items, int n_items, const SyncFlags& sync, cudaStream_t s) {
   if (n_items <= 0) return;
   // one resident wave (2 CTAs per SM), each CTA a contiguous run of items
   launch_frames(frames, output_kernel<NoFrame>, output_kernel<OneFrame>, min(n_items, kNumSMs * 2), 256,
-                size_t(kOutSmem), s, items, n_items);
+                size_t(kOutSmem), s, items, n_items, sync);
 }
 
 }  // namespace av1pf

@@ -68,27 +68,35 @@ struct FrameSet {
   const FrameDesc* dev = nullptr;
   const FrameDesc* one = nullptr;
 };
-// The readiness flags of a launch: a flag is set once it holds `epoch` or a
-// later value, so calls with rising epochs share flags without clearing them.
-// p is null for launches that wait for whole stages.
+// How a call's kernels wait for one another, and for the calls before it,
+// short of whole grids. A flag is set once it holds the call's epoch or a later
+// value, so calls with rising epochs share flags without clearing them. The
+// default is none of it: each kernel waits for the whole kernel before it.
 //
-// Consecutive calls overlap through two more words, each holding the epoch of
-// the last call of one of the context's two buffers that is known to be
-// complete. The loop filter's first CTA, once done with its own tile, waits
-// for the kernel before it on the stream, the previous call's last, and sets
-// *prev. A call whose `war` is not null runs on the scratch of the call before
-// the previous one: its loop filter writes once *war says that call is
-// complete, instead of once the previous call is, and lets CDEF launch at its
-// start; its loop restoration, which writes the caller's planes, waits until
-// *prev says the previous call is complete too (prev_wait).
+// p: the readiness flags between the stages (FrameDesc::lf_flag_base ...), or
+// null.
+//
+// complete: a word that holds the epoch of the last call known to be complete,
+// or null. A call's first kernel raises it to epoch - 1 from one thread that
+// waits for the kernel before it on the stream, the previous call's last; the
+// kernels that must not write before an earlier call is done wait for the word
+// instead of for that kernel. Calls of small frames (`ahead`) run on two
+// scratches in turn: their loop filter and film-grain templates wait for the
+// call before the previous one (lf_wait = epoch - 2), their kernels let the
+// next launch as they start, and loop restoration, which writes the caller's
+// planes, waits for the previous call.
+//
+// grain: set to the epoch by the film-grain template kernel, which then runs
+// first on the call's own stream, one CTA beside the chain (so it has started
+// before the output kernel can wait for it), or null: it runs on another
+// stream, joined by an event.
 struct SyncFlags {
   uint32_t* p = nullptr;
   uint32_t epoch = 1;
-  const uint32_t* war = nullptr;
-  uint32_t war_epoch = 0;
-  uint32_t* prev = nullptr;
-  uint32_t prev_epoch = 0;
-  bool prev_wait = false;
+  uint32_t* complete = nullptr;
+  uint32_t lf_wait = 0;  // the loop filter waits for this in `complete` before it writes; 0: for the previous kernel
+  bool ahead = false;
+  uint32_t* grain = nullptr;
 };
 
 template <typename... PArgs, typename... OArgs, typename... Args>
@@ -190,8 +198,8 @@ cudaError_t lr_init();
 cudaError_t output_init();
 
 // Film grain + output packing (grain.cu)
-void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s);
-void launch_output(const FrameSet& frames, const Item* items, int n_items, cudaStream_t s);
+void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, const SyncFlags& sync, cudaStream_t s);
+void launch_output(const FrameSet& frames, const Item* items, int n_items, const SyncFlags& sync, cudaStream_t s);
 // Uploads the LFSR jump-ahead tables (once per device).
 cudaError_t upload_grain_tables();
 

@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
   __shared__ uint32_t list_v[kFCells], list_h[kFCells];
   __shared__ uint32_t cnt[2][4], base[2][4];
   const int tid = threadIdx.x;
-  if (flags.war) pdl_trigger();
+  if (flags.ahead) pdl_trigger();
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
     const FrameDesc& f = frame_of(one, frames, item.frame);
@@ -470,9 +470,9 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
         }
       }
     }
-    // scratch of its own: the wait for the call that used it before, while the
-    // window loads (barriers follow before anything is written)
-    if (flags.war && tid == 255) flag_wait(flags.war, flags.war_epoch);
+    // the wait for the call that last used this scratch, while the window loads
+    // (barriers follow before anything is written)
+    if (flags.lf_wait && tid == 255) flag_wait(flags.complete, flags.lf_wait);
     // --- decisions: vertical edges of the window's 20 x 17 cells, horizontal
     // edges of the tile's 17 x 16 (postfilter.rs:107-264) ---
     int dv[2] = {0, 0}, dh[2] = {0, 0};
@@ -563,9 +563,12 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
     __syncthreads();
     // Up to here the tile read only this call's inputs (the unfiltered
     // planes, the maps, the descriptor) and worked in shared memory, so it
-    // ran while the previous call's stages drained; cur, which they read
-    // (unless this call has scratch of its own), is written only past this wait.
-    if (!flags.war) pdl_wait();
+    // ran while the previous call's stages drained; cur, which they read, is
+    // written only past this wait or the one above.
+    if (!flags.lf_wait)
+      pdl_wait();
+    else if (!flags.ahead)
+      pdl_trigger();
     // --- write the tile's own samples [x0, x1) x [y0, y1) ---
     {
       const int w = x1 - x0;
@@ -598,10 +601,7 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
       if (tid == 0) flag_set(flags.p + f.lf_flag_base[plane] + (y0 / kFT) * f.lf_tiles_x[plane] + x0 / kFT, flags.epoch);
     }
   }
-  if (flags.prev && blockIdx.x == 0 && tid == 0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous call's last kernel
-    flag_set(flags.prev, flags.prev_epoch);
-  }
+  if (flags.complete && !flags.grain && blockIdx.x == 0 && tid == 0) publish_complete(flags.complete, flags.epoch);
   AV1PF_TRACE_END(1);
 }
 

@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const __grid_constant__
       pdl_trigger();
       lr_wait_cdef(f, flags, p, geo, x0, w, tid);
       // the previous call may write the same planes
-      if (flags.prev_wait && tid == 32) flag_wait(flags.prev, flags.prev_epoch);
+      if (flags.ahead && tid == 32) flag_wait(flags.complete, flags.epoch - 1);
       __syncthreads();
     } else {
       pdl_wait();

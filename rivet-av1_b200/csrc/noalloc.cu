@@ -218,7 +218,7 @@ extern "C" int av1pf_output_noalloc(const av1pf_frame_info* info, const av1pf_pa
   FrameSet frames;
   frames.dev = reinterpret_cast<const FrameDesc*>(d_desc);
   const Item* d_list = reinterpret_cast<const Item*>(d_items);
-  if (grain) launch_grain_prep(frames, d_list, 1, s);
-  launch_output(frames, d_list + first_out, n - first_out, s);
+  if (grain) launch_grain_prep(frames, d_list, 1, SyncFlags{}, s);
+  launch_output(frames, d_list + first_out, n - first_out, SyncFlags{}, s);
   return cuda_status(cudaGetLastError(), "av1pf_output_noalloc: launch");
 }

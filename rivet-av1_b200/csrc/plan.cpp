@@ -540,7 +540,7 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
   plan.off_edges_v = place(size_t(cap) * 8);
   plan.off_edges_h = place(size_t(cap) * 8);
   plan.off_counts = place(16);
-  plan.off_flags = place(plan.flag_sync ? (plan.n_flags + 1) * 4 : 0);
+  plan.off_flags = place(plan.flag_sync ? plan.n_flags * 4 : 0);
   {
     plan.grain_meta.assign(plan.frames.size(), {SIZE_MAX, SIZE_MAX});
     size_t g = 0;
@@ -600,11 +600,8 @@ void pack_meta(const Plan& plan, uint8_t* host) {
 void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                  cudaEvent_t join, const cudaEvent_t* stage_ev, bool counts_zeroed, bool flags,
                  bool grain_private, bool by_value, const SyncFlags& call) {
-  SyncFlags sync;
-  if (flags && plan.flag_sync) {
-    sync = call;
-    sync.p = reinterpret_cast<uint32_t*>(meta + plan.off_flags);
-  }
+  SyncFlags sync = call;
+  sync.p = flags && plan.flag_sync ? reinterpret_cast<uint32_t*>(meta + plan.off_flags) : nullptr;
   auto mark = [&](int k) {
     if (stage_ev) cudaEventRecord(stage_ev[k], s);
   };
@@ -616,7 +613,11 @@ void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t s
   uint64_t* ev = reinterpret_cast<uint64_t*>(meta + plan.off_edges_v);
   uint64_t* eh = reinterpret_cast<uint64_t*>(meta + plan.off_edges_h);
   uint32_t* counts = reinterpret_cast<uint32_t*>(meta + plan.off_counts);
-  if (plan.any_grain) {
+  if (sync.grain) {
+    // the grain templates depend only on the parameters: one CTA ahead of the
+    // chain on its own stream, which the output kernel waits for by a word
+    launch_grain_prep(fset, items(plan.off_grain), int(plan.grain_items.size()), sync, s);
+  } else if (plan.any_grain) {
     // the grain templates depend only on the parameters: run them beside the
     // chain; into a scratch that the previous call's output kernel may still
     // read, only once `s` has got this far
@@ -624,7 +625,7 @@ void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t s
       cudaEventRecord(fork, s);
       cudaStreamWaitEvent(side, fork, 0);
     }
-    launch_grain_prep(fset, items(plan.off_grain), int(plan.grain_items.size()), side);
+    launch_grain_prep(fset, items(plan.off_grain), int(plan.grain_items.size()), sync, side);
     cudaEventRecord(join, side);
   }
   mark(0);
@@ -659,8 +660,8 @@ void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t s
   if (plan.any_lr) launch_lr(fset, items(plan.off_lr), int(plan.lr_items.size()), sync, s);
   mark(4);
   if (plan.any_out) {
-    if (plan.any_grain) cudaStreamWaitEvent(s, join, 0);
-    launch_output(fset, items(plan.off_out), int(plan.out_items.size()), s);
+    if (plan.any_grain && !sync.grain) cudaStreamWaitEvent(s, join, 0);
+    launch_output(fset, items(plan.off_out), int(plan.out_items.size()), sync, s);
   }
   mark(5);
 }

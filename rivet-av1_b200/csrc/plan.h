@@ -111,8 +111,8 @@ void pack_meta(const Plan& plan, uint8_t* host);
 // earlier kernel still reads it), so the template kernel starts on the side
 // stream without waiting for `s`. `by_value` (plan.by_value): the frame's
 // descriptor travels as the kernels' parameter (plan.frames) instead of being
-// read from `meta`. `call`: the call's epoch and how it overlaps the previous
-// ones (its p is set here).
+// read from `meta`. `call`: the call's epoch and how it waits for the calls
+// before it (its p is set here).
 void launch_plan(const Plan& plan, uint8_t* meta, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                  cudaEvent_t join, const cudaEvent_t* stage_ev = nullptr, bool counts_zeroed = false,
                  bool flags = false, bool grain_private = false, bool by_value = false,
