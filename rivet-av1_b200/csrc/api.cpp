@@ -404,7 +404,6 @@ int av1pf_ctx_create(int device, uint64_t hbm_cap_bytes, av1pf_ctx** out) {
     std::lock_guard<std::mutex> lk(g_tables_mu);
     if (device < 64 && !g_tables_ready[device]) {
       if ((e = upload_grain_tables()) != cudaSuccess) return cuda_status(e, "grain tables");
-      if ((e = lr_init()) != cudaSuccess) return cuda_status(e, "loop restoration kernel attributes");
       if ((e = superres_init()) != cudaSuccess) return cuda_status(e, "superres kernel attributes");
       if ((e = cdef_init()) != cudaSuccess) return cuda_status(e, "CDEF kernel attributes");
       if ((e = output_init()) != cudaSuccess) return cuda_status(e, "output kernel attributes");

@@ -192,8 +192,6 @@ cudaError_t superres_init();
 // Loop restoration (lr.cu)
 // `flags`: the readiness flags the kernel waits for.
 void launch_lr(const FrameSet& frames, const Item* items, int n_items, SyncFlags flags, cudaStream_t s);
-// Sets lr_kernel's dynamic shared-memory limit on the current device.
-cudaError_t lr_init();
 // Opts the output kernel into its dynamic shared memory (once per device).
 cudaError_t output_init();
 

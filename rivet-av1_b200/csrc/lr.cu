@@ -4,42 +4,60 @@
 // loop_restoration, lr_stripe, lr_unit_cols, restore_stripe, lr_window,
 // restore_rect_from_window, box_filter_rect, wiener_coefficient).
 //
-// One CTA restores one rectangle: the rows of one stripe (64 luma rows,
-// offset by 8) and up to 64 columns of one restoration unit. 288 threads are
-// 4 row groups x 72 columns (8 x 36 for rectangles of up to 32 columns, as
-// 4:2:0 chroma units are), so every thread owns a column and no loop
-// divides by a runtime width. The window the rectangle reads (3-sample
-// border, the stripe-boundary rule of LrCtx::sample) is staged in shared
-// memory with one row-uniform source choice per row. Wiener runs its
-// horizontal pass into an int16 intermediate, then the vertical pass. The
-// self-guided filter slides each column's box sums down its rows (one new
-// and one old row of horizontal sums per step), then walks each column's
-// output rows with three rows of A and B in registers. The sums are exact in
-// 32 bits for <= 12-bit samples (25 * 4095^2 < 2^31); the products the
-// reference forms in 64 bits (p * s and the B term) are 32x32->64 multiplies
-// here. Rectangles of
-// units without restoration (and planes or frames without it) pass their
-// samples through, so the kernel writes the whole visible area of the
-// reference frame. Every rectangle's output gathers in a shared-memory tile
-// and leaves in 16-byte row chunks: to the reference frame and, for a frame
-// without film grain, to the packed output frame too, so such a frame needs
-// no output pass.
+// A team of threads restores one rectangle: the rows of one stripe (64 luma
+// rows, offset by 8) and up to 64 columns of one restoration unit. The team is
+// a CTA of 128 threads, or for 4:2:0 chroma, whose stripes have 32 rows, half a
+// CTA: one item then holds the U and the V rectangle of a place. The window the
+// rectangle reads (3-sample border, the stripe-boundary rule of LrCtx::sample)
+// is staged in shared memory with one row-uniform source choice per row, behind
+// the only barrier. After it the team's groups work on their own: a group is
+// the lanes across the rectangle, two columns a lane (32 lanes; 16 for
+// rectangles of up to 32 columns), and a run of its rows, which the group
+// walks down with everything it reuses in registers.
+//   Wiener: the horizontal filter of a row, then the vertical filter over the
+//   last seven rows' results. The horizontal taps are 16-bit by 8-bit dot
+//   products on the window's packed samples.
+//   Self-guided, two rows a step: box sums from the rows' horizontal sums
+//   (radius 2 and 1 at once), each position's A and B packed in a word, the
+//   words' neighbours from the lanes on either side, then both filters. The
+//   positions one column outside the group, which no lane owns, are worked out
+//   by the group beforehand, a lane a row.
+// Rectangles of units without restoration (and planes or frames without it)
+// pass their samples through, so the kernel writes the whole visible area of
+// the reference frame and, for a frame without film grain, the packed output
+// frame too, so such a frame needs no output pass.
+//
+// What bounds it: instruction issue and latency (each CTA's chain of item, unit
+// and window loads, then a group's serial walk), at 16 warps on an SM. Against
+// CTAs of 288 threads that passed A, B and the Wiener intermediate through 64 KB
+// of shared memory behind a barrier a phase: 1080p 10-bit 37.5 -> 27.5 us (under
+// ncu), 14.5 M -> 9.4 M warp instructions; the chain call 57.0 -> 51.8 us, 4K
+// 10-bit with superres and grain 231 -> 213 us, 4K 12-bit 4:4:4 478 -> 456 us.
+// 128 registers (4 CTAs a SM): at 96 or 80 the walks spill, and 1080p takes 54.2
+// and 61 us. Items of whole stripes (16 rows a group) instead of 32 rows: 67 us,
+// too few and too long CTAs.
 #include "common.cuh"
 #include "kernels.h"
 
 namespace av1pf {
 
 namespace {
-constexpr int kThreads = 288;
-constexpr int kMaxW = 64;                // columns per rectangle
-constexpr int kMaxH = 64;                // rows per stripe
-constexpr int kWS = 72;                  // window row stride (u16): w + 6 <= 70
-constexpr int kAS = 72;                  // A/B row stride (int32): w + 2 <= 66
-constexpr int kWinBytes = (kMaxH + 6) * kWS * 2;
-constexpr int kABytes = (kMaxH + 2) * kAS * 4;
-constexpr int kF0Bytes = kMaxH * kMaxW * 4;  // the first self-guided filter's output
-constexpr int kSmemBytes = kWinBytes + 2 * kABytes + kF0Bytes;
-static_assert((kMaxH + 6) * kWS * 2 <= kABytes, "Wiener intermediate must fit the A area");
+constexpr int kThreads = 128;
+constexpr int kMaxH = 64;  // rows per stripe
+// window row strides (u16): rectangles of up to 64 columns (w + 6 <= 70), and of
+// up to 32, whose two groups a warp read rows 8 apart: 8 x 22 words are 16 mod
+// 32 banks
+constexpr int kWideWS = 72, kSlimWS = 44;
+// a team's window: 70 wide rows, or two of 38 slim ones (the last rows' loads
+// reach past their columns)
+constexpr int kWinBytes = (kMaxH + 6) * kWideWS * 2 + 16;
+constexpr int kSlimTeamWin = (kMaxH / 2 + 6) * kSlimWS + 8;  // u16
+// per group: the packed A / B of the columns on either side, for the first
+// filter's rows and the second's
+constexpr int kEdgeRows = 18;
+struct GroupEdges {
+  uint32_t first[kEdgeRows / 2][2], second[kEdgeRows][2];
+};
 
 // SGR_A2 (postfilter.rs:884-898), built at compile time into global memory:
 // the self-guided passes read it through the L1, so no CTA sets it up.
@@ -51,9 +69,39 @@ constexpr A2Table make_a2() {
   for (int z = 0; z < 256; z++) t.v[z] = z >= 255 ? 256 : (z == 0 ? 1 : ((z << 8) + z / 2) / (z + 1));
   return t;
 }
+// The scale s of each self-guided parameter set's two filters, times 2^12
+// (postfilter.rs:903-918: ((1 << 20) + n^2 eps / 2) / (n^2 eps)), and 2^16 / n
+// rounded up, for quotients by 1 .. 9 of numbers below 2^12 without a division.
+constexpr int32_t kSgrParams AV1T_SGR_PARAMS_DIMS = AV1T_SGR_PARAMS;
+struct LrConst {
+  uint32_t s12[16][2];
+  int32_t inv[10];
+};
+constexpr LrConst make_lr_const() {
+  LrConst t{};
+  for (int set = 0; set < 16; set++)
+    for (int k = 0; k < 2; k++) {
+      const int n = k ? 9 : 25, n2e = n * n * kSgrParams[set][2 * k + 1];
+      t.s12[set][k] = n2e ? uint32_t(((1 << 20) + n2e / 2) / n2e) << 12 : 0u;
+    }
+  for (int n = 1; n < 10; n++) t.inv[n] = (65536 + n - 1) / n;
+  return t;
+}
 }  // namespace
 
 __device__ const A2Table g_sgr_a2 = make_a2();
+__constant__ LrConst c_lr = make_lr_const();
+
+// The threads that restore one rectangle: `t` of `n`, meeting at barrier `bar`.
+struct Team {
+  int t, n, bar;
+  __device__ __forceinline__ void sync() const {  // (constant barrier names: a kernel that computes them holds all 16)
+    if (bar == 1)
+      asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
+    else
+      asm volatile("bar.sync 2, %0;" ::"r"(n) : "memory");
+  }
+};
 
 struct LrGeom {
   int ss, se, y0, y1, pex, pey;
@@ -94,466 +142,479 @@ __device__ __forceinline__ int ld_row(const uint8_t* row, int sb, int x) {
   return sb == 1 ? int(row[x]) : int(reinterpret_cast<const uint16_t*>(row)[x]);
 }
 
-// Reads the w x h samples at (x0, y0) of `src` (sample width sb) into `tile`
-// (int32, row stride kMaxW): 16-byte chunks where the rows allow them, else
-// single samples. Rows hold MW >> cs chunk slots (w <= MW).
-template <int MW>
-__device__ __forceinline__ void load_tile(const DPlane& src, int sb, int x0, int y0, int w, int h, int32_t* tile,
-                                          int tid) {
-  const uint8_t* s0 = src.p + (int64_t(y0) * src.stride + x0) * sb;
-  const int64_t sp = src.stride * sb;
-  const bool vec = ((reinterpret_cast<uintptr_t>(s0) | uintptr_t(sp)) & 15) == 0;
-  const int cs = sb == 2 ? 3 : 4;                  // log2 samples per chunk
-  const int ls = (MW == 64 ? 6 : 5) - cs;          // log2 chunk slots per row
-  for (int k = tid; k < (h << ls); k += kThreads) {
-    const int r = k >> ls, e0 = (k & ((1 << ls) - 1)) << cs;
-    if (e0 >= w) continue;
-    const uint8_t* row = s0 + int64_t(r) * sp;
-    int32_t* t = tile + r * kMaxW + e0;
-    if (vec && e0 + (1 << cs) <= w) {
-      const uint4 q = *reinterpret_cast<const uint4*>(row + e0 * sb);
-      if (sb == 2) {
-        reinterpret_cast<int4*>(t)[0] = make_int4(q.x & 0xffff, q.x >> 16, q.y & 0xffff, q.y >> 16);
-        reinterpret_cast<int4*>(t)[1] = make_int4(q.z & 0xffff, q.z >> 16, q.w & 0xffff, q.w >> 16);
-      } else {
-        const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-          reinterpret_cast<int4*>(t)[j] =
-              make_int4(wd[j] & 0xff, (wd[j] >> 8) & 0xff, (wd[j] >> 16) & 0xff, wd[j] >> 24);
-      }
-    } else {
-      for (int e = e0; e < min(w, e0 + (1 << cs)); e++) t[e - e0] = ld_row(row, sb, e);
-    }
-  }
-}
-
-// Writes the w x h output samples of `tile` (int32, row stride kMaxW) to
-// rows of `width`-byte samples from `base`, `pitch` bytes apart: 16-byte
-// chunks (8 or 16 samples) where `vec` says the rows allow them, else single
-// samples. Rows hold MW >> cs chunk slots (w <= MW).
-template <int MW>
-__device__ __forceinline__ void store_tile(const int32_t* tile, uint8_t* base, int64_t pitch, int width, bool vec,
-                                           int w, int h, int tid) {
-  const int cs = width == 2 ? 3 : 4;      // log2 samples per chunk
-  const int ls = (MW == 64 ? 6 : 5) - cs;  // log2 chunk slots per row
-  for (int k = tid; k < (h << ls); k += kThreads) {
-    const int r = k >> ls, e0 = (k & ((1 << ls) - 1)) << cs;
-    if (e0 >= w) continue;
-    const int32_t* t = tile + r * kMaxW + e0;
-    uint8_t* row = base + int64_t(r) * pitch;
-    if (vec && e0 + (1 << cs) <= w) {
-      const int4 a = *reinterpret_cast<const int4*>(t);
-      const int4 b = *reinterpret_cast<const int4*>(t + 4);
-      uint4 q;
-      if (width == 2) {
-        q.x = uint32_t(a.x) | (uint32_t(a.y) << 16);
-        q.y = uint32_t(a.z) | (uint32_t(a.w) << 16);
-        q.z = uint32_t(b.x) | (uint32_t(b.y) << 16);
-        q.w = uint32_t(b.z) | (uint32_t(b.w) << 16);
-      } else {
-        const int4 c = *reinterpret_cast<const int4*>(t + 8);
-        const int4 d = *reinterpret_cast<const int4*>(t + 12);
-        q.x = uint32_t(a.x) | (uint32_t(a.y) << 8) | (uint32_t(a.z) << 16) | (uint32_t(a.w) << 24);
-        q.y = uint32_t(b.x) | (uint32_t(b.y) << 8) | (uint32_t(b.z) << 16) | (uint32_t(b.w) << 24);
-        q.z = uint32_t(c.x) | (uint32_t(c.y) << 8) | (uint32_t(c.z) << 16) | (uint32_t(c.w) << 24);
-        q.w = uint32_t(d.x) | (uint32_t(d.y) << 8) | (uint32_t(d.z) << 16) | (uint32_t(d.w) << 24);
-      }
-      *reinterpret_cast<uint4*>(row + e0 * width) = q;
-    } else {
-      for (int e = e0; e < min(w, e0 + (1 << cs)); e++) {
-        if (width == 2)
-          reinterpret_cast<uint16_t*>(row)[e] = uint16_t(t[e - e0]);
-        else
-          row[e] = uint8_t(t[e - e0]);
-      }
-    }
-  }
-}
-
-// Box sums of radius R over the window and the A / B of box_filter_rect
-// (postfilter.rs:935-959) for positions (i, j), i in [0, h+2), j = c - 1,
-// stored at [i][c]. Each of the G row groups owns a contiguous run of rows
-// and slides down it.
-template <int PASS, int G>
-__device__ __forceinline__ void sgr_ab(const uint16_t* win, int32_t* A, int32_t* B, const int32_t* a2tab, int eps,
-                                       int bd, int y0, int h, int w, int c, int g) {
-  constexpr int R = PASS == 0 ? 2 : 1;  // SGR_PARAMS radii: first 0 or 2, second 0 or 1
-  constexpr int n = (2 * R + 1) * (2 * R + 1);
-  const int n2e = n * n * eps;
-  const uint32_t sc = uint32_t(((1 << 20) + n2e / 2) / n2e);
-  constexpr int one_over_n = ((1 << 12) + n / 2) / n;
-  if (c >= w + 2) return;
-  const int rows = h + 2;
-  const int rpg = (rows + G - 1) / G;
-  const int i0 = g * rpg, i1 = min(i0 + rpg, rows);
-  if (i0 >= i1) return;
-  // horizontal sums of window row wr around column c + 2
-  auto hs = [&](int wr, int& s1, int& s2) {
-    s1 = 0;
-    s2 = 0;
-    const uint16_t* rp = win + wr * kWS + c + 2;
-#pragma unroll
-    for (int dx = -R; dx <= R; dx++) {
-      const int v = rp[dx];
-      s1 += v;
-      s2 += v * v;
-    }
-  };
-  // ring of the horizontal sums of the 2R+1 rows in the box: the row that
-  // enters at step i goes to slot (i - i0 + 2R) mod N, the row that leaves
-  // is in slot (i - i0) mod N; unrolling by N makes the slots constants
-  constexpr int N = 2 * R + 1;
-  int r1[N], r2[N];
-  int bsum = 0, bsq = 0;
-#pragma unroll
-  for (int m = 0; m < 2 * R; m++) {
-    hs(i0 + 2 - R + m, r1[m], r2[m]);
-    bsum += r1[m];
-    bsq += r2[m];
-  }
-  for (int ib = i0; ib < i1; ib += N) {
-#pragma unroll
-    for (int u = 0; u < N; u++) {
-      const int i = ib + u;
-      if (i < i1) {
-        const int sn = (u + 2 * R) % N;
-        hs(i + 2 + R, r1[sn], r2[sn]);
-        bsum += r1[sn];
-        bsq += r2[sn];
-        // the first filter weighs only the odd rows' A and B (postfilter.rs:937)
-        if (PASS == 1 || ((y0 + i - 1) & 1) != 0) {
-          const int a = round2(bsq, 2 * (bd - 8));
-          const int d = round2(bsum, bd - 8);
-          const int pp = max(a * n - d * d, 0);
-          const uint64_t z = (uint64_t(uint32_t(pp)) * sc + (1u << 19)) >> 20;
-          const int a2 = __ldg(a2tab + (z > 255 ? 255 : int(z)));
-          const uint32_t k = uint32_t(256 - a2) * uint32_t(one_over_n);
-          const uint64_t b2 = uint64_t(k) * uint32_t(bsum);
-          A[i * kAS + c] = a2;
-          B[i * kAS + c] = int32_t((b2 + (1u << 11)) >> 12);
-        }
-        bsum -= r1[u];
-        bsq -= r2[u];
-      }
-    }
-  }
-}
-
-// The self-guided filter's value at rows [i0, i1) of column c
-// (postfilter.rs:960-989), handed to emit(i, window sample, value). The walk
-// down the column keeps the three A and B rows around row i in registers,
-// each as its centre value and the sum of its left and right neighbours, so
-// a row costs three loads of A and three of B.
-template <int PASS, typename Emit>
-__device__ __forceinline__ void sgr_flt_col(const int32_t* A, const int32_t* B, const uint16_t* win, int c, int i0,
-                                            int i1, int y0, Emit emit) {
-  const int32_t* pa = A + c + 1;
-  const int32_t* pb = B + c + 1;
-  auto row = [&](const int32_t* q, int& m, int& sum) {
-    m = q[0];
-    sum = q[-1] + q[1];
-  };
-  int am0, as0, am1, as1, bm0, bs0, bm1, bs1;
-  row(pa + i0 * kAS, am0, as0);
-  row(pb + i0 * kAS, bm0, bs0);
-  row(pa + (i0 + 1) * kAS, am1, as1);
-  row(pb + (i0 + 1) * kAS, bm1, bs1);
-  for (int i = i0; i < i1; i++) {
-    int am2, as2, bm2, bs2;
-    row(pa + (i + 2) * kAS, am2, as2);
-    row(pb + (i + 2) * kAS, bm2, bs2);
-    const int cd = win[(i + 3) * kWS + c + 3];
-    int a, b, shift;
-    if (PASS == 0) {
-      if ((y0 + i) & 1) {
-        a = 6 * am1 + 5 * as1;
-        b = 6 * bm1 + 5 * bs1;
-        shift = 4;
-      } else {
-        a = 6 * (am0 + am2) + 5 * (as0 + as2);
-        b = 6 * (bm0 + bm2) + 5 * (bs0 + bs2);
-        shift = 5;
-      }
-    } else {
-      a = 4 * (am1 + as1 + am0 + am2) + 3 * (as0 + as2);
-      b = 4 * (bm1 + bs1 + bm0 + bm2) + 3 * (bs0 + bs2);
-      shift = 5;
-    }
-    emit(i, cd, round2(a * cd + b, 8 + shift - 4));
-    am0 = am1;
-    as0 = as1;
-    bm0 = bm1;
-    bs0 = bs1;
-    am1 = am2;
-    as1 = as2;
-    bm1 = bm2;
-    bs1 = bs2;
-  }
-}
-
 // A rectangle without restoration: its samples of the upscaled CDEF frame
 // go straight to the reference frame and (frames without film grain) the
-// packed frame, 8 samples per thread and step, with no shared-memory round
-// trip and no barrier.
-__device__ __forceinline__ void pass_through(const FrameDesc& f, int p, int x0, int y0, int w, int h, int tid) {
+// packed frame, 8 samples per thread and step, two steps' loads in flight.
+__device__ __forceinline__ void pass_through(const FrameDesc& f, int p, int x0, int y0, int w, int h, const Team& tm) {
   const int sb = f.sb, bps = f.bd > 8 ? 2 : 1;
-  const DPlane src = f.up[p], dst = f.ref[p];
-  const int pw = ((f.uw + plane_ssx(f, p)) >> plane_ssx(f, p));
-  uint8_t* out = f.lr_pack ? f.frame_out + f.out_off[p] : nullptr;
-  const int ng = (w + 7) >> 3;
-  for (int k = tid; k < h * ng; k += kThreads) {
-    const int r = k / ng, c = (k - r * ng) * 8;
-    const int n = min(8, w - c);
-    const int y = y0 + r, x = x0 + c;
-    const uint8_t* sp = src.p + (int64_t(y) * src.stride + x) * sb;
-    uint8_t* dp = dst.p + (int64_t(y) * dst.stride + x) * sb;
-    uint8_t* op = out ? out + (int64_t(y) * pw + x) * bps : nullptr;
-    uint32_t v[8];
-    const bool sv = n == 8 && (reinterpret_cast<uintptr_t>(sp) & (8 * sb - 1)) == 0;
-    if (sv && sb == 2) {
-      const uint4 q = *reinterpret_cast<const uint4*>(sp);
-      v[0] = q.x & 0xffffu; v[1] = q.x >> 16; v[2] = q.y & 0xffffu; v[3] = q.y >> 16;
-      v[4] = q.z & 0xffffu; v[5] = q.z >> 16; v[6] = q.w & 0xffffu; v[7] = q.w >> 16;
-    } else if (sv) {
-      const uint2 q = *reinterpret_cast<const uint2*>(sp);
+  const uint8_t* src = f.up[p].p + (int64_t(y0) * f.up[p].stride + x0) * sb;
+  const int64_t spitch = f.up[p].stride * sb, dpitch = f.ref[p].stride * sb;
+  uint8_t* dst = f.ref[p].p + int64_t(y0) * dpitch + x0 * sb;
+  const int64_t opitch = int64_t((f.uw + plane_ssx(f, p)) >> plane_ssx(f, p)) * bps;
+  uint8_t* out = f.lr_pack ? f.frame_out + f.out_off[p] + int64_t(y0) * opitch + x0 * bps : nullptr;
+  const int ng = (w + 7) >> 3;  // 8-sample chunks a row, at most 8
+  const int inv = c_lr.inv[ng];
+  const bool sv = ((reinterpret_cast<uintptr_t>(src) | uintptr_t(spitch)) & uintptr_t(8 * sb - 1)) == 0;
+  constexpr int kBatch = 2;
+#pragma unroll 1
+  for (int k0 = tm.t; k0 < h * ng; k0 += kBatch * tm.n) {
+    uint4 q[kBatch];  // two samples to a word
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        v[e] = (q.x >> (8 * e)) & 0xffu;
-        v[4 + e] = (q.y >> (8 * e)) & 0xffu;
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; e++) v[e] = e < n ? uint32_t(ld_row(sp, sb, e)) : 0u;
-    }
-    auto put = [&](uint8_t* base, int width) {
-      if (n == 8 && (reinterpret_cast<uintptr_t>(base) & (8 * width - 1)) == 0) {
-        if (width == 2)
-          *reinterpret_cast<uint4*>(base) =
-              make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
-        else
-          *reinterpret_cast<uint2*>(base) = make_uint2(v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24),
-                                                       v[4] | (v[5] << 8) | (v[6] << 16) | (v[7] << 24));
-      } else {
-        for (int e = 0; e < n; e++) {
-          if (width == 2)
-            reinterpret_cast<uint16_t*>(base)[e] = uint16_t(v[e]);
-          else
-            base[e] = uint8_t(v[e]);
-        }
-      }
-    };
-    put(dp, sb);
-    if (op) put(op, bps);
-  }
-}
-
-// The shared-memory areas of one CTA.
-struct LrSmem {
-  uint16_t* win;    // the window, rows kWS apart
-  int32_t* A;       // self-guided A (Wiener: the int16 intermediate)
-  int32_t* B;       // self-guided B
-  const int32_t* a2tab;  // SGR_A2 (global memory)
-  int32_t* F0;      // first self-guided output, then every rectangle's output
-  av1pf_lr_unit* unit;
-};
-
-// Restores one rectangle of w <= MW columns into the output tile. CW is the
-// width of a row group (threads per group: 72 for rectangles up to 64
-// columns, 36 for those up to 32, so narrow rectangles keep most threads
-// busy); the window is staged by groups SW threads wide.
-template <int CW>
-__device__ __forceinline__ void restore_rect(const FrameDesc& f, const LrSmem& sm, const LrGeom& geo, int p, int s,
-                                             int x0, int w, int h, int type, const av1pf_lr_unit* unit_p, int tid) {
-  constexpr int G = kThreads / CW;          // row groups
-  constexpr int MW = CW == 72 ? 64 : 32;    // widest rectangle
-  constexpr int SW = CW == 72 ? 72 : 48;    // staging group width (>= MW + 6)
-  constexpr int SG = kThreads / SW;         // staging groups
-  static_assert(G * CW == kThreads && SG * SW == kThreads, "layouts cover the CTA");
-  const int g = tid / CW, c = tid - g * CW;
-  const int sb = f.sb, bd = f.bd;
-  const int maxv = (1 << bd) - 1;
-  int32_t* F0 = sm.F0;
-  if (type != AV1PF_RESTORE_WIENER && type != AV1PF_RESTORE_SGRPROJ) {
-    // a unit without restoration passes its samples through
-    load_tile<MW>(f.up[p], sb, x0, geo.y0, w, h, F0, tid);
-    return;
-  }
-  uint16_t* win = sm.win;
-  // the unit's coefficients wait in shared memory while the window loads
-  if (tid == 0) *sm.unit = *unit_p;
-  // lr_window (postfilter.rs:765-777): a thread's loads all issue before its stores
-  const int ww = w + 6, wh = h + 6;
-  {
-    LrSrc src;
-    src.up = f.up[p].p;
-    src.cur = f.cur[p].p;
-    // superres: upscaled boundary rows; fused horizontal LF pass: the
-    // loop filter's boundary rows; else the loop-filtered plane itself
-    const DPlane lines = f.sr_on ? f.lines[p] : f.prelf[p];
-    src.lines = lines.p;
-    src.up_pitch = int32_t(f.up[p].stride * sb);
-    src.cur_pitch = int32_t(f.cur[p].stride * sb);
-    src.lines_pitch = int32_t(lines.stride * sb);
-    src.sr = f.sr_on != 0 || f.prelf[p].p != nullptr;
-    // Window row r, columns 8q .. 8q+7 (samples x0-3+8q ..) per task. Where
-    // the two aligned 8-sample chunks that hold them lie inside the plane
-    // row (and the row is 16-byte aligned) they come as two vector loads
-    // and are shifted into place; other chunks (the plane's left and right
-    // edges) take one clamped scalar load per sample. The loads of two tasks
-    // issue before their stores.
-    const int nq = (ww + 7) >> 3;  // chunks per window row (<= 9)
-    constexpr int kTasks = ((kMaxH + 6) * 9 + kThreads - 1) / kThreads;
-    const int ntask = wh * nq;
-    constexpr int kBatch = 2;  // tasks whose loads are in flight together
-#pragma unroll
-    for (int m0 = 0; m0 < kTasks; m0 += kBatch) {
-      uint32_t wv[kBatch][5];  // the loaded words a window chunk is cut from
-      bool vec[kBatch];
-#pragma unroll
-      for (int m = 0; m < kBatch; m++) {
-        const int k = tid + (m0 + m) * kThreads;
-        vec[m] = false;
-        if (m0 + m >= kTasks || k >= ntask) continue;
-        const int r = k / nq, q = k - r * nq;
-        const uint8_t* row = lr_row(src, geo, s, geo.y0 + r - 3);
-        const int gx = x0 - 8 + 8 * q;  // first sample of the left chunk
-        if (gx < 0 || gx + 16 > geo.pex + 1 || (reinterpret_cast<uintptr_t>(row) & 15) != 0) continue;
-        vec[m] = true;
+    for (int m = 0; m < kBatch; m++) {
+      const int k = k0 + m * tm.n;
+      if (k >= h * ng) continue;
+      const int r = (k * inv) >> 16, c = (k - r * ng) * 8;
+      const uint8_t* sp = src + int64_t(r) * spitch + c * sb;
+      if (sv && c + 8 <= w) {
         if (sb == 2) {
-          // samples 4..7 of the left chunk and 0..5 of the right one
-          const uint2 a = *reinterpret_cast<const uint2*>(row + int64_t(gx) * 2 + 8);
-          const uint4 b = *reinterpret_cast<const uint4*>(row + int64_t(gx) * 2 + 16);
-          wv[m][0] = a.x; wv[m][1] = a.y; wv[m][2] = b.x; wv[m][3] = b.y; wv[m][4] = b.z;
+          q[m] = *reinterpret_cast<const uint4*>(sp);
         } else {
-          // bytes 4..15 of the 16 samples
-          const uint4 a = *reinterpret_cast<const uint4*>(row + gx);
-          wv[m][0] = a.y; wv[m][1] = a.z; wv[m][2] = a.w;
+          const uint2 b = *reinterpret_cast<const uint2*>(sp);
+          q[m] = make_uint4(__byte_perm(b.x, 0, 0x4140), __byte_perm(b.x, 0, 0x4342), __byte_perm(b.y, 0, 0x4140),
+                            __byte_perm(b.y, 0, 0x4342));
         }
-      }
+      } else {
+        uint32_t v[8];
 #pragma unroll
-      for (int m = 0; m < kBatch; m++) {
-        const int k = tid + (m0 + m) * kThreads;
-        if (m0 + m >= kTasks || k >= ntask) continue;
-        const int r = k / nq, q = k - r * nq;
-        uint16_t* wp = &win[r * kWS + 8 * q];
-        if (vec[m]) {
-          uint4 o;
-          if (sb == 2) {
-            // window sample 2j of the chunk is sample 5 + 2j of the 16 from gx
-            o.x = __funnelshift_r(wv[m][0], wv[m][1], 16);
-            o.y = __funnelshift_r(wv[m][1], wv[m][2], 16);
-            o.z = __funnelshift_r(wv[m][2], wv[m][3], 16);
-            o.w = __funnelshift_r(wv[m][3], wv[m][4], 16);
-          } else {
-            const uint32_t lo = __funnelshift_r(wv[m][0], wv[m][1], 8);  // bytes 5..8
-            const uint32_t hi = __funnelshift_r(wv[m][1], wv[m][2], 8);  // bytes 9..12
-            o.x = __byte_perm(lo, 0, 0x4140);
-            o.y = __byte_perm(lo, 0, 0x4342);
-            o.z = __byte_perm(hi, 0, 0x4140);
-            o.w = __byte_perm(hi, 0, 0x4342);
-          }
-          *reinterpret_cast<uint4*>(wp) = o;
+        for (int e = 0; e < 8; e++) v[e] = c + e < w ? uint32_t(ld_row(sp, sb, e)) : 0u;
+        q[m] = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kBatch; m++) {
+      const int k = k0 + m * tm.n;
+      if (k >= h * ng) continue;
+      const int r = (k * inv) >> 16, c = (k - r * ng) * 8, n = min(8, w - c);
+      auto put = [&](uint8_t* at, int width) {
+        if (n == 8 && (reinterpret_cast<uintptr_t>(at) & uintptr_t(8 * width - 1)) == 0) {
+          if (width == 2)
+            *reinterpret_cast<uint4*>(at) = q[m];
+          else
+            *reinterpret_cast<uint2*>(at) =
+                make_uint2(__byte_perm(q[m].x, q[m].y, 0x6420), __byte_perm(q[m].z, q[m].w, 0x6420));
         } else {
-          const uint8_t* row = lr_row(src, geo, s, geo.y0 + r - 3);
+          const uint32_t wd[4] = {q[m].x, q[m].y, q[m].z, q[m].w};
 #pragma unroll
           for (int e = 0; e < 8; e++) {
-            const int c = 8 * q + e;
-            if (c < ww) wp[e] = uint16_t(ld_row(row, sb, max(min(x0 - 3 + c, geo.pex), 0)));
+            if (e >= n) continue;
+            const uint32_t v = (e & 1) ? wd[e >> 1] >> 16 : wd[e >> 1];
+            if (width == 2)
+              reinterpret_cast<uint16_t*>(at)[e] = uint16_t(v);
+            else
+              at[e] = uint8_t(v);
           }
         }
+      };
+      put(dst + int64_t(r) * dpitch + c * sb, sb);
+      if (out) put(out + int64_t(r) * opitch + c * bps, bps);
+    }
+  }
+}
+
+// Where the window's rows come from: rows[r] is the start of the plane row that
+// window row r reads.
+__device__ __forceinline__ void window_rows(const FrameDesc& f, const uint8_t** rows, const LrGeom& geo, int p, int s, int h,
+                                            const Team& tm) {
+  const int sb = f.sb;
+  LrSrc src;
+  src.up = f.up[p].p;
+  src.cur = f.cur[p].p;
+  // superres: upscaled boundary rows; fused horizontal LF pass: the
+  // loop filter's boundary rows; else the loop-filtered plane itself
+  const DPlane& lines = f.sr_on ? f.lines[p] : f.prelf[p];
+  src.lines = lines.p;
+  src.up_pitch = int32_t(f.up[p].stride * sb);
+  src.cur_pitch = int32_t(f.cur[p].stride * sb);
+  src.lines_pitch = int32_t(lines.stride * sb);
+  src.sr = f.sr_on != 0 || f.prelf[p].p != nullptr;
+  for (int r = tm.t; r < h + 6; r += tm.n) rows[r] = lr_row(src, geo, s, geo.y0 + r - 3);
+}
+
+// lr_window (postfilter.rs:765-777): window row r, columns 8q .. 8q+7 (samples
+// x0-3+8q ..) per task. Where the two aligned 8-sample chunks that hold them
+// lie inside the plane row (and the row is 16-byte aligned) they come as two
+// vector loads and are shifted into place; other chunks (the plane's left and
+// right edges) take one clamped scalar load per sample. The loads of two
+// tasks issue before their stores.
+__device__ __forceinline__ void stage_window(uint16_t* win, int ws, const uint8_t* const* rows, int sb, int pex, int x0,
+                                             int w, int h, const Team& tm) {
+  const int ww = w + 6, wh = h + 6;
+  const int nq = (ww + 7) >> 3;  // chunks per window row (<= 9)
+  const int inv = c_lr.inv[nq];
+  const int ntask = wh * nq;
+  constexpr int kBatch = 2;
+#pragma unroll 1
+  for (int k0 = tm.t; k0 < ntask; k0 += kBatch * tm.n) {
+    uint32_t wv[kBatch][5];  // the loaded words a window chunk is cut from
+    bool vec[kBatch];
+#pragma unroll
+    for (int m = 0; m < kBatch; m++) {
+      const int k = k0 + m * tm.n;
+      vec[m] = false;
+      if (k >= ntask) continue;
+      const int r = (k * inv) >> 16, q = k - r * nq;
+      const uint8_t* row = rows[r];
+      const int gx = x0 - 8 + 8 * q;  // first sample of the left chunk
+      if (gx < 0 || gx + 16 > pex + 1 || (reinterpret_cast<uintptr_t>(row) & 15) != 0) continue;
+      vec[m] = true;
+      if (sb == 2) {
+        // samples 4..7 of the left chunk and 0..5 of the right one
+        const uint2 a = *reinterpret_cast<const uint2*>(row + int64_t(gx) * 2 + 8);
+        const uint4 b = *reinterpret_cast<const uint4*>(row + int64_t(gx) * 2 + 16);
+        wv[m][0] = a.x; wv[m][1] = a.y; wv[m][2] = b.x; wv[m][3] = b.y; wv[m][4] = b.z;
+      } else {
+        // bytes 4..15 of the 16 samples
+        const uint4 a = *reinterpret_cast<const uint4*>(row + gx);
+        wv[m][0] = a.y; wv[m][1] = a.z; wv[m][2] = a.w;
       }
     }
-  }
-  __syncthreads();
-  const av1pf_lr_unit& unit = *sm.unit;
-  // each row group's contiguous run of output rows
-  const int per = (h + G - 1) / G;
-  const int i0 = g * per, i1 = min(h, i0 + per);
-  const bool col = c < w && i0 < i1;
-  if (type == AV1PF_RESTORE_WIENER) {
-    // postfilter.rs:795-822
-    int16_t* inter = reinterpret_cast<int16_t*>(sm.A);
-    const int round0 = bd == 12 ? 5 : 3, round1 = bd == 12 ? 9 : 11;
-    const int offset = 1 << (bd + 7 - round0 - 1);
-    const int limit = (1 << (bd + 1 + 7 - round0)) - 1;
-    const int h0 = unit.wiener[1][0], h1 = unit.wiener[1][1], h2 = unit.wiener[1][2];
-    const int v0 = unit.wiener[0][0], v1 = unit.wiener[0][1], v2 = unit.wiener[0][2];
-    const int h3 = 128 - 2 * (h0 + h1 + h2), v3 = 128 - 2 * (v0 + v1 + v2);
-    // horizontal pass: two adjacent outputs per task from 8 window samples
-    // (four aligned 32-bit loads), packed into one 32-bit store
-    constexpr int LP = MW == 64 ? 5 : 4;  // log2 column pairs per row
-    for (int k = tid; k < (wh << LP); k += kThreads) {
-      const int r = k >> LP, c2 = (k & ((1 << LP) - 1)) * 2;
-      if (c2 >= w) continue;
-      const uint32_t* sp = reinterpret_cast<const uint32_t*>(&win[r * kWS + c2]);
-      const uint32_t q0 = sp[0], q1 = sp[1], q2 = sp[2], q3 = sp[3];
-      const int s0 = int(q0 & 0xffffu), s1 = int(q0 >> 16), s2 = int(q1 & 0xffffu), s3 = int(q1 >> 16);
-      const int s4 = int(q2 & 0xffffu), s5 = int(q2 >> 16), s6 = int(q3 & 0xffffu), s7 = int(q3 >> 16);
-      const int a0 = h0 * (s0 + s6) + h1 * (s1 + s5) + h2 * (s2 + s4) + h3 * s3;
-      const int a1 = h0 * (s1 + s7) + h1 * (s2 + s6) + h2 * (s3 + s5) + h3 * s4;
-      const int o0 = clip3(-offset, limit - offset, round2(a0, round0));
-      const int o1 = clip3(-offset, limit - offset, round2(a1, round0));
-      *reinterpret_cast<uint32_t*>(&inter[r * kWS + c2]) = uint32_t(uint16_t(o0)) | (uint32_t(uint16_t(o1)) << 16);
-    }
-    __syncthreads();
-    // vertical pass: each row group slides a 7-row window down its column
-    if (col) {
-      const int16_t* ip = &inter[i0 * kWS + c];
-      int t0 = ip[0], t1 = ip[kWS], t2 = ip[2 * kWS], t3 = ip[3 * kWS], t4 = ip[4 * kWS], t5 = ip[5 * kWS];
-      for (int i = i0; i < i1; i++) {
-        const int t6 = inter[(i + 6) * kWS + c];
-        const int acc = v0 * (t0 + t6) + v1 * (t1 + t5) + v2 * (t2 + t4) + v3 * t3;
-        F0[i * kMaxW + c] = clip3(0, maxv, round2(acc, round1));
-        t0 = t1;
-        t1 = t2;
-        t2 = t3;
-        t3 = t4;
-        t4 = t5;
-        t5 = t6;
-      }
-    }
-    return;
-  }
-  // postfilter.rs:823-851 with box_filter_rect (postfilter.rs:901-991)
-  int32_t* A = sm.A;
-  int32_t* B = sm.B;
-  const int set = unit.sgr_set & 15;
-  const int r0 = c_sgr_params[set][0], r1 = c_sgr_params[set][2];
-  if (r0) {
-    sgr_ab<0, G>(win, A, B, sm.a2tab, c_sgr_params[set][1], bd, geo.y0, h, w, c, g);
-    __syncthreads();
-    if (col) sgr_flt_col<0>(A, B, win, c, i0, i1, geo.y0, [&](int i, int, int v) { F0[i * kMaxW + c] = v; });
-    __syncthreads();
-  }
-  if (r1) {
-    sgr_ab<1, G>(win, A, B, sm.a2tab, c_sgr_params[set][3], bd, geo.y0, h, w, c, g);
-    __syncthreads();
-  }
-  const int w0 = unit.sgr_xqd[0], w1 = unit.sgr_xqd[1];
-  const int w2 = (1 << 7) - w0 - w1;
-  if (col) {
-    // the weighted sum of the two filters and the sample itself; this
-    // thread's own slot of the output tile
-    auto combine = [&](int i, int cd, int flt1) {
-      const int u = cd << 4;
-      int v = w1 * u;
-      v += r0 != 0 ? w0 * F0[i * kMaxW + c] : w0 * u;
-      v += w2 * flt1;
-      F0[i * kMaxW + c] = clip3(0, maxv, round2(v, 11));
-    };
-    if (r1) {
-      sgr_flt_col<1>(A, B, win, c, i0, i1, geo.y0, combine);
-    } else {
-      for (int i = i0; i < i1; i++) {
-        const int cd = win[(i + 3) * kWS + c + 3];
-        combine(i, cd, cd << 4);
+#pragma unroll
+    for (int m = 0; m < kBatch; m++) {
+      const int k = k0 + m * tm.n;
+      if (k >= ntask) continue;
+      const int r = (k * inv) >> 16, q = k - r * nq;
+      uint16_t* wp = &win[r * ws + 8 * q];
+      if (vec[m]) {
+        uint4 o;
+        if (sb == 2) {
+          // window sample 2j of the chunk is sample 5 + 2j of the 16 from gx
+          o.x = __funnelshift_r(wv[m][0], wv[m][1], 16);
+          o.y = __funnelshift_r(wv[m][1], wv[m][2], 16);
+          o.z = __funnelshift_r(wv[m][2], wv[m][3], 16);
+          o.w = __funnelshift_r(wv[m][3], wv[m][4], 16);
+        } else {
+          const uint32_t lo = __funnelshift_r(wv[m][0], wv[m][1], 8);  // bytes 5..8
+          const uint32_t hi = __funnelshift_r(wv[m][1], wv[m][2], 8);  // bytes 9..12
+          o.x = __byte_perm(lo, 0, 0x4140);
+          o.y = __byte_perm(lo, 0, 0x4342);
+          o.z = __byte_perm(hi, 0, 0x4140);
+          o.w = __byte_perm(hi, 0, 0x4342);
+        }
+        // (slim rows are 8-byte aligned)
+        reinterpret_cast<uint2*>(wp)[0] = make_uint2(o.x, o.y);
+        if (8 * q + 4 < ws) reinterpret_cast<uint2*>(wp)[1] = make_uint2(o.z, o.w);
+      } else {
+        const uint8_t* row = rows[r];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          const int c = 8 * q + e;
+          if (c < ww) wp[e] = uint16_t(ld_row(row, sb, max(min(x0 - 3 + c, pex), 0)));
+        }
       }
     }
   }
 }
 
-// With readiness flags: waits (threads 0..15, one flag each) for the CDEF
+// What a group restores: rows i0 .. of the rectangle, `per` of them walked (the
+// same for a warp's groups) and `left` of them written; the lane's columns c and
+// c + 1, and where they go: the next row in the reference frame and (not null)
+// the packed frame, in samples of rw and ow bytes.
+struct Group {
+  int i0, per, left, c;
+  int cols;             // how many of the lane's columns are inside the rectangle
+  const uint16_t* win;  // window row 0, column c
+  int ws;
+  uint8_t *ref, *out;
+  int64_t ref_pitch, out_pitch;
+  int rw, ow;
+};
+
+// Writes the next row's samples. PAIRS: both of every lane's are written, and
+// are aligned as a pair in every row.
+template <bool PAIRS>
+__device__ __forceinline__ void emit(Group& g, uint32_t a, uint32_t b) {
+  auto put = [&](uint8_t* at, int width) {
+    if (PAIRS) {
+      if (width == 2)
+        *reinterpret_cast<uint32_t*>(at) = a | (b << 16);
+      else
+        *reinterpret_cast<uint16_t*>(at) = uint16_t(a | (b << 8));
+      return;
+    }
+    if (width == 2) {
+      if (g.cols > 0) reinterpret_cast<uint16_t*>(at)[0] = uint16_t(a);
+      if (g.cols > 1) reinterpret_cast<uint16_t*>(at)[1] = uint16_t(b);
+    } else {
+      if (g.cols > 0) at[0] = uint8_t(a);
+      if (g.cols > 1) at[1] = uint8_t(b);
+    }
+  };
+  if (g.left > 0) {
+    put(g.ref, g.rw);
+    if (g.out) {
+      put(g.out, g.ow);
+      g.out += g.out_pitch;
+    }
+  }
+  g.left--;
+  g.ref += g.ref_pitch;
+}
+
+// Four 8-bit coefficients in a word.
+__device__ __forceinline__ int bytes4(int a, int b, int c, int d) {
+  return int((uint32_t(a) & 255u) | ((uint32_t(b) & 255u) << 8) | ((uint32_t(c) & 255u) << 16) | (uint32_t(d) << 24));
+}
+
+// postfilter.rs:795-822
+template <bool PAIRS>
+__device__ __forceinline__ void wiener_group(Group& g, const av1pf_lr_unit& u, int bd) {
+  const int round0 = bd == 12 ? 5 : 3, round1 = bd == 12 ? 9 : 11;
+  const int offset = 1 << (bd + 7 - round0 - 1);
+  const int limit = (1 << (bd + 1 + 7 - round0)) - 1;
+  const int maxv = (1 << bd) - 1;
+  const int h0 = u.wiener[1][0], h1 = u.wiener[1][1], h2 = u.wiener[1][2];
+  const int v0 = u.wiener[0][0], v1 = u.wiener[0][1], v2 = u.wiener[0][2];
+  const int h3 = 128 - 2 * (h0 + h1 + h2), v3 = 128 - 2 * (v0 + v1 + v2);
+  // the taps but the middle one (which can exceed 8 bits) against the samples
+  // c .. c + 7, for the first column and the second
+  const int e0 = bytes4(h0, h1, h2, 0), e1 = bytes4(h2, h1, h0, 0);
+  const int o0 = bytes4(0, h0, h1, h2), o1 = bytes4(0, h2, h1, h0);
+  const int rnd0 = 1 << (round0 - 1), rnd1 = 1 << (round1 - 1);
+  const uint16_t* row = g.win + g.i0 * g.ws;
+  auto across = [&](int& a, int& b) {
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(row);
+    row += g.ws;
+    const int q0 = int(q[0]), q1 = int(q[1]), q2 = int(q[2]), q3 = int(q[3]);
+    int x = int(uint32_t(q1) >> 16) * h3 + rnd0, y = (q2 & 0xffff) * h3 + rnd0;
+    x = __dp2a_hi(q3, e1, __dp2a_lo(q2, e1, __dp2a_hi(q1, e0, __dp2a_lo(q0, e0, x))));
+    y = __dp2a_hi(q3, o1, __dp2a_lo(q2, o1, __dp2a_hi(q1, o0, __dp2a_lo(q0, o0, y))));
+    a = clip3(-offset, limit - offset, x >> round0);
+    b = clip3(-offset, limit - offset, y >> round0);
+  };
+  // the last six rows' results and four new ones a step
+  int a[10], b[10];
+#pragma unroll
+  for (int k = 0; k < 6; k++) across(a[k], b[k]);
+  auto down = [&](const int* t) {
+    const int acc = v0 * (t[0] + t[6]) + v1 * (t[1] + t[5]) + v2 * (t[2] + t[4]) + v3 * t[3] + rnd1;
+    return uint32_t(clip3(0, maxv, acc >> round1));
+  };
+#pragma unroll 1
+  for (int i = 0; i < g.per; i += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      across(a[6 + k], b[6 + k]);
+      emit<PAIRS>(g, down(a + k), down(b + k));
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      a[k] = a[k + 4];
+      b[k] = b[k + 4];
+    }
+  }
+}
+
+// A and B of box_filter_rect (postfilter.rs:935-959) packed in a word, A above
+// B, from the sum and the sum of squares over a box of radius R. B is at most
+// (255 * ((4096 + n / 2) / n) * n * (2^bitdepth - 1) + 2^11) >> 12 < 2^20 for 12
+// bits, and all products fit 32 bits but p * s.
+constexpr int kAB = 21;  // bits of B: room for the sum of two at 12 bits, of five at 10
+template <int R>
+__device__ __forceinline__ uint32_t sgr_word(uint32_t sum, uint32_t sq, uint32_t s12, int sh) {
+  constexpr uint32_t n = (2 * R + 1) * (2 * R + 1), one_over_n = ((1u << 12) + n / 2) / n;
+  const uint32_t half = (1u << sh) >> 1;
+  const uint32_t a = (sq + ((1u << (2 * sh)) >> 1)) >> (2 * sh), d = (sum + half) >> sh;
+  const int pp = max(int(a * n - d * d), 0);
+  // (p * s + 2^19) >> 20, as the high word of p * (s << 12) + 2^31
+  const uint32_t z = uint32_t((uint64_t(uint32_t(pp)) * s12 + (1u << 31)) >> 32);
+  const uint32_t a2 = uint32_t(__ldg(&g_sgr_a2.v[min(z, 255u)]));
+  const uint32_t b = ((256u - a2) * one_over_n * sum + (1u << 11)) >> 12;
+  return (a2 << kAB) | b;
+}
+
+// postfilter.rs:823-851 with box_filter_rect (postfilter.rs:901-991). Window
+// row i + 3, columns c + 3 and c + 4 are the lane's samples of row i. DEEP: 12
+// bits, where sums of more than two B's leave their field and the sum over a
+// 5x5 box its 16 bits.
+template <bool DEEP, bool PAIRS>
+__device__ __forceinline__ void sgr_group(Group& g, const av1pf_lr_unit& u, int bd, GroupEdges& edges, int gl, int gn) {
+  const int set = u.sgr_set & 15;
+  const int r0 = c_sgr_params[set][0], r1 = c_sgr_params[set][2];
+  const uint32_t sa = c_lr.s12[set][0], sb = c_lr.s12[set][1];
+  // the weights of the first filter, the sample and the second filter; a filter
+  // that is off (radius 0) gives the sample, whose weight then takes its own
+  int w0 = u.sgr_xqd[0], w1 = u.sgr_xqd[1], w2 = (1 << 7) - w0 - w1;
+  if (!r0) {
+    w1 += w0;
+    w0 = 0;
+  }
+  if (!r1) {
+    w1 += w2;
+    w2 = 0;
+  }
+  w1 *= 16;
+  const int maxv = (1 << bd) - 1, sh = bd - 8;
+  const int ws = g.ws;
+  // --- the words of the columns at either side of the group: one at a time, a
+  // lane a (row, side). Row j of `second` is output row i0 - 1 + j, of `first`
+  // i0 - 1 + 2j ---
+  {
+    const uint16_t* base = g.win - g.c + g.i0 * ws;  // window row i0, the group's first column
+    const int width = 2 * gn;
+    if (r1)
+#pragma unroll 1
+      for (int k = gl; k < 2 * (g.per + 2); k += gn) {
+        const int j = k >> 1, side = k & 1;
+        const uint16_t* at = base + (j + 2) * ws + (side ? width : -1) + 3;
+        uint32_t s = 0, q = 0;
+#pragma unroll
+        for (int y = -1; y <= 1; y++)
+#pragma unroll
+          for (int x = -1; x <= 1; x++) {
+            const uint32_t v = at[y * ws + x];
+            s += v;
+            q += v * v;
+          }
+        edges.second[j][side] = sgr_word<1>(s, q, sb, sh);
+      }
+    if (r0)
+#pragma unroll 1
+      for (int k = gl; k < g.per + 2; k += gn) {
+        const int j = k >> 1, side = k & 1;
+        const uint16_t* at = base + (2 * j + 2) * ws + (side ? width : -1) + 3;
+        uint32_t s = 0, q = 0;
+#pragma unroll
+        for (int y = -2; y <= 2; y++)
+#pragma unroll
+          for (int x = -2; x <= 2; x++) {
+            const uint32_t v = at[y * ws + x];
+            s += v;
+            q += v * v;
+          }
+        edges.first[j][side] = sgr_word<2>(s, q, sa, sh);
+      }
+    __syncwarp();
+  }
+  const bool at_left = gl == 0, at_right = gl == gn - 1;
+  // A word's two columns in x, and the sums of each one's neighbours in y
+  struct Words {
+    uint32_t x0, x1, y0, y1;
+  };
+  auto with_neighbours = [&](uint32_t x0, uint32_t x1, const uint32_t (&edge)[2]) {
+    uint32_t l = __shfl_up_sync(0xffffffffu, x1, 1), r = __shfl_down_sync(0xffffffffu, x0, 1);
+    if (at_left) l = edge[0];
+    if (at_right) r = edge[1];
+    return Words{x0, x1, l + x1, x0 + r};
+  };
+  // Horizontal sums of a window row around the lane's two columns: the samples
+  // (both columns' in the halves of a word) and their squares, radius 2 and 1.
+  struct Rows {
+    uint32_t s5, s3, q5a, q5b, q3a, q3b;
+  };
+  const uint16_t* row = g.win + g.i0 * ws;
+  auto across = [&]() {
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(row);
+    row += ws;
+    // window columns c .. c + 7; the lane's columns are 3 and 4 of them
+    const uint32_t k0 = q[0], k1 = q[1], k2 = q[2], k3 = q[3];
+    const uint32_t m1 = __byte_perm(k0, k1, 0x5432), m2 = __byte_perm(k1, k2, 0x5432), m3 = __byte_perm(k2, k3, 0x5432);
+    Rows t;
+    t.s3 = k1 + m2 + k2;                 // (2,3) + (3,4) + (4,5)
+    t.s5 = t.s3 + m1 + m3;               // + (1,2) + (5,6)
+    const uint32_t p1 = k0 >> 16, p2 = k1 & 0xffffu, p3 = k1 >> 16, p4 = k2 & 0xffffu, p5 = k2 >> 16, p6 = k3 & 0xffffu;
+    const uint32_t m = p3 * p3 + p4 * p4;
+    t.q3a = p2 * p2 + m;
+    t.q3b = p5 * p5 + m;
+    t.q5a = p1 * p1 + (p5 * p5 + t.q3a);
+    t.q5b = p6 * p6 + (p2 * p2 + t.q3b);
+    return t;
+  };
+  auto lo = [](uint32_t v) { return v & 0xffffu; };
+  auto hi = [](uint32_t v) { return v >> 16; };
+  // The sums of the rows so far, of step row i: radius 2, row i - 1 (p), rows i
+  // and i + 1 together (g) and row i + 1 (o); radius 1, rows i and i + 1 together
+  // (g3) and row i + 1 (o3). Samples of both columns in a word, squares apart.
+  struct Sums {
+    uint32_t s, a, b;
+    __device__ __forceinline__ Sums operator+(const Sums& t) const { return Sums{s + t.s, a + t.a, b + t.b}; }
+  };
+  auto of5 = [](const Rows& t) { return Sums{t.s5, t.q5a, t.q5b}; };
+  auto of3 = [](const Rows& t) { return Sums{t.s3, t.q3a, t.q3b}; };
+  auto words1 = [&](const Sums& t, const uint32_t (&edge)[2]) {
+    return with_neighbours(sgr_word<1>(lo(t.s), t.a, sb, sh), sgr_word<1>(hi(t.s), t.b, sb, sh), edge);
+  };
+  // (DEEP: the five rows' sample sums leave 16 bits; x is the sum of three rows' at most, y of two)
+  auto words2 = [&](const Sums& x, const Sums& y, const uint32_t (&edge)[2]) {
+    const uint32_t s = x.s + y.s;
+    return with_neighbours(sgr_word<2>(DEEP ? lo(x.s) + lo(y.s) : lo(s), x.a + y.a, sa, sh),
+                           sgr_word<2>(DEEP ? hi(x.s) + hi(y.s) : hi(s), x.b + y.b, sa, sh), edge);
+  };
+  Sums p{}, g5{}, o{}, g3{}, o3{};
+  Words f0{}, b0{}, b1{};  // first filter: row i - 1; second: rows i - 1 and i
+  {
+    const Rows t0 = across(), t1 = across(), t2 = across(), t3 = across(), t4 = across();  // rows i0 - 3 .. i0 + 1
+    p = of5(t2);
+    o = of5(t4);
+    g5 = of5(t3) + o;
+    o3 = of3(t4);
+    g3 = of3(t3) + o3;
+    if (r0) f0 = words2(of5(t0) + of5(t1) + p, g5, edges.first[0]);
+    if (r1) {
+      b0 = words1(of3(t1) + of3(t2) + of3(t3), edges.second[0]);
+      b1 = words1(of3(t2) + g3, edges.second[1]);
+    }
+  }
+  constexpr uint32_t kB = (1u << kAB) - 1;
+  // (wa * A's + wb * B's) of words x and y weighed wx and wy, times the sample
+  auto blend = [&](uint32_t x, uint32_t y, int wx, int wy, uint32_t cd) {
+    return int((wx * (x >> kAB) + wy * (y >> kAB)) * cd + (wx * (x & kB) + wy * (y & kB)));
+  };
+  auto blend2 = [&](uint32_t x, uint32_t x2, uint32_t y, uint32_t y2, int wx, int wy, uint32_t cd) {
+    return DEEP ? int((wx * ((x >> kAB) + (x2 >> kAB)) + wy * ((y >> kAB) + (y2 >> kAB))) * cd +
+                      (wx * ((x & kB) + (x2 & kB)) + wy * ((y & kB) + (y2 & kB))))
+                : blend(x + x2, y + y2, wx, wy, cd);
+  };
+  auto blend5 = [&](uint32_t x, uint32_t y, uint32_t x0, uint32_t x2, uint32_t y0, uint32_t y2, uint32_t cd) {
+    return DEEP ? int((4 * ((x >> kAB) + (y >> kAB) + (x0 >> kAB) + (x2 >> kAB)) + 3 * ((y0 >> kAB) + (y2 >> kAB))) * cd +
+                      (4 * ((x & kB) + (y & kB) + (x0 & kB) + (x2 & kB)) + 3 * ((y0 & kB) + (y2 & kB))))
+                : blend(x + y + x0 + x2, y0 + y2, 4, 3, cd);
+  };
+  auto finish = [&](uint32_t cd, int flt0, int flt1) {
+    return uint32_t(clip3(0, maxv, (w1 * int(cd) + (1 << 10) + w0 * flt0 + w2 * flt1) >> 11));
+  };
+#pragma unroll 1  // (and the loops below and above: unrolled, they take more registers than a CTA has)
+  for (int step = 0; step < g.per / 2; step++) {
+    // row i + 2 completes the second filter's row i + 1, and its output row i
+    Rows t = across();
+    Words b2{};
+    Sums n5 = of5(t);
+    const Sums n3 = of3(t);
+    if (r1) b2 = words1(g3 + n3, edges.second[2 * step + 2]);
+    const uint16_t* mid = row - 3 * ws + 2;  // samples (c - 1, c) and (c + 1, ..) of row i
+    uint32_t ca = hi(*reinterpret_cast<const uint32_t*>(mid)), cb = lo(*reinterpret_cast<const uint32_t*>(mid + 2));
+    const int sa1 = (blend5(b1.x0, b1.y0, b0.x0, b2.x0, b0.y0, b2.y0, ca) + 256) >> 9;
+    const int sb1 = (blend5(b1.x1, b1.y1, b0.x1, b2.x1, b0.y1, b2.y1, cb) + 256) >> 9;
+    // row i + 3 completes the first filter's row i + 1: the even output row takes
+    // it and row i - 1
+    t = across();
+    Words f1{};
+    const Sums m5 = of5(t);
+    if (r0) f1 = words2(p + g5, n5 + m5, edges.first[step + 1]);
+    emit<PAIRS>(g, finish(ca, (blend2(f0.x0, f1.x0, f0.y0, f1.y0, 6, 5, ca) + 256) >> 9, sa1),
+           finish(cb, (blend2(f0.x1, f1.x1, f0.y1, f1.y1, 6, 5, cb) + 256) >> 9, sb1));
+    f0 = f1;
+    b0 = b1;
+    b1 = b2;
+    // and the second filter's row i + 2: the odd row
+    if (r1) b2 = words1(o3 + n3 + of3(t), edges.second[2 * step + 3]);
+    mid += ws;
+    ca = hi(*reinterpret_cast<const uint32_t*>(mid));
+    cb = lo(*reinterpret_cast<const uint32_t*>(mid + 2));
+    emit<PAIRS>(g, finish(ca, (blend(f0.x0, f0.y0, 6, 5, ca) + 128) >> 8,
+                  (blend5(b1.x0, b1.y0, b0.x0, b2.x0, b0.y0, b2.y0, ca) + 256) >> 9),
+           finish(cb, (blend(f0.x1, f0.y1, 6, 5, cb) + 128) >> 8,
+                  (blend5(b1.x1, b1.y1, b0.x1, b2.x1, b0.y1, b2.y1, cb) + 256) >> 9));
+    b0 = b1;
+    b1 = b2;
+    p = o;
+    o = m5;
+    g5 = n5 + m5;
+    o3 = of3(t);
+    g3 = n3 + o3;
+  }
+}
+
+// With readiness flags: waits (team threads 0..15, one flag each) for the CDEF
 // half superblocks under a rectangle: the stripe's rows y0 .. y1, which it
 // reads from the CDEF planes, over its columns and 3 on either side. (The
 // rows past the stripe come from the loop filter's output: the half
@@ -564,32 +625,37 @@ __device__ __forceinline__ void lr_wait_cdef(const FrameDesc& f, const SyncFlags
   if (tid >= 16) return;
   const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
   const int xa = max(x0 - 3, 0), xb = min(x0 + w + 2, geo.pex);
-  const int h0 = (geo.y0 << sy) >> 5, h1 = ((geo.y1 << sy) + sy) >> 5;
+  // (an item of part of a stripe reads 3 more of the stripe's rows on either side)
+  const int ya = max(geo.y0 - 3, max(geo.ss, 0)), yb = min(geo.y1 + 3, min(geo.se, geo.pey));
+  const int h0 = (ya << sy) >> 5, h1 = ((yb << sy) + sy) >> 5;
   const int c0 = (xa << sx) >> 6, c1 = min(((xb << sx) + sx) >> 6, f.cdef_sbc - 1);
   const int hr = h0 + (tid >> 2), c = c0 + (tid & 3);
   if (hr > h1 || c > c1) return;
   flag_wait(flags.p + f.cdef_flag_base + hr * f.cdef_sbc + c, flags.epoch);
 }
 
+// Item: the rectangle x0 .. x1 - 1 of stripe a and unit column b of `plane`;
+// kind 1: of planes 1 and 2, the CTA's halves a plane each (at most 32 columns
+// and rows).
 template <class F>
-__global__ void __launch_bounds__(kThreads, 3) lr_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
-                                                     const Item* __restrict__ items, int n_items, SyncFlags flags) {
+__global__ void __launch_bounds__(kThreads, 4) lr_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+                                                      const Item* __restrict__ items, int n_items, SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ av1pf_lr_unit s_unit;
-  LrSmem sm;
-  sm.win = reinterpret_cast<uint16_t*>(smem);
-  sm.A = reinterpret_cast<int32_t*>(smem + kWinBytes);
-  sm.B = reinterpret_cast<int32_t*>(smem + kWinBytes + kABytes);
-  sm.a2tab = g_sgr_a2.v;
-  sm.F0 = reinterpret_cast<int32_t*>(smem + kWinBytes + 2 * kABytes);
-  sm.unit = &s_unit;
+  __shared__ __align__(16) uint16_t window[kWinBytes / 2];
+  __shared__ GroupEdges edges[kThreads / 16];
+  __shared__ const uint8_t* rows[2][kMaxH + 6];
   const int tid = threadIdx.x;
 
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
     const FrameDesc& f = frame_of(one, frames, item.frame);
-    const int p = item.plane;
+    const bool pair = item.kind != 0;
+    Team tm;
+    const int half = pair ? tid >> 6 : 0;
+    tm.t = pair ? tid & 63 : tid;
+    tm.n = pair ? 64 : kThreads;
+    tm.bar = 1 + half;
+    const int p = item.plane + half;
     const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
     // lr_stripe (postfilter.rs:640-661)
     LrGeom geo;
@@ -601,6 +667,9 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const __grid_constant__
     geo.y0 = max(geo.ss, 0);
     geo.y1 = min(geo.se, geo.pey);
     const int x0 = item.x0, w = int(item.x1) - int(item.x0);
+    // the item's rows of the stripe
+    geo.y0 += item.y0;
+    geo.y1 = min(geo.y1, geo.y0 + int(item.y1) - int(item.y0) - 1);
     const int h = geo.y1 - geo.y0 + 1;
     if (h <= 0 || w <= 0) {
       // without flags every CTA waits, so the kernel never completes before
@@ -612,75 +681,77 @@ __global__ void __launch_bounds__(kThreads, 3) lr_kernel(const __grid_constant__
       continue;
     }
     int type = AV1PF_RESTORE_NONE;
-    const av1pf_lr_unit* unit_p = nullptr;
+    av1pf_lr_unit unit{};
     if (f.lr_on && f.lr_type[p] != AV1PF_RESTORE_NONE) {
       const int unit_size = f.lr_unit_size[p];
       const int luma_row = max(s * 64 - 8, 0);
-      const int unit_row = min(f.lr_unit_rows[p] - 1, ((luma_row + 8) >> sy) / unit_size);
-      unit_p = &f.lru[p][unit_row * f.lr_unit_cols[p] + item.b];
-      type = unit_p->type;
+      const int unit_row = min(f.lr_unit_rows[p] - 1, ((luma_row + 8) >> sy) >> floor_log2(uint32_t(unit_size)));  // 32 .. 256
+      unit = f.lru[p][unit_row * f.lr_unit_cols[p] + item.b];
+      type = unit.type;
     }
     // the descriptor and the unit are inputs of the chain; the planes below
     // are the previous stage's output: all of it, or with readiness flags
     // the half superblocks under the rectangle
     if (flags.p) {
       pdl_trigger();
-      lr_wait_cdef(f, flags, p, geo, x0, w, tid);
+      lr_wait_cdef(f, flags, p, geo, x0, w, tm.t);
       // the previous call may write the same planes
-      if (flags.ahead && tid == 32) flag_wait(flags.complete, flags.epoch - 1);
-      __syncthreads();
+      if (flags.ahead && tm.t == 32) flag_wait(flags.complete, flags.epoch - 1);
     } else {
       pdl_wait();
     }
-    if (type != AV1PF_RESTORE_WIENER && type != AV1PF_RESTORE_SGRPROJ) {
-      pass_through(f, p, x0, geo.y0, w, h, tid);  // uniform across the CTA: no barrier needed
+    const bool restores = type == AV1PF_RESTORE_WIENER || type == AV1PF_RESTORE_SGRPROJ;
+    if (restores) window_rows(f, rows[half], geo, p, s, h, tm);
+    tm.sync();  // (also: the team is done with the previous item's window)
+    if (!restores) {
+      pass_through(f, p, x0, geo.y0, w, h, tm);
       continue;
     }
-    if (w > 32)
-      restore_rect<72>(f, sm, geo, p, s, x0, w, h, type, unit_p, tid);
+    const bool wide = w > 32;
+    Group g;
+    g.ws = wide ? kWideWS : kSlimWS;
+    uint16_t* win = window + half * kSlimTeamWin;
+    stage_window(win, g.ws, rows[half], f.sb, geo.pex, x0, w, h, tm);
+    const int gs = wide ? 5 : 4, gn = 1 << gs;  // lanes of a group
+    const int gl = tm.t & (gn - 1), gi = tm.t >> gs, lgroups = (pair ? 6 : 7) - gs;
+    // an even number of rows a group (y0 is even: row i has the parity of y0 + i)
+    g.per = (((h + (1 << lgroups) - 1) >> lgroups) + 1) & ~1;
+    g.i0 = gi * g.per;
+    g.left = min(h - g.i0, g.per);
+    g.c = 2 * gl;
+    g.cols = min(w - g.c, 2);
+    g.win = win + g.c;
+    const int bd = f.bd;
+    const int y = geo.y0 + g.i0, x = x0 + g.c;
+    g.rw = f.sb;
+    g.ref_pitch = f.ref[p].stride * g.rw;
+    g.ref = f.ref[p].p + y * g.ref_pitch + x * g.rw;
+    // the packed frame: u8 samples at 8 bits, little-endian u16 above
+    // (frame.rs:153-158), rows of the plane's width (decoder/mod.rs:846-917)
+    g.ow = bd > 8 ? 2 : 1;
+    g.out_pitch = int64_t(geo.pex + 1) * g.ow;
+    g.out = f.lr_pack ? f.frame_out + f.out_off[p] + y * g.out_pitch + x * g.ow : nullptr;
+    const bool odd = ((reinterpret_cast<uintptr_t>(g.ref) | uintptr_t(g.ref_pitch)) & uintptr_t(2 * g.rw - 1)) != 0 ||
+                     (g.out && ((reinterpret_cast<uintptr_t>(g.out) | uintptr_t(g.out_pitch)) & uintptr_t(2 * g.ow - 1)) != 0);
+    const bool pairs = __all_sync(0xffffffffu, g.cols > 1 && !odd);
+    tm.sync();
+    GroupEdges& ed = edges[tid >> gs];
+    if (type == AV1PF_RESTORE_WIENER)
+      pairs ? wiener_group<true>(g, unit, bd) : wiener_group<false>(g, unit, bd);
+    else if (bd > 10)
+      pairs ? sgr_group<true, true>(g, unit, bd, ed, gl, gn) : sgr_group<true, false>(g, unit, bd, ed, gl, gn);
     else
-      restore_rect<36>(f, sm, geo, p, s, x0, w, h, type, unit_p, tid);
-    __syncthreads();
-    // the rectangle's output samples, from shared memory to the reference
-    // frame and (frames without film grain) the packed frame: u8 samples at
-    // 8 bits, little-endian u16 above (frame.rs:153-158), rows of the plane's
-    // width (decoder/mod.rs:846-917)
-    {
-      const int sb = f.sb, bd = f.bd;
-      const DPlane dst = f.ref[p];
-      uint8_t* d0 = dst.p + (int64_t(geo.y0) * dst.stride + x0) * sb;
-      const int64_t dp = dst.stride * sb;
-      const bool d_vec = ((reinterpret_cast<uintptr_t>(d0) | uintptr_t(dp)) & 15) == 0;
-      const int bps = bd > 8 ? 2 : 1;
-      const int64_t op = int64_t(geo.pex + 1) * bps;
-      uint8_t* o0 = f.lr_pack ? f.frame_out + f.out_off[p] + int64_t(geo.y0) * op + int64_t(x0) * bps : nullptr;
-      const bool o_vec = ((reinterpret_cast<uintptr_t>(o0) | uintptr_t(op)) & 15) == 0;
-      if (w > 32) {
-        store_tile<64>(sm.F0, d0, dp, sb, d_vec, w, h, tid);
-        if (o0) store_tile<64>(sm.F0, o0, op, bps, o_vec, w, h, tid);
-      } else {
-        store_tile<32>(sm.F0, d0, dp, sb, d_vec, w, h, tid);
-        if (o0) store_tile<32>(sm.F0, o0, op, bps, o_vec, w, h, tid);
-      }
-    }
-    __syncthreads();
+      pairs ? sgr_group<false, true>(g, unit, bd, ed, gl, gn) : sgr_group<false, false>(g, unit, bd, ed, gl, gn);
   }
   AV1PF_TRACE_END(3);
 }
 
-cudaError_t lr_init() {
-  cudaError_t e = cudaFuncSetAttribute(lr_kernel<NoFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(lr_kernel<OneFrame>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-  return e;
-}
-
 void launch_lr(const FrameSet& frames, const Item* items, int n_items, SyncFlags flags, cudaStream_t s) {
   if (n_items <= 0) return;
-  // one CTA per rectangle: the block scheduler hands rectangles of uneven
-  // cost (copy, Wiener, self-guided) to SMs as they free up
-  launch_frames(frames, lr_kernel<NoFrame>, lr_kernel<OneFrame>, min(n_items, kItemGrid), kThreads,
-                size_t(kSmemBytes), s, items, n_items, flags);
+  // one CTA per item: the block scheduler hands items of uneven cost (copy,
+  // Wiener, self-guided) to SMs as they free up
+  launch_frames(frames, lr_kernel<NoFrame>, lr_kernel<OneFrame>, min(n_items, kItemGrid), kThreads, 0, s, items, n_items,
+                flags);
 }
 
 }  // namespace av1pf

@@ -434,6 +434,12 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
         const int us = has_lr ? p->loop_restoration_size[k] : 1 << 30;
         const int ucols = has_lr ? p->lr_unit_cols[k] : 1;
         const int rw = j.lr_cols == 32 ? 32 : kTile;  // rectangle width (the kernel takes <= 64)
+        // 4:2:0 chroma with the same units in both planes: a rectangle of up to
+        // 32 columns (and its 32 rows) leaves half of a CTA idle, so one item
+        // holds those of U and V
+        const bool pairs = k > 0 && i->subsampling_y && (p->frame_restoration_type[1] != 0) == (p->frame_restoration_type[2] != 0) &&
+                           (!has_lr || (p->loop_restoration_size[1] == p->loop_restoration_size[2] &&
+                                        p->lr_unit_cols[1] == p->lr_unit_cols[2]));
         for (int s = 0; items && s < d.stripes; s++) {
           const int sy = k ? d.ssy : 0;
           const int ss = (-8 + s * 64) >> sy;
@@ -452,7 +458,16 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
               it.x1 = uint16_t(std::min(cx + rw, x1 + 1));
               it.a = uint16_t(s);
               it.b = uint16_t(uc);
-              if (items) plan.lr_items.push_back(it);
+              if (pairs && it.x1 - it.x0 <= 32) {
+                if (k == 2) continue;
+                it.kind = 1;
+              }
+              const int part = it.x1 - it.x0 <= 32 ? kTile : 32;
+              for (int y = 0; y <= y1 - y0; y += part) {
+                it.y0 = uint16_t(y);
+                it.y1 = uint16_t(y + part);
+                plan.lr_items.push_back(it);
+              }
             }
           }
         }
