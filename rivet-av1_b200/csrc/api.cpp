@@ -406,6 +406,7 @@ int av1pf_ctx_create(int device, uint64_t hbm_cap_bytes, av1pf_ctx** out) {
       if ((e = upload_grain_tables()) != cudaSuccess) return cuda_status(e, "grain tables");
       if ((e = superres_init()) != cudaSuccess) return cuda_status(e, "superres kernel attributes");
       if ((e = cdef_init()) != cudaSuccess) return cuda_status(e, "CDEF kernel attributes");
+      if ((e = search_init()) != cudaSuccess) return cuda_status(e, "search kernel attributes");
       if ((e = output_init()) != cudaSuccess) return cuda_status(e, "output kernel attributes");
       g_tables_ready[device] = true;
     }

@@ -18,6 +18,7 @@
 // search each thread takes one 8x8 block and two of the 8 directions (one
 // pair per warp), so the partial-sum bins are compile-time register indices.
 #include "av1_tables.h"
+#include "cdef_search.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "lf_core.cuh"
@@ -607,26 +608,6 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const __grid_const
   AV1PF_TRACE_END(2);
 }
 
-// Sum of a u32 over the warp, exactly (two 16-bit halves, so no lane sum
-// overflows).
-__device__ __forceinline__ uint64_t warp_sum_u32(uint32_t v) {
-  const uint32_t lo = __reduce_add_sync(0xffffffffu, v & 0xffffu);
-  const uint32_t hi = __reduce_add_sync(0xffffffffu, v >> 16);
-  return (uint64_t(hi) << 16) + lo;
-}
-
-// The search's candidate strengths (encoder/cdef.rs:60-80): primaries of
-// the fast and thorough lists, secondaries decoded (coded 3 is 4).
-__host__ __device__ constexpr int search_y_pri(bool th, int i) {
-  constexpr int f[7] = {0, 1, 2, 4, 6, 9, 12}, t[11] = {0, 1, 2, 3, 4, 5, 6, 8, 10, 12, 15};
-  return th ? t[i] : f[i];
-}
-__host__ __device__ constexpr int search_uv_pri(bool th, int i) {
-  constexpr int f[5] = {0, 1, 2, 4, 7}, t[8] = {0, 1, 2, 3, 4, 6, 8, 11};
-  return th ? t[i] : f[i];
-}
-__host__ __device__ constexpr int search_sec(int j) { return j == 3 ? 4 : j; }
-
 // |constrain(d)| (cdef.rs:48-51) from |d|: min(|d|, max(0, str - (|d| >> adj))).
 // `mone` is -1 at run time but opaque to the compiler, so the subtraction
 // is a multiply-add (the integer ALU pipe is this kernel's bound).
@@ -794,7 +775,7 @@ __device__ __forceinline__ void warp_reduce_pairs(const uint32_t (&acc)[N], uint
 // grid covers every block of n frames: frame i's blocks start at CTA
 // ds[i].block0.
 template <bool TH>
-__global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDesc* __restrict__ ds, int n) {
+__global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDesc* __restrict__ ds, int n, int min_bd) {
   constexpr int NYP = TH ? 11 : 7, NUVP = TH ? 8 : 5, NYS = 4, NUVS = 3;
   constexpr int NY = NYP * NYS, NUV = NUVP * NUVS;
   constexpr int R = 64, top = 2, wrows = R + 2 * top;
@@ -809,16 +790,9 @@ __global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDes
   __shared__ uint8_t uvdir[2][2][8];
   __shared__ int s_one;
   __shared__ uint64_t red[8][kSearchMaxY + kSearchMaxUV];
-  int fi = 0;
-  for (int hi = n - 1; fi < hi;) {  // the last frame whose first block is at or before this CTA
-    const int mid = (fi + hi + 1) >> 1;
-    if (ds[mid].block0 <= int(blockIdx.x))
-      fi = mid;
-    else
-      hi = mid - 1;
-  }
-  const CdefSearchDesc& d = ds[fi];
+  const CdefSearchDesc& d = ds[search_frame(ds, n, int(blockIdx.x))];
   const FrameDesc& f = *d.frame;
+  if (f.bd < min_bd) return;  // the packed kernel's
   CdefGreedy* g = d.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int fb = int(blockIdx.x) - d.block0, nfb = d.fb_rows * d.fb_cols;
@@ -1060,12 +1034,17 @@ void launch_cdef(const FrameSet& frames, const Item* items, int n_items, const C
                   items, n_items, wrows, min_bd, flags);
 }
 
-void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, cudaStream_t s) {
+void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, bool shallow, bool deep,
+                        cudaStream_t s) {
   if (blocks <= 0) return;
+  // Frames of up to 10 bits take the packed kernel; a launch of both kinds runs
+  // both over every block, each leaving the other's frames alone.
+  if (shallow) launch_cdef_search_packed(ds, n, blocks, thorough, s);
+  if (!deep) return;
   if (thorough)
-    cdef_search_kernel<true><<<blocks, 256, kSearchSmem, s>>>(ds, n);
+    cdef_search_kernel<true><<<blocks, 256, kSearchSmem, s>>>(ds, n, 11);
   else
-    cdef_search_kernel<false><<<blocks, 256, kSearchSmem, s>>>(ds, n);
+    cdef_search_kernel<false><<<blocks, 256, kSearchSmem, s>>>(ds, n, 11);
   note_launch();
 }
 

@@ -24,6 +24,7 @@
 // load fall in 32 different banks. Row strides of 8 columns a lane would put
 // blocks 32 columns apart in one bank.
 #include "cdef_packed.cuh"
+#include "cdef_search.cuh"
 #include "kernels.h"
 
 namespace av1pf {
@@ -481,6 +482,318 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __gri
   AV1PF_TRACE_END(2);
 }
 
+// ---------------------------------------------------------------------------
+// The encoder's CDEF search, error tables (encoder/cdef.rs:103-190), for bit
+// depths up to 10.
+// ---------------------------------------------------------------------------
+namespace {
+
+// A strength of a block: its terms and, of a primary, the tap weights.
+struct alignas(16) SearchStrength {
+  PStrength s;
+  uint32_t w0, w1;
+  uint32_t pad[3];
+};
+
+constexpr int kSR = 32;  // luma rows of a CTA: half a block
+
+constexpr int8_t kSearchDirs[8][2][2] = AV1T_CDEF_DIRECTIONS;
+constexpr int search_off(int dir, int k) { return (kSearchDirs[dir][k][0] * kPS + kSearchDirs[dir][k][1]) * 4; }
+
+__device__ __forceinline__ SearchStrength search_strength(int str, int damping, int cs) {
+  SearchStrength t;
+  t.s = packed_strength(str, str ? max(damping - floor_log2(uint32_t(str)), 0) : 0);
+  const bool odd = (str >> cs) & 1;
+  t.w0 = odd ? 0x42004200u : 0x44004400u;
+  t.w1 = odd ? 0x42004200u : 0x40004000u;
+  return t;
+}
+
+// Adds the squares of e's halves (those that count) to acc: exact while acc
+// stays below 2^24.
+__device__ __forceinline__ void add_squares(float& acc, uint32_t e, bool lo, bool hi) {
+  if (lo) asm("{ .reg .f16 l, h; mov.b32 {l, h}, %1; fma.rn.f32.f16 %0, l, l, %0; }" : "+f"(acc) : "r"(e));
+  if (hi) asm("{ .reg .f16 l, h; mov.b32 {l, h}, %1; fma.rn.f32.f16 %0, h, h, %0; }" : "+f"(acc) : "r"(e));
+}
+
+// The squared errors of one word's two samples under every (primary,
+// secondary) pair of a plane's list, added to acc[i * NS + j]
+// (encoder/cdef.rs:113-188). A pair's filter sum is P(primary) + S(secondary):
+// each distinct P and S is computed once, and a pair costs an addition, the
+// rounding, the clamp, the difference from the source and two multiply-adds.
+// Pairs with primary strength 0 filter in direction 0 (secondary taps at
+// directions 6 and 2); the others in the block's direction (offsets `o` in
+// bytes: primary k0, k1, secondary lo k0, hi k0, lo k1, hi k1). With one kind
+// of tap the weights sum to 12 < 16 and the result needs no clamp.
+template <int NP, int NS>
+__device__ __forceinline__ void word_pairs(const uint32_t* c, uint32_t src, bool lo, bool hi, const int16_t* o,
+                                           const SearchStrength* pri, const SearchStrength* sec, float (&acc)[NP * NS]) {
+  const uint32_t xw = c[0];
+  const __half2 x = as_h2(xw), nx = as_h2(xw ^ 0x80008000u), ns = as_h2(src ^ 0x80008000u);
+  auto at = [&](int off) { return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(c) + off); };
+  auto score = [&](int k, __half2 v) { add_squares(acc[k], as_u32(__hadd2(v, ns)), lo, hi); };
+  // weight-2 taps, then weight-1
+  auto sec_sum = [&](const __half2 (&d)[8], const PStrength& s) {
+    __half2 s2 = packed_constrain(d[0], s), s1 = packed_constrain(d[4], s);
+#pragma unroll
+    for (int k = 1; k < 4; k++) {
+      s2 = __hadd2(s2, packed_constrain(d[k], s));
+      s1 = __hadd2(s1, packed_constrain(d[4 + k], s));
+    }
+    return __hfma2(s2, as_h2(0x40004000u), s1);
+  };
+  {  // primary strength 0: secondary taps alone, in direction 0
+    constexpr int offs[4] = {search_off(6, 0), search_off(2, 0), search_off(6, 1), search_off(2, 1)};
+    __half2 d[8];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      d[2 * k] = __hadd2(as_h2(at(offs[k])), nx);
+      d[2 * k + 1] = __hadd2(as_h2(at(-offs[k])), nx);
+    }
+    score(0, x);
+#pragma unroll
+    for (int j = 1; j < NS; j++) score(j, packed_round(sec_sum(d, sec[j].s), x));
+  }
+  __half2 mx = x;
+  uint32_t mn = xw;
+  __half2 d[12];
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const uint32_t p0 = at(o[k]), p1 = at(-o[k]);
+    mx = __hmax2(mx, __hmax2(as_h2(p0), as_h2(p1)));
+    mn = __vminu2(mn, __vminu2(p0, p1));
+    d[2 * k] = __hadd2(as_h2(p0), nx);
+    d[2 * k + 1] = __hadd2(as_h2(p1), nx);
+  }
+  __half2 S[NS];
+  {
+    const __half2 ds[8] = {d[4], d[5], d[6], d[7], d[8], d[9], d[10], d[11]};
+#pragma unroll
+    for (int j = 1; j < NS; j++) S[j] = sec_sum(ds, sec[j].s);
+  }
+#pragma unroll
+  for (int i = 1; i < NP; i++) {
+    const SearchStrength t = pri[i];
+    const __half2 q0 = __hadd2(packed_constrain(d[0], t.s), packed_constrain(d[1], t.s));
+    const __half2 q1 = __hadd2(packed_constrain(d[2], t.s), packed_constrain(d[3], t.s));
+    const __half2 P = __hfma2(q0, as_h2(t.w0), __hmul2(q1, as_h2(t.w1)));
+    score(i * NS, packed_round(P, x));
+#pragma unroll
+    for (int j = 1; j < NS; j++)
+      score(i * NS + j, __hmax2(__hmin2(packed_round(__hadd2(P, S[j]), x), mx), as_h2(mn)));
+  }
+}
+
+// Adds warp sums of acc[] to red[base + k].
+template <int N>
+__device__ __forceinline__ void flush_pairs(float (&acc)[N], uint64_t* red, int lane, int base) {
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const uint64_t ws = warp_sum_u32(uint32_t(acc[k]));
+    if (lane == 0) red[base + k] += ws;
+    acc[k] = 0.f;
+  }
+}
+
+template <bool TH>
+struct SearchSmem {
+  static constexpr int NYP = TH ? 11 : 7, NUVP = TH ? 8 : 5, NYS = 4, NUVS = 3;
+  static constexpr int NY = NYP * NYS, NUV = NUVP * NUVS;
+  SearchStrength ypri[kSR][NYP];
+  SearchStrength ysec[NYS], uvpri[NUVP], uvsec[NUVS];
+  uint64_t red[kSR / 8][NY + NUV];
+  int16_t off[2][kSR][8];  // luma, chroma: a block's tap offsets
+};
+template <bool TH>
+constexpr int search_smem() {
+  return packed_smem(kSR, true) + int(sizeof(SearchSmem<TH>));
+}
+static_assert(packed_smem(kSR, true) % 16 == 0, "SearchSmem follows the windows");
+
+}  // namespace
+
+// One CTA per half (32 rows) of a 64x64 block, 128 threads: the decoder kernel's
+// windows and direction search; then a warp per row of 8x8 blocks scores every
+// candidate pair on every filtered sample, two samples a lane as in the decoder
+// kernel (luma: rows r and r + 4; chroma: U and V, whose errors are summed). A
+// thread scores 16 samples before its float sums of squares, each at most
+// 16 * 1023^2 < 2^24, go to the warp's 64-bit totals; the halves' totals are
+// added in the (cleared) table. TH: the thorough lists.
+//
+// What bounds it: instruction issue, about 560 instructions for two luma
+// samples against 710 for one in cdef_search_kernel, whose integer pipe was the
+// limit; half-precision instructions issue every second clock, as the integer
+// pipe's do. 1080p 10-bit, fast lists: 115 us for that kernel, 68 for this one.
+// (Whole blocks a CTA, 5 CTAs an SM, and source samples loaded ahead: the same.)
+template <bool TH>
+__global__ void __launch_bounds__(4 * kSR, 4) cdef_search_packed_kernel(const CdefSearchDesc* __restrict__ ds, int n) {
+  using Smem = SearchSmem<TH>;
+  constexpr int NYP = Smem::NYP, NUVP = Smem::NUVP, NYS = Smem::NYS, NUVS = Smem::NUVS, NY = Smem::NY, NUV = Smem::NUV;
+  constexpr int R = kSR;
+  extern __shared__ __align__(16) uint8_t packed_base[];
+  uint16_t* const dwin = reinterpret_cast<uint16_t*>(packed_base);
+  uint32_t* const lw = reinterpret_cast<uint32_t*>(packed_base + R * kDS * 2);
+  uint32_t* const cw = lw + R * kPS;
+  Smem& sm = *reinterpret_cast<Smem*>(packed_base + packed_smem(R, true));
+  __shared__ uint32_t cost[8][R];
+  __shared__ uint8_t bstate[R];
+  __shared__ int16_t doff[8][2];
+  const int half = blockIdx.x & 1, block = blockIdx.x >> 1;
+  const CdefSearchDesc& d = ds[search_frame(ds, n, block)];
+  const FrameDesc& f = *d.frame;
+  if (f.bd > 10) return;  // cdef_search_kernel's
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int fb = block - d.block0, nfb = d.fb_rows * d.fb_cols;
+  const int fr = fb / d.fb_cols, fc = fb - fr * d.fb_cols;
+  const int y0 = fr * 64 + half * R;
+  const int idx = f.cdef_idx[int64_t(fr) * f.cdef_stride + fc];
+  if (idx < 0) {  // codes no index: zero errors, and no part in the greedy's sums
+    if (tid == 0 && half == 0) d.best[fb] = 0;
+    return;
+  }
+  if (tid == 0 && half == 0) {
+    d.best[fb] = ~uint64_t(0);
+    atomicAdd(&d.g->nb, 1u);
+  }
+  if (y0 >= f.mi_rows * 4) return;  // a half past the mode-info area
+  if (tid < 16) doff[tid >> 1][tid & 1] = int16_t((c_cdef_dirs[tid >> 1][tid & 1][0] * kPS + c_cdef_dirs[tid >> 1][tid & 1][1]) * 4);
+  const int np = f.np, sb = f.sb, cs = f.bd - 8, sx = f.ssx, sy = f.ssy;
+  const int damping = d.damping + cs;
+  // --- the 8x8 blocks CDEF filters (encoder/cdef.rs:106-112) ---
+  if (tid < R) {
+    const int r = (y0 >> 2) + 2 * (tid >> 3), c = fc * 16 + 2 * (tid & 7);
+    uint8_t st = 0;
+    if (r < f.mi_rows && c < f.mi_cols) {
+      const av1pf_mi* m = f.mi + int64_t(r) * f.mi_stride + c;
+      const int ms = f.mi_stride;
+      if (!(m[0].skip_segment & m[ms].skip_segment & m[1].skip_segment & m[ms + 1].skip_segment & AV1PF_MI_SKIP)) st = 2;
+    }
+    bstate[tid] = st;
+  }
+  // strengths that no block changes, and cleared totals
+  if (tid < NYS) sm.ysec[tid] = search_strength(search_sec(tid) << cs, damping, cs);
+  if (tid >= 32 && tid < 32 + NUVP) sm.uvpri[tid - 32] = search_strength(search_uv_pri(TH, tid - 32) << cs, damping - 1, cs);
+  if (tid >= 64 && tid < 64 + NUVS) sm.uvsec[tid - 64] = search_strength(search_sec(tid - 64) << cs, damping - 1, cs);
+  for (int k = tid; k < R / 8 * (NY + NUV); k += blockDim.x) (&sm.red[0][0])[k] = 0;
+  if (fc > 0 && fc * 64 + 80 <= f.mi_cols * 4 && y0 > 0 && y0 + R + 4 <= f.mi_rows * 4)
+    stage_windows<R, true>(f, fc, y0, lw, cw, dwin, tid);
+  else
+    stage_windows<R, false>(f, fc, y0, lw, cw, dwin, tid);
+  __syncthreads();
+  // --- direction search (postfilter.rs:345-401), as in the decoder's kernel ---
+  {
+    const int pair = warp & 3, b = (warp >> 2) * 32 + lane;
+    if (bstate[b] == 2) {
+      const uint16_t* s = &dwin[(b >> 3) * 8 * kDS + (b & 7) * 8];
+      uint32_t c1, c2;
+      switch (pair) {
+        case 0: packed_cost_pair<0>(s, c1, c2); break;
+        case 1: packed_cost_pair<1>(s, c1, c2); break;
+        case 2: packed_cost_pair<2>(s, c1, c2); break;
+        default: packed_cost_pair<3>(s, c1, c2); break;
+      }
+      cost[pair][b] = c1;
+      cost[pair + 4][b] = c2;
+    }
+  }
+  __syncthreads();
+  // --- each block's directions, and its primary strengths after the variance
+  // adjustment (postfilter.rs:318-323): 4 threads a block ---
+  {
+    const int b = tid >> 2, q = tid & 3;
+    if (bstate[b] == 2) {
+      uint32_t best = cost[0][b];
+      int y_dir = 0;
+#pragma unroll
+      for (int k = 1; k < 8; k++) {
+        const uint32_t ck = cost[k][b];
+        if (ck > best) {
+          best = ck;
+          y_dir = k;
+        }
+      }
+      const int32_t var = int32_t(best - cost[(y_dir + 4) & 7][b]) >> 10;
+      const int var_str = (var >> 6) != 0 ? min(floor_log2(uint32_t(var >> 6)), 12) : 0;
+      for (int i = q; i < NYP; i += 4) {
+        const int p0 = search_y_pri(TH, i) << cs;
+        sm.ypri[b][i] = search_strength(var != 0 ? (p0 * (4 + var_str) + 8) >> 4 : 0, damping, cs);
+      }
+      if (q < 2) {
+        const int dir = q ? c_cdef_uv_dir[sx][sy][y_dir] : y_dir;
+        const int dlo = (dir + 6) & 7, dhi = (dir + 2) & 7;
+        int16_t* o = sm.off[q][b];
+        o[0] = doff[dir][0];
+        o[1] = doff[dir][1];
+        o[2] = doff[dlo][0];
+        o[3] = doff[dhi][0];
+        o[4] = doff[dlo][1];
+        o[5] = doff[dhi][1];
+      }
+    }
+  }
+  __syncthreads();
+  // --- every pair on every filtered sample (encoder/cdef.rs:113-188) inside the
+  // frame (block_sse's crop, encoder/cdef.rs:261-285). Lanes as in the decoder's
+  // kernel: 4 blocks x 4 rows x 2 columns, or 8 x 2 x 2 for 4-wide chroma ---
+  const int h = lane & 1;
+  {
+    float acc[NY];
+#pragma unroll
+    for (int k = 0; k < NY; k++) acc[k] = 0.f;
+    const DPlane src = d.src[0];
+    const int fw = f.fw, fh = f.fh;
+#pragma unroll 1
+    for (int k = 0; k < 8; k++) {  // half of the blocks, column
+      const int b = warp * 8 + (k >> 2) * 4 + (lane >> 3);
+      if (bstate[b] != 2) continue;
+      const int x = (b & 7) * 8 + 2 * (k & 3) + h, y = warp * 8 + ((lane >> 1) & 3);
+      const int gx = fc * 64 + x, gy = y0 + y;
+      const bool lo = gx < fw && gy < fh, hi = gx < fw && gy + 4 < fh;
+      const uint32_t s = kPBias | (lo ? uint32_t(ld_sample(src, sb, gx, gy)) : 0u) |
+                         (hi ? uint32_t(ld_sample(src, sb, gx, gy + 4)) << 16 : 0u);
+      word_pairs<NYP, NYS>(lw + (y + 2) * kPS + 2 + x, s, lo, hi, sm.off[0][b], sm.ypri[b], sm.ysec, acc);
+    }
+    flush_pairs<NY>(acc, sm.red[warp], lane, 0);
+  }
+  if (np > 1) {
+    float acc[NUV];
+#pragma unroll
+    for (int k = 0; k < NUV; k++) acc[k] = 0.f;
+    const int bw = 8 >> sx, bh = 8 >> sy;
+    const int fw = (f.fw + sx) >> sx, fh = (f.fh + sy) >> sy;
+    const DPlane su = d.src[1], sv = d.src[2];
+    // words a lane: 4-wide 2 columns x bh / 2 rows; 8-wide 2 halves x 4 columns x bh / 4 rows
+    const int words = sx ? bh : 2 * bh;
+#pragma unroll 1
+    for (int k = 0; k < words; k++) {
+      const int b = warp * 8 + (sx ? lane >> 2 : (k & 1) * 4 + (lane >> 3));
+      const int x = (b & 7) * bw + (sx ? 2 * (k & 1) : 2 * ((k >> 1) & 3)) + h;
+      const int y = warp * bh + (sx ? ((lane >> 1) & 1) + (k >> 1) * 2 : ((lane >> 1) & 3) + (k >> 3) * 4);
+      const int gx = ((fc * 64) >> sx) + x, gy = (y0 >> sy) + y;
+      if (bstate[b] == 2 && gx < fw && gy < fh) {
+        const uint32_t s = kPBias | uint32_t(ld_sample(su, sb, gx, gy)) | (uint32_t(ld_sample(sv, sb, gx, gy)) << 16);
+        word_pairs<NUVP, NUVS>(cw + (y + 2) * kPS + 2 + x, s, true, true, sm.off[1][b], sm.uvpri, sm.uvsec, acc);
+      }
+      if ((k & 7) == 7) flush_pairs<NUV>(acc, sm.red[warp], lane, NY);
+    }
+    if (words & 7) flush_pairs<NUV>(acc, sm.red[warp], lane, NY);
+  }
+  __syncthreads();
+  for (int k = tid; k < NY + NUV; k += blockDim.x) {
+    uint64_t s = 0;
+    for (int w4 = 0; w4 < R / 8; w4++) s += sm.red[w4][k];
+    if (s) atomicAdd(reinterpret_cast<unsigned long long*>(&d.sse[int64_t(k) * nfb + fb]), static_cast<unsigned long long>(s));
+  }
+}
+
+void launch_cdef_search_packed(const CdefSearchDesc* ds, int n, int blocks, bool thorough, cudaStream_t s) {
+  if (thorough)
+    cdef_search_packed_kernel<true><<<2 * blocks, 4 * kSR, search_smem<true>(), s>>>(ds, n);
+  else
+    cdef_search_packed_kernel<false><<<2 * blocks, 4 * kSR, search_smem<false>(), s>>>(ds, n);
+  note_launch();
+}
+
 cudaError_t cdef_packed_init() {
   cudaError_t e = cudaSuccess;
   auto opt_in = [&](auto kernel, int bytes) {
@@ -490,6 +803,8 @@ cudaError_t cdef_packed_init() {
   opt_in(cdef_packed_kernel<OneFrame, 64>, packed_smem(64, true));
   opt_in(cdef_packed_kernel<NoFrame, 32>, packed_smem(32, true));
   opt_in(cdef_packed_kernel<OneFrame, 32>, packed_smem(32, true));
+  opt_in(cdef_search_packed_kernel<false>, search_smem<false>());
+  opt_in(cdef_search_packed_kernel<true>, search_smem<true>());
   return e;
 }
 

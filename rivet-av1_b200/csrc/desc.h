@@ -117,6 +117,7 @@ struct CdefSearchDesc {
   int8_t y_pri[kSearchMaxY], y_sec[kSearchMaxY];     // secondary decoded (coded 3 -> 4)
   int8_t uv_pri[kSearchMaxUV], uv_sec[kSearchMaxUV];
   uint64_t* sse;           // [ny + nuv][fb_rows * fb_cols], candidate-major
+  uint64_t* sse_out;       // the same [fb_rows * fb_cols][ny + nuv], block-major, or null
   uint64_t* best;          // [fb_rows * fb_cols]: the greedy's per-block minimum
   // one frame of a batched search: its descriptor, greedy state, candidate
   // totals, input table and outputs, and its first CTA in each grid

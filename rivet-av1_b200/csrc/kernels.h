@@ -147,17 +147,22 @@ void launch_dsp_cdef(const int32_t* win, const av1pf_cdef_taps* taps, uint16_t* 
 // The encoder's CDEF search: per-block squared errors of every candidate
 // (one CTA per 64x64 block of n frames, `blocks` in all); counts each
 // frame's coding blocks into its greedy state.
-void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, cudaStream_t s);
+// `shallow`: some frame has at most 10 bits; `deep`: some has 12.
+void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, bool shallow, bool deep,
+                        cudaStream_t s);
+// The part of it for frames of up to 10 bits (cdef_packed.cu).
+void launch_cdef_search_packed(const CdefSearchDesc* ds, int n, int blocks, bool thorough, cudaStream_t s);
 
 // Encoder searches (search.cu)
-// One greedy step of the CDEF search for n frames side by side: every pair
-// not yet chosen is scored and the best is added (the last CTA of a frame
-// to finish picks).
-void launch_cdef_greedy_step(const CdefSearchDesc* ds, int n, int ncand, cudaStream_t s);
-// The CDEF search's outcome: each coding block's index into each frame's
-// table (a copy of its cdef_idx) and the chosen pairs into its result
-// (`total` table entries over all frames).
-void launch_cdef_greedy_finish(const CdefSearchDesc* ds, int n, int total, cudaStream_t s);
+// The greedy choice of the CDEF search for n frames side by side (ny x nuv pairs,
+// at most nfb_max blocks a frame), and its outcome: each coding block's index into
+// each frame's table (a copy of its cdef_idx; `entries` over all frames) and the
+// chosen pairs into its result.
+void launch_cdef_greedy(const CdefSearchDesc* ds, int n, int ny, int nuv, int nfb_max, int entries, cudaStream_t s);
+// The error tables of the frames that ask for them (sse_out), block-major.
+void launch_sse_transpose(const CdefSearchDesc* ds, int n, int nfb_max, int nc, cudaStream_t s);
+// Sets the cluster kernel's dynamic shared-memory limit on the current device.
+cudaError_t search_init();
 // Squared error of planes against the source over each plane's frame area:
 // sse[i] += sum over plane job i (a, b: plane pointers and strides; `jobs`
 // in device memory, at most 65535).

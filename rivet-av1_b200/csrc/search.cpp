@@ -146,12 +146,24 @@ int av1pf_cdef_search_many(av1pf_ctx* ctx, int n, const av1pf_cdef_search_job* j
     blocks += G.nfb;
     entries += int(G.table_bytes);
   }
-  const size_t o_results = off, dev_bytes = o_results + res_bytes;
+  // the block-major error tables that the callers take follow the results
   size_t sse_bytes = 0;
-  for (int i = 0; i < n; i++)
+  int nfb_max = 0;
+  for (int i = 0; i < n; i++) {
     if (jobs[i].block_sse) sse_bytes += size_t(nc) * size_t(geo[size_t(i)].nfb) * 8;
+    nfb_max = std::max(nfb_max, geo[size_t(i)].nfb);
+  }
+  const size_t o_results = off, dev_bytes = o_results + res_bytes + sse_bytes;
   const size_t host_bytes = o_g + res_bytes + sse_bytes;
-  if ((rc = ctx->ensure(ctx->search_dev, dev_bytes)) != AV1PF_OK) return rc;
+  // (where there is no room for them, the candidate-major tables come back and
+  // the host turns them)
+  rc = ctx->ensure(ctx->search_dev, dev_bytes);
+  const bool turned = rc == AV1PF_OK;
+  if (!turned && sse_bytes) {
+    cudaGetLastError();
+    rc = ctx->ensure(ctx->search_dev, dev_bytes - sse_bytes);
+  }
+  if (rc != AV1PF_OK) return rc;
   if ((rc = ctx->ensure_host(ctx->search_host, host_bytes)) != AV1PF_OK) return rc;
   uint8_t* dv = static_cast<uint8_t*>(ctx->search_dev.ptr);
   uint8_t* hs = static_cast<uint8_t*>(ctx->search_host.ptr);
@@ -160,6 +172,7 @@ int av1pf_cdef_search_many(av1pf_ctx* ctx, int n, const av1pf_cdef_search_job* j
   const auto* dframes = reinterpret_cast<const FrameDesc*>(dv);
   auto* dg = reinterpret_cast<CdefGreedy*>(dv + o_g);
   int block0 = 0, table0 = 0;
+  size_t sse_off = o_results + res_bytes;
   for (int i = 0; i < n; i++) {
     const av1pf_cdef_search_job& jb = jobs[i];
     const av1pf_frame_info* info = jb.info;
@@ -199,6 +212,10 @@ int av1pf_cdef_search_many(av1pf_ctx* ctx, int n, const av1pf_cdef_search_job* j
     }
     d.sse = reinterpret_cast<uint64_t*>(dv + G.o_sse);
     d.best = reinterpret_cast<uint64_t*>(dv + G.o_best);
+    if (jb.block_sse && turned) {
+      d.sse_out = reinterpret_cast<uint64_t*>(dv + sse_off);
+      sse_off += size_t(nc) * size_t(G.nfb) * 8;
+    }
     d.frame = dframes + i;
     d.g = dg + i;
     d.tot = reinterpret_cast<uint64_t*>(dv + G.o_tot);
@@ -215,14 +232,18 @@ int av1pf_cdef_search_many(av1pf_ctx* ctx, int n, const av1pf_cdef_search_job* j
   }
   const auto* ddescs = reinterpret_cast<const CdefSearchDesc*>(dv + o_descs);
   cudaError_t e = cudaMemcpyAsync(dv, hs, o_g, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dg, 0, size_t(n) * sizeof(CdefGreedy), s);
+  // the greedy states and, with them, everything up to the results: the error
+  // tables, into which the halves of a block are added
+  if (e == cudaSuccess) e = cudaMemsetAsync(dg, 0, o_results - o_g, s);
   if (e != cudaSuccess) return cuda_status(e, "search upload");
-  launch_cdef_search(ddescs, n, blocks, thorough != 0, s);
-  for (int step = 0; step < 8; step++) launch_cdef_greedy_step(ddescs, n, ncand, s);
-  launch_cdef_greedy_finish(ddescs, n, entries, s);
-  e = cudaMemcpyAsync(hs + o_g, dv + o_results, res_bytes, cudaMemcpyDeviceToHost, s);
+  bool shallow = false, deep = false;
+  for (int i = 0; i < n; i++) (jobs[i].info->bit_depth > 10 ? deep : shallow) = true;
+  launch_cdef_search(ddescs, n, blocks, thorough != 0, shallow, deep, s);
+  launch_cdef_greedy(ddescs, n, ny, nuv, nfb_max, entries, s);
+  if (sse_bytes && turned) launch_sse_transpose(ddescs, n, nfb_max, nc, s);
+  e = cudaMemcpyAsync(hs + o_g, dv + o_results, res_bytes + (turned ? sse_bytes : 0), cudaMemcpyDeviceToHost, s);
   size_t so = o_g + res_bytes;
-  for (int i = 0; i < n && e == cudaSuccess; i++) {
+  for (int i = 0; i < n && e == cudaSuccess && !turned; i++) {
     if (!jobs[i].block_sse) continue;
     const size_t bytes = size_t(nc) * size_t(geo[size_t(i)].nfb) * 8;
     e = cudaMemcpyAsync(hs + so, dv + geo[size_t(i)].o_sse, bytes, cudaMemcpyDeviceToHost, s);
@@ -249,10 +270,13 @@ int av1pf_cdef_search_many(av1pf_ctx* ctx, int n, const av1pf_cdef_search_job* j
       }
     }
     if (jb.cdef_idx_out) std::memcpy(jb.cdef_idx_out, hs + o_g + G.o_res + 18 * sizeof(int32_t), G.table_bytes);
-    if (jb.block_sse) {  // candidate-major on the device, block-major for the caller
+    if (jb.block_sse) {
       const uint64_t* t = reinterpret_cast<const uint64_t*>(hs + so);
-      for (int k = 0; k < nc; k++)
-        for (int b = 0; b < G.nfb; b++) jb.block_sse[size_t(b) * size_t(nc) + size_t(k)] = t[size_t(k) * size_t(G.nfb) + size_t(b)];
+      if (turned)
+        std::memcpy(jb.block_sse, t, size_t(nc) * size_t(G.nfb) * 8);
+      else
+        for (int k = 0; k < nc; k++)
+          for (int b = 0; b < G.nfb; b++) jb.block_sse[size_t(b) * size_t(nc) + size_t(k)] = t[size_t(k) * size_t(G.nfb) + size_t(b)];
       so += size_t(nc) * size_t(G.nfb) * 8;
     }
   }
