@@ -165,8 +165,8 @@ struct LrSearchDesc {
   const LrSearchFrame* frames;
   int32_t wmax, hmax;      // the widest unit and tallest rectangle
   int32_t step;            // fit on every step-th row and column
-  int32_t band, cache_px;  // self-guided rows per band; filter outputs kept per unit
-  int32_t both;            // 1: radius-2 and radius-1 box sums from one sweep (their buffers fit)
+  int32_t spc;             // self-guided sets a CTA fits (1 or 2)
+  int32_t deep;            // 1: some frame has more than 10 bits
   int32_t multi_rect;      // 1: some job has several stripe rectangles (the first-pass kernel runs)
   int32_t nsets, sets[16];
   const LrSearchJob* jobs;

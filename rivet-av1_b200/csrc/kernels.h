@@ -176,11 +176,7 @@ struct SsePlane {
 // The loop-restoration search (lr_search.cu): per unit job, the no-filter
 // error and the Wiener passes on `s` (the first pass in a kernel of its own
 // for jobs of several rectangles), the self-guided fits (one CTA per job
-// and set) on `side` beside them, then the choice. Shared memory per kind:
-// 0 the first-pass kernel, 1 the Wiener kernel, 2 the self-guided kernel.
-size_t lr_search_smem(int wmax, int hmax, int kind, int band, int cache_px, int both);
-// The self-guided band height and filter-output cache that fit shared memory.
-void lr_search_shape(int wmax, int hmax, int upx_max, int& band, int& cache_px, int& both);
+// and d.spc sets) on `side` beside them, then the choice.
 // Raises the kernels' dynamic shared-memory limits to the device's maximum
 // (the same value on every call) on the current device.
 cudaError_t lr_search_init();

@@ -4,10 +4,10 @@
 // for each parameter set, priced with lambda; the cheapest is the unit's
 // choice.
 //
-// One CTA per unit, 256 threads. Each of the unit's stripe rectangles is
-// staged as the decoder's restoration window (postfilter.rs:765-777:
-// clamped to the plane, rows beyond the stripe from the deblocked frame)
-// in shared memory, once per phase.
+// One CTA per unit (per unit and two parameter sets for the self-guided
+// fits). Each of the unit's stripe rectangles is staged as the decoder's
+// restoration window (postfilter.rs:765-777: clamped to the plane, rows beyond
+// the stripe from the deblocked frame) in shared memory.
 //
 // Exactness. The reference fits in f64, summing over the unit's samples in
 // row-major order. Sums whose terms are integers (the first Wiener pass,
@@ -23,24 +23,24 @@
 // file is compiled without floating-point contraction, and the sums use
 // the explicit _rn intrinsics).
 #include <cfloat>
+#include <type_traits>
 
 #include "av1_tables.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "lr_walk.cuh"
 
 namespace av1pf {
 
 namespace {
 
 constexpr int kB = 3;            // window border (postfilter.rs:744 LRB)
-constexpr int kSgrCachePx = 6144;  // filter outputs kept between the fit and its error (units up to 96 x 64)
 constexpr int kThreads = 256;
 constexpr int kWienerChunk = 4;  // rows of Wiener terms handed from the producing warps to the adding lanes at a time
 constexpr int kWienerErrBand = 32;  // output rows per band of the Wiener error pass (its int16 rows fit the term region)
 __constant__ int32_t kSgrParams[16][4] = AV1T_SGR_PARAMS;
 __constant__ int32_t kWienerMin[3] = AV1T_WIENER_TAPS_MIN, kWienerMax[3] = AV1T_WIENER_TAPS_MAX;
 __constant__ int32_t kXqdMin[2] = AV1T_SGRPROJ_XQD_MIN, kXqdMax[2] = AV1T_SGRPROJ_XQD_MAX;
-constexpr uint64_t kExact = uint64_t(1) << 53;
 
 __device__ __forceinline__ int ld(const DPlane& p, int sb, int x, int y) { return ld_sample(p, sb, x, y); }
 
@@ -60,15 +60,13 @@ struct Win {
 
 // lr_window (postfilter.rs:765-777) of rectangle `rc` into shared memory.
 __device__ void stage_window(const LrSearchFrame& d, int p, const LrSearchRect& rc, int x0, int w, int16_t* win,
-                             int ws, int16_t* srcw = nullptr) {
+                             int ws) {
   // a warp per window row, lanes along it (no index division), eight rows'
-  // loads in flight before their stores; with `srcw`, the rectangle's source
-  // samples too (row stride w)
+  // loads in flight before their stores
   constexpr int kR = 8;
   const int ww = w + 2 * kB, wh = rc.h + 2 * kB, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int pex = d.pex[p], pey = d.pey[p];
-  const int rows_all = wh + (srcw ? rc.h : 0);
-  for (int r0 = threadIdx.x >> 5; r0 < rows_all; r0 += kR * nw) {
+  for (int r0 = threadIdx.x >> 5; r0 < wh; r0 += kR * nw) {
     for (int c = lane; c < ww; c += 32) {
       int v[kR];
 #pragma unroll
@@ -80,33 +78,15 @@ __device__ void stage_window(const LrSearchFrame& d, int p, const LrSearchRect& 
           const DPlane& pl = y < rc.ss || y > rc.se ? d.cur[p] : d.cdef[p];
           const int yy = y < rc.ss ? max(rc.ss - 2, y) : (y > rc.se ? min(rc.se + 2, y) : y);
           v[m] = ld(pl, d.sb, max(min(x0 + c - kB, pex), 0), yy);
-        } else if (r < rows_all && c < w) {
-          v[m] = ld(d.src[p], d.sb, x0 + c, rc.y0 + r - wh);
         }
       }
 #pragma unroll
       for (int m = 0; m < kR; m++) {
         const int r = r0 + m * nw;
-        if (r < wh)
-          win[r * ws + c] = int16_t(v[m]);
-        else if (r < rows_all && c < w)
-          srcw[(r - wh) * w + c] = int16_t(v[m]);
+        if (r < wh) win[r * ws + c] = int16_t(v[m]);
       }
     }
   }
-}
-
-// Block sum of 64-bit values (every thread gets the result).
-__device__ int64_t block_sum_i64(int64_t v, int64_t* red) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int64_t t = 0;
-  for (int w = 0; w < kThreads / 32; w++) t += red[w];
-  __syncthreads();
-  return t;
 }
 
 // Block sums of N 64-bit values in one round (every thread gets the totals).
@@ -183,9 +163,22 @@ __device__ __forceinline__ void wiener_line(const Win& W, bool vertical, int i, 
   }
 }
 
+// The window of a rectangle, read from the planes: row r, column c.
+struct PlaneWin {
+  const LrSearchFrame& F;
+  const LrSearchRect& rc;
+  int p, x0;
+  __device__ int at(int r, int c) const {
+    const int x = max(min(x0 + c - kB, F.pex[p]), 0), y = max(min(rc.y0 + r - kB, F.pey[p]), 0);
+    return y < rc.ss   ? ld(F.cur[p], F.sb, x, max(rc.ss - 2, y))
+           : y > rc.se ? ld(F.cur[p], F.sb, x, min(rc.se + 2, y))
+                       : ld(F.cdef[p], F.sb, x, y);
+  }
+};
+
 // One self-guided A/B pair (postfilter.rs:918-948) at A/B position (ai, aj)
 // of the rectangle (window position ai + 2, aj + 2).
-__device__ __forceinline__ void sgr_ab(const Win& W, int ai, int aj, int r, int n, int s, int one_over_n, int bd,
+__device__ __forceinline__ void sgr_ab(const PlaneWin& W, int ai, int aj, int r, int n, int s, int one_over_n, int bd,
                                        int32_t& A, int32_t& B) {
   const int wy = ai + kB - 1, wx = aj + kB - 1;
   int32_t bs = 0;
@@ -222,33 +215,9 @@ __device__ __forceinline__ SgrPass sgr_pass(int set, int pass) {
   return q;
 }
 
-// A self-guided filter output (postfilter.rs:950-988) at (i, j) from A/B
-// rows held in shared memory (`ab`: rows ai0.., stride aw; A then B).
-__device__ __forceinline__ int32_t sgr_flt(int pass, int yabs, int i_rel, int j, const int32_t* Ab, const int32_t* Bb,
-                                           int aw, int cval) {
-  int32_t a = 0, b = 0;
-#pragma unroll
-  for (int dy = -1; dy <= 1; dy++) {
-#pragma unroll
-    for (int dx = -1; dx <= 1; dx++) {
-      int wgt;
-      if (pass == 0)
-        wgt = ((yabs + dy) & 1) ? (dx == 0 ? 6 : 5) : 0;
-      else
-        wgt = (dx == 0 || dy == 0) ? 4 : 3;
-      if (wgt) {
-        const int k = (i_rel + 1 + dy) * aw + (j + 1 + dx);
-        a += wgt * Ab[k];
-        b += wgt * Bb[k];
-      }
-    }
-  }
-  const int shift = (pass == 0 && (yabs & 1)) ? 4 : 5;
-  return round2(a * cval + b, 8 + shift - 4);
-}
-
-// The same output with A/B computed on the spot (the in-order fallback).
-__device__ int32_t sgr_flt_direct(const Win& W, int pass, const SgrPass& q, int bd, int yabs, int i, int j, int cval) {
+// A self-guided filter output (postfilter.rs:950-988) at (i, j), its A/B
+// computed on the spot (the in-order fallback).
+__device__ int32_t sgr_flt_direct(const PlaneWin& W, int pass, const SgrPass& q, int bd, int yabs, int i, int j, int cval) {
   int32_t a = 0, b = 0;
   for (int dy = -1; dy <= 1; dy++)
     for (int dx = -1; dx <= 1; dx++) {
@@ -268,162 +237,14 @@ __device__ int32_t sgr_flt_direct(const Win& W, int pass, const SgrPass& q, int 
   return round2(a * cval + b, 8 + shift - 4);
 }
 
-// SGR_A2 (postfilter.rs:884-898), built at compile time.
-struct LrsA2 {
-  int32_t v[256];
-};
-constexpr LrsA2 make_lrs_a2() {
-  LrsA2 t{};
-  for (int z = 0; z < 256; z++) t.v[z] = z >= 255 ? 256 : (z == 0 ? 1 : ((z << 8) + z / 2) / (z + 1));
-  return t;
-}
-__device__ const LrsA2 g_lrs_a2 = make_lrs_a2();
-
-// Fills A/B rows for output rows [i0, i0 + rows) of a rectangle (A/B rows
-// i0 .. i0 + rows + 1) for one pass (postfilter.rs:918-948), with separable
-// box sums: first each window row's horizontal sums of the samples and of
-// their squares (int32: 25 squares of 12-bit samples fit), then the
-// vertical sums. Pass 0 computes odd absolute rows only (the others have
-// weight 0). `hs`/`hq` hold (rows + 2 + 2r) x (w + 2) sums.
-// The vertical half: A/B rows 0 .. rows + 1 of the band from the window
-// rows' horizontal sums `hs`/`hq` (rows + 2 + 2r rows of stride w + 2).
-template <int r>
-__device__ __forceinline__ void sgr_vert_ab(const SgrPass& q, int pass, int bd, int y0, int i0, int rows, int w,
-                                            int32_t* Ab, int32_t* Bb, int aw, const int32_t* hs, const int32_t* hq) {
-  // n and 1/n follow from the radius (sgr_pass computes the same values)
-  constexpr int n = (2 * r + 1) * (2 * r + 1), one_over_n = ((1 << 12) + n / 2) / n;
-  const int cw = w + 2;
-  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sh = 2 * (bd - 8);
-  for (int ir = warp; ir < rows + 2; ir += nw) {
-    if (pass == 0 && ((y0 + i0 + ir - 1) & 1) == 0) continue;
-    for (int aj = lane; aj < cw; aj += 32) {
-      int32_t bs = 0, as = 0;
-#pragma unroll
-      for (int dy = 0; dy <= 2 * r; dy++) {
-        bs += hs[(ir + dy) * cw + aj];
-        as += hq[(ir + dy) * cw + aj];
-      }
-      // a * n and dd^2 stay below 2^31 (25 * 25 * 255^2); p * s needs 64 bits
-      const int32_t a = round2(as, sh);
-      const int32_t dd = round2(bs, bd - 8);
-      const int32_t p = max(a * n - dd * dd, 0);
-      const int64_t z = (int64_t(p) * q.s + (int64_t(1) << 19)) >> 20;  // SGRPROJ_MTABLE_BITS
-      const int32_t a2 = g_lrs_a2.v[z < 255 ? int(z) : 255];
-      const int64_t b2 = int64_t((256 - a2) * bs) * one_over_n;
-      Ab[ir * aw + aj] = a2;
-      Bb[ir * aw + aj] = int32_t((b2 + (1 << 11)) >> 12);  // SGRPROJ_RECIP_BITS
-    }
-  }
-}
-
-// Fills A/B rows for output rows [i0, i0 + rows) of a rectangle (A/B rows
-// i0 .. i0 + rows + 1) for one pass (postfilter.rs:918-948), with separable
-// box sums: first each window row's horizontal sums of the samples and of
-// their squares (int32: 25 squares of 12-bit samples fit), then the
-// vertical sums. Pass 0 computes odd absolute rows only (the others have
-// weight 0). `hs`/`hq` hold (rows + 2 + 2r) x (w + 2) sums.
-template <int r>
-__device__ void sgr_band_ab_r(const Win& W, const SgrPass& q, int pass, int bd, int y0, int i0, int rows, int w,
-                              int32_t* Ab, int32_t* Bb, int aw, int32_t* hs, int32_t* hq) {
-  const int cw = w + 2;
-  const int nrow = rows + 2 + 2 * r, wy0 = i0 + kB - 1 - r;
-  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();  // the previous users of hs / hq are done
-  for (int rr = warp; rr < nrow; rr += nw) {
-    const int wy = wy0 + rr;
-    for (int aj = lane; aj < cw; aj += 32) {
-      const int wx = aj + kB - 1;
-      int32_t sum = 0, sq = 0;
-#pragma unroll
-      for (int dx = -r; dx <= r; dx++) {
-        const int v = W.at(wy, wx + dx);
-        sum += v;
-        sq += v * v;
-      }
-      hs[rr * cw + aj] = sum;
-      hq[rr * cw + aj] = sq;
-    }
-  }
-  __syncthreads();
-  sgr_vert_ab<r>(q, pass, bd, y0, i0, rows, w, Ab, Bb, aw, hs, hq);
-}
-
-// Both passes of a band (pass 0 of radius 2, pass 1 of radius 1) from one
-// horizontal sweep: a row's 3-wide sums are the middle of its 5-wide ones.
-// `hs5`/`hq5` hold rows + 6 rows, `hs3`/`hq3` rows + 4 (window rows one
-// lower).
-__device__ void sgr_band_ab_both(const Win& W, const SgrPass& q0, const SgrPass& q1, int bd, int y0, int i0, int rows,
-                                 int w, int32_t* Ab0, int32_t* Bb0, int32_t* Ab1, int32_t* Bb1, int aw, int32_t* hs5,
-                                 int32_t* hq5, int32_t* hs3, int32_t* hq3) {
-  const int cw = w + 2;
-  const int nrow = rows + 6, wy0 = i0 + kB - 3;
-  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();  // the previous users of the sums are done
-  for (int rr = warp; rr < nrow; rr += nw) {
-    const int wy = wy0 + rr;
-    const bool mid = rr >= 1 && rr < nrow - 1;  // also a row of the radius-1 sums (row rr - 1)
-    for (int aj = lane; aj < cw; aj += 32) {
-      const int wx = aj + kB - 1;
-      const int v0 = W.at(wy, wx - 2), v1 = W.at(wy, wx - 1), v2 = W.at(wy, wx), v3 = W.at(wy, wx + 1),
-                v4 = W.at(wy, wx + 2);
-      const int32_t s3 = v1 + v2 + v3, q3 = v1 * v1 + v2 * v2 + v3 * v3;
-      hs5[rr * cw + aj] = s3 + v0 + v4;
-      hq5[rr * cw + aj] = q3 + v0 * v0 + v4 * v4;
-      if (mid) {
-        hs3[(rr - 1) * cw + aj] = s3;
-        hq3[(rr - 1) * cw + aj] = q3;
-      }
-    }
-  }
-  __syncthreads();
-  sgr_vert_ab<2>(q0, 0, bd, y0, i0, rows, w, Ab0, Bb0, aw, hs5, hq5);
-  sgr_vert_ab<1>(q1, 1, bd, y0, i0, rows, w, Ab1, Bb1, aw, hs3, hq3);
-}
-
-// The band's A/B for the pass's radius (1 or 2): the box sums' loops unrolled.
-__device__ __forceinline__ void sgr_band_ab(const Win& W, const SgrPass& q, int pass, int bd, int y0, int i0, int rows,
-                                            int w, int32_t* Ab, int32_t* Bb, int aw, int32_t* hs, int32_t* hq) {
-  if (q.r == 2)
-    sgr_band_ab_r<2>(W, q, pass, bd, y0, i0, rows, w, Ab, Bb, aw, hs, hq);
-  else
-    sgr_band_ab_r<1>(W, q, pass, bd, y0, i0, rows, w, Ab, Bb, aw, hs, hq);
-}
-
 }  // namespace
 
-// Shared memory of a search kernel: the window, then a region used as the
-// Wiener pass's term rows or the self-guided A/B bands.
-size_t lr_window_bytes(int wmax, int hmax) {
+// Shared memory of the first-pass kernel (kind 0: the window) and of the Wiener
+// kernel (1: the window and the term rows).
+size_t lr_search_smem(int wmax, int hmax, int kind) {
   const size_t ws = size_t(wmax + 2 * kB + 1) & ~size_t(1);
-  return ((size_t(hmax + 2 * kB) * ws * 2) + 15) & ~size_t(15);
-}
-size_t lr_search_smem(int wmax, int hmax, int kind, int band, int cache_px, int both) {
-  const size_t win = lr_window_bytes(wmax, hmax);
-  if (kind == 0) return win;  // the first-pass kernel
-  if (kind == 1) return win + size_t(2) * 4 * kWienerChunk * size_t(wmax + 1) * sizeof(double);  // Wiener passes
-  // self-guided: A/B of both passes, the band's box sums, the filter-output cache
-  return win + size_t(4) * (band + 2) * size_t(wmax + 2) * sizeof(int32_t) +
-         size_t(2) * (band + 6) * size_t(wmax + 2) * sizeof(int32_t) +
-         size_t(both ? 2 : 0) * (band + 4) * size_t(wmax + 2) * sizeof(int32_t) +
-         size_t(cache_px) * 2 * sizeof(int32_t) +
-         ((size_t(hmax) * size_t(wmax) * sizeof(int16_t) + 15) & ~size_t(15));
-}
-
-void lr_search_shape(int wmax, int hmax, int upx_max, int& band, int& cache_px, int& both) {
-  // Filter outputs are kept when every unit's fit fits the cache; then the
-  // tallest band that leaves room for two CTAs per SM, else the tallest that
-  // fits at all; the one-sweep box sums where their buffers fit beside that
-  // band.
-  constexpr size_t kTwo = 113 * 1024, kLimit = 220 * 1024;
-  cache_px = upx_max <= kSgrCachePx ? upx_max : 0;
-  for (size_t lim : {kTwo, kLimit})
-    for (band = 32; band >= 4; band /= 2)
-      for (both = 1; both >= 0; both--)
-        if (lr_search_smem(wmax, hmax, 2, band, cache_px, both) <= lim) return;
-  band = 4;
-  cache_px = 0;
-  both = 0;
+  const size_t win = ((size_t(hmax + 2 * kB) * ws * 2) + 15) & ~size_t(15);
+  return kind == 0 ? win : win + size_t(2) * 4 * kWienerChunk * size_t(wmax + 1) * sizeof(double);
 }
 
 namespace {
@@ -753,25 +574,16 @@ __global__ void __launch_bounds__(128, 4) lr_search_wiener_kernel(const LrSearch
 
 // The self-guided fit's f64 sums in the reference's sample order, on one
 // thread (rare: very large units with large errors at 12 bits, where the
-// exact integer sums could round differently); the thread rebuilds each
-// rectangle's window itself.
+// exact integer sums could round differently), from the planes.
 __device__ __noinline__ void sgr_fit_in_order(const LrSearchDesc& d, const LrSearchFrame& F, const LrSearchJob& job,
-                                              const LrSearchRect* rects,
-                                              const Win& W, const Smem& sm, const SgrPass& q0, const SgrPass& q1,
+                                              const LrSearchRect* rects, const SgrPass& q0, const SgrPass& q1,
                                               double& m00, double& m01, double& m11, double& v0, double& v1) {
   const int p = job.plane, x0 = job.x0, w = job.w, sb = F.sb, step = d.step, bd = F.bd;
   const int r0 = q0.r, r1 = q1.r;
   m00 = m01 = m11 = v0 = v1 = 0.0;
   for (int ri = 0; ri < job.nr; ri++) {
     const LrSearchRect rc = rects[ri];
-    const int ww = w + 2 * kB, wh = rc.h + 2 * kB;
-    for (int k = 0; k < ww * wh; k++) {
-      const int rr = k / ww, c = k - rr * ww;
-      const int x = max(min(x0 + c - kB, F.pex[p]), 0), y = max(min(rc.y0 + rr - kB, F.pey[p]), 0);
-      sm.win[rr * sm.ws + c] = int16_t(y < rc.ss   ? ld(F.cur[p], sb, x, max(rc.ss - 2, y))
-                                       : y > rc.se ? ld(F.cur[p], sb, x, min(rc.se + 2, y))
-                                                   : ld(F.cdef[p], sb, x, y));
-    }
+    const PlaneWin W{F, rc, p, x0};
     for (int i = 0; i < rc.h; i += step)
       for (int j = 0; j < w; j += step) {
         const int yabs = rc.y0 + i;
@@ -789,183 +601,314 @@ __device__ __noinline__ void sgr_fit_in_order(const LrSearchDesc& d, const LrSea
   }
 }
 
-// Phase 3, one CTA per (unit, parameter set) (256 threads): the self-guided
-// fit (encoder/lr.rs:330-430) — the two box filters in bands of rows, the
-// fit's sums exact in int64 under the 2^53 magnitude bound (else in order
-// on one thread), the projection weights — and the restoration's error.
-__global__ void __launch_bounds__(kThreads, 2) lr_search_sgr_kernel(const LrSearchDesc d) {
-  extern __shared__ __align__(16) uint8_t lrs_smem[];
-  __shared__ int64_t red[kThreads / 32];
-  __shared__ int s_xqd[2];
-  const int ji = blockIdx.x / d.nsets, si = blockIdx.x - ji * d.nsets;
-  const LrSearchJob job = d.jobs[ji];
-  const LrSearchFrame& F = d.frames[job.frame];
-  const int p = job.plane, x0 = job.x0, w = job.w, sb = F.sb, tid = threadIdx.x, step = d.step;
-  const Smem sm = smem_of(lrs_smem, d);
-  const Win W{sm.win, sm.ws};
-  const LrSearchRect* rects = d.rects + job.r0;
-  const int bd = F.bd, maxv = (1 << bd) - 1;
-  const int set = d.sets[si];
+namespace {
+
+// The self-guided fits' shared memory: a strip's window, its source samples and
+// both filters' outputs less the sample (int16 pairs up to 10 bits, where they
+// stay below 2^15; else int32 pairs) of up to two sets.
+constexpr int kStrip = 64;
+constexpr int kStripPx = kStrip * kMaxH;
+constexpr int kSgrSrcOff = kWinBytes, kSgrCacheOff = kSgrSrcOff + kStripPx * 2;
+static_assert(kSgrSrcOff % 16 == 0, "vector access");
+
+struct SgrSums {  // of a warp: a = first filter - sample, b = second filter - sample, t = source - sample
+  int64_t aa, ab, bb, at, bt, tt;
+};
+
+__device__ __forceinline__ int64_t warp_sum_i64(int64_t v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The lane's part of a strip: columns c, c + 1 (`cols` of them inside) of rows
+// i0 .. i0 + left - 1; `per` rows are walked.
+struct SgrLane {
+  int i0, per, left, c, cols, ws;
+  const uint16_t *win, *src;  // window row 0 at column c; source row 0 at column c
+};
+
+// Both filters of a set over a lane's samples: their outputs less the sample to
+// `cache`, and the fit's sums added to `sum` by the warp's first lane. step:
+// every step-th row and column is fitted (1 or 2).
+template <bool DEEP>
+__device__ __forceinline__ void sgr_fit_strip(const SgrLane& g, int set, int step, int bd, GroupEdges& edges, int gl, int gn,
+                                              uint8_t* cache, SgrSums* sum) {
+  using Cross = typename std::conditional<DEEP, int64_t, int32_t>::type;  // 32 products below 2^24, or below 2^28
+  const int r0 = kSgrParams[set][0], r1 = kSgrParams[set][2];
+  const int k0 = r0 ? 16 : 0, k1 = r1 ? 16 : 0;
+  int64_t aa = 0, ab = 0, bb = 0;
+  Cross at = 0, bt = 0;
+  uint32_t tt = 0;  // (32 squares below 2^24)
+  auto fit = [&](int a, int b, int t) {
+    aa += int64_t(a) * a;
+    ab += int64_t(a) * b;
+    bb += int64_t(b) * b;
+    at += Cross(a) * t;
+    bt += Cross(b) * t;
+    tt += uint32_t(t * t);
+  };
+  int i = 0;
+  const uint16_t* sp = g.src + g.i0 * kStrip;
+  uint8_t* cp = cache + (g.i0 * kStrip + g.c) * (DEEP ? 8 : 4);
+  sgr_walk<DEEP>(g.win, g.ws, g.c, g.i0, g.per, r0, r1, c_lr.s12[set][0], c_lr.s12[set][1], bd - 8, edges, gl, gn,
+                 [&](uint32_t ca, uint32_t cb, int f0a, int f0b, int f1a, int f1b) {
+                   if (i < g.left) {
+                     const uint32_t s = *reinterpret_cast<const uint32_t*>(sp);
+                     const int aa0 = f0a - int(ca) * k0, ba0 = f1a - int(ca) * k1;
+                     const int ab0 = f0b - int(cb) * k0, bb0 = f1b - int(cb) * k1;
+                     if (DEEP)
+                       *reinterpret_cast<int4*>(cp) = make_int4(aa0, ba0, ab0, bb0);
+                     else
+                       *reinterpret_cast<uint2*>(cp) = make_uint2(__byte_perm(uint32_t(aa0), uint32_t(ba0), 0x5410),
+                                                                  __byte_perm(uint32_t(ab0), uint32_t(bb0), 0x5410));
+                     if (step == 1 || !(i & 1)) {
+                       fit(aa0, ba0, int(s & 0xffffu) - int(ca));
+                       if (step == 1 && g.cols > 1) fit(ab0, bb0, int(s >> 16) - int(cb));
+                     }
+                   }
+                   i++;
+                   sp += kStrip;
+                   cp += kStrip * (DEEP ? 8 : 4);
+                 });
+  const int64_t taa = warp_sum_i64(aa), tab = warp_sum_i64(ab), tbb = warp_sum_i64(bb);
+  const int64_t tat = warp_sum_i64(int64_t(at)), tbt = warp_sum_i64(int64_t(bt)), ttt = warp_sum_i64(int64_t(tt));
+  if ((threadIdx.x & 31) == 0) {
+    sum->aa += taa;
+    sum->ab += tab;
+    sum->bb += tbb;
+    sum->at += tat;
+    sum->bt += tbt;
+    sum->tt += ttt;
+  }
+}
+
+// The squared error of the lane's samples restored with weights w0, w2 from the
+// outputs that sgr_fit_strip kept: the sample, which the two weights' rest to 128
+// goes to, plus the weighted differences (postfilter.rs:836-850).
+template <bool DEEP>
+__device__ __forceinline__ uint32_t sgr_error_strip(const SgrLane& g, int w0, int w2, int maxv, const uint8_t* cache) {
+  uint32_t acc = 0;  // (32 squares below 2^24)
+  const uint16_t* wp = g.win + (g.i0 + 3) * g.ws + 2;  // samples (c - 1, c), (c + 1, ..)
+  const uint16_t* sp = g.src + g.i0 * kStrip;
+  const uint8_t* cp = cache + (g.i0 * kStrip + g.c) * (DEEP ? 8 : 4);
+  auto error = [&](int c, int a, int b, int s) {
+    const int e = clip3(0, maxv, c + ((w0 * a + w2 * b + (1 << 10)) >> 11)) - s;
+    return uint32_t(e * e);
+  };
+#pragma unroll 2
+  for (int i = 0; i < g.left; i++) {
+    const int ca = int(*reinterpret_cast<const uint32_t*>(wp) >> 16), cb = int(*reinterpret_cast<const uint32_t*>(wp + 2) & 0xffffu);
+    const uint32_t s = *reinterpret_cast<const uint32_t*>(sp);
+    int4 v;
+    if (DEEP) {
+      v = *reinterpret_cast<const int4*>(cp);
+    } else {
+      const uint2 q = *reinterpret_cast<const uint2*>(cp);
+      v = make_int4(int16_t(q.x), int32_t(q.x) >> 16, int16_t(q.y), int32_t(q.y) >> 16);
+    }
+    acc += error(ca, v.x, v.y, int(s & 0xffffu));
+    if (g.cols > 1) acc += error(cb, v.z, v.w, int(s >> 16));
+    wp += g.ws;
+    sp += kStrip;
+    cp += kStrip * (DEEP ? 8 : 4);
+  }
+  return acc;
+}
+
+// A set's weights from its fit (encoder/lr.rs:389-430).
+__device__ __noinline__ void sgr_weights(const LrSearchDesc& d, const LrSearchFrame& F, const LrSearchJob& job,
+                                         const LrSearchRect* rects, int set, const SgrSums& t, int32_t* xqd) {
   const SgrPass q0 = sgr_pass(set, 0), q1 = sgr_pass(set, 1);
   const int r0 = q0.r, r1 = q1.r;
-  const int aw = d.wmax + 2, band = d.band;
-  int32_t* Ab[2];
-  int32_t* Bb[2];
-  int32_t* reg = reinterpret_cast<int32_t*>(sm.region);
-  for (int q = 0; q < 2; q++) {
-    Ab[q] = reg + (2 * q) * (band + 2) * aw;
-    Bb[q] = reg + (2 * q + 1) * (band + 2) * aw;
+  // The reference's target is (128 * 16) times ours. Its f64 partial sums are
+  // exact, so any order gives them, while the terms' magnitudes sum below 2^53:
+  // the squares' own sums do, and by Cauchy-Schwarz a product's does where the
+  // product of its squares' sums is below 2^106 (2^105 here: it is rounded).
+  constexpr int64_t kExact = int64_t(1) << 53;
+  constexpr double kBound = 4.056481920730334e31;  // 2^105
+  const double tt = double(t.tt) * 4194304.0;      // 2048^2
+  double m00, m01, m11, v0, v1;
+  if (t.aa < kExact && t.bb < kExact && double(t.aa) * tt < kBound && double(t.bb) * tt < kBound) {
+    m00 = double(t.aa);
+    m01 = double(t.ab);
+    m11 = double(t.bb);
+    v0 = double(t.at * 2048);
+    v1 = double(t.bt * 2048);
+  } else {
+    sgr_fit_in_order(d, F, job, rects, q0, q1, m00, m01, m11, v0, v1);
   }
-  int32_t* hs = reg + 4 * (band + 2) * aw;
-  int32_t* hq = hs + (band + 6) * aw;
-  int32_t* hs3 = hq + (band + 6) * aw;  // the radius-1 sums of the one-sweep box sums
-  int32_t* hq3 = hs3 + (band + 4) * aw;
-  int32_t* cache = d.both ? hq3 + (band + 4) * aw : hs3;  // [px][2] filter outputs of the unit
-  int16_t* srcw = reinterpret_cast<int16_t*>(cache + 2 * d.cache_px);  // the rectangle's source samples
-  int upx = 0;
-  for (int ri = 0; ri < job.nr; ri++) upx += rects[ri].h * w;
-  const bool cached = upx <= d.cache_px;
-  int64_t f00 = 0, f01 = 0, f11 = 0, g0 = 0, g1 = 0, acc = 0;
-  uint64_t b01 = 0, bg0 = 0, bg1 = 0;
-  for (int pass_sse = 0; pass_sse < 2; pass_sse++) {
-    // pass_sse 0: the fit; 1: the error with the quantised weights
-    int pw0 = 0, pw1 = 0, pw2 = 0;
-    if (pass_sse == 1) {
-      pw0 = s_xqd[0];
-      pw1 = s_xqd[1];
-      pw2 = (1 << 7) - pw0 - pw1;
-    }
-    if (pass_sse == 1 && cached) {
-      // the fit pass kept every filter output
-      int off = 0;
-      for (int ri = 0; ri < job.nr; ri++) {
-        const LrSearchRect rc = rects[ri];
-        for (int i = tid >> 5; i < rc.h; i += blockDim.x >> 5)
-          for (int j = tid & 31; j < w; j += 32) {
-          const int k = i * w + j;
-          // one rectangle: its window and source are still staged
-          const int u = (job.nr == 1 ? W.at(i + kB, j + kB) : ld(F.cdef[p], sb, x0 + j, rc.y0 + i)) << 4;
-          const int fl0 = cache[2 * (off + k)], fl1 = cache[2 * (off + k) + 1];
-          int32_t val = pw1 * u;
-          val += r0 ? pw0 * fl0 : pw0 * u;
-          val += r1 ? pw2 * fl1 : pw2 * u;
-          const int out = min(max(round2(val, 4 + 7), 0), maxv);
-          const int e = out - (job.nr == 1 ? srcw[k] : ld(F.src[p], sb, x0 + j, rc.y0 + i));
-          acc += int64_t(e) * e;
-          }
-        off += rc.h * w;
+  double w0, w2;
+  if (r0 && r1) {
+    double m[2][2] = {{m00, m01}, {m01, m11}}, v[2] = {v0, v1}, x2[2];
+    solve<2>(m, v, x2);
+    w0 = x2[0];
+    w2 = x2[1];
+  } else if (r0) {
+    w0 = m00 > 0.0 ? __ddiv_rn(v0, m00) : 0.0;
+    w2 = 0.0;
+  } else {
+    w0 = 0.0;
+    w2 = m11 > 0.0 ? __ddiv_rn(v1, m11) : 0.0;
+  }
+  const int x0q = r0 ? min(max(f64_to_i32(round(w0)), kXqdMin[0]), kXqdMax[0]) : 0;
+  int x1q;
+  if (r1) {
+    // i32 arithmetic wraps as the reference's release build does
+    const int diff = int(uint32_t(1 << 7) - uint32_t(x0q) - uint32_t(f64_to_i32(round(w2))));
+    x1q = min(max(diff, kXqdMin[1]), kXqdMax[1]);
+  } else {
+    x1q = min(max((1 << 7) - x0q, kXqdMin[1]), kXqdMax[1]);
+  }
+  xqd[0] = x0q;
+  xqd[1] = x1q;
+}
+
+// The start of plane row y of window row `r` of a rectangle.
+__device__ __forceinline__ const uint8_t* search_row(const LrSearchFrame& F, int p, const LrSearchRect& rc, int r) {
+  const int y = max(min(rc.y0 + r - kB, F.pey[p]), 0);
+  const DPlane& pl = y < rc.ss || y > rc.se ? F.cur[p] : F.cdef[p];
+  const int yy = y < rc.ss ? max(rc.ss - 2, y) : (y > rc.se ? min(rc.se + 2, y) : y);
+  return pl.p + int64_t(yy) * pl.stride * F.sb;
+}
+
+// The source samples of a strip (columns x .. x + w - 1, rows y .. y + h - 1),
+// kStrip apart, eight at a time where they lie in an aligned row.
+__device__ __forceinline__ void stage_source(const LrSearchFrame& F, int p, int x, int w, int y, int h, uint16_t* out) {
+  const int64_t pitch = F.src[p].stride * F.sb;
+  const uint8_t* base = F.src[p].p + int64_t(y) * pitch + int64_t(x) * F.sb;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(base) | uintptr_t(pitch)) & uintptr_t(8 * F.sb - 1)) == 0;
+  for (int k = threadIdx.x; k < h * (kStrip / 8); k += kLrThreads) {
+    const int i = k / (kStrip / 8), j = (k % (kStrip / 8)) * 8;
+    if (j >= w) continue;
+    const uint8_t* row = base + int64_t(i) * pitch;
+    uint16_t* o = out + i * kStrip + j;
+    if (aligned && j + 8 <= w) {
+      uint4 v;
+      if (F.sb == 2) {
+        v = *reinterpret_cast<const uint4*>(row + j * 2);
+      } else {
+        const uint2 b = *reinterpret_cast<const uint2*>(row + j);
+        v = make_uint4(__byte_perm(b.x, 0, 0x4140), __byte_perm(b.x, 0, 0x4342), __byte_perm(b.y, 0, 0x4140),
+                       __byte_perm(b.y, 0, 0x4342));
       }
-      break;
+      *reinterpret_cast<uint4*>(o) = v;
+    } else {
+      for (int e = 0; e < 8 && j + e < w; e++) o[e] = uint16_t(ld_row(row, F.sb, j + e));
     }
-    int off = 0;
+  }
+}
+
+}  // namespace
+
+// Phase 3, one CTA per unit and d.spc (1 or 2) parameter sets: the self-guided
+// fit (encoder/lr.rs:330-430), the projection weights, and the restoration's
+// error. What bounds it is instruction issue; so the filters are the decoder's,
+// which walk the rows in registers (lr_walk.cuh), in strips of 64 columns and a
+// stripe. Of a unit that is one strip the window is staged once for all sets, and
+// each sample's filter outputs, kept from the fit, give its error; others stage
+// and walk their strips again. A strip of up to 32 columns holds work for two
+// warps: two sets take a half of the CTA each.
+// 6 sets of a 1080p 4:2:0 frame in units of 64: 740 us with the
+// filters in bands of shared memory (778 instructions a sample and set), 195 now.
+__global__ void __launch_bounds__(kLrThreads, 4) lr_search_sgr_kernel(const LrSearchDesc d) {
+  extern __shared__ __align__(16) uint8_t lrs_smem[];
+  __shared__ GroupEdges edges[kLrThreads / 16];
+  __shared__ const uint8_t* rows[kMaxH + 6];
+  __shared__ SgrSums sums[2][kLrThreads / 32];
+  __shared__ uint64_t s_err[2][kLrThreads / 32];
+  __shared__ int32_t s_xqd[2][2];
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int per_job = (d.nsets + d.spc - 1) / d.spc;
+  const int ji = blockIdx.x / per_job, si = (blockIdx.x - ji * per_job) * d.spc;
+  const int nk = min(d.spc, d.nsets - si);  // this CTA's sets
+  const LrSearchJob job = d.jobs[ji];
+  const LrSearchFrame& F = d.frames[job.frame];
+  const LrSearchRect* rects = d.rects + job.r0;
+  const int p = job.plane, bd = F.bd, maxv = (1 << bd) - 1;
+  uint16_t* win = reinterpret_cast<uint16_t*>(lrs_smem);
+  uint16_t* src = reinterpret_cast<uint16_t*>(lrs_smem + kSgrSrcOff);
+  uint8_t* cache = lrs_smem + kSgrCacheOff;
+  const bool deep = bd > 10;
+  const int slot = kStripPx * (deep ? 8 : 4);  // bytes of a set's kept outputs
+  const bool single = job.nr == 1 && job.w <= kStrip;
+  const bool halves = single && job.w <= kStrip / 2 && nk == 2;
+  const Team all{tid, kLrThreads, 1};
+  if (tid < 2 * (kLrThreads / 32)) {
+    sums[tid & 1][tid >> 1] = SgrSums{};
+    s_err[tid & 1][tid >> 1] = 0;
+  }
+  for (int pass = 0; pass < 2; pass++) {  // the fit, then the error with the quantised weights
     for (int ri = 0; ri < job.nr; ri++) {
       const LrSearchRect rc = rects[ri];
-      __syncthreads();
-      stage_window(F, p, rc, x0, w, sm.win, sm.ws, srcw);
-      for (int i0 = 0; i0 < rc.h; i0 += band) {
-        const int rows = min(band, rc.h - i0);
-        __syncthreads();
-        if (d.both && r0 == 2 && r1 == 1) {
-          sgr_band_ab_both(W, q0, q1, bd, rc.y0, i0, rows, w, Ab[0], Bb[0], Ab[1], Bb[1], aw, hs, hq, hs3, hq3);
-        } else {
-          if (r0) sgr_band_ab(W, q0, 0, bd, rc.y0, i0, rows, w, Ab[0], Bb[0], aw, hs, hq);
-          if (r1) sgr_band_ab(W, q1, 1, bd, rc.y0, i0, rows, w, Ab[1], Bb[1], aw, hs, hq);
+      for (int x = 0; x < job.w; x += kStrip) {
+        const int w = min(job.w - x, kStrip), h = rc.h;
+        SgrLane g;
+        g.ws = w > 32 ? kWideWS : kSlimWS;
+        const int gs = w > 32 ? 5 : 4, gn = 1 << gs;  // lanes of a group
+        const int half = halves ? tid >> 6 : 0, t = halves ? tid & 63 : tid;
+        const int gl = t & (gn - 1), lgroups = (halves ? 6 : 7) - gs;
+        g.per = (((h + (1 << lgroups) - 1) >> lgroups) + 1) & ~1;  // (the stripe's first row is even)
+        g.i0 = (t >> gs) * g.per;
+        g.c = 2 * gl;
+        g.cols = min(w - g.c, 2);
+        g.left = g.cols > 0 ? min(h - g.i0, g.per) : 0;
+        g.win = win + g.c;
+        g.src = src + g.c;
+        const int k0 = half, k1 = halves ? half + 1 : nk;  // the sets of this half
+        if (pass == 0 || !single) {
+          __syncthreads();  // (everyone is done with the previous strip)
+          for (int r = tid; r < h + 6; r += kLrThreads) rows[r] = search_row(F, p, rc, r);
+          __syncthreads();
+          stage_window(win, g.ws, rows, F.sb, F.pex[p], job.x0 + x, w, h, all);
+          stage_source(F, p, job.x0 + x, w, rc.y0, h, src);
+          __syncthreads();
         }
-        __syncthreads();
-        for (int ir = tid >> 5; ir < rows; ir += blockDim.x >> 5)
-          for (int j = tid & 31; j < w; j += 32) {
-          const int i = i0 + ir, yabs = rc.y0 + i;
-          const bool fit_px = ((i | j) & (step - 1)) == 0;  // step is 1 or 2
-          if (pass_sse == 0 && !fit_px && !cached) continue;
-          const int cval = W.at(i + kB, j + kB);  // the rectangle's rows lie in its stripe: CDEF output
-          const int u = cval << 4;  // SGRPROJ_RST_BITS
-          const int fl0 = r0 ? sgr_flt(0, yabs, ir, j, Ab[0], Bb[0], aw, cval) : 0;
-          const int fl1 = r1 ? sgr_flt(1, yabs, ir, j, Ab[1], Bb[1], aw, cval) : 0;
-          if (pass_sse == 0 && cached) {
-            cache[2 * (off + i * w + j)] = fl0;
-            cache[2 * (off + i * w + j) + 1] = fl1;
+#pragma unroll 1
+        for (int k = k0; k < k1; k++) {
+          uint8_t* kept = cache + k * slot;
+          // (the second walk's sums go where nothing reads them)
+          if (pass == 0 || !single) {
+            if (deep)
+              sgr_fit_strip<true>(g, d.sets[si + k], d.step, bd, edges[tid >> gs], gl, gn, kept, &sums[k][warp]);
+            else
+              sgr_fit_strip<false>(g, d.sets[si + k], d.step, bd, edges[tid >> gs], gl, gn, kept, &sums[k][warp]);
+            __syncwarp();  // (the next set's walk writes the group's edges)
           }
-          if (pass_sse == 0 && !fit_px) continue;
-          const int sv = srcw[i * w + j];
-          if (pass_sse == 0) {
-            // |a|, |b| < 2^17 and |t| < 2^23: 32-bit operands, 64-bit products
-            const int32_t a = r0 ? fl0 - u : 0, b = r1 ? fl1 - u : 0;
-            const int32_t t = 128 * ((sv << 4) - u);
-            f00 += int64_t(a) * a;
-            f01 += int64_t(a) * b;
-            f11 += int64_t(b) * b;
-            g0 += int64_t(a) * t;
-            g1 += int64_t(b) * t;
-            const uint32_t ua = uint32_t(abs(a)), ub = uint32_t(abs(b)), ut = uint32_t(abs(t));
-            b01 += uint64_t(ua) * ub;
-            bg0 += uint64_t(ua) * ut;
-            bg1 += uint64_t(ub) * ut;
-          } else {
-            int32_t val = pw1 * u;
-            val += r0 ? pw0 * fl0 : pw0 * u;
-            val += r1 ? pw2 * fl1 : pw2 * u;
-            const int out = min(max(round2(val, 4 + 7), 0), maxv);
-            const int e = out - sv;
-            acc += int64_t(e) * e;
+          if (pass == 1) {
+            const int w0 = s_xqd[k][0], w2 = (1 << 7) - w0 - s_xqd[k][1];
+            const uint32_t e = deep ? sgr_error_strip<true>(g, w0, w2, maxv, kept) : sgr_error_strip<false>(g, w0, w2, maxv, kept);
+            const int64_t te = warp_sum_i64(int64_t(e));
+            if ((tid & 31) == 0) s_err[k][warp] += uint64_t(te);
           }
         }
       }
-      off += rc.h * w;
-    }
-    if (pass_sse == 1) break;
-    const int64_t t00 = block_sum_i64(f00, red), t01 = block_sum_i64(f01, red), t11 = block_sum_i64(f11, red);
-    const int64_t tg0 = block_sum_i64(g0, red), tg1 = block_sum_i64(g1, red);
-    // each f64 partial sum is exact (so any order gives the reference's sums)
-    // while the terms' magnitudes sum below 2^53
-    const uint64_t sb01 = uint64_t(block_sum_i64(int64_t(b01), red));
-    const uint64_t sbg0 = uint64_t(block_sum_i64(int64_t(bg0), red));
-    const uint64_t sbg1 = uint64_t(block_sum_i64(int64_t(bg1), red));
-    const bool exact = uint64_t(t00) < kExact && uint64_t(t11) < kExact && sb01 < kExact && sbg0 < kExact &&
-                       sbg1 < kExact;
-    if (tid == 0) {
-      double m00, m01, m11, v0, v1;
-      if (exact) {
-        m00 = double(t00);
-        m01 = double(t01);
-        m11 = double(t11);
-        v0 = double(tg0);
-        v1 = double(tg1);
-      } else {
-        sgr_fit_in_order(d, F, job, rects, W, sm, q0, q1, m00, m01, m11, v0, v1);
-      }
-      double w0, w2;
-      if (r0 && r1) {
-        double m[2][2] = {{m00, m01}, {m01, m11}}, v[2] = {v0, v1}, x2[2];
-        solve<2>(m, v, x2);
-        w0 = x2[0];
-        w2 = x2[1];
-      } else if (r0) {
-        w0 = m00 > 0.0 ? __ddiv_rn(v0, m00) : 0.0;
-        w2 = 0.0;
-      } else {
-        w0 = 0.0;
-        w2 = m11 > 0.0 ? __ddiv_rn(v1, m11) : 0.0;
-      }
-      const int x0q = r0 ? min(max(f64_to_i32(round(w0)), kXqdMin[0]), kXqdMax[0]) : 0;
-      int x1q;
-      if (r1) {
-        // i32 arithmetic wraps as the reference's release build does
-        const int diff = int(uint32_t(1 << 7) - uint32_t(x0q) - uint32_t(f64_to_i32(round(w2))));
-        x1q = min(max(diff, kXqdMin[1]), kXqdMax[1]);
-      } else {
-        x1q = min(max((1 << 7) - x0q, kXqdMin[1]), kXqdMax[1]);
-      }
-      s_xqd[0] = x0q;
-      s_xqd[1] = x1q;
     }
     __syncthreads();
-  }
-  const int64_t e = block_sum_i64(acc, red);
-  if (tid == 0) {
-    LrSgrResult& r = d.sgr[blockIdx.x];
-    r.xqd[0] = s_xqd[0];
-    r.xqd[1] = s_xqd[1];
-    r.sse = uint64_t(e);
+    // a thread per set: in the first warp of the half that fits it
+    if ((tid & 63) == 0 && tid >> 6 < nk) {
+      const int k = tid >> 6;
+      if (pass == 0) {
+        SgrSums t{};
+        for (int q = 0; q < kLrThreads / 32; q++) {
+          t.aa += sums[k][q].aa;
+          t.ab += sums[k][q].ab;
+          t.bb += sums[k][q].bb;
+          t.at += sums[k][q].at;
+          t.bt += sums[k][q].bt;
+          t.tt += sums[k][q].tt;
+        }
+        sgr_weights(d, F, job, rects, d.sets[si + k], t, s_xqd[k]);
+      } else {
+        LrSgrResult& r = d.sgr[ji * d.nsets + si + k];
+        r.xqd[0] = s_xqd[k][0];
+        r.xqd[1] = s_xqd[k][1];
+        uint64_t e = 0;
+        for (int q = 0; q < kLrThreads / 32; q++) e += s_err[k][q];
+        r.sse = e;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -1029,13 +972,13 @@ cudaError_t lr_search_init() {
 void launch_lr_search(const LrSearchDesc& d, int njobs, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                       cudaEvent_t join) {
   if (njobs <= 0) return;
-  const size_t s0 = lr_search_smem(d.wmax, d.hmax, 0, d.band, d.cache_px, d.both);
-  const size_t s1 = lr_search_smem(d.wmax, d.hmax, 1, d.band, d.cache_px, d.both);
-  const size_t s2 = lr_search_smem(d.wmax, d.hmax, 2, d.band, d.cache_px, d.both);
+  const size_t s0 = lr_search_smem(d.wmax, d.hmax, 0);
+  const size_t s1 = lr_search_smem(d.wmax, d.hmax, 1);
+  const size_t s2 = size_t(kSgrCacheOff) + size_t(d.spc) * kStripPx * (d.deep ? 8 : 4);
   // the self-guided fits depend on nothing else: they run beside the Wiener passes
   cudaEventRecord(fork, s);
   cudaStreamWaitEvent(side, fork, 0);
-  lr_search_sgr_kernel<<<njobs * d.nsets, kThreads, s2, side>>>(d);
+  lr_search_sgr_kernel<<<njobs * ((d.nsets + d.spc - 1) / d.spc), kLrThreads, s2, side>>>(d);
   if (d.multi_rect) lr_search_prep_kernel<<<njobs, kThreads, s0, s>>>(d);
   lr_search_wiener_kernel<<<njobs, 128, s1, s>>>(d);
   cudaEventRecord(join, side);

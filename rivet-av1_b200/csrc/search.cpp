@@ -537,14 +537,14 @@ int av1pf_lr_search_many(av1pf_ctx* ctx, int n, av1pf_lr_search_job* jobs_in, in
   }
   std::vector<av1pf_lr_unit> chosen(jobs.size());
   if (!jobs.empty()) {
-    int upx_max = 0;
-    for (const LrSearchJob& jb : jobs) {
-      int px = 0;
-      for (int r = 0; r < jb.nr; r++) px += rects[size_t(jb.r0 + r)].h * jb.w;
-      upx_max = std::max(upx_max, px);
+    for (const LrSearchJob& jb : jobs)
       if (jb.nr > 1) d.multi_rect = 1;
-    }
-    lr_search_shape(d.wmax, d.hmax, upx_max, d.band, d.cache_px, d.both);
+    for (const LrSearchFrame& f : frames)
+      if (f.bd > 10) d.deep = 1;
+    // Two sets a CTA share a unit's window and source, where that leaves four
+    // CTAs for each SM; the kept outputs of two sets above 10 bits would leave an
+    // SM two CTAs.
+    d.spc = !d.deep && int64_t(jobs.size()) * (d.nsets / 2) >= 4 * 148 ? 2 : 1;
     cudaError_t e = lr_search_init();
     if (e != cudaSuccess) return cuda_status(e, "loop-restoration search attributes");
     const size_t fb = frames.size() * sizeof(LrSearchFrame);
