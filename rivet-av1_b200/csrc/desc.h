@@ -149,11 +149,10 @@ struct LrSearchRect {
   int32_t ss, se;  // StripeStartY, StripeEndY
   int32_t y0, h;   // rows restored
 };
-// Per unit: the unfiltered error, the first Wiener pass's vertical
-// solution, the quantised Wiener coefficients and their error.
+// Per unit: the unfiltered error, the quantised Wiener coefficients and their
+// error.
 struct LrJobState {
   uint64_t none, wiener;
-  double vc[3];  // first-pass solution of a unit of several rectangles
   int32_t coef[2][3];
 };
 // Per (unit, self-guided set): the projection weights and their error.
@@ -167,7 +166,6 @@ struct LrSearchDesc {
   int32_t step;            // fit on every step-th row and column
   int32_t spc;             // self-guided sets a CTA fits (1 or 2)
   int32_t deep;            // 1: some frame has more than 10 bits
-  int32_t multi_rect;      // 1: some job has several stripe rectangles (the first-pass kernel runs)
   int32_t nsets, sets[16];
   const LrSearchJob* jobs;
   const LrSearchRect* rects;

@@ -174,8 +174,7 @@ struct SsePlane {
   int32_t sb;       // bytes per sample
 };
 // The loop-restoration search (lr_search.cu): per unit job, the no-filter
-// error and the Wiener passes on `s` (the first pass in a kernel of its own
-// for jobs of several rectangles), the self-guided fits (one CTA per job
+// error and the Wiener passes on `s`, the self-guided fits (one CTA per job
 // and d.spc sets) on `side` beside them, then the choice.
 // Raises the kernels' dynamic shared-memory limits to the device's maximum
 // (the same value on every call) on the current device.

@@ -57,7 +57,7 @@ constexpr LrConst make_lr_const() {
       const int n = k ? 9 : 25, n2e = n * n * kSgrParams[set][2 * k + 1];
       t.s12[set][k] = n2e ? uint32_t(((1 << 20) + n2e / 2) / n2e) << 12 : 0u;
     }
-  for (int n = 1; n < 10; n++) t.inv[n] = (65536 + n - 1) / n;
+  for (int n = 1; n < 50; n++) t.inv[n] = ((1u << 22) + n - 1) / n;
   return t;
 }
 }  // namespace
@@ -76,7 +76,7 @@ __device__ __forceinline__ void pass_through(const FrameDesc& f, int p, int x0, 
   const int64_t opitch = int64_t((f.uw + plane_ssx(f, p)) >> plane_ssx(f, p)) * bps;
   uint8_t* out = f.lr_pack ? f.frame_out + f.out_off[p] + int64_t(y0) * opitch + x0 * bps : nullptr;
   const int ng = (w + 7) >> 3;  // 8-sample chunks a row, at most 8
-  const int inv = c_lr.inv[ng];
+  const uint32_t inv = c_lr.inv[ng];
   const bool sv = ((reinterpret_cast<uintptr_t>(src) | uintptr_t(spitch)) & uintptr_t(8 * sb - 1)) == 0;
   constexpr int kBatch = 2;
 #pragma unroll 1
@@ -86,7 +86,7 @@ __device__ __forceinline__ void pass_through(const FrameDesc& f, int p, int x0, 
     for (int m = 0; m < kBatch; m++) {
       const int k = k0 + m * tm.n;
       if (k >= h * ng) continue;
-      const int r = (k * inv) >> 16, c = (k - r * ng) * 8;
+      const int r = int((uint32_t(k) * inv) >> 22), c = (k - r * ng) * 8;
       const uint8_t* sp = src + int64_t(r) * spitch + c * sb;
       if (sv && c + 8 <= w) {
         if (sb == 2) {
@@ -107,7 +107,7 @@ __device__ __forceinline__ void pass_through(const FrameDesc& f, int p, int x0, 
     for (int m = 0; m < kBatch; m++) {
       const int k = k0 + m * tm.n;
       if (k >= h * ng) continue;
-      const int r = (k * inv) >> 16, c = (k - r * ng) * 8, n = min(8, w - c);
+      const int r = int((uint32_t(k) * inv) >> 22), c = (k - r * ng) * 8, n = min(8, w - c);
       auto put = [&](uint8_t* at, int width) {
         if (n == 8 && (reinterpret_cast<uintptr_t>(at) & uintptr_t(8 * width - 1)) == 0) {
           if (width == 2)
@@ -179,58 +179,11 @@ __device__ __forceinline__ void emit(Group& g, uint32_t a, uint32_t b) {
   g.ref += g.ref_pitch;
 }
 
-// Four 8-bit coefficients in a word.
-__device__ __forceinline__ int bytes4(int a, int b, int c, int d) {
-  return int((uint32_t(a) & 255u) | ((uint32_t(b) & 255u) << 8) | ((uint32_t(c) & 255u) << 16) | (uint32_t(d) << 24));
-}
-
 // postfilter.rs:795-822
 template <bool PAIRS>
 __device__ __forceinline__ void wiener_group(Group& g, const av1pf_lr_unit& u, int bd) {
-  const int round0 = bd == 12 ? 5 : 3, round1 = bd == 12 ? 9 : 11;
-  const int offset = 1 << (bd + 7 - round0 - 1);
-  const int limit = (1 << (bd + 1 + 7 - round0)) - 1;
-  const int maxv = (1 << bd) - 1;
-  const int h0 = u.wiener[1][0], h1 = u.wiener[1][1], h2 = u.wiener[1][2];
-  const int v0 = u.wiener[0][0], v1 = u.wiener[0][1], v2 = u.wiener[0][2];
-  const int h3 = 128 - 2 * (h0 + h1 + h2), v3 = 128 - 2 * (v0 + v1 + v2);
-  // the taps but the middle one (which can exceed 8 bits) against the samples
-  // c .. c + 7, for the first column and the second
-  const int e0 = bytes4(h0, h1, h2, 0), e1 = bytes4(h2, h1, h0, 0);
-  const int o0 = bytes4(0, h0, h1, h2), o1 = bytes4(0, h2, h1, h0);
-  const int rnd0 = 1 << (round0 - 1), rnd1 = 1 << (round1 - 1);
-  const uint16_t* row = g.win + g.i0 * g.ws;
-  auto across = [&](int& a, int& b) {
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(row);
-    row += g.ws;
-    const int q0 = int(q[0]), q1 = int(q[1]), q2 = int(q[2]), q3 = int(q[3]);
-    int x = int(uint32_t(q1) >> 16) * h3 + rnd0, y = (q2 & 0xffff) * h3 + rnd0;
-    x = __dp2a_hi(q3, e1, __dp2a_lo(q2, e1, __dp2a_hi(q1, e0, __dp2a_lo(q0, e0, x))));
-    y = __dp2a_hi(q3, o1, __dp2a_lo(q2, o1, __dp2a_hi(q1, o0, __dp2a_lo(q0, o0, y))));
-    a = clip3(-offset, limit - offset, x >> round0);
-    b = clip3(-offset, limit - offset, y >> round0);
-  };
-  // the last six rows' results and four new ones a step
-  int a[10], b[10];
-#pragma unroll
-  for (int k = 0; k < 6; k++) across(a[k], b[k]);
-  auto down = [&](const int* t) {
-    const int acc = v0 * (t[0] + t[6]) + v1 * (t[1] + t[5]) + v2 * (t[2] + t[4]) + v3 * t[3] + rnd1;
-    return uint32_t(clip3(0, maxv, acc >> round1));
-  };
-#pragma unroll 1
-  for (int i = 0; i < g.per; i += 4) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      across(a[6 + k], b[6 + k]);
-      emit<PAIRS>(g, down(a + k), down(b + k));
-    }
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-      a[k] = a[k + 4];
-      b[k] = b[k + 4];
-    }
-  }
+  wiener_walk(g.win, g.ws, g.i0, g.per, u.wiener[0][0], u.wiener[0][1], u.wiener[0][2], u.wiener[1][0], u.wiener[1][1],
+              u.wiener[1][2], bd, [](int) {}, [&](int, uint32_t a, uint32_t b) { emit<PAIRS>(g, a, b); });
 }
 
 // postfilter.rs:823-851

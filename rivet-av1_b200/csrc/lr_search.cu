@@ -16,9 +16,8 @@
 // sum of the terms' magnitudes stays below 2^53: they are summed in int64
 // in parallel (the self-guided sums check that bound and otherwise redo the
 // sum in order on one thread). The second and third Wiener passes have
-// real-valued terms, so their sums run in the reference's order: warps 1-3
-// produce four rows of terms at a time into shared memory while lanes of
-// warp 0 each add one accumulator's terms in sample order. Every f64 operation is a
+// real-valued terms, so their sums run in the reference's order: lanes of one
+// warp each add one accumulator's terms in sample order. Every f64 operation is a
 // round-to-nearest multiply, add or divide in the reference's order (this
 // file is compiled without floating-point contraction, and the sums use
 // the explicit _rn intrinsics).
@@ -35,9 +34,10 @@ namespace av1pf {
 namespace {
 
 constexpr int kB = 3;            // window border (postfilter.rs:744 LRB)
-constexpr int kThreads = 256;
-constexpr int kWienerChunk = 4;  // rows of Wiener terms handed from the producing warps to the adding lanes at a time
-constexpr int kWienerErrBand = 32;  // output rows per band of the Wiener error pass (its int16 rows fit the term region)
+constexpr int kStrip = 64;  // columns of a strip
+constexpr int kStripPx = kStrip * kMaxH;
+constexpr int kWienerThreads = 160;  // a warp that adds and four that produce
+constexpr int kWienerCols = 6;  // columns a producing lane has: units reach 256 + 127 columns, two warps a row
 __constant__ int32_t kSgrParams[16][4] = AV1T_SGR_PARAMS;
 __constant__ int32_t kWienerMin[3] = AV1T_WIENER_TAPS_MIN, kWienerMax[3] = AV1T_WIENER_TAPS_MAX;
 __constant__ int32_t kXqdMin[2] = AV1T_SGRPROJ_XQD_MIN, kXqdMax[2] = AV1T_SGRPROJ_XQD_MAX;
@@ -52,46 +52,52 @@ __device__ __forceinline__ int32_t f64_to_i32(double x) {
   return int32_t(x);
 }
 
-struct Win {
-  const int16_t* w;
-  int ws;  // row stride
-  __device__ __forceinline__ int at(int r, int c) const { return w[r * ws + c]; }
-};
+// The start of the plane row that window row r of a rectangle reads.
+__device__ __forceinline__ const uint8_t* search_row(const LrSearchFrame& F, int p, const LrSearchRect& rc, int r) {
+  const int y = max(min(rc.y0 + r - kB, F.pey[p]), 0);
+  const DPlane& pl = y < rc.ss || y > rc.se ? F.cur[p] : F.cdef[p];
+  const int yy = y < rc.ss ? max(rc.ss - 2, y) : (y > rc.se ? min(rc.se + 2, y) : y);
+  return pl.p + int64_t(yy) * pl.stride * F.sb;
+}
 
-// lr_window (postfilter.rs:765-777) of rectangle `rc` into shared memory.
-__device__ void stage_window(const LrSearchFrame& d, int p, const LrSearchRect& rc, int x0, int w, int16_t* win,
-                             int ws) {
-  // a warp per window row, lanes along it (no index division), eight rows'
-  // loads in flight before their stores
-  constexpr int kR = 8;
-  const int ww = w + 2 * kB, wh = rc.h + 2 * kB, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
-  const int pex = d.pex[p], pey = d.pey[p];
-  for (int r0 = threadIdx.x >> 5; r0 < wh; r0 += kR * nw) {
-    for (int c = lane; c < ww; c += 32) {
-      int v[kR];
-#pragma unroll
-      for (int m = 0; m < kR; m++) {
-        const int r = r0 + m * nw;
-        v[m] = 0;
-        if (r < wh) {
-          const int y = max(min(rc.y0 + r - kB, pey), 0);
-          const DPlane& pl = y < rc.ss || y > rc.se ? d.cur[p] : d.cdef[p];
-          const int yy = y < rc.ss ? max(rc.ss - 2, y) : (y > rc.se ? min(rc.se + 2, y) : y);
-          v[m] = ld(pl, d.sb, max(min(x0 + c - kB, pex), 0), yy);
-        }
+// The window of columns x .. x + w - 1 of a rectangle, by the whole CTA.
+__device__ __forceinline__ void stage_rect(const LrSearchFrame& F, int p, const LrSearchRect& rc, int x, int w, uint16_t* win,
+                                           int ws, const uint8_t** rows) {
+  for (int r = threadIdx.x; r < rc.h + 2 * kB; r += blockDim.x) rows[r] = search_row(F, p, rc, r);
+  __syncthreads();
+  stage_window(win, ws, rows, F.sb, F.pex[p], x, w, rc.h, Team{int(threadIdx.x), int(blockDim.x), 1});
+}
+
+// The source samples of a strip (columns x .. x + w - 1, rows y .. y + h - 1),
+// kStrip apart, eight at a time where they lie in an aligned row.
+__device__ __forceinline__ void stage_source(const LrSearchFrame& F, int p, int x, int w, int y, int h, uint16_t* out) {
+  const int64_t pitch = F.src[p].stride * F.sb;
+  const uint8_t* base = F.src[p].p + int64_t(y) * pitch + int64_t(x) * F.sb;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(base) | uintptr_t(pitch)) & uintptr_t(8 * F.sb - 1)) == 0;
+  for (int k = threadIdx.x; k < h * (kStrip / 8); k += blockDim.x) {
+    const int i = k / (kStrip / 8), j = (k % (kStrip / 8)) * 8;
+    if (j >= w) continue;
+    const uint8_t* row = base + int64_t(i) * pitch;
+    uint16_t* o = out + i * kStrip + j;
+    if (aligned && j + 8 <= w) {
+      uint4 v;
+      if (F.sb == 2) {
+        v = *reinterpret_cast<const uint4*>(row + j * 2);
+      } else {
+        const uint2 b = *reinterpret_cast<const uint2*>(row + j);
+        v = make_uint4(__byte_perm(b.x, 0, 0x4140), __byte_perm(b.x, 0, 0x4342), __byte_perm(b.y, 0, 0x4140),
+                       __byte_perm(b.y, 0, 0x4342));
       }
-#pragma unroll
-      for (int m = 0; m < kR; m++) {
-        const int r = r0 + m * nw;
-        if (r < wh) win[r * ws + c] = int16_t(v[m]);
-      }
+      *reinterpret_cast<uint4*>(o) = v;
+    } else {
+      for (int e = 0; e < 8 && j + e < w; e++) o[e] = uint16_t(ld_row(row, F.sb, j + e));
     }
   }
 }
 
 // Block sums of N 64-bit values in one round (every thread gets the totals).
 template <int N>
-__device__ void block_sums_i64(int64_t (&v)[N], int64_t (*red)[kThreads / 32]) {
+__device__ void block_sums_i64(int64_t (&v)[N], int64_t (*red)[kWienerThreads / 32]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
   for (int q = 0; q < N; q++) {
@@ -110,57 +116,81 @@ __device__ void block_sums_i64(int64_t (&v)[N], int64_t (*red)[kThreads / 32]) {
 
 // Gaussian elimination with partial pivoting (encoder/lr.rs:212-233): the
 // last row of largest magnitude is the pivot (Iterator::max_by); zeros when
-// singular.
+// singular. All in registers: rows are swapped by selection.
 template <int N>
-__device__ __noinline__ void solve(double (&m)[N][N], double (&v)[N], double (&x)[N]) {
+__device__ __forceinline__ void solve(double (&m)[N][N], double (&v)[N], double (&x)[N]) {
+#pragma unroll
   for (int i = 0; i < N; i++) {
     int piv = i;
-    for (int a = i + 1; a < N; a++)
-      if (!(fabs(m[a][i]) < fabs(m[piv][i]))) piv = a;
-    for (int c = 0; c < N; c++) {
-      const double t = m[i][c];
-      m[i][c] = m[piv][c];
-      m[piv][c] = t;
+    double most = fabs(m[i][i]);
+#pragma unroll
+    for (int a = i + 1; a < N; a++) {
+      const double mag = fabs(m[a][i]);
+      if (!(mag < most)) piv = a, most = mag;
     }
-    const double tv = v[i];
-    v[i] = v[piv];
-    v[piv] = tv;
+#pragma unroll
+    for (int a = i + 1; a < N; a++) {
+      const bool swap = piv == a;
+      auto exchange = [&](double& p, double& q) {
+        const double t = p;
+        p = swap ? q : p;
+        q = swap ? t : q;
+      };
+#pragma unroll
+      for (int c = 0; c < N; c++) exchange(m[i][c], m[a][c]);
+      exchange(v[i], v[a]);
+    }
     if (fabs(m[i][i]) < 1e-9) {
+#pragma unroll
       for (int k = 0; k < N; k++) x[k] = 0.0;
       return;
     }
+#pragma unroll
     for (int r = 0; r < N; r++) {
       if (r != i) {
         const double f = __ddiv_rn(m[r][i], m[i][i]);
+#pragma unroll
         for (int c = i; c < N; c++) m[r][c] = __dsub_rn(m[r][c], __dmul_rn(f, m[i][c]));
         v[r] = __dsub_rn(v[r], __dmul_rn(f, v[i]));
       }
     }
   }
+#pragma unroll
   for (int i = 0; i < N; i++) x[i] = __ddiv_rn(v[i], m[i][i]);
 }
 
-// The 7 samples of a Wiener line at (i, j) with the other direction's
-// filter applied first (encoder/lr.rs:265-285); the line's taps run along
-// columns (vertical) or rows.
-__device__ __forceinline__ void wiener_line(const Win& W, bool vertical, int i, int j, const double* other,
-                                            double (&line)[7]) {
-#pragma unroll
-  for (int t = 0; t < 7; t++) {
-    const int r = vertical ? i + t : i + kB, c = vertical ? j + kB : j + t;
-    const int center = W.at(r, c);
-    double s = double(center);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const int dd = 3 - k;
-      const int a = vertical ? W.at(r, c - dd) : W.at(r - dd, c);
-      const int b = vertical ? W.at(r, c + dd) : W.at(r + dd, c);
-      // a + b - 2 * center is an integer below 2^17: the f64 expression of
-      // encoder/lr.rs is exact, so integer arithmetic gives the same value
-      s = __dadd_rn(s, __dmul_rn(other[k], double(a + b - 2 * center)));
-    }
-    line[t] = s;
+// A Wiener pass's solution from its sums (m00 m01 m02 m11 m12 m22 v0 v1 v2);
+// chroma filters have no outermost tap.
+__device__ __noinline__ void wiener_solve(const double* t, bool luma, double* sol) {
+  if (luma) {
+    double m[3][3] = {{t[0], t[1], t[2]}, {t[1], t[3], t[4]}, {t[2], t[4], t[5]}}, v[3] = {t[6], t[7], t[8]}, x[3];
+    solve<3>(m, v, x);
+    sol[0] = x[0];
+    sol[1] = x[1];
+    sol[2] = x[2];
+  } else {
+    double m[2][2] = {{t[3], t[4]}, {t[4], t[5]}}, v[2] = {t[7], t[8]}, x[2];
+    solve<2>(m, v, x);
+    sol[0] = 0.0;
+    sol[1] = x[0];
+    sol[2] = x[1];
   }
+}
+
+// A sample with the other direction's filter applied (encoder/lr.rs:265-285):
+// `at` is the sample's place in the window, `step` the distance to its neighbour
+// along that direction.
+__device__ __forceinline__ double wiener_other(const uint16_t* at, int step, const double (&other)[3]) {
+  const int center = at[0];
+  double s = double(center);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int dd = (3 - k) * step;
+    // a + b - 2 * center is an integer below 2^17: the f64 expression of
+    // encoder/lr.rs is exact, so integer arithmetic gives the same value
+    s = __dadd_rn(s, __dmul_rn(other[k], double(at[-dd] + at[dd] - 2 * center)));
+  }
+  return s;
 }
 
 // The window of a rectangle, read from the planes: row r, column c.
@@ -239,334 +269,377 @@ __device__ int32_t sgr_flt_direct(const PlaneWin& W, int pass, const SgrPass& q,
 
 }  // namespace
 
-// Shared memory of the first-pass kernel (kind 0: the window) and of the Wiener
-// kernel (1: the window and the term rows).
-size_t lr_search_smem(int wmax, int hmax, int kind) {
-  const size_t ws = size_t(wmax + 2 * kB + 1) & ~size_t(1);
-  const size_t win = ((size_t(hmax + 2 * kB) * ws * 2) + 15) & ~size_t(15);
-  return kind == 0 ? win : win + size_t(2) * 4 * kWienerChunk * size_t(wmax + 1) * sizeof(double);
+namespace {
+// The Wiener kernel's shared memory: the window; the source samples of a unit
+// of one strip (64 columns of one stripe); the rows of samples filtered in the
+// other direction; and two buffers of the nine products, a product's chunk of fit
+// rows one after another (rows of a multiple of 8) and the products on different
+// banks for 16-byte loads. A chunk is two rows, of units of up to 32 columns four:
+// a column for each producing lane of a 64-column unit and of a 32-column one.
+__host__ __device__ constexpr int lr_window_stride(int wmax) { return (wmax + 2 * kB + 7) & ~7; }
+__host__ __device__ constexpr size_t lr_window_bytes(int wmax, int hmax) {
+  return size_t(((hmax + 3) & ~3) + 2 * kB) * lr_window_stride(wmax) * 2;  // (rows are walked in fours)
+}
+__host__ __device__ constexpr int wiener_cols(int w, int step) { return (w + step - 1) / step; }
+__host__ __device__ constexpr int wiener_row(int cols) { return (cols + 7) & ~7; }
+__host__ __device__ constexpr int wiener_chunk(int w) { return w > 32 ? 2 : 4; }
+// rows of a vertical pass's ring: a chunk's lines reach over (rows - 1) * step + 7
+// window rows, and the next chunk's rows * step more are written beside them
+__host__ __device__ constexpr int wiener_rows(int w, int step) { return w <= 32 && step == 2 ? 32 : 16; }
+__host__ __device__ constexpr int wiener_term(int wmax, int step) {
+  int n = 0;
+  for (int w = wmax < 32 ? wmax : 32; w <= wmax; w += wmax > w ? wmax - w : 1) {
+    const int k = wiener_chunk(w) * wiener_row(wiener_cols(w, step));
+    n = k > n ? k : n;
+  }
+  return n + ((2 - n) & 15);  // 2 mod 16 doubles: 4 mod 32 banks
+}
+__host__ __device__ constexpr int wiener_ring(int wmax, int step) {
+  int n = 0;
+  for (int w = wmax < 32 ? wmax : 32; w <= wmax; w += wmax > w ? wmax - w : 1) {
+    const int across = 2 * wiener_chunk(w) * (w + 2 * kB), down = wiener_rows(w, step) * wiener_cols(w, step);
+    n = across > n ? across : n;
+    n = down > n ? down : n;
+  }
+  return (n + 1) & ~1;
+}
+constexpr size_t kUnitSrc = size_t(kStripPx) * 2;
+}  // namespace
+
+size_t lr_search_smem(int wmax, int hmax, int step) {
+  return lr_window_bytes(wmax, hmax) + kUnitSrc +
+         sizeof(double) * (size_t(wiener_ring(wmax, step)) + size_t(2) * 9 * wiener_term(wmax, step));
 }
 
 namespace {
 
 // Window stride and the region after the window.
 struct Smem {
-  int16_t* win;
+  uint16_t* win;
   int ws;
   uint8_t* region;
 };
 __device__ __forceinline__ Smem smem_of(uint8_t* base, const LrSearchDesc& d) {
   Smem m;
-  m.ws = (d.wmax + 2 * kB + 1) & ~1;
-  m.win = reinterpret_cast<int16_t*>(base);
-  m.region = base + ((((size_t(d.hmax + 2 * kB) * m.ws * 2) + 15) & ~size_t(15)));
+  m.ws = lr_window_stride(d.wmax);
+  m.win = reinterpret_cast<uint16_t*>(base);
+  m.region = base + lr_window_bytes(d.wmax, d.hmax);
   return m;
 }
 
 }  // namespace
 
-// For units of several stripe rectangles, one CTA per unit (256 threads):
-// the error without a filter (encoder/lr.rs:134-146), and the first Wiener
-// pass (vertical, the other direction's filter still zero: its lines are
-// plain samples, so its sums are exact integer sums in any order) and its
-// solve. A one-rectangle unit's Wiener CTA does this itself, on the window
-// it keeps for its other passes.
-__global__ void __launch_bounds__(kThreads, 2) lr_search_prep_kernel(const LrSearchDesc d) {
-  extern __shared__ __align__(16) uint8_t lrs_smem[];
-  __shared__ int64_t red10[10][kThreads / 32];
-  const LrSearchJob job = d.jobs[blockIdx.x];
-  if (job.nr == 1) return;
-  const LrSearchFrame& F = d.frames[job.frame];
-  const int p = job.plane, x0 = job.x0, w = job.w, sb = F.sb, tid = threadIdx.x, step = d.step;
-  const Smem sm = smem_of(lrs_smem, d);
-  const Win W{sm.win, sm.ws};
-  const LrSearchRect* rects = d.rects + job.r0;
-  LrJobState& st = d.state[blockIdx.x];
-  int64_t acc = 0, m00 = 0, m01 = 0, m02 = 0, m11 = 0, m12 = 0, m22 = 0, v0 = 0, v1 = 0, v2 = 0;
-  const int nci = (w + step - 1) / step;
-  for (int ri = 0; ri < job.nr; ri++) {
-    const LrSearchRect rc = rects[ri];
-    __syncthreads();
-    stage_window(F, p, rc, x0, w, sm.win, sm.ws);
-    __syncthreads();
-    // no filter: the window's interior is the rectangle's CDEF output (its
-    // rows lie in its stripe, its columns in the plane)
-    for (int i = tid >> 5; i < rc.h; i += blockDim.x >> 5)
-      for (int j = tid & 31; j < w; j += 32) {
-        const int e = W.at(i + kB, j + kB) - ld(F.src[p], sb, x0 + j, rc.y0 + i);
-        acc += int64_t(e) * e;
-      }
-    const int nri = (rc.h + step - 1) / step;
-    for (int ii = tid >> 5; ii < nri; ii += blockDim.x >> 5)
-      for (int jj = tid & 31; jj < nci; jj += 32) {
-      const int i = ii * step, j = jj * step;
-      int ln[7];
+namespace {
+
+// The unfiltered error and the first Wiener pass (encoder/lr.rs:134-146; vertical,
+// the other direction's filter still zero: its lines are plain samples) over a
+// lane's two columns and rows i0 .. i0 + left - 1 of a rectangle, walked down the
+// window: `per` rows, a multiple of 4. sums: m00 m01 m02 m11 m12 m22 v0 v1 v2 and
+// the error, exact integers.
+template <class Source>
+__device__ __forceinline__ void wiener_first(const uint16_t* win, int ws, int i0, int per, int left, int cols, int step,
+                                             Source source, int64_t (&sums)[10]) {
+  const uint16_t* row = win + i0 * ws + kB;
+  auto next = [&]() {  // (columns c and c + 1 start at an odd one of the window)
+    const uint32_t v = uint32_t(row[0]) | (uint32_t(row[1]) << 16);
+    row += ws;
+    return v;
+  };
+  uint32_t t[10];
 #pragma unroll
-      for (int t = 0; t < 7; t++) ln[t] = W.at(i + t, j + kB);
-      const int64_t tg = ld(F.src[p], sb, x0 + j, rc.y0 + i) - ln[3];
-      const int64_t d0 = ln[0] + ln[6] - 2 * ln[3], d1 = ln[1] + ln[5] - 2 * ln[3], d2 = ln[2] + ln[4] - 2 * ln[3];
-      m00 += d0 * d0;
-      m01 += d0 * d1;
-      m02 += d0 * d2;
-      m11 += d1 * d1;
-      m12 += d1 * d2;
-      m22 += d2 * d2;
-      v0 += d0 * tg;
-      v1 += d1 * tg;
-      v2 += d2 * tg;
-      }
-  }
-  int64_t sums[10] = {m00, m01, m02, m11, m12, m22, v0, v1, v2, acc};
-  block_sums_i64(sums, red10);
-  double tot[9];
+  for (int k = 0; k < 6; k++) t[k] = next();
+#pragma unroll 1
+  for (int i = 0; i < per; i += 4) {
+    uint32_t src[4];
 #pragma unroll
-  for (int q = 0; q < 9; q++) tot[q] = double(sums[q]);
-  if (tid == 0) {
-    st.none = uint64_t(sums[9]);
-    double sol[3] = {0.0, 0.0, 0.0};
-    if (p == 0) {
-      double m[3][3] = {{tot[0], tot[1], tot[2]}, {tot[1], tot[3], tot[4]}, {tot[2], tot[4], tot[5]}};
-      double v[3] = {tot[6], tot[7], tot[8]};
-      solve<3>(m, v, sol);
-    } else {
-      double m[2][2] = {{tot[3], tot[4]}, {tot[4], tot[5]}}, v[2] = {tot[7], tot[8]}, x2[2];
-      solve<2>(m, v, x2);
-      sol[1] = x2[0];
-      sol[2] = x2[1];
+    for (int k = 0; k < 4; k++) {
+      src[k] = source(i0 + i + k);
+      t[6 + k] = next();
     }
-    for (int k = 0; k < 3; k++) st.vc[k] = sol[k];
+    int32_t part[10] = {};  // eight products below 2^26 each
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t s06 = t[k] + t[k + 6], s15 = t[k + 1] + t[k + 5], s24 = t[k + 2] + t[k + 4];  // no carry: below 2^13
+      auto add = [&](int c, int s, int a06, int a15, int a24, bool fit) {
+        const int e = s - c;
+        part[9] += e * e;
+        if (!fit) return;
+        const int d0 = a06 - 2 * c, d1 = a15 - 2 * c, d2 = a24 - 2 * c;
+        part[0] += d0 * d0;
+        part[1] += d0 * d1;
+        part[2] += d0 * d2;
+        part[3] += d1 * d1;
+        part[4] += d1 * d2;
+        part[5] += d2 * d2;
+        part[6] += d0 * e;
+        part[7] += d1 * e;
+        part[8] += d2 * e;
+      };
+      if (i + k < left) {
+        add(t[k + 3] & 0xffffu, src[k] & 0xffffu, s06 & 0xffffu, s15 & 0xffffu, s24 & 0xffffu, step == 1 || !(k & 1));
+        if (cols > 1) add(t[k + 3] >> 16, src[k] >> 16, s06 >> 16, s15 >> 16, s24 >> 16, step == 1);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 10; q++) sums[q] += part[q];
+#pragma unroll
+    for (int k = 0; k < 6; k++) t[k] = t[k + 4];
   }
 }
 
-// One CTA per unit (128 threads). For a one-rectangle unit, first the error
-// without a filter and the first Wiener pass and its solve, as the kernel
-// above does for the others. Then the second
-// (horizontal) and third (vertical) Wiener passes, whose terms are
-// real-valued, so each of their sums runs in the reference's sample order:
-// warps 1-3 produce four rows of terms into shared memory (two buffers)
-// while lane q of warp 0 adds accumulator q's terms (m00 m01 m02 m11 m12 m22
-// v0 v1 v2). Then the solves, the quantised coefficients
-// (encoder/lr.rs:316-327) and the filter's error.
-__global__ void __launch_bounds__(128, 4) lr_search_wiener_kernel(const LrSearchDesc d) {
+}  // namespace
+
+// One CTA per unit: the error without a filter and the first Wiener pass; then
+// the second (horizontal) and third (vertical) passes, whose terms are
+// real-valued, so each of their sums runs in the reference's sample order: warps
+// 1-4 produce two or four rows of products into shared memory (two buffers) while
+// lane q of warp 0 adds accumulator q's (m00 m01 m02 m11 m12 m22 v0 v1 v2). Then
+// the solves, the quantised coefficients (encoder/lr.rs:316-327) and the filter's
+// error.
+//
+// What bounds it is the chain of f64 additions, two for each sample of a unit, 8
+// cycles each: so the adding warp does nothing but read products, eight ahead,
+// and add; the producers apply the other direction's filter once for each sample
+// (not for each of the seven lines that it is on). The first pass and the filter's
+// error walk down the rows in registers, and a unit of one strip keeps its source
+// samples beside its window. 1080p 4:2:0: units of 64, 241 us -> 152 (of which the
+// chains alone are 40); units of 256, 1590 us -> 1330 (690).
+__global__ void __launch_bounds__(kWienerThreads, 4) lr_search_wiener_kernel(const LrSearchDesc d) {
   extern __shared__ __align__(16) uint8_t lrs_smem[];
-  __shared__ int64_t red[4];
-  __shared__ int64_t red10[10][kThreads / 32];
-  __shared__ double s_m[3][3], s_v[3], s_other[3], s_vc[3];
+  __shared__ int64_t red[kWienerThreads / 32];
+  __shared__ int64_t red10[10][kWienerThreads / 32];
+  __shared__ double s_sums[9], s_other[3], s_vc[3];
   __shared__ int s_coef[2][3];
+  __shared__ const uint8_t* s_rows[kMaxH + 6];
   const LrSearchJob job = d.jobs[blockIdx.x];
   const LrSearchFrame& F = d.frames[job.frame];
   const int p = job.plane, x0 = job.x0, w = job.w, sb = F.sb, tid = threadIdx.x, step = d.step;
   const int lane = tid & 31, warp = tid >> 5;
+  constexpr int nw = kWienerThreads / 32;
+  const bool unit = job.nr == 1 && w <= kStrip;  // one strip: its source and window are staged once
   const Smem sm = smem_of(lrs_smem, d);
-  const Win W{sm.win, sm.ws};
+  uint16_t* usrc = reinterpret_cast<uint16_t*>(sm.region);
   const LrSearchRect* rects = d.rects + job.r0;
   LrJobState& st = d.state[blockIdx.x];
   const int first = p == 0 ? 0 : 1;
-  const int bd = F.bd, maxv = (1 << bd) - 1;
-  const int nci = (w + step - 1) / step;
-  if (job.nr == 1) {  // the no-filter error and the first pass (CTA-uniform)
-    int64_t acc = 0, m00 = 0, m01 = 0, m02 = 0, m11 = 0, m12 = 0, m22 = 0, v0 = 0, v1 = 0, v2 = 0;
+  const int bd = F.bd;
+  const int nci = wiener_cols(w, step);
+  auto source = [&](const LrSearchRect& rc, int i, int j) {
+    return unit ? int(usrc[i * kStrip + j]) : ld(F.src[p], sb, x0 + j, rc.y0 + i);
+  };
+  // Each rectangle's columns in strips of 64, two a lane, its rows a warp's share
+  // of them (a multiple of 4): run(rc, x, win, i0, per, left, cols, pair), where
+  // pair(i) is a row's two source samples, clamped to the rectangle.
+  auto strips = [&](const LrSearchRect& rc, auto run) {
+    const int per = ((rc.h + nw - 1) / nw + 3) & ~3, i0 = warp * per;
+    if (i0 >= rc.h) return;
+    for (int x = 0; x < w; x += kStrip) {
+      const int c = x + 2 * lane, cols = min(w - c, 2), left = cols > 0 ? min(rc.h - i0, per) : 0;
+      run(sm.win + min(c, (w - 1) & ~1), i0, per, left, cols, [&](int i) {
+        i = min(i, rc.h - 1);
+        if (unit) return *reinterpret_cast<const uint32_t*>(usrc + i * kStrip + c);
+        const int c0 = min(c, w - 1), c1 = min(c + 1, w - 1);
+        return uint32_t(ld(F.src[p], sb, x0 + c0, rc.y0 + i)) | (uint32_t(ld(F.src[p], sb, x0 + c1, rc.y0 + i)) << 16);
+      });
+    }
+  };
+  {
+    int64_t sums[10] = {};
     for (int ri = 0; ri < job.nr; ri++) {
       const LrSearchRect rc = rects[ri];
       __syncthreads();
-      stage_window(F, p, rc, x0, w, sm.win, sm.ws);
+      stage_rect(F, p, rc, x0, w, sm.win, sm.ws, s_rows);
+      if (unit) stage_source(F, p, x0, w, rc.y0, rc.h, usrc);
       __syncthreads();
-      // no filter: the window's interior is the rectangle's CDEF output (its
-      // rows lie in its stripe, its columns in the plane)
-      for (int i = tid >> 5; i < rc.h; i += blockDim.x >> 5)
-        for (int j = tid & 31; j < w; j += 32) {
-          const int e = W.at(i + kB, j + kB) - ld(F.src[p], sb, x0 + j, rc.y0 + i);
-          acc += int64_t(e) * e;
-        }
-      const int nri = (rc.h + step - 1) / step;
-      for (int ii = tid >> 5; ii < nri; ii += blockDim.x >> 5)
-        for (int jj = tid & 31; jj < nci; jj += 32) {
-        const int i = ii * step, j = jj * step;
-        int ln[7];
-#pragma unroll
-        for (int t = 0; t < 7; t++) ln[t] = W.at(i + t, j + kB);
-        const int64_t tg = ld(F.src[p], sb, x0 + j, rc.y0 + i) - ln[3];
-        const int64_t d0 = ln[0] + ln[6] - 2 * ln[3], d1 = ln[1] + ln[5] - 2 * ln[3], d2 = ln[2] + ln[4] - 2 * ln[3];
-        m00 += d0 * d0;
-        m01 += d0 * d1;
-        m02 += d0 * d2;
-        m11 += d1 * d1;
-        m12 += d1 * d2;
-        m22 += d2 * d2;
-        v0 += d0 * tg;
-        v1 += d1 * tg;
-        v2 += d2 * tg;
-        }
+      strips(rc, [&](const uint16_t* win, int i0, int per, int left, int cols, auto pair) {
+        wiener_first(win, sm.ws, i0, per, left, cols, step, pair, sums);
+      });
     }
-    int64_t sums[10] = {m00, m01, m02, m11, m12, m22, v0, v1, v2, acc};
     block_sums_i64(sums, red10);
     if (tid == 0) {
       st.none = uint64_t(sums[9]);
-      double sol[3] = {0.0, 0.0, 0.0};
-      const double tot[9] = {double(sums[0]), double(sums[1]), double(sums[2]), double(sums[3]), double(sums[4]),
-                             double(sums[5]), double(sums[6]), double(sums[7]), double(sums[8])};
-      if (p == 0) {
-        double m[3][3] = {{tot[0], tot[1], tot[2]}, {tot[1], tot[3], tot[4]}, {tot[2], tot[4], tot[5]}};
-        double v[3] = {tot[6], tot[7], tot[8]};
-        solve<3>(m, v, sol);
-      } else {
-        double m[2][2] = {{tot[3], tot[4]}, {tot[4], tot[5]}}, v[2] = {tot[7], tot[8]}, x2[2];
-        solve<2>(m, v, x2);
-        sol[1] = x2[0];
-        sol[2] = x2[1];
-      }
-      for (int k = 0; k < 3; k++) s_vc[k] = sol[k];
+      double tot[9];
+#pragma unroll
+      for (int q = 0; q < 9; q++) tot[q] = double(sums[q]);
+      wiener_solve(tot, p == 0, s_vc);
     }
-  } else if (tid < 3) {
-    s_vc[tid] = st.vc[tid];  // from the kernel above
   }
   __syncthreads();
-  double vc[3] = {s_vc[0], s_vc[1], s_vc[2]}, hc[3] = {0.0, 0.0, 0.0};
-  const int qa = lane < 6 ? (lane < 3 ? 0 : (lane < 5 ? 1 : 2)) : lane - 6;
-  const int qb = lane < 6 ? (lane < 3 ? lane : (lane < 5 ? lane - 2 : 2)) : 3;  // 3: the target
-  const bool owner = warp == 0 && lane < 9 && qa >= first && (qb == 3 || qb >= first);
-  // [2 buffers][4 terms: d0 d1 d2 t][kWienerChunk rows][wmax + 1]: the odd
-  // row stride puts the four terms of a sample on different banks for the
-  // accumulating lanes
-  double* terms = reinterpret_cast<double*>(sm.region);
-  const int ts = d.wmax + 1, tq_stride = kWienerChunk * ts;
+  double hc[3] = {0.0, 0.0, 0.0};
+  const bool owner = warp == 0 && lane < 9 && (p == 0 || (lane >= 3 && lane != 6));
+  // [2 buffers][9 products][chunk rows][row8]
+  double* ring = reinterpret_cast<double*>(sm.region + kUnitSrc);
+  double* terms = ring + wiener_ring(d.wmax, step);
+  const int row8 = wiener_row(nci), tq_stride = wiener_term(d.wmax, step);
+  const int chunk = wiener_chunk(w), rmask = wiener_rows(w, step) - 1, across = w + 2 * kB;
+  // a producing lane's row of a chunk, and its columns: every pstep-th from pcol
+  const int prow = chunk == 4 ? warp - 1 : (warp - 1) >> 1;
+  const int pstep = chunk == 4 ? 32 : 64, pcol = chunk == 4 ? lane : ((warp - 1) & 1) * 32 + lane;
+  constexpr int kProducers = kWienerThreads - 32;
   for (int iter = 1; iter < 3; iter++) {
     const bool vertical = iter == 2;
-    if (tid < 3) s_other[tid] = vertical ? hc[tid] : vc[tid];
+    if (tid < 3) s_other[tid] = vertical ? hc[tid] : s_vc[tid];
     double macc = 0.0;
     for (int ri = 0; ri < job.nr; ri++) {
       const LrSearchRect rc = rects[ri];
       __syncthreads();
       // one rectangle: its window, staged for the first pass, stays in place
       // (the term rows and band rows lie outside it)
-      if (job.nr > 1) stage_window(F, p, rc, x0, w, sm.win, sm.ws);
+      if (job.nr > 1) stage_rect(F, p, rc, x0, w, sm.win, sm.ws, s_rows);
       __syncthreads();
-      const int nri = (rc.h + step - 1) / step, nch = (nri + kWienerChunk - 1) / kWienerChunk;
-      // chunks of rows in turn, two buffers: warps 1.. fill chunk c + 1 while
-      // warp 0 adds chunk c, row by row in sample order
+      const int nri = (rc.h + step - 1) / step, nch = (nri + chunk - 1) / chunk;
+      const double oth[3] = {s_other[0], s_other[1], s_other[2]};
+      // the samples of a chunk's lines, filtered in the other direction:
+      // horizontal lines take the fit rows' window columns, vertical ones the fit
+      // columns of the window rows from the chunk's first (the ring has those that
+      // the chunk before takes too)
+      auto filter = [&](int ch) {
+        if (vertical) {
+          const int hend = (min((ch + 1) * chunk, nri) - 1) * step + 7;
+          for (int r = (ch ? (ch * chunk - 1) * step + 7 : 0) + prow; r < hend; r += chunk)
+            for (int c = pcol; c < nci; c += pstep)
+              ring[(r & rmask) * nci + c] = wiener_other(&sm.win[r * sm.ws + c * step + kB], 1, oth);
+        } else if (ch * chunk + prow < nri) {
+          const uint16_t* row = sm.win + ((ch * chunk + prow) * step + kB) * sm.ws;
+          double* to = ring + ((ch & 1) * chunk + prow) * across;
+          for (int c = pcol; c < across; c += pstep) to[c] = wiener_other(row + c, sm.ws, oth);
+        }
+      };
+      if (warp > 0) {
+        filter(0);
+        asm volatile("bar.sync 1, %0;" ::"n"(kProducers) : "memory");
+      }
+      // chunks of rows in turn, two buffers: warps 1.. fill chunk c + 1 (and
+      // filter for chunk c + 2) while warp 0 adds chunk c, row by row in sample
+      // order
       for (int ch = 0; ch <= nch; ch++) {
         if (ch < nch && warp > 0) {
-          double* tb = terms + (ch & 1) * 4 * tq_stride;
-          const int rows = min(kWienerChunk, nri - ch * kWienerChunk);
-          const double oth[3] = {s_other[0], s_other[1], s_other[2]};
-          for (int k = tid - 32; k < rows * nci; k += blockDim.x - 32) {
-            const int r = k / nci, jj = k - r * nci;
-            const int i = (ch * kWienerChunk + r) * step, j = jj * step;
-            double line[7];
-            wiener_line(W, vertical, i, j, oth, line);
-            const double two3 = __dmul_rn(2.0, line[3]);
-            double* tr = tb + r * ts + jj;
-            tr[0 * tq_stride] = __dsub_rn(__dadd_rn(line[0], line[6]), two3);
-            tr[1 * tq_stride] = __dsub_rn(__dadd_rn(line[1], line[5]), two3);
-            tr[2 * tq_stride] = __dsub_rn(__dadd_rn(line[2], line[4]), two3);
-            tr[3 * tq_stride] = __dsub_rn(double(ld(F.src[p], sb, x0 + j, rc.y0 + i)), line[3]);
+          double* tr = terms + (ch & 1) * 9 * tq_stride + prow * row8;
+          const int i = (ch * chunk + prow) * step;
+          const bool row = ch * chunk + prow < nri;
+          int sv[kWienerCols];
+#pragma unroll
+          for (int u = 0; u < kWienerCols; u++) {
+            if (u * pstep >= nci) break;
+            const int c = pcol + u * pstep;
+            sv[u] = row && c < nci ? source(rc, i, c * step) : 0;
+          }
+          if (ch + 1 < nch) filter(ch + 1);
+          // the row's lines: sample q of column c's is tap[q][c * next]
+          const double* tap[7];
+#pragma unroll
+          for (int q = 0; q < 7; q++) tap[q] = ring + (vertical ? ((i + q) & rmask) * nci : ((ch & 1) * chunk + prow) * across + q);
+          const int next = vertical ? 1 : step;
+#pragma unroll
+          for (int u = 0; u < kWienerCols; u++) {
+            if (u * pstep >= row8) break;
+            const int c = pcol + u * pstep;
+            if (c >= row8) continue;
+            // past a row's end, and past the last row: products that add nothing
+            double d0 = 0.0, d1 = 0.0, d2 = 0.0, t = 0.0;
+            if (row && c < nci) {
+              double line[7];
+#pragma unroll
+              for (int q = 0; q < 7; q++) line[q] = tap[q][c * next];
+              const double two3 = __dmul_rn(2.0, line[3]);
+              d0 = __dsub_rn(__dadd_rn(line[0], line[6]), two3);
+              d1 = __dsub_rn(__dadd_rn(line[1], line[5]), two3);
+              d2 = __dsub_rn(__dadd_rn(line[2], line[4]), two3);
+              t = __dsub_rn(double(sv[u]), line[3]);
+            }
+            if (p == 0) {
+              tr[0 * tq_stride + c] = __dmul_rn(d0, d0);
+              tr[1 * tq_stride + c] = __dmul_rn(d0, d1);
+              tr[2 * tq_stride + c] = __dmul_rn(d0, d2);
+              tr[6 * tq_stride + c] = __dmul_rn(d0, t);
+            }
+            tr[3 * tq_stride + c] = __dmul_rn(d1, d1);
+            tr[4 * tq_stride + c] = __dmul_rn(d1, d2);
+            tr[5 * tq_stride + c] = __dmul_rn(d2, d2);
+            tr[7 * tq_stride + c] = __dmul_rn(d1, t);
+            tr[8 * tq_stride + c] = __dmul_rn(d2, t);
           }
         }
         if (ch > 0 && owner) {
-          const double* tb = terms + ((ch - 1) & 1) * 4 * tq_stride;
-          const int rows = min(kWienerChunk, nri - (ch - 1) * kWienerChunk);
-          for (int r = 0; r < rows; r++) {
-            const double* ta = tb + qa * tq_stride + r * ts;
-            const double* tq = tb + qb * tq_stride + r * ts;
-            // the products of 8 terms are independent of the sum: form them
-            // first, then add them one after another in sample order
-            int jj = 0;
-            for (; jj + 8 <= nci; jj += 8) {
-              double pr[8];
+          // the sum runs in sample order, eight products while the next eight are read
+          const int n = chunk * row8;  // a multiple of 16
+          const double2* tp = reinterpret_cast<const double2*>(terms + ((ch - 1) & 1) * 9 * tq_stride + lane * tq_stride);
+          double2 a[4], b[4];
+          auto load = [&](double2 (&q)[4]) {
 #pragma unroll
-              for (int u = 0; u < 8; u++) pr[u] = __dmul_rn(ta[jj + u], tq[jj + u]);
+            for (int u = 0; u < 4; u++) q[u] = tp[u];
+            tp += 4;
+          };
+          auto add = [&](const double2 (&q)[4]) {
 #pragma unroll
-              for (int u = 0; u < 8; u++) macc = __dadd_rn(macc, pr[u]);
-            }
-            for (; jj < nci; jj++) macc = __dadd_rn(macc, __dmul_rn(ta[jj], tq[jj]));
+            for (int u = 0; u < 4; u++) macc = __dadd_rn(__dadd_rn(macc, q[u].x), q[u].y);
+          };
+          load(a);
+#pragma unroll 1
+          for (int left = n; left > 16; left -= 16) {
+            load(b);
+            add(a);
+            load(a);
+            add(b);
           }
+          load(b);
+          add(a);
+          add(b);
         }
         __syncthreads();
       }
     }
-    if (owner) {
-      if (qb == 3)
-        s_v[qa] = macc;
-      else
-        s_m[qa][qb] = s_m[qb][qa] = macc;
-    }
+    if (owner) s_sums[lane] = macc;
     __syncthreads();
-    if (tid == 0) {
-      double sol[3] = {0.0, 0.0, 0.0};
-      if (first == 0) {
-        double m[3][3], v[3];
-        for (int a = 0; a < 3; a++) {
-          v[a] = s_v[a];
-          for (int b = 0; b < 3; b++) m[a][b] = s_m[a][b];
-        }
-        solve<3>(m, v, sol);
-      } else {
-        double m[2][2] = {{s_m[1][1], s_m[1][2]}, {s_m[2][1], s_m[2][2]}}, v[2] = {s_v[1], s_v[2]}, x2[2];
-        solve<2>(m, v, x2);
-        sol[1] = x2[0];
-        sol[2] = x2[1];
-      }
-      for (int k = 0; k < 3; k++) s_other[k] = sol[k];  // the pass's solution
-    }
+    if (tid == 0) wiener_solve(s_sums, p == 0, s_other);  // the pass's solution
     __syncthreads();
-    for (int k = 0; k < 3; k++) (vertical ? vc : hc)[k] = s_other[k];
+    if (vertical) {
+      if (tid < 3) s_vc[tid] = s_other[tid];
+    } else {
+      for (int k = 0; k < 3; k++) hc[k] = s_other[k];
+    }
     __syncthreads();
   }
-  if (tid == 0) {
-    for (int k = 0; k < 3; k++) {
-      s_coef[0][k] = k < first ? 0 : min(max(f64_to_i32(round(vc[k] * 128.0)), kWienerMin[k]), kWienerMax[k]);
-      s_coef[1][k] = k < first ? 0 : min(max(f64_to_i32(round(hc[k] * 128.0)), kWienerMin[k]), kWienerMax[k]);
-    }
+  if (tid < 3) {
+    const double vk = s_vc[tid], hk = tid == 0 ? hc[0] : tid == 1 ? hc[1] : hc[2];
+    s_coef[0][tid] = tid < first ? 0 : min(max(f64_to_i32(round(vk * 128.0)), kWienerMin[tid]), kWienerMax[tid]);
+    s_coef[1][tid] = tid < first ? 0 : min(max(f64_to_i32(round(hk * 128.0)), kWienerMin[tid]), kWienerMax[tid]);
   }
   __syncthreads();
   // the Wiener filter's error (postfilter.rs:781-822 restoration)
-  int vf[7], hf[7];
-  vf[3] = hf[3] = 128;
-  for (int k = 0; k < 3; k++) {
-    vf[k] = vf[6 - k] = s_coef[0][k];
-    hf[k] = hf[6 - k] = s_coef[1][k];
-    vf[3] -= 2 * s_coef[0][k];
-    hf[3] -= 2 * s_coef[1][k];
-  }
-  const int round0 = bd == 12 ? 5 : 3, round1 = bd == 12 ? 9 : 11;
-  const int off = 1 << (bd + 7 - round0 - 1), lim = (1 << (bd + 1 + 7 - round0)) - 1;
-  // separable: each band's horizontally filtered window rows go to the term
-  // region as int16 (clipped to [-off, lim - off], within [-2^13, 2^15)),
-  // then the vertical taps run over them
-  int16_t* hrow = reinterpret_cast<int16_t*>(sm.region);
-  const int nw = blockDim.x >> 5;
   int64_t acc = 0;
   for (int ri = 0; ri < job.nr; ri++) {
     const LrSearchRect rc = rects[ri];
-    __syncthreads();
-    if (job.nr > 1) stage_window(F, p, rc, x0, w, sm.win, sm.ws);  // else still staged
-    for (int i0 = 0; i0 < rc.h; i0 += kWienerErrBand) {
-      const int rows = min(kWienerErrBand, rc.h - i0);
-      __syncthreads();  // the window is staged; the previous band's rows are read
-      for (int r = warp; r < rows + 2 * kB; r += nw)
-        for (int j = lane; j < w; j += 32) {
-          int h = 0;
-#pragma unroll
-          for (int u = 0; u < 7; u++) h += hf[u] * W.at(i0 + r, j + u);
-          hrow[r * w + j] = int16_t(clip3(-off, lim - off, round2(h, round0)));
-        }
+    if (job.nr > 1) {  // else still staged
       __syncthreads();
-      for (int ir = warp; ir < rows; ir += nw)
-        for (int j = lane; j < w; j += 32) {
-          int sv = 0;
-#pragma unroll
-          for (int t = 0; t < 7; t++) sv += vf[t] * hrow[(ir + t) * w + j];
-          const int e = min(max(round2(sv, round1), 0), maxv) - ld(F.src[p], sb, x0 + j, rc.y0 + i0 + ir);
-          acc += int64_t(e) * e;
-        }
+      stage_rect(F, p, rc, x0, w, sm.win, sm.ws, s_rows);
+      __syncthreads();
     }
+    strips(rc, [&](const uint16_t* win, int i0, int per, int left, int cols, auto pair) {
+      uint32_t src[4], part = 0;  // (32 squares below 2^24)
+      wiener_walk(
+          win, sm.ws, i0, per, s_coef[0][0], s_coef[0][1], s_coef[0][2], s_coef[1][0], s_coef[1][1], s_coef[1][2], bd,
+          [&](int i) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) src[k] = pair(i0 + i + k);
+          },
+          [&](int i, uint32_t a, uint32_t b) {
+            if (i >= left) return;
+            const int ea = int(a) - int(src[i & 3] & 0xffffu), eb = int(b) - int(src[i & 3] >> 16);
+            part += uint32_t(ea * ea);
+            if (cols > 1) part += uint32_t(eb * eb);
+          });
+      acc += part;
+    });
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) red[warp] = acc;
   __syncthreads();
   if (tid == 0) {
-    st.wiener = uint64_t(red[0] + red[1] + red[2] + red[3]);
+    int64_t all = 0;
+    for (int q = 0; q < nw; q++) all += red[q];
+    st.wiener = uint64_t(all);
     for (int a = 0; a < 2; a++)
       for (int b = 0; b < 3; b++) st.coef[a][b] = s_coef[a][b];
   }
@@ -606,8 +679,6 @@ namespace {
 // The self-guided fits' shared memory: a strip's window, its source samples and
 // both filters' outputs less the sample (int16 pairs up to 10 bits, where they
 // stay below 2^15; else int32 pairs) of up to two sets.
-constexpr int kStrip = 64;
-constexpr int kStripPx = kStrip * kMaxH;
 constexpr int kSgrSrcOff = kWinBytes, kSgrCacheOff = kSgrSrcOff + kStripPx * 2;
 static_assert(kSgrSrcOff % 16 == 0, "vector access");
 
@@ -764,41 +835,6 @@ __device__ __noinline__ void sgr_weights(const LrSearchDesc& d, const LrSearchFr
   xqd[1] = x1q;
 }
 
-// The start of plane row y of window row `r` of a rectangle.
-__device__ __forceinline__ const uint8_t* search_row(const LrSearchFrame& F, int p, const LrSearchRect& rc, int r) {
-  const int y = max(min(rc.y0 + r - kB, F.pey[p]), 0);
-  const DPlane& pl = y < rc.ss || y > rc.se ? F.cur[p] : F.cdef[p];
-  const int yy = y < rc.ss ? max(rc.ss - 2, y) : (y > rc.se ? min(rc.se + 2, y) : y);
-  return pl.p + int64_t(yy) * pl.stride * F.sb;
-}
-
-// The source samples of a strip (columns x .. x + w - 1, rows y .. y + h - 1),
-// kStrip apart, eight at a time where they lie in an aligned row.
-__device__ __forceinline__ void stage_source(const LrSearchFrame& F, int p, int x, int w, int y, int h, uint16_t* out) {
-  const int64_t pitch = F.src[p].stride * F.sb;
-  const uint8_t* base = F.src[p].p + int64_t(y) * pitch + int64_t(x) * F.sb;
-  const bool aligned = ((reinterpret_cast<uintptr_t>(base) | uintptr_t(pitch)) & uintptr_t(8 * F.sb - 1)) == 0;
-  for (int k = threadIdx.x; k < h * (kStrip / 8); k += kLrThreads) {
-    const int i = k / (kStrip / 8), j = (k % (kStrip / 8)) * 8;
-    if (j >= w) continue;
-    const uint8_t* row = base + int64_t(i) * pitch;
-    uint16_t* o = out + i * kStrip + j;
-    if (aligned && j + 8 <= w) {
-      uint4 v;
-      if (F.sb == 2) {
-        v = *reinterpret_cast<const uint4*>(row + j * 2);
-      } else {
-        const uint2 b = *reinterpret_cast<const uint2*>(row + j);
-        v = make_uint4(__byte_perm(b.x, 0, 0x4140), __byte_perm(b.x, 0, 0x4342), __byte_perm(b.y, 0, 0x4140),
-                       __byte_perm(b.y, 0, 0x4342));
-      }
-      *reinterpret_cast<uint4*>(o) = v;
-    } else {
-      for (int e = 0; e < 8 && j + e < w; e++) o[e] = uint16_t(ld_row(row, F.sb, j + e));
-    }
-  }
-}
-
 }  // namespace
 
 // Phase 3, one CTA per unit and d.spc (1 or 2) parameter sets: the self-guided
@@ -833,7 +869,6 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_search_sgr_kernel(const LrSe
   const int slot = kStripPx * (deep ? 8 : 4);  // bytes of a set's kept outputs
   const bool single = job.nr == 1 && job.w <= kStrip;
   const bool halves = single && job.w <= kStrip / 2 && nk == 2;
-  const Team all{tid, kLrThreads, 1};
   if (tid < 2 * (kLrThreads / 32)) {
     sums[tid & 1][tid >> 1] = SgrSums{};
     s_err[tid & 1][tid >> 1] = 0;
@@ -858,9 +893,7 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_search_sgr_kernel(const LrSe
         const int k0 = half, k1 = halves ? half + 1 : nk;  // the sets of this half
         if (pass == 0 || !single) {
           __syncthreads();  // (everyone is done with the previous strip)
-          for (int r = tid; r < h + 6; r += kLrThreads) rows[r] = search_row(F, p, rc, r);
-          __syncthreads();
-          stage_window(win, g.ws, rows, F.sb, F.pex[p], job.x0 + x, w, h, all);
+          stage_rect(F, p, rc, job.x0 + x, w, win, g.ws, rows);
           stage_source(F, p, job.x0 + x, w, rc.y0, h, src);
           __syncthreads();
         }
@@ -963,7 +996,6 @@ cudaError_t lr_search_init() {
   int dev = 0, optin = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e == cudaSuccess) e = allow_max_smem(lr_search_prep_kernel, optin);
   if (e == cudaSuccess) e = allow_max_smem(lr_search_wiener_kernel, optin);
   if (e == cudaSuccess) e = allow_max_smem(lr_search_sgr_kernel, optin);
   return e;
@@ -972,19 +1004,17 @@ cudaError_t lr_search_init() {
 void launch_lr_search(const LrSearchDesc& d, int njobs, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                       cudaEvent_t join) {
   if (njobs <= 0) return;
-  const size_t s0 = lr_search_smem(d.wmax, d.hmax, 0);
-  const size_t s1 = lr_search_smem(d.wmax, d.hmax, 1);
+  const size_t s1 = lr_search_smem(d.wmax, d.hmax, d.step);
   const size_t s2 = size_t(kSgrCacheOff) + size_t(d.spc) * kStripPx * (d.deep ? 8 : 4);
   // the self-guided fits depend on nothing else: they run beside the Wiener passes
   cudaEventRecord(fork, s);
   cudaStreamWaitEvent(side, fork, 0);
+  lr_search_wiener_kernel<<<njobs, kWienerThreads, s1, s>>>(d);
   lr_search_sgr_kernel<<<njobs * ((d.nsets + d.spc - 1) / d.spc), kLrThreads, s2, side>>>(d);
-  if (d.multi_rect) lr_search_prep_kernel<<<njobs, kThreads, s0, s>>>(d);
-  lr_search_wiener_kernel<<<njobs, 128, s1, s>>>(d);
   cudaEventRecord(join, side);
   cudaStreamWaitEvent(s, join, 0);
   lr_search_choose_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(d, njobs);
-  note_launch(d.multi_rect ? 4 : 3);
+  note_launch(3);
 }
 
 }  // namespace av1pf

@@ -35,11 +35,12 @@ struct A2Table {
 };
 extern __device__ const A2Table g_sgr_a2;
 // The scale s of each self-guided parameter set's two filters, times 2^12
-// (postfilter.rs:903-918: ((1 << 20) + n^2 eps / 2) / (n^2 eps)), and 2^16 / n
-// rounded up, for quotients by 1 .. 9 of numbers below 2^12 without a division.
+// (postfilter.rs:903-918: ((1 << 20) + n^2 eps / 2) / (n^2 eps)), and 2^22 / n
+// rounded up, for quotients k / n of k < 2^22 / n without a division (chunks of
+// eight columns of a unit of up to 383, in 70 rows).
 struct LrConst {
   uint32_t s12[16][2];
-  int32_t inv[10];
+  uint32_t inv[50];
 };
 extern __constant__ LrConst c_lr;
 
@@ -109,8 +110,8 @@ __device__ __forceinline__ void window_rows(const LrSrc& src, const uint8_t** ro
 __device__ __forceinline__ void stage_window(uint16_t* win, int ws, const uint8_t* const* rows, int sb, int pex, int x0,
                                              int w, int h, const Team& tm) {
   const int ww = w + 6, wh = h + 6;
-  const int nq = (ww + 7) >> 3;  // chunks per window row (<= 9)
-  const int inv = c_lr.inv[nq];
+  const int nq = (ww + 7) >> 3;  // chunks per window row
+  const uint32_t inv = c_lr.inv[nq];
   const int ntask = wh * nq;
   constexpr int kBatch = 2;
 #pragma unroll 1
@@ -122,7 +123,7 @@ __device__ __forceinline__ void stage_window(uint16_t* win, int ws, const uint8_
       const int k = k0 + m * tm.n;
       vec[m] = false;
       if (k >= ntask) continue;
-      const int r = (k * inv) >> 16, q = k - r * nq;
+      const int r = int((uint32_t(k) * inv) >> 22), q = k - r * nq;
       const uint8_t* row = rows[r];
       const int gx = x0 - 8 + 8 * q;  // first sample of the left chunk
       if (gx < 0 || gx + 16 > pex + 1 || (reinterpret_cast<uintptr_t>(row) & 15) != 0) continue;
@@ -142,7 +143,7 @@ __device__ __forceinline__ void stage_window(uint16_t* win, int ws, const uint8_
     for (int m = 0; m < kBatch; m++) {
       const int k = k0 + m * tm.n;
       if (k >= ntask) continue;
-      const int r = (k * inv) >> 16, q = k - r * nq;
+      const int r = int((uint32_t(k) * inv) >> 22), q = k - r * nq;
       uint16_t* wp = &win[r * ws + 8 * q];
       if (vec[m]) {
         uint4 o;
@@ -171,6 +172,65 @@ __device__ __forceinline__ void stage_window(uint16_t* win, int ws, const uint8_
           if (c < ww) wp[e] = uint16_t(ld_row(row, sb, max(min(x0 - 3 + c, pex), 0)));
         }
       }
+    }
+  }
+}
+
+// Four 8-bit coefficients in a word.
+__device__ __forceinline__ int bytes4(int a, int b, int c, int d) {
+  return int((uint32_t(a) & 255u) | ((uint32_t(b) & 255u) << 8) | ((uint32_t(c) & 255u) << 16) | (uint32_t(d) << 24));
+}
+
+// The Wiener filter (postfilter.rs:795-822) with vertical taps v0 v1 v2 (and
+// the middle one that makes their sum 128) and horizontal ones h0 h1 h2: two
+// columns a lane, rows i0 .. i0 + per - 1, four a step (per is rounded up to
+// fours, and the window has those rows). `win` is window row 0 at the first
+// column. begin(i) is called before rows i .. i + 3 (from 0), emit(i, a, b) takes
+// row i's outputs.
+template <class Begin, class Emit>
+__device__ __forceinline__ void wiener_walk(const uint16_t* win, int ws, int i0, int per, int v0, int v1, int v2, int h0,
+                                            int h1, int h2, int bd, Begin begin, Emit emit) {
+  const int round0 = bd == 12 ? 5 : 3, round1 = bd == 12 ? 9 : 11;
+  const int offset = 1 << (bd + 7 - round0 - 1);
+  const int limit = (1 << (bd + 1 + 7 - round0)) - 1;
+  const int maxv = (1 << bd) - 1;
+  const int h3 = 128 - 2 * (h0 + h1 + h2), v3 = 128 - 2 * (v0 + v1 + v2);
+  // the taps but the middle one (which can exceed 8 bits) against the samples
+  // c .. c + 7, for the first column and the second
+  const int e0 = bytes4(h0, h1, h2, 0), e1 = bytes4(h2, h1, h0, 0);
+  const int o0 = bytes4(0, h0, h1, h2), o1 = bytes4(0, h2, h1, h0);
+  const int rnd0 = 1 << (round0 - 1), rnd1 = 1 << (round1 - 1);
+  const uint16_t* row = win + i0 * ws;
+  auto across = [&](int& a, int& b) {
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(row);
+    row += ws;
+    const int q0 = int(q[0]), q1 = int(q[1]), q2 = int(q[2]), q3 = int(q[3]);
+    int x = int(uint32_t(q1) >> 16) * h3 + rnd0, y = (q2 & 0xffff) * h3 + rnd0;
+    x = __dp2a_hi(q3, e1, __dp2a_lo(q2, e1, __dp2a_hi(q1, e0, __dp2a_lo(q0, e0, x))));
+    y = __dp2a_hi(q3, o1, __dp2a_lo(q2, o1, __dp2a_hi(q1, o0, __dp2a_lo(q0, o0, y))));
+    a = clip3(-offset, limit - offset, x >> round0);
+    b = clip3(-offset, limit - offset, y >> round0);
+  };
+  // the last six rows' results and four new ones a step
+  int a[10], b[10];
+#pragma unroll
+  for (int k = 0; k < 6; k++) across(a[k], b[k]);
+  auto down = [&](const int* t) {
+    const int acc = v0 * (t[0] + t[6]) + v1 * (t[1] + t[5]) + v2 * (t[2] + t[4]) + v3 * t[3] + rnd1;
+    return uint32_t(clip3(0, maxv, acc >> round1));
+  };
+#pragma unroll 1
+  for (int i = 0; i < per; i += 4) {
+    begin(i);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      across(a[6 + k], b[6 + k]);
+      emit(i + k, down(a + k), down(b + k));
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      a[k] = a[k + 4];
+      b[k] = b[k + 4];
     }
   }
 }

@@ -537,8 +537,6 @@ int av1pf_lr_search_many(av1pf_ctx* ctx, int n, av1pf_lr_search_job* jobs_in, in
   }
   std::vector<av1pf_lr_unit> chosen(jobs.size());
   if (!jobs.empty()) {
-    for (const LrSearchJob& jb : jobs)
-      if (jb.nr > 1) d.multi_rect = 1;
     for (const LrSearchFrame& f : frames)
       if (f.bd > 10) d.deep = 1;
     // Two sets a CTA share a unit's window and source, where that leaves four
