@@ -439,7 +439,7 @@ int av1pf_ctx_destroy(av1pf_ctx* ctx) {
       if (ev) cudaEventDestroy(ev);
   }
   if (ctx->upload) cudaStreamDestroy(ctx->upload);
-  for (auto* b : {&ctx->h_in, &ctx->h_ref, &ctx->h_maps, &ctx->h_frame, &ctx->search_dev, &ctx->search_planes})
+  for (auto* b : {&ctx->h_in, &ctx->h_ref, &ctx->h_maps, &ctx->h_frame, &ctx->search_dev})
     ctx->release(*b);
   if (ctx->search_host.ptr) cudaFreeHost(ctx->search_host.ptr);
   if (ctx->h_maps_stage.ptr) cudaFreeHost(ctx->h_maps_stage.ptr);

@@ -60,9 +60,9 @@ struct Ctx {
   DevBuf scratch;
   DevBuf h_in, h_ref, h_maps, h_frame;  // av1pf_chain_host
   HostBuf h_maps_stage;                  // its small maps, packed for one upload
-  // encoder searches: descriptors, error tables and greedy state; the
-  // loop-filter search's filtered copies; pinned staging of both
-  DevBuf search_dev, search_planes;
+  // encoder searches: descriptors, error tables and greedy state, and their
+  // pinned staging
+  DevBuf search_dev;
   HostBuf search_host;
   // av1pf_chain_host_many: device frame slots used in turn (`threads` of
   // them), with the events that order a slot's upload (pipe_up), chain

@@ -132,6 +132,17 @@ struct CdefSearchDesc {
   int32_t block0, table0;  // first CTA in the table kernel, first entry in the finish kernel
 };
 
+// One frame of the encoder's loop-filter level search (encoder/mod.rs:1457-1506).
+constexpr int kLfScales = 6;
+struct LfSearchDesc {
+  FrameDesc f;                   // the reconstruction (in), its maps and level deltas
+  DPlane src[3];                 // the source; w x h the frame area
+  int32_t levels[kLfScales][4];  // the frame's levels at each scale
+  uint32_t filtered[3];          // bit s: scale s filters the plane
+  int32_t tiles_x[3], tile0[3];  // 64x64 tiles a row of the frame area; the plane's first tile in the launch
+  uint64_t* sse;                 // [scale][plane]
+};
+
 // The encoder's loop-restoration search (encoder/lr.rs:64-430): one job
 // per restoration unit, its stripe rectangles, and the chosen filter.
 struct LrSearchJob {

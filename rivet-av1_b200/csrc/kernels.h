@@ -163,16 +163,9 @@ void launch_cdef_greedy(const CdefSearchDesc* ds, int n, int ny, int nuv, int nf
 void launch_sse_transpose(const CdefSearchDesc* ds, int n, int nfb_max, int nc, cudaStream_t s);
 // Sets the cluster kernel's dynamic shared-memory limit on the current device.
 cudaError_t search_init();
-// Squared error of planes against the source over each plane's frame area:
-// sse[i] += sum over plane job i (a, b: plane pointers and strides; `jobs`
-// in device memory, at most 65535).
-struct SsePlane {
-  const uint8_t* a;
-  const uint8_t* b;
-  int64_t sa, sb_;  // strides in samples
-  int32_t w, h;
-  int32_t sb;       // bytes per sample
-};
+// The loop-filter level search (lf.cu): the errors of every (frame, scale,
+// plane), added to each frame's sse. `tiles`: 64x64 tiles over all frames.
+void launch_lf_search(const LfSearchDesc* ds, int n, int tiles, cudaStream_t s);
 // The loop-restoration search (lr_search.cu): per unit job, the no-filter
 // error and the Wiener passes on `s`, the self-guided fits (one CTA per job
 // and d.spc sets) on `side` beside them, then the choice.
@@ -181,7 +174,6 @@ struct SsePlane {
 cudaError_t lr_search_init();
 void launch_lr_search(const LrSearchDesc& d, int njobs, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                       cudaEvent_t join);
-void launch_plane_sse(const SsePlane* jobs, int n, int rows_max, uint64_t* sse, cudaStream_t s);
 
 // Super-resolution (superres.cu)
 // `row_max`: the most source samples in a row among the launch's frames.

@@ -605,6 +605,238 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
   AV1PF_TRACE_END(1);
 }
 
+// The loop-filter level search (encoder/mod.rs:1457-1506): the squared error
+// against the source of one 64x64 tile of the frame area, unfiltered or
+// filtered by both passes at each of a group's scales (scales g, g + groups,
+// ...; one CTA a tile and group). The window, the edges, their filter sizes
+// and every scale's levels are staged and worked out once; a scale then
+// restores the window, filters it as lf_fused_kernel does and adds up the
+// tile's errors, so no filtered plane is ever written. A thread restores and
+// scores the same 8-sample chunks, so those steps need no barrier between
+// them. 256 threads.
+__global__ void __launch_bounds__(256, 4) lf_search_kernel(const LfSearchDesc* __restrict__ ds, int n, int groups) {
+  const LfTables& tb = g_lf_tables;
+  __shared__ __align__(16) uint16_t W0[kFW * kFS], W[kFW * kFS], S[kFT * kFT];
+  __shared__ uint16_t list_v[kFCells], list_h[kFCells];
+  __shared__ uint8_t lv_v[kLfScales][kFCells], lv_h[kLfScales][kFCells];
+  __shared__ uint32_t cnt[2][4], base[2][4];
+  __shared__ unsigned long long s_sum[kLfScales];
+  const int tid = threadIdx.x;
+  const int tile = int(blockIdx.x) / groups, grp = int(blockIdx.x) - tile * groups;
+  int lo = 0;
+  for (int hi = n; hi - lo > 1;) {  // the frame: the last whose first tile is not past this one
+    const int mid = (lo + hi) >> 1;
+    if (ds[mid].tile0[0] <= tile)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  const LfSearchDesc& d = ds[lo];
+  const FrameDesc& f = d.f;
+  const int plane = f.np == 1 || tile < d.tile0[1] ? 0 : (tile < d.tile0[2] ? 1 : 2);
+  const int at = tile - d.tile0[plane], tx = d.tiles_x[plane];
+  const int y0 = at / tx * kFT, x0 = at % tx * kFT;
+  const DPlane cur = f.in[plane], src = d.src[plane];
+  const int sb = f.sb;
+  const int rows = min(kFT, src.h - y0), cols = min(kFT, src.w - x0);
+  uint32_t filtered = 0;  // this group's scales that filter the plane
+  for (int s = grp; s < kLfScales; s += groups) filtered |= d.filtered[plane] & (1u << s);
+  const bool filt = filtered != 0;
+  if (tid < 8) (&cnt[0][0])[tid] = 0u;
+  if (tid < kLfScales) s_sum[tid] = 0u;
+  __syncthreads();
+  // --- stage this thread's chunks of the window and, inside the tile, of the source ---
+  uint2 q8[4], p8[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    const int k = tid + m * 256;
+    const int r = k / 10, ch = k - r * 10;
+    q8[m] = p8[m] = make_uint2(0u, 0u);
+    if (k >= kFChunks) continue;
+    const int ty = r - kFH, txo = (ch - 1) * 8;
+    const bool own = ty >= 0 && ty < rows && txo >= 0 && txo < cols;
+    if (!filt && !own) continue;
+    const int gy = y0 + ty, gx = x0 + txo;
+    uint16_t* wp = &W0[r * kFS + ch * 8];
+    if (gy < 0 || gy >= cur.h) {
+      *reinterpret_cast<uint4*>(wp) = make_uint4(0u, 0u, 0u, 0u);
+      continue;
+    }
+    const uint8_t* rp = cur.p + int64_t(gy) * cur.stride * sb;
+    if (gx >= 0 && gx + 8 <= cur.w) {
+      if (sb == 2)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(wp)), "l"(rp + int64_t(gx) * 2)
+                     : "memory");
+      else
+        q8[m] = *reinterpret_cast<const uint2*>(rp + gx);
+    } else {
+      for (int e = 0; e < 8; e++) {
+        const int x = gx + e;
+        wp[e] = (x >= 0 && x < cur.w) ? uint16_t(sb == 1 ? rp[x] : reinterpret_cast<const uint16_t*>(rp)[x]) : 0;
+      }
+    }
+    if (!own) continue;
+    uint16_t* sp = &S[ty * kFT + txo];
+    const uint8_t* srp = src.p + int64_t(gy) * src.stride * sb;
+    if (txo + 8 <= cols) {
+      if (sb == 2)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(sp)), "l"(srp + int64_t(gx) * 2)
+                     : "memory");
+      else
+        p8[m] = *reinterpret_cast<const uint2*>(srp + gx);
+    } else {
+      for (int e = 0; e < cols - txo; e++)
+        sp[e] = uint16_t(sb == 1 ? srp[gx + e] : reinterpret_cast<const uint16_t*>(srp)[gx + e]);
+    }
+  }
+  if (filt) {
+    // --- the edges, as lf_fused_kernel decides them, grouped by filter size ---
+    const int sx = plane_ssx(f, plane), sy = plane_ssy(f, plane);
+    const int gw = f.mi_cols >> sx, gh = f.mi_rows >> sy;
+    const int cx0 = x0 >> 2, cy0 = (y0 >> 2) - 2;
+    int cv[2], chh[2], row[2], col[2];
+    uint2 raw[2];
+    uint32_t iv[2], ih[2];
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      const int k = tid + m * 256;
+      const int i = k / kFCC, j = k - i * kFCC;
+      const int cx = cx0 + j, cy = cy0 + i;
+      cv[m] = chh[m] = row[m] = col[m] = 0;
+      raw[m] = make_uint2(0u, 0u);
+      if (k < kFCells && cy >= 0 && cx < gw && cy < gh)
+        lf_edges2(f, tb, plane, cx, cy, cv[m], chh[m], raw[m], row[m], col[m]);
+      if (!(i >= 2 && i <= 2 + kFT / 4 && j < kFT / 4)) chh[m] = 0;
+    }
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      iv[m] = cv[m] ? atomicAdd(&cnt[0][cv[m]], 1u) : 0u;
+      ih[m] = chh[m] ? atomicAdd(&cnt[1][chh[m]], 1u) : 0u;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      uint32_t run = 0;
+      for (int c = 3; c >= 1; c--) {
+        base[tid][c] = run;
+        run += cnt[tid][c];
+      }
+      cnt[tid][0] = run;  // the pass's edge count
+    }
+    __syncthreads();
+    // an edge's place and its level at each scale
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      const int k = tid + m * 256;
+      const int i = k / kFCC, j = k - i * kFCC;
+#pragma unroll
+      for (int pass = 0; pass < 2; pass++) {
+        const int c = pass ? chh[m] : cv[m];
+        if (!c) continue;
+        const uint32_t e = base[pass][c] + (pass ? ih[m] : iv[m]);
+        (pass ? list_h : list_v)[e] = uint16_t(j | ((pass ? i - 2 : i) << 5) | (c << 10));
+        const int li = plane == 0 ? pass : plane + 1;
+        const int first = pass ? (cy0 + i) * 4 : (cx0 + j) * 4;  // of q0, across the edge
+        // a conformant map keeps wide edges off the plane start
+        const bool bad = first < (c == 3 ? 8 : 4);
+        for (int s = grp; s < kLfScales; s += groups) {
+          int lvl = 0;
+          if (filtered >> s & 1u) {
+            lvl = lf_level_from(f, raw[m], li, d.levels[s][li]);
+            if (lvl == 0) {
+              const int nr = pass ? row[m] - (1 << sy) : row[m], nc = pass ? col[m] : col[m] - (1 << sx);
+              lvl = lf_level_from(f, *reinterpret_cast<const uint2*>(f.mi + int64_t(nr) * f.mi_stride + nc), li,
+                                  d.levels[s][li]);
+            }
+            if (lvl && bad) {
+              atomicOr(&g_error_flags, ERRF_BAD_MAP);
+              lvl = 0;
+            }
+          }
+          (pass ? lv_h : lv_v)[s][e] = uint8_t(lvl);
+        }
+      }
+    }
+  }
+  // u8 samples widen to 16 bits
+  auto widen = [](uint2 q) {
+    return make_uint4(__byte_perm(q.x, 0, 0x4140), __byte_perm(q.x, 0, 0x4342), __byte_perm(q.y, 0, 0x4140),
+                      __byte_perm(q.y, 0, 0x4342));
+  };
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    const int k = tid + m * 256;
+    const int r = k / 10, ch = k - r * 10;
+    if (sb != 1 || k >= kFChunks) continue;
+    const int ty = r - kFH, txo = (ch - 1) * 8;
+    const bool own = ty >= 0 && ty < rows && txo >= 0 && txo < cols;
+    const int gy = y0 + ty, gx = x0 + txo;
+    if ((!filt && !own) || gy < 0 || gy >= cur.h) continue;
+    if (gx >= 0 && gx + 8 <= cur.w) *reinterpret_cast<uint4*>(&W0[r * kFS + ch * 8]) = widen(q8[m]);
+    if (own && txo + 8 <= cols) *reinterpret_cast<uint4*>(&S[ty * kFT + txo]) = widen(p8[m]);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  const int bd = f.bd, sharp = f.sharpness;
+  const bool chroma = plane != 0;
+  for (int s = grp; s < kLfScales; s += groups) {
+    const bool on = filtered >> s & 1u;
+    if (on) {
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        const int k = tid + m * 256;
+        const int r = k / 10, o = r * kFS + (k - r * 10) * 8;
+        if (k < kFChunks) *reinterpret_cast<uint4*>(&W[o]) = *reinterpret_cast<const uint4*>(&W0[o]);
+      }
+      __syncthreads();
+      const int nv = int(cnt[0][0]) * 4;
+      for (int t = tid; t < nv; t += 256) {
+        const int e = list_v[t >> 2], lvl = lv_v[s][t >> 2];
+        if (lvl)
+          lf_filter_smem(&W[(((e >> 5) & 31) * 4 + (t & 3)) * kFS + kFH + (e & 31) * 4], 1, e >> 10, chroma, bd, lvl,
+                         sharp);
+      }
+      __syncthreads();
+      const int nh = int(cnt[1][0]) * 4;
+      for (int t = tid; t < nh; t += 256) {
+        const int e = list_h[t >> 2], lvl = lv_h[s][t >> 2];
+        if (lvl)
+          lf_filter_smem(&W[(kFH + ((e >> 5) & 31) * 4) * kFS + kFH + (e & 31) * 4 + (t & 3)], kFS, e >> 10, chroma,
+                         bd, lvl, sharp);
+      }
+      __syncthreads();
+    }
+    // at most 16 samples a thread, squares below 2^24: the sum fits 32 bits
+    uint32_t acc = 0;
+    const uint16_t* P = on ? W : W0;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int k = tid + m * 256;
+      const int r = k / 10, ch = k - r * 10;
+      const int ty = r - kFH, txo = (ch - 1) * 8;
+      if (k >= kFChunks || ty < 0 || ty >= rows || txo < 0 || txo >= cols) continue;
+      const uint16_t *wp = &P[r * kFS + ch * 8], *sp = &S[ty * kFT + txo];
+      if (txo + 8 <= cols) {
+        const uint4 a = *reinterpret_cast<const uint4*>(wp), b = *reinterpret_cast<const uint4*>(sp);
+        const uint32_t dw[4] = {a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {  // both differences from one subtraction: hi * 2^16 + lo
+          const int l = int16_t(dw[e]), h = (int(dw[e]) - l) >> 16;
+          acc += uint32_t(l * l) + uint32_t(h * h);
+        }
+      } else {
+        for (int e = 0; e < cols - txo; e++) {
+          const int l = int(wp[e]) - int(sp[e]);
+          acc += uint32_t(l * l);
+        }
+      }
+    }
+    const uint32_t l16 = __reduce_add_sync(~0u, acc & 0xffffu), h16 = __reduce_add_sync(~0u, acc >> 16);
+    if ((tid & 31) == 0) atomicAdd(&s_sum[s], (static_cast<unsigned long long>(h16) << 16) + l16);
+  }
+  __syncthreads();
+  if (tid < kLfScales && s_sum[tid])
+    atomicAdd(reinterpret_cast<unsigned long long*>(&d.sse[tid * 3 + plane]), s_sum[tid]);
+}
+
 // dsp::lf::filter (lf.rs:25) on independent edges: one thread per lane.
 __global__ void dsp_lf_kernel(int32_t* __restrict__ edges, const av1pf_lf_edge_params* __restrict__ prm, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -641,6 +873,18 @@ void launch_lf_fused(const FrameSet& frames, const Item* items, int n_items, Syn
   if (n_items <= 0) return;
   launch_frames(frames, lf_fused_kernel<NoFrame>, lf_fused_kernel<OneFrame>, min(n_items, kItemGrid), 256, 0, s,
                 items, n_items, flags);
+}
+
+void launch_lf_search(const LfSearchDesc* ds, int n, int tiles, cudaStream_t s) {
+  if (n <= 0 || tiles <= 0) return;
+  // Every group stages the window and decides the edges again, so one group
+  // where the tiles fill the GPU; half a wave of them or less (4 CTAs a SM) is
+  // split. us a call with 1 / 3 / 6 groups: 640x360 (90 tiles) 55 / 42 / 34,
+  // 1280x720 (360) 59 / 58 / 68, 1920x1080 (780) 93 / 94 / 117, 3840x2160
+  // (3060) 231 / 299 / 377.
+  const int groups = tiles <= kNumSMs ? 6 : (tiles <= 2 * kNumSMs ? 3 : 1);
+  lf_search_kernel<<<tiles * groups, 256, 0, s>>>(ds, n, groups);
+  note_launch();
 }
 
 void launch_lf_edges(int pass, const FrameDesc* frames, const uint64_t* list, const uint32_t* count, uint32_t cap,

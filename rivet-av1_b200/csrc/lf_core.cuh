@@ -12,16 +12,16 @@
 namespace av1pf {
 
 // 7.14.4-5 filter_strength (postfilter.rs:207-246): the level of one 4x4
-// from its mode-info words.
-__device__ __forceinline__ int lf_level_raw(const FrameDesc& f, uint2 raw, int plane, int pass) {
+// from its mode-info words, where the frame's level i (0, 1 luma's passes,
+// 2, 3 chroma) is `base`.
+__device__ __forceinline__ int lf_level_from(const FrameDesc& f, uint2 raw, int i, int base) {
   const int mi_segment = int((raw.x >> 24) & 7u);
   const int rf = int(int8_t((raw.x >> 16) & 0xffu));
   const int mode = int((raw.x >> 8) & 0xffu);
   const int mode_type = (mode >= 14 && mode != 16 && mode != 24) ? 1 : 0;  // NEARESTMV.., !GLOBALMV, !GLOBAL_GLOBALMV
-  const int i = plane == 0 ? pass : plane + 1;
   const int didx = f.delta_lf_multi ? i : 0;
   const int delta_lf = int(int8_t((raw.y >> (8 * didx)) & 0xffu));
-  int lvl = clip3(0, 63, delta_lf + f.lf_level[i]);
+  int lvl = clip3(0, 63, delta_lf + base);
   if (f.seg_enabled && f.seg_lf_on[mi_segment][i]) lvl = clip3(0, 63, f.seg_lf_data[mi_segment][i] + lvl);
   if (f.delta_enabled) {
     const int n_shift = lvl >> 5;
@@ -33,6 +33,11 @@ __device__ __forceinline__ int lf_level_raw(const FrameDesc& f, uint2 raw, int p
     lvl = clip3(0, 63, lvl);
   }
   return lvl;
+}
+
+__device__ __forceinline__ int lf_level_raw(const FrameDesc& f, uint2 raw, int plane, int pass) {
+  const int i = plane == 0 ? pass : plane + 1;
+  return lf_level_from(f, raw, i, f.lf_level[i]);
 }
 
 __device__ __forceinline__ int lf_level(const FrameDesc& f, int row, int col, int plane, int pass) {
@@ -84,16 +89,17 @@ constexpr LfTables make_lf_tables() {
 extern __device__ const LfTables g_lf_tables;  // lf.cu
 
 // edge_loop_filter's decisions (postfilter.rs:107-172) for the 4x4 at plane
-// position (cx, cy), both passes: 0 = not filtered, else (size code << 6) |
-// lvl with size code 1 = 4, 2 = 8, 3 = 16. Block and transform sizes are
-// powers of two, so the edge tests are masks. The mode-info word and the
-// three transform sizes (this 4x4, its left and upper neighbours) are all
-// loaded before any is used.
-__device__ __forceinline__ void lf_decide2(const FrameDesc& f, const LfTables& tb, int plane, int cx, int cy,
-                                           int& dv, int& dh) {
-  dv = dh = 0;
+// position (cx, cy), both passes, up to the level: cv, ch = 0 where there is
+// no edge to filter, else its size code, 1 = 4, 2 = 8, 3 = 16; with the 4x4's
+// mode-info word and place. Block and transform sizes are powers of two, so
+// the edge tests are masks. The mode-info word and the three transform sizes
+// (this 4x4, its left and upper neighbours) are all loaded before any is used.
+__device__ __forceinline__ void lf_edges2(const FrameDesc& f, const LfTables& tb, int plane, int cx, int cy,
+                                          int& cv, int& ch, uint2& raw, int& row, int& col) {
+  cv = ch = 0;
   const int sx = plane_ssx(f, plane), sy = plane_ssy(f, plane);
-  int row = cy << sy, col = cx << sx;
+  row = cy << sy;
+  col = cx << sx;
   const int x = col * 4, y = row * 4;
   if (x >= f.fw || y >= f.fh) return;
   const int xp = x >> sx, yp = y >> sy;
@@ -102,7 +108,7 @@ __device__ __forceinline__ void lf_decide2(const FrameDesc& f, const LfTables& t
   const int ms = f.mi_stride;
   const uint8_t* txm = f.tx[plane];
   const bool has_v = x != 0, has_h = y != 0;
-  const uint2 raw = *reinterpret_cast<const uint2*>(f.mi + int64_t(row) * ms + col);
+  raw = *reinterpret_cast<const uint2*>(f.mi + int64_t(row) * ms + col);
   const int tx_sz = txm[int64_t(row >> sy) * ms + (col >> sx)];
   const int tx_v = has_v ? txm[int64_t(row >> sy) * ms + ((col - (1 << sx)) >> sx)] : 0;
   const int tx_h = has_h ? txm[int64_t((row - (1 << sy)) >> sy) * ms + (col >> sx)] : 0;
@@ -124,9 +130,7 @@ __device__ __forceinline__ void lf_decide2(const FrameDesc& f, const LfTables& t
     const bool is_tx_edge = (xp & ((1 << tb.txw_log2[tx_sz]) - 1)) == 0;
     if (is_tx_edge && (is_block_edge || !skip || is_intra)) {
       const int size = min(cap, min(int(tb.txw[tx_v]), int(tb.txw[tx_sz])));
-      int lvl = lf_level_raw(f, raw, plane, 0);
-      if (lvl == 0) lvl = lf_level(f, row, col - (1 << sx), plane, 0);
-      if (lvl) dv = ((size >= 16 ? 3 : (size >= 8 ? 2 : 1)) << 6) | lvl;
+      cv = size >= 16 ? 3 : (size >= 8 ? 2 : 1);
     }
   }
   if (has_h) {
@@ -134,10 +138,28 @@ __device__ __forceinline__ void lf_decide2(const FrameDesc& f, const LfTables& t
     const bool is_tx_edge = (yp & ((1 << tb.txh_log2[tx_sz]) - 1)) == 0;
     if (is_tx_edge && (is_block_edge || !skip || is_intra)) {
       const int size = min(cap, min(int(tb.txh[tx_h]), int(tb.txh[tx_sz])));
-      int lvl = lf_level_raw(f, raw, plane, 1);
-      if (lvl == 0) lvl = lf_level(f, row - (1 << sy), col, plane, 1);
-      if (lvl) dh = ((size >= 16 ? 3 : (size >= 8 ? 2 : 1)) << 6) | lvl;
+      ch = size >= 16 ? 3 : (size >= 8 ? 2 : 1);
     }
+  }
+}
+
+// The same with the level: 0 = not filtered, else (size code << 6) | lvl. An
+// edge's level is its 4x4's, or, where that is 0, the one's on its other side.
+__device__ __forceinline__ void lf_decide2(const FrameDesc& f, const LfTables& tb, int plane, int cx, int cy,
+                                           int& dv, int& dh) {
+  int cv, ch, row, col;
+  uint2 raw;
+  dv = dh = 0;
+  lf_edges2(f, tb, plane, cx, cy, cv, ch, raw, row, col);
+  if (cv) {
+    int lvl = lf_level_raw(f, raw, plane, 0);
+    if (lvl == 0) lvl = lf_level(f, row, col - (1 << plane_ssx(f, plane)), plane, 0);
+    if (lvl) dv = (cv << 6) | lvl;
+  }
+  if (ch) {
+    int lvl = lf_level_raw(f, raw, plane, 1);
+    if (lvl == 0) lvl = lf_level(f, row - (1 << plane_ssy(f, plane)), col, plane, 1);
+    if (lvl) dh = (ch << 6) | lvl;
   }
 }
 

@@ -297,15 +297,8 @@ int av1pf_lf_search_many(av1pf_ctx* ctx, int n, av1pf_lf_search_job* jobs, void*
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   std::string why;
   // the six scales of the starting levels (encoder/mod.rs:1470-1472)
-  static const double kScales[6] = {0.0, 0.5, 0.75, 1.0, 1.25, 1.5};
-  struct Frame {
-    int32_t levels[6][4];
-    size_t bytes, plane_off[3];
-    int filtered[6];  // index of the filtered copy of each scale, or -1
-  };
-  std::vector<Frame> fr(static_cast<size_t>(n));
-  size_t copy_bytes = 0;
-  int copies = 0;
+  static const double kScales[kLfScales] = {0.0, 0.5, 0.75, 1.0, 1.25, 1.5};
+  std::vector<FrameJob> fjobs(static_cast<size_t>(n));
   for (int fi = 0; fi < n; fi++) {
     const av1pf_lf_search_job& jb = jobs[fi];
     const av1pf_frame_info* info = jb.info;
@@ -316,109 +309,66 @@ int av1pf_lf_search_many(av1pf_ctx* ctx, int n, av1pf_lf_search_job* jobs, void*
     if (!maps || !maps->mi || maps->mi_stride < info->mi_cols) return fail_input("mi map missing or mi_stride < mi_cols");
     for (int p = 0; p < info->num_planes; p++)
       if (!maps->lf_tx_size[p]) return fail_input("lf_tx_size map missing");
-    Frame& F = fr[size_t(fi)];
-    F.bytes = 0;
-    for (int p = 0; p < info->num_planes; p++) {
-      F.plane_off[p] = F.bytes;
-      F.bytes += align256(size_t(jb.cur[p].height) * size_t(jb.cur[p].stride) * size_t(info->sample_bytes));
-    }
-    for (int si = 0; si < 6; si++) {
-      for (int k = 0; k < 4; k++)
-        F.levels[si][k] = std::min(int32_t(std::round(double(jb.params->loop_filter_level[k]) * kScales[si])), 63);
-      F.filtered[si] = (F.levels[si][0] || F.levels[si][1]) ? copies++ : -1;
-      if (F.filtered[si] >= 0) copy_bytes += F.bytes;
-    }
+    fjobs[size_t(fi)] = FrameJob{info, jb.params, maps, jb.cur, nullptr, nullptr, nullptr, ST_LF, true};
   }
-  // filtered copies, one per (frame, scale that filters), filtered in place as one batch
-  if ((rc = ctx->ensure(ctx->search_planes, std::max<size_t>(1, copy_bytes))) != AV1PF_OK) return rc;
-  uint8_t* base = static_cast<uint8_t*>(ctx->search_planes.ptr);
-  std::vector<uint8_t*> copy_at(static_cast<size_t>(copies));
-  std::vector<av1pf_params> prm(static_cast<size_t>(copies));
-  std::vector<std::array<av1pf_plane, 3>> planes(static_cast<size_t>(copies));
-  std::vector<FrameJob> fjobs;
-  cudaError_t e = cudaSuccess;
-  size_t at = 0;
-  for (int fi = 0; fi < n; fi++) {
-    const av1pf_lf_search_job& jb = jobs[fi];
-    const Frame& F = fr[size_t(fi)];
-    for (int si = 0; si < 6; si++) {
-      const int ci = F.filtered[si];
-      if (ci < 0) continue;
-      copy_at[size_t(ci)] = base + at;
-      prm[size_t(ci)] = *jb.params;
-      for (int k = 0; k < 4; k++) prm[size_t(ci)].loop_filter_level[k] = F.levels[si][k];
-      for (int p = 0; p < jb.info->num_planes; p++) {
-        uint8_t* dst = base + at + F.plane_off[p];
-        const size_t bytes = size_t(jb.cur[p].height) * size_t(jb.cur[p].stride) * size_t(jb.info->sample_bytes);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, jb.cur[p].data, bytes, cudaMemcpyDeviceToDevice, s);
-        planes[size_t(ci)][size_t(p)] = jb.cur[p];
-        planes[size_t(ci)][size_t(p)].data = dst;
-      }
-      fjobs.push_back(FrameJob{jb.info, &prm[size_t(ci)], jb.maps, planes[size_t(ci)].data(), nullptr,
-                               planes[size_t(ci)].data(), nullptr, ST_LF, true});
-      at += F.bytes;
-    }
-  }
-  if (e != cudaSuccess) return cuda_status(e, "loop-filter search copies");
-  if (!fjobs.empty() && (rc = ctx->run(fjobs.data(), int(fjobs.size()), s)) != AV1PF_OK) return rc;
-  // the errors of every (frame, scale, plane) in one launch
-  std::vector<SsePlane> sj;
-  int rows_max = 0;
-  for (int fi = 0; fi < n; fi++) {
-    const av1pf_lf_search_job& jb = jobs[fi];
-    const av1pf_frame_info* info = jb.info;
-    const Frame& F = fr[size_t(fi)];
-    for (int si = 0; si < 6; si++)
-      for (int p = 0; p < info->num_planes; p++) {
-        const int sx = p ? info->subsampling_x : 0, sy = p ? info->subsampling_y : 0;
-        SsePlane j{};
-        j.a = F.filtered[si] < 0 ? static_cast<const uint8_t*>(jb.cur[p].data)
-                                 : copy_at[size_t(F.filtered[si])] + F.plane_off[p];
-        j.b = static_cast<const uint8_t*>(jb.src[p].data);
-        j.sa = jb.cur[p].stride;
-        j.sb_ = jb.src[p].stride;
-        j.w = (info->frame_width + sx) >> sx;
-        j.h = (info->frame_height + sy) >> sy;
-        j.sb = info->sample_bytes;
-        rows_max = std::max(rows_max, j.h);
-        sj.push_back(j);
-      }
-  }
-  const size_t jb_bytes = sj.size() * sizeof(SsePlane), o_sse = align256(jb_bytes);
-  const size_t total = o_sse + align256(sj.size() * sizeof(uint64_t));
+  Plan plan;
+  if ((rc = build_plan(fjobs.data(), n, nullptr, plan, &why, false)) != AV1PF_OK) return set_error(why), rc;
+  // one upload: the frames' descriptors and their zeroed error sums
+  const size_t o_sse = align256(size_t(n) * sizeof(LfSearchDesc)), nsse = size_t(n) * kLfScales * 3;
+  const size_t total = o_sse + nsse * sizeof(uint64_t);
   if ((rc = ctx->ensure(ctx->search_dev, total)) != AV1PF_OK) return rc;
   if ((rc = ctx->ensure_host(ctx->search_host, total)) != AV1PF_OK) return rc;
   uint8_t* dv = static_cast<uint8_t*>(ctx->search_dev.ptr);
   uint8_t* hs = static_cast<uint8_t*>(ctx->search_host.ptr);
-  std::memcpy(hs, sj.data(), jb_bytes);
-  e = cudaMemcpyAsync(dv, hs, jb_bytes, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dv + o_sse, 0, sj.size() * sizeof(uint64_t), s);
+  auto* descs = reinterpret_cast<LfSearchDesc*>(hs);
+  auto* hsse = reinterpret_cast<uint64_t*>(hs + o_sse);
+  int tiles = 0;
+  for (int fi = 0; fi < n; fi++) {
+    const av1pf_lf_search_job& jb = jobs[fi];
+    LfSearchDesc d{};
+    d.f = plan.frames[size_t(fi)];
+    for (int si = 0; si < kLfScales; si++)
+      for (int k = 0; k < 4; k++)
+        d.levels[si][k] = std::min(int32_t(std::round(double(jb.params->loop_filter_level[k]) * kScales[si])), 63);
+    for (int p = 0; p < jb.info->num_planes; p++) {
+      const int w = plane_w(jb.info, p, jb.info->frame_width), h = plane_h(jb.info, p);
+      d.src[p] = DPlane{static_cast<uint8_t*>(jb.src[p].data), jb.src[p].stride, w, h};
+      for (int si = 0; si < kLfScales; si++) {  // postfilter.rs:67-70, decoder/mod.rs:748
+        const int32_t* l = d.levels[si];
+        if ((l[0] || l[1]) && (p == 0 || l[1 + p])) d.filtered[p] |= 1u << si;
+      }
+      d.tiles_x[p] = (w + 63) / 64;
+      d.tile0[p] = tiles;
+      tiles += d.tiles_x[p] * ((h + 63) / 64);
+    }
+    d.sse = reinterpret_cast<uint64_t*>(dv + o_sse) + size_t(fi) * kLfScales * 3;
+    descs[fi] = d;
+  }
+  std::memset(hsse, 0, nsse * sizeof(uint64_t));
+  cudaError_t e = cudaMemcpyAsync(dv, hs, total, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return cuda_status(e, "loop-filter search");
-  launch_plane_sse(reinterpret_cast<const SsePlane*>(dv), int(sj.size()), rows_max,
-                   reinterpret_cast<uint64_t*>(dv + o_sse), s);
-  e = cudaMemcpyAsync(hs + o_sse, dv + o_sse, sj.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
+  launch_lf_search(reinterpret_cast<const LfSearchDesc*>(dv), n, tiles, s);
+  e = cudaMemcpyAsync(hsse, dv + o_sse, nsse * sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e, "loop-filter search");
   // each plane's level with the least error, the first scale on ties
   // (encoder/mod.rs:1477-1492)
-  const uint64_t* hsse = reinterpret_cast<const uint64_t*>(hs + o_sse);
-  size_t k = 0;
   for (int fi = 0; fi < n; fi++) {
     av1pf_lf_search_job& jb = jobs[fi];
     const int np = jb.info->num_planes;
-    const Frame& F = fr[size_t(fi)];
+    const int32_t(*levels)[4] = descs[fi].levels;
     uint64_t best_e[3] = {UINT64_MAX, UINT64_MAX, UINT64_MAX};
     int32_t best_l[3] = {0, 0, 0};
     if (jb.sse_out)
       for (int q = 0; q < 18; q++) jb.sse_out[q] = 0;
-    for (int si = 0; si < 6; si++)
+    for (int si = 0; si < kLfScales; si++)
       for (int p = 0; p < np; p++) {
-        const uint64_t err = hsse[k++];
+        const uint64_t err = hsse[(fi * kLfScales + si) * 3 + p];
         if (jb.sse_out) jb.sse_out[si * 3 + p] = err;
         if (err < best_e[p]) {
           best_e[p] = err;
-          best_l[p] = p == 0 ? F.levels[si][0] : F.levels[si][1 + p];
+          best_l[p] = p == 0 ? levels[si][0] : levels[si][1 + p];
         }
       }
     if (best_l[0] == 0) {

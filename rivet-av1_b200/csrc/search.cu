@@ -416,62 +416,6 @@ __global__ void cdef_greedy_finish_kernel(const CdefSearchDesc* __restrict__ ds,
   d.table[e] = v;
 }
 
-// Squared error of one plane pair over rows [4*blockIdx.x, +4) of job
-// blockIdx.y: 16-byte loads (planes and rows are 16-byte aligned), the
-// ragged end of a row sample by sample.
-__global__ void __launch_bounds__(256) plane_sse_kernel(const SsePlane* __restrict__ jobs, uint64_t* __restrict__ sse) {
-  const SsePlane j = jobs[blockIdx.y];
-  const int sb = j.sb;
-  const int y0 = blockIdx.x * 4;
-  uint64_t acc = 0;
-  if (y0 < j.h) {
-    const int per = 16 / sb;  // samples per 16 bytes
-    const int nv = j.w / per;
-    const int rows = min(4, j.h - y0);
-    for (int k = threadIdx.x; k < rows * nv; k += blockDim.x) {
-      const int r = y0 + k / nv, v = k % nv;
-      const uint4 qa = *reinterpret_cast<const uint4*>(j.a + (int64_t(r) * j.sa + int64_t(v) * per) * sb);
-      const uint4 qb = *reinterpret_cast<const uint4*>(j.b + (int64_t(r) * j.sb_ + int64_t(v) * per) * sb);
-      const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
-      uint32_t s = 0;  // 8 squares below 4096^2, or 16 below 256^2: fits
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (sb == 2) {
-          const int d0 = int(wa[q] & 0xffffu) - int(wb[q] & 0xffffu), d1 = int(wa[q] >> 16) - int(wb[q] >> 16);
-          s += uint32_t(d0 * d0) + uint32_t(d1 * d1);
-        } else {
-#pragma unroll
-          for (int h = 0; h < 4; h++) {
-            const int dd = int((wa[q] >> (8 * h)) & 0xffu) - int((wb[q] >> (8 * h)) & 0xffu);
-            s += uint32_t(dd * dd);
-          }
-        }
-      }
-      acc += s;
-    }
-    const int tail = j.w - nv * per;
-    for (int k = threadIdx.x; k < rows * tail; k += blockDim.x) {
-      const int r = y0 + k / tail, x = nv * per + k % tail;
-      int dd;
-      if (sb == 2)
-        dd = int(reinterpret_cast<const uint16_t*>(j.a)[int64_t(r) * j.sa + x]) -
-             int(reinterpret_cast<const uint16_t*>(j.b)[int64_t(r) * j.sb_ + x]);
-      else
-        dd = int(j.a[int64_t(r) * j.sa + x]) - int(j.b[int64_t(r) * j.sb_ + x]);
-      acc += uint64_t(dd * dd);
-    }
-  }
-  __shared__ uint64_t s_sum[8];
-  acc = warp_sum_u64(acc);
-  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint64_t t = 0;
-    for (int w = 0; w < 8; w++) t += s_sum[w];
-    if (t) atomicAdd(reinterpret_cast<unsigned long long*>(&sse[blockIdx.y]), static_cast<unsigned long long>(t));
-  }
-}
-
 }  // namespace
 
 cudaError_t search_init() {
@@ -507,12 +451,6 @@ void launch_cdef_greedy(const CdefSearchDesc* ds, int n, int ny, int nuv, int nf
 
 void launch_sse_transpose(const CdefSearchDesc* ds, int n, int nfb_max, int nc, cudaStream_t s) {
   sse_transpose_kernel<<<dim3(unsigned((nfb_max + 31) / 32), unsigned((nc + 31) / 32), unsigned(n)), 256, 0, s>>>(ds);
-  note_launch();
-}
-
-void launch_plane_sse(const SsePlane* jobs, int n, int rows_max, uint64_t* sse, cudaStream_t s) {
-  if (n <= 0 || rows_max <= 0) return;
-  plane_sse_kernel<<<dim3(unsigned((rows_max + 3) / 4), unsigned(n)), 256, 0, s>>>(jobs, sse);
   note_launch();
 }
 
