@@ -414,7 +414,8 @@ constexpr int kFChunks = kFW / 8 * kFW;  // 8-sample chunks of the window (800)
 // same property as the in-place passes: for conformant maps no edge of a
 // pass reads a sample another edge of that pass changes. The active edges of
 // each pass are listed in shared memory grouped by filter size, so a warp's
-// lanes mostly take one filter path. 256 threads.
+// lanes mostly take one filter path, two lanes of an edge a thread
+// (lf_filter_pair). 256 threads.
 template <class F>
 __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
                                                      const Item* __restrict__ items, int n_items, SyncFlags flags) {
@@ -544,20 +545,20 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
       __syncthreads();
       const int bd = f.bd, sharp = f.sharpness;
       const bool chroma = plane != 0;
-      // --- vertical edges: (edge, row lane) per thread ---
-      const int nv = int(cnt[0][0]) * 4;
+      // --- vertical edges: (edge, two rows) per thread ---
+      const int nv = int(cnt[0][0]) * 2;
       for (int t = tid; t < nv; t += 256) {
-        const uint32_t e = list_v[t >> 2];
+        const uint32_t e = list_v[t >> 1];
         const int j = int(e & 31u), i = int((e >> 5) & 31u), d = int(e >> 10);
-        lf_filter_smem(&W[(i * 4 + (t & 3)) * kFS + kFH + j * 4], 1, d >> 6, chroma, bd, d & 63, sharp);
+        lf_pair_rows(&W[(i * 4 + (t & 1) * 2) * kFS + kFH + j * 4], kFS, d >> 6, chroma, bd, d & 63, sharp);
       }
       __syncthreads();
-      // --- horizontal edges: (edge, column lane) per thread ---
-      const int nh = int(cnt[1][0]) * 4;
+      // --- horizontal edges: (edge, two columns) per thread ---
+      const int nh = int(cnt[1][0]) * 2;
       for (int t = tid; t < nh; t += 256) {
-        const uint32_t e = list_h[t >> 2];
+        const uint32_t e = list_h[t >> 1];
         const int j = int(e & 31u), i = int((e >> 5) & 31u), d = int(e >> 10);
-        lf_filter_smem(&W[(kFH + i * 4) * kFS + kFH + j * 4 + (t & 3)], kFS, d >> 6, chroma, bd, d & 63, sharp);
+        lf_pair_cols(&W[(kFH + i * 4) * kFS + kFH + j * 4 + (t & 1) * 2], kFS, d >> 6, chroma, bd, d & 63, sharp);
       }
     }
     __syncthreads();
@@ -613,7 +614,10 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
 // restores the window, filters it as lf_fused_kernel does and adds up the
 // tile's errors, so no filtered plane is ever written. A thread restores and
 // scores the same 8-sample chunks, so those steps need no barrier between
-// them. 256 threads.
+// them. Bound by issued instructions (the filters of five scales; staging and
+// decisions are a fifth). A 1080p 10-bit call takes 80 us; filtered copies,
+// one in-place pass a direction over all of them and a pass for the errors
+// took 200. 256 threads.
 __global__ void __launch_bounds__(256, 4) lf_search_kernel(const LfSearchDesc* __restrict__ ds, int n, int groups) {
   const LfTables& tb = g_lf_tables;
   __shared__ __align__(16) uint16_t W0[kFW * kFS], W[kFW * kFS], S[kFT * kFT];
@@ -787,20 +791,20 @@ __global__ void __launch_bounds__(256, 4) lf_search_kernel(const LfSearchDesc* _
         if (k < kFChunks) *reinterpret_cast<uint4*>(&W[o]) = *reinterpret_cast<const uint4*>(&W0[o]);
       }
       __syncthreads();
-      const int nv = int(cnt[0][0]) * 4;
+      const int nv = int(cnt[0][0]) * 2;
       for (int t = tid; t < nv; t += 256) {
-        const int e = list_v[t >> 2], lvl = lv_v[s][t >> 2];
+        const int e = list_v[t >> 1], lvl = lv_v[s][t >> 1];
         if (lvl)
-          lf_filter_smem(&W[(((e >> 5) & 31) * 4 + (t & 3)) * kFS + kFH + (e & 31) * 4], 1, e >> 10, chroma, bd, lvl,
-                         sharp);
+          lf_pair_rows(&W[(((e >> 5) & 31) * 4 + (t & 1) * 2) * kFS + kFH + (e & 31) * 4], kFS, e >> 10, chroma, bd,
+                       lvl, sharp);
       }
       __syncthreads();
-      const int nh = int(cnt[1][0]) * 4;
+      const int nh = int(cnt[1][0]) * 2;
       for (int t = tid; t < nh; t += 256) {
-        const int e = list_h[t >> 2], lvl = lv_h[s][t >> 2];
+        const int e = list_h[t >> 1], lvl = lv_h[s][t >> 1];
         if (lvl)
-          lf_filter_smem(&W[(kFH + ((e >> 5) & 31) * 4) * kFS + kFH + (e & 31) * 4 + (t & 3)], kFS, e >> 10, chroma,
-                         bd, lvl, sharp);
+          lf_pair_cols(&W[(kFH + ((e >> 5) & 31) * 4) * kFS + kFH + (e & 31) * 4 + (t & 1) * 2], kFS, e >> 10, chroma,
+                       bd, lvl, sharp);
       }
       __syncthreads();
     }
@@ -879,9 +883,9 @@ void launch_lf_search(const LfSearchDesc* ds, int n, int tiles, cudaStream_t s) 
   if (n <= 0 || tiles <= 0) return;
   // Every group stages the window and decides the edges again, so one group
   // where the tiles fill the GPU; half a wave of them or less (4 CTAs a SM) is
-  // split. us a call with 1 / 3 / 6 groups: 640x360 (90 tiles) 55 / 42 / 34,
-  // 1280x720 (360) 59 / 58 / 68, 1920x1080 (780) 93 / 94 / 117, 3840x2160
-  // (3060) 231 / 299 / 377.
+  // split. us a call with 1 / 3 / 6 groups: 640x360 (90 tiles) 43 / 33 / 33,
+  // 1280x720 (360) 56 / 55 / 58, 1920x1080 (780) 80 / 82 / 105, 3840x2160
+  // (3060) 191 / 253 / 327.
   const int groups = tiles <= kNumSMs ? 6 : (tiles <= 2 * kNumSMs ? 3 : 1);
   lf_search_kernel<<<tiles * groups, 256, 0, s>>>(ds, n, groups);
   note_launch();

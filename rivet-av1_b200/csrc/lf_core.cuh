@@ -290,4 +290,180 @@ __device__ __forceinline__ void lf_filter_smem(T* q0p, int step, int code, bool 
     if (k >= lo && k < hi) q0p[(k - 7) * step] = T(v[k]);
 }
 
+// ---------------------------------------------------------------------------
+// Two lanes of one edge at once: the same process on words of two 16-bit
+// samples. A sample has at most 12 bits, so the wide filters' tap sums stay
+// below 2^16 and plain 32-bit additions, subtractions and shifts (with the
+// bits that cross over masked off) work on both halves; signed values are
+// held plus 2^15; minima and maxima are single instructions. Rows of a
+// vertical edge come by 8-byte loads, two columns of a horizontal one are a
+// word. The tile kernels are bound by issued instructions, and the filters
+// took about a third of them: one lane a thread, against two, per call
+// 1080p 10-bit 52.3 / 50.4 us, 853x477 24.7 / 23.5, 4K 12-bit 4:4:4 434 / 422,
+// the level search at 1080p 92 / 80.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kHi2 = 0x80008000u;
+__device__ __forceinline__ uint32_t lf_diff2(uint32_t a, uint32_t b) { return __vmaxu2(a, b) - __vminu2(a, b); }
+__device__ __forceinline__ uint32_t lf_clamp2(uint32_t x, uint32_t lo, uint32_t hi) {
+  return __vmaxu2(__vminu2(x, hi), lo);
+}
+__device__ __forceinline__ uint32_t lf_half_mask(uint32_t bits) { return ((bits >> 15) & 0x10001u) * 0xffffu; }
+__device__ __forceinline__ uint32_t lf_pick(uint32_t mask, uint32_t a, uint32_t b) { return (a & mask) | (b & ~mask); }
+
+// lf_wide on words; only the lanes in `lanes` are changed.
+template <int N, int N2, int LOG2>
+__device__ __forceinline__ void lf_wide2(uint32_t v[14], uint32_t lanes) {
+  uint32_t o[14];
+#pragma unroll
+  for (int k = 0; k < 14; k++) o[k] = v[k];
+  auto at = [&](int k) { return o[7 + (k < -(N + 1) ? -(N + 1) : (k > N ? N : k))]; };
+  uint32_t sum = 0x10001u << (LOG2 - 1);  // of the first output (i = -N), rounding included
+#pragma unroll
+  for (int j = -N; j <= N; j++) sum += at(-N + j);
+#pragma unroll
+  for (int j = -N2; j <= N2; j++) sum += at(-N + j);
+#pragma unroll
+  for (int i = -N; i < N; i++) {
+    v[7 + i] = lf_pick(lanes, (sum >> LOG2) & ((0xffffu >> LOG2) * 0x10001u), o[7 + i]);
+    sum += at(i + N + 1) - at(i - N) + at(i + N2 + 1) - at(i - N2);
+  }
+}
+
+// lf_filter_one for two lanes. lo, hi: the samples that either lane's filter
+// changes; the other lane's among them keep their values.
+__device__ __forceinline__ void lf_filter_pair(uint32_t v[14], int code, bool chroma, int bd, int lvl, int sharp,
+                                               int& lo, int& hi) {
+  lo = hi = 0;
+  int limit, blimit, thresh;
+  lf_limits(lvl, sharp, limit, blimit, thresh);
+  const uint32_t unit = 0x10001u << (bd - 8);
+  const uint32_t p0 = v[6], p1 = v[5], q0 = v[7], q1 = v[8];
+  const uint32_t step = __vmaxu2(lf_diff2(p1, p0), lf_diff2(q1, q0));
+  uint32_t steps = step;
+  if (code > 1) {
+    steps = __vmaxu2(steps, __vmaxu2(lf_diff2(v[4], p1), lf_diff2(v[9], q1)));
+    if (!chroma) steps = __vmaxu2(steps, __vmaxu2(lf_diff2(v[3], v[4]), lf_diff2(v[10], v[9])));
+  }
+  // bit 15 of a half: x <= limit, as limit - x + 2^15
+  const uint32_t edge = (lf_diff2(p0, q0) << 1) + ((lf_diff2(p1, q1) >> 1) & 0x7fff7fffu);
+  const uint32_t ok = (kHi2 + unit * uint32_t(limit) - steps) & (kHi2 + unit * uint32_t(blimit) - edge) & kHi2;
+  if (!ok) return;
+  uint32_t flat = 0;
+  if (code > 1) {
+    uint32_t m = __vmaxu2(step, __vmaxu2(lf_diff2(v[4], p0), lf_diff2(v[9], q0)));
+    if (!chroma) m = __vmaxu2(m, __vmaxu2(lf_diff2(v[3], p0), lf_diff2(v[10], q0)));
+    flat = ok & (kHi2 + unit - m);
+  }
+  uint32_t flat2 = 0;
+  if (code == 3 && flat && !chroma) {
+    uint32_t m = __vmaxu2(lf_diff2(v[0], p0), lf_diff2(v[13], q0));
+    m = __vmaxu2(m, __vmaxu2(lf_diff2(v[1], p0), lf_diff2(v[12], q0)));
+    m = __vmaxu2(m, __vmaxu2(lf_diff2(v[2], p0), lf_diff2(v[11], q0)));
+    flat2 = flat & (kHi2 + unit - m);
+  }
+  uint32_t n_p1 = p1, n_p0 = p0, n_q0 = q0, n_q1 = q1;
+  const uint32_t narrow = lf_half_mask(ok & ~flat);
+  if (narrow) {
+    // 7.14.6.3, signed values plus 2^15. The offset by half the range that the
+    // text takes off and puts back only moves its clamps to 0 and the maximum.
+    const uint32_t half = 0x10001u << (bd - 1), low = kHi2 - half, high = kHi2 + half - 0x10001u;
+    const uint32_t top = kHi2 + (half << 1) - 0x10001u;
+    const uint32_t flat_side = lf_half_mask(kHi2 + unit * uint32_t(thresh) - step);  // not hev
+    const uint32_t base = lf_pick(flat_side, kHi2, lf_clamp2(p1 + kHi2 - q1, low, high));
+    const uint32_t fl = lf_clamp2(base + 3u * q0 - 3u * p0, low, high);
+    // filter1, filter2 plus half / 8
+    const uint32_t f1 = ((__vminu2(fl + 0x40004u, high) - low) >> 3) & 0x1fff1fffu;
+    const uint32_t f2 = ((__vminu2(fl + 0x30003u, high) - low) >> 3) & 0x1fff1fffu;
+    n_q0 = lf_pick(narrow, lf_clamp2(q0 + (kHi2 + (half >> 3)) - f1, kHi2, top) ^ kHi2, q0);
+    n_p0 = lf_pick(narrow, lf_clamp2(p0 + (kHi2 - (half >> 3)) + f2, kHi2, top) ^ kHi2, p0);
+    const uint32_t fr = ((f1 + 0x10001u) >> 1) & 0x7fff7fffu;  // plus half / 16
+    const uint32_t outer = narrow & flat_side;
+    n_q1 = lf_pick(outer, lf_clamp2(q1 + (kHi2 + (half >> 4)) - fr, kHi2, top) ^ kHi2, q1);
+    n_p1 = lf_pick(outer, lf_clamp2(p1 + (kHi2 - (half >> 4)) + fr, kHi2, top) ^ kHi2, p1);
+  }
+  lo = 5;
+  hi = 9;
+  if (flat) {
+    // 7.14.6.4: on lanes of their own, and the narrow filter's samples put
+    // back afterwards (a lane takes one filter, from the unfiltered samples)
+    const uint32_t w2 = lf_half_mask(flat2), w1 = lf_half_mask(flat) & ~w2;
+    if (w1) {
+      if (chroma) {
+        lf_wide2<2, 1, 3>(v, w1);
+      } else {
+        lf_wide2<3, 0, 3>(v, w1);
+        lo = 4;
+        hi = 10;
+      }
+    }
+    if (w2) {
+      lf_wide2<6, 1, 4>(v, w2);
+      lo = 1;
+      hi = 13;
+    }
+  }
+  v[5] = lf_pick(narrow, n_p1, v[5]);
+  v[6] = lf_pick(narrow, n_p0, v[6]);
+  v[7] = lf_pick(narrow, n_q0, v[7]);
+  v[8] = lf_pick(narrow, n_q1, v[8]);
+}
+
+// Two rows of a vertical edge in shared memory: q0p points at q0 of the upper
+// one, rows `stride` samples apart; q0 lies on a multiple of 4 samples and
+// rows on 8 bytes. Only samples that an edge of this size may change are
+// written, beside luma's outermost that only the edge itself reads.
+__device__ __forceinline__ void lf_pair_rows(uint16_t* q0p, int stride, int code, bool chroma, int bd, int lvl,
+                                             int sharp) {
+  uint32_t v[14];
+  const bool w16 = code == 3 && !chroma;
+  auto load = [&](int at, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+    const uint2 u = *reinterpret_cast<const uint2*>(q0p + at), l = *reinterpret_cast<const uint2*>(q0p + stride + at);
+    a = __byte_perm(u.x, l.x, 0x5410);
+    b = __byte_perm(u.x, l.x, 0x7632);
+    c = __byte_perm(u.y, l.y, 0x5410);
+    d = __byte_perm(u.y, l.y, 0x7632);
+  };
+  uint32_t unused;
+  v[0] = v[1] = v[2] = v[11] = v[12] = v[13] = 0;
+  if (w16) {
+    load(-8, unused, v[0], v[1], v[2]);
+    load(4, v[11], v[12], v[13], unused);
+  }
+  load(-4, v[3], v[4], v[5], v[6]);
+  load(0, v[7], v[8], v[9], v[10]);
+  int lo, hi;
+  lf_filter_pair(v, code, chroma, bd, lvl, sharp, lo, hi);
+  if (lo == hi) return;
+  auto store = [&](int at, uint32_t a, uint32_t b) {
+    *reinterpret_cast<uint32_t*>(q0p + at) = __byte_perm(a, b, 0x5410);
+    *reinterpret_cast<uint32_t*>(q0p + stride + at) = __byte_perm(a, b, 0x7632);
+  };
+  if (lo < 5) {
+    store(-4, v[3], v[4]);
+    store(2, v[9], v[10]);
+    if (lo < 4) {
+      store(-6, v[1], v[2]);
+      store(4, v[11], v[12]);
+    }
+  }
+  store(-2, v[5], v[6]);
+  store(0, v[7], v[8]);
+}
+
+// Two columns of a horizontal edge: q0p points at q0 of the left one (on 4
+// bytes), the samples across the edge `stride` apart.
+__device__ __forceinline__ void lf_pair_cols(uint16_t* q0p, int stride, int code, bool chroma, int bd, int lvl,
+                                             int sharp) {
+  uint32_t v[14];
+  const bool w16 = code == 3 && !chroma;
+#pragma unroll
+  for (int k = 0; k < 14; k++)
+    v[k] = (k >= 3 && k < 11) || w16 ? *reinterpret_cast<const uint32_t*>(q0p + (k - 7) * stride) : 0u;
+  int lo, hi;
+  lf_filter_pair(v, code, chroma, bd, lvl, sharp, lo, hi);
+#pragma unroll
+  for (int k = 1; k < 13; k++)
+    if (k >= lo && k < hi) *reinterpret_cast<uint32_t*>(q0p + (k - 7) * stride) = v[k];
+}
+
 }  // namespace av1pf
