@@ -228,8 +228,8 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   const bool resident = m.ready && m.key == key_scratch;
   // Calls of small frames wait for the calls before them by words (SyncFlags).
   // With film grain the template kernel then runs first on the call's stream
-  // and the output kernel starts early and waits on the SMs; its CTAs take half
-  // a SM's registers each, so only where at most one lands on a SM (us a call,
+  // and the output kernel starts early and waits on the SMs; its CTAs take a
+  // third of a SM's registers each, so only where at most one lands on a SM (us a call,
   // against templates on the side stream and no overlap: 640x360 27.8 / 44.7,
   // 1280x720 53.9 / 52.1, 1920x1080 70.8 / 72.4, 3840x2160 235 / 233).
   const bool chained = scratch_turns && plan.by_value && !plan.lff_items.empty() && !capturing && !prof &&

@@ -737,8 +737,15 @@ constexpr int kOutWaitLimit = 1 << 16;  // bulk-copy waits of about 1 us each be
 // a new plane's template and scaling table as two more), all completing on
 // one barrier, while 18 threads fetch the stripe's block offsets; then 256
 // threads take 8 consecutive samples (one grain block) each per row.
+//
+// Bound by the latency of each item's copies and barriers, so by the CTAs a SM
+// holds: 3 with the descriptor as a parameter (us a call against 2: 1080p 10-bit
+// 63.1 / 64.8, 2560x1440 103.9 / 107.1, 4K 10-bit superres 185.5 / 189.6, 4K
+// 12-bit 4:4:4 409 / 415); with descriptors in memory 80 registers would spill.
 template <class F>
-__global__ void __launch_bounds__(256, 2) output_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+constexpr int kOutCtas = sizeof(F) == sizeof(OneFrame) ? 3 : 2;
+template <class F>
+__global__ void __launch_bounds__(256, kOutCtas<F>) output_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
                                                      const Item* __restrict__ items, int n_items, SyncFlags sync) {
   AV1PF_TRACE_BEGIN();
   if (sync.ahead) pdl_trigger();
@@ -926,9 +933,10 @@ void launch_grain_prep(const FrameSet& frames, const Item* items, int n_items, c
 
 void launch_output(const FrameSet& frames, const Item* items, int n_items, const SyncFlags& sync, cudaStream_t s) {
   if (n_items <= 0) return;
-  // one resident wave (2 CTAs per SM), each CTA a contiguous run of items
-  launch_frames(frames, output_kernel<NoFrame>, output_kernel<OneFrame>, min(n_items, kNumSMs * 2), 256,
-                size_t(kOutSmem), s, items, n_items, sync);
+  // one resident wave, each CTA a contiguous run of items
+  const int ctas = kNumSMs * (frames.one ? kOutCtas<OneFrame> : kOutCtas<NoFrame>);
+  launch_frames(frames, output_kernel<NoFrame>, output_kernel<OneFrame>, min(n_items, ctas), 256, size_t(kOutSmem), s,
+                items, n_items, sync);
 }
 
 }  // namespace av1pf
