@@ -1,4 +1,7 @@
-// cdef.cu — the constrained directional enhancement filter (7.15).
+// cdef.cu — the constrained directional enhancement filter (7.15) with the
+// horizontal loop-filter pass fused in, one sample a lane; launches without that
+// pass take the packed kernels (cdef_packed.cu). Also the 12-bit frames of the
+// encoder's search.
 //
 // Reference: rivet-av1 src/decoder/postfilter.rs:266-513 (cdef, cdef_block,
 // cdef_direction, cdef_filter, cdef_filter_block) and src/dsp/cdef.rs:13-90
@@ -44,9 +47,9 @@ constexpr int16_t kNA = -32768;  // unavailable sample
 // 4-way conflict on every load.)
 constexpr int kDS = 72;
 // dynamic shared memory: the direction-search copy, then the three windows
-// of R + 2*2 rows, or R + 2*11 with the horizontal loop-filter pass fused in
+// of R + 2*11 rows
 constexpr int cdef_dir_bytes(int R) { return R * kDS * 2; }
-constexpr int cdef_smem(int R, bool lfh) { return cdef_dir_bytes(R) + 3 * (R + 2 * (lfh ? kTopLfh : 2)) * kS * 2; }
+constexpr int cdef_smem(int R) { return cdef_dir_bytes(R) + 3 * (R + 2 * kTopLfh) * kS * 2; }
 
 // Per 8x8 block and plane: strengths, tap weights and window offsets.
 struct BlkTaps {
@@ -388,33 +391,11 @@ __device__ __forceinline__ void write_prelf(const FrameDesc& f, int p, int sc, i
 // Item: R luma rows of a superblock (x0 = SB column, y0 = SB row, a = which
 // R rows). 4R threads, one warp per 8x8 block row. Item kind 1: the frame's
 // horizontal loop-filter edges (planes in f.lfh_mask) are filtered here, on
-// the staged window, before CDEF. `wrows` is the rows of one plane's window
-// (R + 22 when the launch has kind-1 items, else R + 4).
-// LFH: the launch has kind-1 items (the fused horizontal loop-filter pass);
-// without it the kernel carries none of that pass's code, which keeps the
-// default kernel's instruction footprint small.
-// With readiness flags: waits (threads 0..47, one flag each) for the
-// loop-filter tiles under the CTA's windows, the rows and columns
-// stage_plane reads: plane rows (y0 >> sy) - 2 .. ((y0 + R) >> sy) + 1 and
-// 8 columns past the superblock on either side, within the plane.
+// the staged window, before CDEF. The launches with such items take this kernel;
+// `wrows` is the rows of one plane's window (R + 22).
 template <int R>
-__device__ __forceinline__ void cdef_wait_lf(const FrameDesc& f, const SyncFlags& flags, int sc, int y0, int tid) {
-  if (tid >= 48) return;
-  const int p = tid >> 4, dy = (tid >> 2) & 3, dx = tid & 3;
-  if (p >= f.np || f.lf_tiles_x[p] == 0) return;
-  const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
-  const int W = f.cur[p].w, H = f.cur[p].h;
-  const int r0 = max((y0 >> sy) - 2, 0), r1 = min(((y0 + R) >> sy) + 1, H - 1);
-  const int c0 = max(((sc * 64) >> sx) - 8, 0), c1 = min(((sc * 64 + 64) >> sx) + 7, W - 1);
-  const int ty = (r0 >> 6) + dy, tx = (c0 >> 6) + dx;
-  if (r0 > r1 || c0 > c1 || ty > (r1 >> 6) || tx > (c1 >> 6)) return;
-  flag_wait(flags.p + f.lf_flag_base[p] + ty * f.lf_tiles_x[p] + tx, flags.epoch);
-}
-
-template <class F, int R, bool LFH>
-__global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
-                                                     const Item* __restrict__ items, int n_items, int wrows,
-                                                           int min_bd, SyncFlags flags) {
+__global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const FrameDesc* __restrict__ frames,
+                                                     const Item* __restrict__ items, int n_items, int wrows) {
   AV1PF_TRACE_BEGIN();
   extern __shared__ __align__(16) int16_t cdef_smem_base[];  // [R][kDS] direction copy, then [3][wrows * kS]
   int16_t* const dwin = cdef_smem_base;
@@ -435,13 +416,13 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const __grid_const
   if (tid == 0) s_one = 1;
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
-    const FrameDesc& f = frame_of(one, frames, item.frame);
+    const FrameDesc& f = frames[item.frame];
     const int sc = item.x0, sr = item.y0;
     const int y0 = sr * 64 + item.a * R;  // luma row of the CTA's first row
     const int np = f.np, sb = f.sb;
     const int cs = f.bd - 8;
     const int idx = f.cdef_idx[int64_t(sr) * f.cdef_stride + sc];  // postfilter.rs:285
-    const bool lfh = LFH && item.kind != 0;
+    const bool lfh = item.kind != 0;
     const int top = lfh ? kTopLfh : 2;  // window row of the superblock's first row
     // --- per 8x8: inside the MI area? skipped? (postfilter.rs:281-287, 306-310) ---
     // (the maps are inputs of the chain: read before waiting for the loop filter)
@@ -460,14 +441,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const __grid_const
         }
       }
     }
-    if (flags.p) {
-      // only the loop-filter tiles this CTA reads
-      pdl_trigger();
-      cdef_wait_lf<R>(f, flags, sc, y0, tid);
-    } else {
-      pdl_wait();  // the loop filter's output is complete past this point
-      if (f.bd < min_bd) continue;
-    }
+    pdl_wait();  // the loop filter's output is complete past this point
     __syncthreads();  // the previous item is done with the windows and block states
     if (tid < R) bstate[tid] = st;
     // --- stage the windows (postfilter.rs:464-488): 8-sample chunks ---
@@ -594,16 +568,6 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_kernel(const __grid_const
       }
     }
     __syncthreads();
-    if (flags.p && tid == 0) {
-      // the rows are in the CDEF planes: the half superblocks' flags
-      uint32_t* fl = flags.p + f.cdef_flag_base + 2 * sr * f.cdef_sbc + sc;
-      if (R == 64) {
-        flag_set(fl, flags.epoch);
-        flag_set(fl + f.cdef_sbc, flags.epoch);
-      } else {
-        flag_set(fl + item.a * f.cdef_sbc, flags.epoch);
-      }
-    }
   }
   AV1PF_TRACE_END(2);
 }
@@ -990,12 +954,8 @@ cudaError_t cdef_init() {
   auto opt_in = [&](auto kernel, int bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   };
-  opt_in(cdef_kernel<NoFrame, 64, true>, cdef_smem(64, true));
-  opt_in(cdef_kernel<NoFrame, 32, true>, cdef_smem(32, true));
-  opt_in(cdef_kernel<NoFrame, 64, false>, cdef_smem(64, false));
-  opt_in(cdef_kernel<NoFrame, 32, false>, cdef_smem(32, false));
-  opt_in(cdef_kernel<OneFrame, 64, false>, cdef_smem(64, false));
-  opt_in(cdef_kernel<OneFrame, 32, false>, cdef_smem(32, false));
+  opt_in(cdef_kernel<64>, cdef_smem(64));
+  opt_in(cdef_kernel<32>, cdef_smem(32));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(cdef_search_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSearchSmem);
   if (e == cudaSuccess)
@@ -1007,31 +967,18 @@ cudaError_t cdef_init() {
 void launch_cdef(const FrameSet& frames, const Item* items, int n_items, const CdefShape& c, SyncFlags flags,
                  cudaStream_t s) {
   if (n_items <= 0) return;
-  // Frames of up to 10 bits take the packed kernel, whose half precision holds
-  // their samples exactly (1080p 10-bit: 25.5 against 36.0 us); 12-bit frames,
-  // and launches with the fused horizontal pass, this file's. A launch of both kinds runs both kernels
-  // over the whole list, each leaving the other's frames alone.
-  const bool packed = c.shallow && !c.lfh;
-  if (packed) launch_cdef_packed(frames, items, n_items, c.half, c.tall, flags, s);
-  if (packed && !c.deep) return;
-  const int min_bd = packed ? 11 : 0;
-  // without the fused horizontal pass the windows hold 2 border rows each
-  // side: smaller windows, more CTAs per SM
+  // Launches with the fused horizontal pass take this file's kernel (one sample
+  // a lane, 32 bits), all others the packed kernels (two): 1080p 10-bit 25.5
+  // against 36.0 us, 4K 12-bit 4:4:4 coded at 3072 columns 104 against 140. A
+  // launch with frames of up to 10 bits and of 12 runs both packed kernels over
+  // the whole list, each leaving the other's frames alone.
+  if (!c.lfh) return launch_cdef_packed(frames, items, n_items, c, flags, s);
   const int R = c.half ? 32 : 64;
-  const int wrows = R + 2 * (c.lfh ? kTopLfh : 2);
-  const int grid = min(n_items, kItemGrid);
-  const size_t smem = size_t(cdef_smem(R, c.lfh));
   auto by_ptr = [&](auto kernel) {
-    launch_pdl(kernel, grid, 4 * R, smem, s, NoFrame{}, frames.dev, items, n_items, wrows, min_bd, flags);
+    launch_pdl(kernel, min(n_items, kItemGrid), 4 * R, size_t(cdef_smem(R)), s, frames.dev, items, n_items,
+               R + 2 * kTopLfh);
   };
-  if (c.lfh)
-    c.half ? by_ptr(cdef_kernel<NoFrame, 32, true>) : by_ptr(cdef_kernel<NoFrame, 64, true>);
-  else if (c.half)
-    launch_frames(frames, cdef_kernel<NoFrame, 32, false>, cdef_kernel<OneFrame, 32, false>, grid, 4 * R, smem, s,
-                  items, n_items, wrows, min_bd, flags);
-  else
-    launch_frames(frames, cdef_kernel<NoFrame, 64, false>, cdef_kernel<OneFrame, 64, false>, grid, 4 * R, smem, s,
-                  items, n_items, wrows, min_bd, flags);
+  c.half ? by_ptr(cdef_kernel<32>) : by_ptr(cdef_kernel<64>);
 }
 
 void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorough, bool shallow, bool deep,

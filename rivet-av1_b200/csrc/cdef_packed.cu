@@ -1,11 +1,13 @@
-// cdef_packed.cu — the constrained directional enhancement filter (7.15) for
-// bit depths up to 10, two samples per lane in half precision
-// (cdef_packed.cuh shows why that is exact). 12-bit frames, and launches with
-// the horizontal loop-filter pass fused in, take cdef_kernel (cdef.cu).
+// cdef_packed.cu — the constrained directional enhancement filter (7.15), two
+// samples per lane: in half precision for bit depths up to 10, in 16-bit
+// integers for 12 (cdef_packed.cuh shows why both are exact). Launches with the
+// horizontal loop-filter pass fused in take cdef_kernel (cdef.cu).
 //
 // Reference: rivet-av1 src/decoder/postfilter.rs:266-513, src/dsp/cdef.rs:13-90.
 //
-// What bounds it: instruction issue. The constrained taps of the 32-bit
+// What bounds it: instruction issue. (Half precision first; a tap in integers
+// is 12 instructions for two samples: 4K 12-bit 4:4:4 coded at 3072 columns 140
+// -> 104 us against the 32-bit kernel, the chain call 409 -> 378.) The constrained taps of the 32-bit
 // kernel were 70% of its 16.2 M warp instructions per 1080p frame, on the
 // integer ALU pipe (one instruction per two clocks). Here a tap is about 10
 // instructions for two samples instead of 12 for one, half of them on the
@@ -38,22 +40,32 @@ constexpr int packed_smem(int R, bool tall) { return R * kDS * 2 + R * kPS * 4 +
 
 // The taps of one block (postfilter.rs:489-511), 48 bytes.
 struct alignas(16) PackedTaps {
-  PStrength pri;
-  uint32_t w0, w1;  // primary weights, in both halves
+  PStrength pri;    // (12-bit frames: strength, shift, mask of what it leaves, per half)
+  uint32_t w0, w1;  // primary weights, in both halves (12-bit frames: as integers)
   PStrength sec;
   int16_t off[6];  // bytes: primary k0, k1, secondary lo k0, hi k0, lo k1, hi k1
   int32_t mode;    // 0 both kinds, 1 primary only, 2 secondary only, 3 copy
 };
 static_assert(sizeof(PackedTaps) == 48, "three 16-byte loads");
 
+template <bool DEEP>
 __device__ __forceinline__ PackedTaps make_packed_taps(int pri, int sec, int damping, int dir, int cs,
                                                        const int16_t (*doff)[2]) {
   PackedTaps t;
-  t.pri = packed_strength(pri, pri ? max(damping - floor_log2(uint32_t(pri)), 0) : 0);
-  t.sec = packed_strength(sec, sec ? max(damping - floor_log2(uint32_t(sec)), 0) : 0);
+  const int pri_adj = pri ? max(damping - floor_log2(uint32_t(pri)), 0) : 0;
+  const int sec_adj = sec ? max(damping - floor_log2(uint32_t(sec)), 0) : 0;
   const bool odd = (pri >> cs) & 1;  // CDEF_PRI_TAPS: [4, 2] / [3, 3]
-  t.w0 = odd ? 0x42004200u : 0x44004400u;
-  t.w1 = odd ? 0x42004200u : 0x40004000u;
+  if (DEEP) {
+    t.pri = deep_strength(pri, pri_adj);
+    t.sec = deep_strength(sec, sec_adj);
+    t.w0 = odd ? 3u : 4u;
+    t.w1 = odd ? 3u : 2u;
+  } else {
+    t.pri = packed_strength(pri, pri_adj);
+    t.sec = packed_strength(sec, sec_adj);
+    t.w0 = odd ? 0x42004200u : 0x44004400u;
+    t.w1 = odd ? 0x42004200u : 0x40004000u;
+  }
   const int dlo = (dir + 6) & 7, dhi = (dir + 2) & 7;
   t.off[0] = doff[dir][0];
   t.off[1] = doff[dir][1];
@@ -98,6 +110,43 @@ __device__ __forceinline__ void packed_px2(const uint32_t* c, const PackedTaps& 
     if (MODE == 0) v = __hmax2(__hmin2(v, mx[e]), as_h2(mn[e]));
     (e ? o1 : o0) = as_u32(v);
   }
+}
+
+// The same for 12-bit frames, in 16-bit integers (cdef_packed.cuh).
+template <int MODE>
+__device__ __forceinline__ void deep_px2(const uint32_t* c, const PackedTaps& t, uint32_t& o0, uint32_t& o1) {
+  const uint32_t xw[2] = {c[0], c[2]};
+  uint32_t sum[2], mx[2], mn[2];
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    sum[e] = 0u - (MODE == 0 ? 24u : 12u) * xw[e];
+    mx[e] = mn[e] = xw[e];
+  }
+#pragma unroll
+  for (int k = MODE == 2 ? 2 : 0; k < (MODE == 1 ? 2 : 6); k++) {
+    const uint32_t w = k == 0 ? t.w0 : k == 1 ? t.w1 : k < 4 ? 2u : 1u;  // CDEF_SEC_TAPS [2, 1]
+    const int off = t.off[k];
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(c) + (side ? -off : off));
+#pragma unroll
+      for (int e = 0; e < 2; e++) deep_tap<MODE == 0>(p[2 * e], xw[e], k < 2 ? t.pri : t.sec, w, sum[e], mx[e], mn[e]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    uint32_t v = deep_round(sum[e], xw[e]);
+    if (MODE == 0) v = __vmaxu2(__vminu2(v, mx[e]), mn[e]);
+    (e ? o1 : o0) = v;
+  }
+}
+
+template <int MODE, bool DEEP>
+__device__ __forceinline__ void px2(const uint32_t* c, const PackedTaps& t, uint32_t& o0, uint32_t& o1) {
+  if (DEEP)
+    deep_px2<MODE>(c, t, o0, o1);
+  else
+    packed_px2<MODE>(c, t, o0, o1);
 }
 
 // Costs of directions P and P + 4 of the 8x8 block at `s` (rows kDS apart,
@@ -188,20 +237,22 @@ __device__ __forceinline__ uint4 load_chunk(const uint8_t* at, int sb, int gx, i
   const uint2 h = *reinterpret_cast<const uint2*>(at);
   return make_uint4(h.x, h.y, 0u, 0u);
 }
-template <bool INSIDE>
+template <bool INSIDE, bool DEEP = false>
 __device__ __forceinline__ uint4 bias_chunk(const uint4& q, const uint8_t* at, int sb, int gx, int gy, int xlim, int ylim) {
+  constexpr uint32_t bias = DEEP ? kDeepBias : kPBias;
   if (!INSIDE && (gy < 0 || gy >= ylim || gx < 0 || gx + 8 > xlim)) {
-    uint32_t o[4] = {kPNA, kPNA, kPNA, kPNA};
+    constexpr uint32_t na = DEEP ? kDeepNA : kPNA;
+    uint32_t o[4] = {na, na, na, na};
     if (gy >= 0 && gy < ylim && gx >= 0)
 #pragma unroll
       for (int e = 0; e < 8; e++)
         if (gx + e < xlim) {
-          const uint32_t v = 0x6400u | uint32_t(sb == 1 ? at[e] : reinterpret_cast<const uint16_t*>(at)[e]);
+          const uint32_t v = (bias & 0xffffu) | uint32_t(sb == 1 ? at[e] : reinterpret_cast<const uint16_t*>(at)[e]);
           o[e >> 1] = (e & 1) ? ((o[e >> 1] & 0xffffu) | (v << 16)) : ((o[e >> 1] & 0xffff0000u) | v);
         }
     return make_uint4(o[0], o[1], o[2], o[3]);
   }
-  if (sb == 2) return make_uint4(q.x | kPBias, q.y | kPBias, q.z | kPBias, q.w | kPBias);
+  if (DEEP || sb == 2) return make_uint4(q.x | bias, q.y | bias, q.z | bias, q.w | bias);
   return make_uint4(__byte_perm(q.x, 0x64646464u, 0x4140), __byte_perm(q.x, 0x64646464u, 0x4342),
                     __byte_perm(q.y, 0x64646464u, 0x4140), __byte_perm(q.y, 0x64646464u, 0x4342));
 }
@@ -226,7 +277,7 @@ __device__ __forceinline__ void put_words(uint32_t* row, int ch, int nch, const 
 // and high halves of three word rows, so a row is loaded once and (but for the
 // thread's first and last) used twice. Chroma: one chunk of a U and of a V
 // row. All of a thread's first loads are in flight together.
-template <int R, bool INSIDE>
+template <int R, bool INSIDE, bool DEEP = false>
 __device__ __forceinline__ void stage_windows(const FrameDesc& f, int sc, int y0, uint32_t* lw, uint32_t* cw,
                                               uint16_t* dwin, int tid) {
   constexpr int NT = 4 * R;
@@ -260,12 +311,12 @@ __device__ __forceinline__ void stage_windows(const FrameDesc& f, int sc, int y0
   };
   if (tid < nc) load_chroma(tid);
   if (ltask) {
-    uint4 a = bias_chunk<INSIDE>(l[0], lat, sb, lgx, lgy, lxl, lyl);
+    uint4 a = bias_chunk<INSIDE, DEEP>(l[0], lat, sb, lgx, lgy, lxl, lyl);
 #pragma unroll
     for (int e = 0; e < 3; e++) {
       const int i = li + 4 * e;
       if (i >= R) break;
-      const uint4 b = bias_chunk<INSIDE>(l[e + 1], lat + (e + 1) * pitch4, sb, lgx, lgy + 4 * (e + 1), lxl, lyl);
+      const uint4 b = bias_chunk<INSIDE, DEEP>(l[e + 1], lat + (e + 1) * pitch4, sb, lgx, lgy + 4 * (e + 1), lxl, lyl);
       put_words(lw + i * kPS, lch, 10, a, b);
       if (lch != 0 && lch != 9) {
         // the superblock's own rows, at 8 bits, for the direction search: the
@@ -282,8 +333,8 @@ __device__ __forceinline__ void stage_windows(const FrameDesc& f, int sc, int y0
     }
   }
   for (int k = tid; k < nc;) {
-    put_words(cw + ci * kPS, cc, cch, bias_chunk<INSIDE>(u, uat, sb, gx, gy, cxl, cyl),
-              bias_chunk<INSIDE>(v, vat, sb, gx, gy, cxl, cyl));
+    put_words(cw + ci * kPS, cc, cch, bias_chunk<INSIDE, DEEP>(u, uat, sb, gx, gy, cxl, cyl),
+              bias_chunk<INSIDE, DEEP>(v, vat, sb, gx, gy, cxl, cyl));
     k += NT;  // more chunks than threads: chroma without vertical subsampling
     if (k < nc) load_chroma(k);
   }
@@ -309,10 +360,10 @@ __device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const SyncFla
 }  // namespace
 
 // Item: R luma rows of a superblock (x0 = SB column, y0 = SB row, a = which R
-// rows). 4R threads, one warp per row of 8x8 blocks. Frames above 10 bits are
-// left to cdef_kernel. The chroma window has room for `R` rows and 4 more
+// rows). 4R threads, one warp per row of 8x8 blocks. DEEP takes the launch's
+// 12-bit frames and leaves the others, and the other way round. The chroma window has room for `R` rows and 4 more
 // when the launch was sized for frames without vertical subsampling.
-template <class F, int R>
+template <class F, int R, bool DEEP>
 __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
                                                      const Item* __restrict__ items, int n_items,
                                                                   SyncFlags flags) {
@@ -357,16 +408,16 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __gri
       packed_wait_lf<R>(f, flags, sc, y0, tid);  // only the loop-filter tiles this CTA reads
     } else {
       pdl_wait();  // the loop filter's output is complete past this point
-      if (f.bd > 10) continue;
+      if ((f.bd > 10) != DEEP) continue;
     }
     __syncthreads();  // the previous item is done with the windows and block states
     if (tid < R) bstate[tid] = st;
     const int csx = f.ssx, csy = f.ssy;
     // the chunks reach 8 columns past the superblock, 16 luma columns in subsampled chroma
     if (sc > 0 && sc * 64 + 80 <= f.mi_cols * 4 && y0 >= 4 && y0 + R + 4 <= f.mi_rows * 4)
-      stage_windows<R, true>(f, sc, y0, lw, cw, dwin, tid);
+      stage_windows<R, true, DEEP>(f, sc, y0, lw, cw, dwin, tid);
     else
-      stage_windows<R, false>(f, sc, y0, lw, cw, dwin, tid);
+      stage_windows<R, false, DEEP>(f, sc, y0, lw, cw, dwin, tid);
     __syncthreads();
     // --- direction search (postfilter.rs:345-401): each thread two directions of one block ---
     {
@@ -414,7 +465,7 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __gri
           pri = var != 0 ? (p0 * (4 + var_str) + 8) >> 4 : 0;
         }
       }
-      taps[uv][b] = make_packed_taps(pri, sec, f.cdef_damping + cs - uv, dir, cs, doff);
+      taps[uv][b] = make_packed_taps<DEEP>(pri, sec, f.cdef_damping + cs - uv, dir, cs, doff);
     }
     __syncthreads();
     // --- filter + write (postfilter.rs:405-442): a warp per block row. Luma
@@ -443,17 +494,17 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __gri
         for (int cols = wide ? 2 : 1; cols > 0; cols--) {
           uint32_t o0, o1;
           if (t.mode == 0) {
-            packed_px2<0>(c, t, o0, o1);
+            px2<0, DEEP>(c, t, o0, o1);
           } else if (t.mode == 1) {
-            packed_px2<1>(c, t, o0, o1);
+            px2<1, DEEP>(c, t, o0, o1);
           } else if (t.mode == 2) {
-            packed_px2<2>(c, t, o0, o1);
+            px2<2, DEEP>(c, t, o0, o1);
           } else {
             o0 = c[0];
             o1 = c[2];
           }
-          o0 ^= kPBias;  // 0x6400 | v in each half, v < 1024
-          o1 ^= kPBias;
+          o0 ^= DEEP ? kDeepBias : kPBias;  // bias | v in each half
+          o1 ^= DEEP ? kDeepBias : kPBias;
           const uint32_t p0 = __shfl_xor_sync(0xffffffffu, o0, 1), p1 = __shfl_xor_sync(0xffffffffu, o1, 1);
           const uint32_t w0 = __byte_perm(h ? p0 : o0, h ? o0 : p0, sel), w1 = __byte_perm(h ? p1 : o1, h ? o1 : p1, sel);
           if (live) {
@@ -799,25 +850,38 @@ cudaError_t cdef_packed_init() {
   auto opt_in = [&](auto kernel, int bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   };
-  opt_in(cdef_packed_kernel<NoFrame, 64>, packed_smem(64, true));
-  opt_in(cdef_packed_kernel<OneFrame, 64>, packed_smem(64, true));
-  opt_in(cdef_packed_kernel<NoFrame, 32>, packed_smem(32, true));
-  opt_in(cdef_packed_kernel<OneFrame, 32>, packed_smem(32, true));
+  opt_in(cdef_packed_kernel<NoFrame, 64, false>, packed_smem(64, true));
+  opt_in(cdef_packed_kernel<NoFrame, 32, false>, packed_smem(32, true));
+  opt_in(cdef_packed_kernel<OneFrame, 64, false>, packed_smem(64, true));
+  opt_in(cdef_packed_kernel<OneFrame, 32, false>, packed_smem(32, true));
+  opt_in(cdef_packed_kernel<NoFrame, 64, true>, packed_smem(64, true));
+  opt_in(cdef_packed_kernel<NoFrame, 32, true>, packed_smem(32, true));
+  opt_in(cdef_packed_kernel<OneFrame, 64, true>, packed_smem(64, true));
+  opt_in(cdef_packed_kernel<OneFrame, 32, true>, packed_smem(32, true));
   opt_in(cdef_search_packed_kernel<false>, search_smem<false>());
   opt_in(cdef_search_packed_kernel<true>, search_smem<true>());
   return e;
 }
 
-void launch_cdef_packed(const FrameSet& frames, const Item* items, int n_items, bool half, bool tall, SyncFlags flags,
-                        cudaStream_t s) {
-  if (n_items <= 0) return;
+namespace {
+template <bool DEEP>
+void launch_packed(const FrameSet& frames, const Item* items, int n_items, bool half, bool tall, SyncFlags flags,
+                   cudaStream_t s) {
   const int grid = min(n_items, kItemGrid);
   if (half)
-    launch_frames(frames, cdef_packed_kernel<NoFrame, 32>, cdef_packed_kernel<OneFrame, 32>, grid, 128,
+    launch_frames(frames, cdef_packed_kernel<NoFrame, 32, DEEP>, cdef_packed_kernel<OneFrame, 32, DEEP>, grid, 128,
                   size_t(packed_smem(32, tall)), s, items, n_items, flags);
   else
-    launch_frames(frames, cdef_packed_kernel<NoFrame, 64>, cdef_packed_kernel<OneFrame, 64>, grid, 256,
+    launch_frames(frames, cdef_packed_kernel<NoFrame, 64, DEEP>, cdef_packed_kernel<OneFrame, 64, DEEP>, grid, 256,
                   size_t(packed_smem(64, tall)), s, items, n_items, flags);
+}
+}  // namespace
+
+void launch_cdef_packed(const FrameSet& frames, const Item* items, int n_items, const CdefShape& c, SyncFlags flags,
+                        cudaStream_t s) {
+  if (n_items <= 0) return;
+  if (c.shallow) launch_packed<false>(frames, items, n_items, c.half, c.tall, flags, s);
+  if (c.deep) launch_packed<true>(frames, items, n_items, c.half, c.tall, flags, s);
 }
 
 }  // namespace av1pf

@@ -1,6 +1,7 @@
 // cdef_packed.cuh — CDEF's constrained taps (7.15.2) on two samples at once,
-// in half precision, exactly, for bit depths up to 10.
+// exactly: in half precision for bit depths up to 10, in 16-bit integers for 12.
 //
+// Half precision, bit depths up to 10.
 // A sample v (0 .. 1023) is held as the half 1024 + v: its bits are 0x6400 | v,
 // so packing and unpacking are integer operations, and every half in
 // [1024, 2048) is an integer. Two samples that take the same taps share a
@@ -23,6 +24,19 @@
 // sample is -infinity: its limit is 0 (so it adds nothing), a max never takes
 // it, and a min of the bits as unsigned integers never takes it (0xfc00 is
 // above every 0x6400 | v, whose order is that of v).
+//
+// Integers, 12 bits. A sample v is held as 4096 + v (0x1000 | v), two to a word.
+//   |d| = max(p, x) - min(p, x)      no borrow between the halves;
+//   lim = str - min(|d| >> adj, str) the shift's bits from the upper half
+//         masked off;
+//   p clamped to [x - lim, x + lim]  x plus the constrained difference; both
+//         ends stay in (0, 2^15), a limit being at most 240.
+// The weighted sum of those words less the weights times x is hi * 2^16 + lo of
+// the two sums, at most 12 * 240 + 12 * 64 in magnitude: one 32-bit
+// multiply-add a tap, whatever crosses the halves on the way. An unavailable
+// sample is 0xf000: |d| >= 0xd001, and |d| >> adj is no less than str (str <<
+// adj is at most 2^11), so its limit is 0; a signed max and an unsigned min
+// never take it.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -73,5 +87,32 @@ __device__ __forceinline__ void packed_tap(uint32_t p, __half2 nx, const PStreng
 
 // 1024 + x + (sum / 16 rounded to nearest, halves away from 0), x biased.
 __device__ __forceinline__ __half2 packed_round(__half2 sum, __half2 x) { return __hfma2(sum, as_h2(0x2c012c01u), x); }
+
+constexpr uint32_t kDeepBias = 0x10001000u;  // 4096 in both halves
+constexpr uint32_t kDeepNA = 0xf000f000u;
+
+// Strength terms in integers: str and the mask of |d| >> adj in both halves, adj.
+__device__ __forceinline__ PStrength deep_strength(int str, int adj) {
+  return PStrength{uint32_t(str) * 0x10001u, uint32_t(adj), (0xffffu >> adj) * 0x10001u};
+}
+
+template <bool CLAMP>
+__device__ __forceinline__ void deep_tap(uint32_t p, uint32_t x, const PStrength& s, uint32_t w, uint32_t& sum,
+                                         uint32_t& mx, uint32_t& mn) {
+  const uint32_t d = __vmaxu2(p, x) - __vminu2(p, x);
+  const uint32_t lim = s.c - __vminu2((d >> s.k) & s.o, s.c);
+  sum += w * __vminu2(__vmaxu2(p, x - lim), x + lim);
+  if (CLAMP) {
+    mx = __vmaxs2(mx, p);
+    mn = __vminu2(mn, p);
+  }
+}
+
+// x + (8 + sum - (sum < 0) >> 4) in both halves, of the sums hi * 2^16 + lo.
+__device__ __forceinline__ uint32_t deep_round(uint32_t sum, uint32_t x) {
+  const int lo = int16_t(sum & 0xffffu), hi = (int(sum) - lo) >> 16;
+  const int rl = (8 + lo + (lo >> 31)) >> 4, rh = (8 + hi + (hi >> 31)) >> 4;
+  return x + (uint32_t(rh) << 16) + uint32_t(rl);
+}
 
 }  // namespace av1pf

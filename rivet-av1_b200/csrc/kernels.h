@@ -137,8 +137,8 @@ struct CdefShape {
 // latter needs the descriptors in device memory).
 void launch_cdef(const FrameSet& frames, const Item* items, int n_items, const CdefShape& c, SyncFlags flags,
                  cudaStream_t s);
-// The part of it for frames of up to 10 bits (cdef_packed.cu).
-void launch_cdef_packed(const FrameSet& frames, const Item* items, int n_items, bool half, bool tall, SyncFlags flags,
+// The part of it for launches without the fused horizontal pass (cdef_packed.cu).
+void launch_cdef_packed(const FrameSet& frames, const Item* items, int n_items, const CdefShape& c, SyncFlags flags,
                         cudaStream_t s);
 cudaError_t cdef_packed_init();
 // Sets cdef_kernel's dynamic shared-memory limit on the current device.

@@ -1,5 +1,5 @@
-"""CDEF's two-samples-a-lane kernel (bit depths up to 10) against the oracle,
-bit for bit: windows inside the frame and at each of its edges, half and whole
+"""CDEF's two-samples-a-lane kernels (in half precision for bit depths up to 10,
+in integers for 12) against the oracle, bit for bit: windows inside the frame and at each of its edges, half and whole
 superblock CTAs, every chroma layout, extreme samples and strengths, and a
 batch whose frames need both CDEF kernels."""
 import ctypes as C
@@ -24,6 +24,12 @@ SHAPES = {
     "422_10bit": dict(width=296, height=212, bit_depth=10, subsampling_x=1, subsampling_y=0),
     "444_8bit_u16": dict(width=264, height=140, bit_depth=8, sample_bytes=2, subsampling_x=0, subsampling_y=0),
     "mono_10bit": dict(width=328, height=200, bit_depth=10, mono=1),
+    "tiny_12bit": dict(width=20, height=12, bit_depth=12),
+    "ragged_12bit": dict(width=292, height=196, bit_depth=12),
+    "422_12bit": dict(width=296, height=212, bit_depth=12, subsampling_x=1, subsampling_y=0),
+    "444_12bit": dict(width=261, height=139, bit_depth=12, subsampling_x=0, subsampling_y=0),
+    "mono_12bit": dict(width=328, height=200, bit_depth=12, mono=1),
+    "whole_420_12bit": dict(width=2564, height=1044, bit_depth=12),
     # more superblocks than one wave of half superblocks: whole-superblock CTAs
     "whole_420_8bit": dict(width=2564, height=1044, bit_depth=8, sample_bytes=1),
     "whole_444_10bit": dict(width=2564, height=1036, bit_depth=10, subsampling_x=0, subsampling_y=0),
@@ -37,22 +43,24 @@ def ctx():
     c.close()
 
 
-@pytest.mark.parametrize("content", ["field", "extremes"])
+@pytest.mark.parametrize("content", ["field", "extremes", "noise"])
 @pytest.mark.parametrize("name", sorted(SHAPES))
 def test_cdef_stage_matches_oracle(ctx, name, content):
     sf = A.SynthHandle(**SHAPES[name], seed=91, skip_pct=15)
     info, params, maps = sf.f.info, sf.f.params, sf.f.maps
     cur = O.HostPlanes.like_synth(sf)
-    if content == "extremes":  # samples at and next to the range's ends, the strongest and weakest filters
+    if content != "field":  # samples at and next to the range's ends, or anywhere; the strongest and weakest filters
         rng = np.random.default_rng(5)
         top = (1 << info.bit_depth) - 1
         for a in cur.arrays:
-            a[...] = rng.choice(np.array([0, 1, 2, top // 2, top - 1, top], a.dtype), size=a.shape)
+            a[...] = (rng.choice(np.array([0, 1, 2, top // 2, top - 1, top], a.dtype), size=a.shape)
+                      if content == "extremes" else
+                      np.clip(top // 2 + rng.normal(0, top / 24, a.shape), 0, top).astype(a.dtype))
         for k, (yp, ys, up, us) in enumerate([(15, 4, 15, 4), (15, 0, 0, 4), (0, 4, 15, 0), (1, 1, 1, 1),
                                               (0, 0, 0, 0), (8, 2, 7, 1), (3, 4, 2, 4), (0, 1, 1, 0)]):
             params.cdef_y_pri_strength[k], params.cdef_y_sec_strength[k] = yp, ys
             params.cdef_uv_pri_strength[k], params.cdef_uv_sec_strength[k] = up, us
-        params.cdef_damping = 6
+        params.cdef_damping = 6 if content == "extremes" else 4
     want = O.HostPlanes.zeros_like(cur)
     assert O.lib().oracle_cdef(C.byref(info), C.byref(params), C.byref(maps), cur.c, want.c, 0) == 0
     df = G.DevFrame(sf)
