@@ -5,10 +5,10 @@
 //
 // Reference: rivet-av1 src/decoder/postfilter.rs:266-513, src/dsp/cdef.rs:13-90.
 //
-// What bounds it: instruction issue. (Half precision first; a tap in integers
-// is 12 instructions for two samples: 4K 12-bit 4:4:4 coded at 3072 columns 140
-// -> 104 us against the 32-bit kernel, the chain call 409 -> 378.) The constrained taps of the 32-bit
-// kernel were 70% of its 16.2 M warp instructions per 1080p frame, on the
+// What bounds it: instruction issue. A tap in integers is 12 instructions for
+// two samples: 4K 12-bit 4:4:4 coded at 3072 columns takes 104 us against the
+// 32-bit kernel's 140, the chain call 378 against 409. In half precision: the
+// constrained taps of the 32-bit kernel were 70% of its 16.2 M warp instructions per 1080p frame, on the
 // integer ALU pipe (one instruction per two clocks). Here a tap is about 10
 // instructions for two samples instead of 12 for one, half of them on the
 // multiply-add pipe, which issues every clock. 1080p 10-bit 4:2:0 against the
