@@ -416,8 +416,15 @@ constexpr int kFChunks = kFW / 8 * kFW;  // 8-sample chunks of the window (800)
 // each pass are listed in shared memory grouped by filter size, so a warp's
 // lanes mostly take one filter path, two lanes of an edge a thread
 // (lf_filter_pair). 256 threads.
+//
+// CTAs a SM: five (48 registers, a few spills) for launches of many frames, a
+// batch of 16 mixed frames 608 against 617 us with four; four for single frames,
+// whose next stage wants the room: 1080p 10-bit 50.3 against 51.1 us, 853x477 23.9
+// against 24.3 (4K 12-bit 4:4:4 would take 374 with five, 377 with four).
 template <class F>
-__global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
+constexpr int kFusedCtas = sizeof(F) == sizeof(OneFrame) ? 4 : 5;
+template <class F>
+__global__ void __launch_bounds__(256, kFusedCtas<F>) lf_fused_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
                                                      const Item* __restrict__ items, int n_items, SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
   const LfTables& tb = g_lf_tables;
@@ -615,10 +622,11 @@ __global__ void __launch_bounds__(256, 4) lf_fused_kernel(const __grid_constant_
 // tile's errors, so no filtered plane is ever written. A thread restores and
 // scores the same 8-sample chunks, so those steps need no barrier between
 // them. Bound by issued instructions (the filters of five scales; staging and
-// decisions are a fifth). A 1080p 10-bit call takes 80 us; filtered copies,
+// decisions are a fifth). A 1080p 10-bit call takes 77 us (79 with four CTAs a SM
+// instead of five); filtered copies,
 // one in-place pass a direction over all of them and a pass for the errors
 // took 200. 256 threads.
-__global__ void __launch_bounds__(256, 4) lf_search_kernel(const LfSearchDesc* __restrict__ ds, int n, int groups) {
+__global__ void __launch_bounds__(256, 5) lf_search_kernel(const LfSearchDesc* __restrict__ ds, int n, int groups) {
   const LfTables& tb = g_lf_tables;
   __shared__ __align__(16) uint16_t W0[kFW * kFS], W[kFW * kFS], S[kFT * kFT];
   __shared__ uint16_t list_v[kFCells], list_h[kFCells];
@@ -882,7 +890,7 @@ void launch_lf_fused(const FrameSet& frames, const Item* items, int n_items, Syn
 void launch_lf_search(const LfSearchDesc* ds, int n, int tiles, cudaStream_t s) {
   if (n <= 0 || tiles <= 0) return;
   // Every group stages the window and decides the edges again, so one group
-  // where the tiles fill the GPU; half a wave of them or less (4 CTAs a SM) is
+  // where the tiles fill the GPU; two of them a SM or less are
   // split. us a call with 1 / 3 / 6 groups: 640x360 (90 tiles) 43 / 33 / 33,
   // 1280x720 (360) 56 / 55 / 58, 1920x1080 (780) 80 / 82 / 105, 3840x2160
   // (3060) 191 / 253 / 327.
