@@ -59,17 +59,17 @@ METRIC = "bit-exact post-filtered Mpx/s"
 HEADLINE = dict(width=1920, height=1080, bit_depth=10)
 L2_BYTES = 126 * 2**20
 HEADLINE_WORKLOAD = "1920x1080 10-bit 4:2:0 single-frame post-filter chain (LF+CDEF+LR+pack)"
-# Per launch of each stage's kernels on the headline workload, from one ncu capture of the headline
-# bench (profiles/metrics_1080p10_chain.md gives the command): DRAM bytes read and written
+# Per launch of each stage's kernels on the headline workload, from one ncu capture of a headline
+# frame (profiles/kernels.md gives the command): DRAM bytes read and written
 # (dram__bytes_read.sum, dram__bytes_write.sum) and warp-instructions executed
 # (smsp__inst_executed.sum). ncu flushes the caches before a captured launch, so the reads are cold;
 # a frame's 6-19 MB of writes stay in the 126 MB L2 when the launch ends, so the writes read near 0
 # (they reach DRAM later, during the next launches). The headline frames have no film grain: the
 # loop-restoration kernel packs them and no output kernel runs.
 NCU_HEADLINE = {
-    "loop_filter": {"dram_read": 8345344, "dram_write": 0, "warp_inst": 10128792},  # lf_fused_kernel (mode 3)
-    "cdef": {"dram_read": 6999808, "dram_write": 0, "warp_inst": 16245271},
-    "loop_restoration": {"dram_read": 8367872, "dram_write": 13312, "warp_inst": 14475086},
+    "loop_filter": {"dram_read": 8354048, "dram_write": 0, "warp_inst": 8443133},  # lf_fused_kernel (mode 3)
+    "cdef": {"dram_read": 7251456, "dram_write": 4608, "warp_inst": 10472039},
+    "loop_restoration": {"dram_read": 6830592, "dram_write": 0, "warp_inst": 9491721},
 }
 B200_SMS, ISSUE_PER_SM_CLK = 148, 4  # four schedulers per SM, one warp-instruction each per clock
 
