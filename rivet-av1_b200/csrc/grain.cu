@@ -319,11 +319,39 @@ __device__ __forceinline__ void ar_plane(int lag, int16_t (*T)[kTW], const int16
   }
 }
 
+// The same for a plane whose coefficients do not all fit the 8 bits that the
+// dot products take (no stream codes such values, but the parameters' fields
+// hold them): a warp walks the cells one by one, a lane a tap, in 32 bits.
+__device__ __noinline__ void ar_wide(int lag, int16_t (*T)[kTW], const int16_t (*Y)[kTW], const int32_t* coef, int H,
+                                     int W, int ar_shift, int gmin, int gmax, int sub_x, int sub_y, bool luma_on) {
+  const int lane = threadIdx.x & 31, taps = 2 * lag * (lag + 1), row = 2 * lag + 1;
+  const int dy = lane / row - lag, dx = lane % row - lag;
+  const bool tap = lane < taps, luma = lane == taps && luma_on;
+  const int c = tap || luma ? coef[lane] : 0;
+  for (int y = 3; y < H; y++)
+    for (int x = 3; x < W - 3; x++) {
+      int v = 0;
+      if (tap) v = T[y + dy][x + dx];
+      if (luma) {
+        const int16_t* at = &Y[((y - 3) << sub_y) + 3][((x - 3) << sub_x) + 3];
+        v = at[0];
+        if (sub_x) v += at[1];
+        if (sub_y) v += at[kTW];
+        if (sub_x && sub_y) v += at[kTW + 1];
+        v = round2(v, sub_x + sub_y);
+      }
+      const int sum = __reduce_add_sync(0xffffffffu, v * c);
+      if (lane == 0) T[y][x] = int16_t(clip3(gmin, gmax, T[y][x] + round2(sum, ar_shift)));
+      __syncwarp();
+    }
+}
+
 // One CTA of 256 threads per frame. All threads fill the templates with
 // Gaussian values (one template row each). Then warps 0, 1 and 2 run the
 // luma, Cb and Cr auto-regressions side by side, chroma trailing luma,
 // while warps 3-7 build the scaling tables (one entry per thread) and the
-// per-stripe block offsets (one stripe per thread).
+// per-stripe block offsets (one stripe per thread). (With a coefficient beyond
+// 8 bits warp 0 does all three planes, ar_wide.)
 template <class F>
 __global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__ F one, const FrameDesc* __restrict__ frames,
                                                      const Item* __restrict__ items, int n_items, SyncFlags sync) {
@@ -370,7 +398,11 @@ __global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__
       coef[2][tid] = g.ar_coeffs_cr_plus_128[tid] - 128;
     }
     if (tid == 0) progress = 0u;
-    __syncthreads();
+    const int lag = g.ar_coeff_lag;
+    // (the last coefficient, chroma's luma term, is not packed)
+    auto beyond8 = [&](int v) { return v != int(int8_t(v)); };
+    const bool wide = __syncthreads_or(tid < 2 * lag * (lag + 1) &&
+                                       (beyond8(coef[0][tid]) || (!mono && (beyond8(coef[1][tid]) || beyond8(coef[2][tid])))));
     {
       int plane = -1, row = tid;
       if (row < kTH) {
@@ -403,9 +435,13 @@ __global__ void __launch_bounds__(256) grain_prep_kernel(const __grid_constant__
       }
     }
     __syncthreads();
-    const int lag = g.ar_coeff_lag;
     const int ar_shift = g.ar_coeff_shift_minus_6 + 6;
-    if (warp == 0) {
+    if (wide && warp <= 2) {
+      if (warp == 0)
+        for (int p = 0; p < (mono ? 1 : 3); p++)
+          ar_wide(lag, T[p], T[0], coef[p], p ? chroma_h : kTH, p ? chroma_w : kTW, ar_shift, grain_min, grain_max,
+                  p ? sub_x : 0, p ? sub_y : 0, p && g.num_y_points > 0);
+    } else if (warp == 0) {
       // --- luma auto-regression (grain.rs:55-73) ---
       ar_plane<false>(lag, T[0], T[0], coef[0], kTH, kTW, ar_shift, grain_min, grain_max, 0, 0, false, &progress);
     } else if (warp <= 2) {

@@ -47,3 +47,22 @@ def test_grain_lags_match_oracle(ctx, name, lag, coefs):
     for p, (a, b) in enumerate(zip(ref_gpu, ref_cpu.arrays)):
         assert np.array_equal(a, b), f"reference plane {p}"
     assert np.array_equal(fb_gpu, fb_cpu), f"{(fb_gpu != fb_cpu).sum()} bytes differ"
+
+
+@pytest.mark.parametrize("lag", [0, 1, 2, 3])
+@pytest.mark.parametrize("name", ["420_8bit", "422_10bit", "444_12bit", "mono_12bit"])
+def test_grain_coefficients_beyond_8_bits(ctx, name, lag):
+    """The coefficients' fields are 32 bits wide and are not checked: values that
+    no stream codes are multiplied as they are, in one plane or in all."""
+    sf = A.SynthHandle(width=200, height=136, enable_grain=1, seed=60 + lag, frame_index=5 + lag, **LAYOUTS[name])
+    g = sf.f.params.film_grain
+    g.ar_coeff_lag = lag
+    g.ar_coeff_shift_minus_6 = 3
+    results = []
+    for arr in (g.ar_coeffs_y_plus_128, g.ar_coeffs_cb_plus_128, g.ar_coeffs_cr_plus_128):
+        arr[0], arr[2 * lag * (lag + 1) - 1 if lag else 0] = 128 + 200, 128 - 700
+        results.append((O.chain(sf), G.gpu_chain(ctx, G.DevFrame(sf))))
+    for k, ((ref_cpu, fb_cpu), (ref_gpu, fb_gpu)) in enumerate(results):
+        for p, (a, b) in enumerate(zip(ref_gpu, ref_cpu.arrays)):
+            assert np.array_equal(a, b), f"step {k} reference plane {p}"
+        assert np.array_equal(fb_gpu, fb_cpu), f"step {k}: {(fb_gpu != fb_cpu).sum()} bytes differ"
