@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 
 #include <cfloat>
+#include <utility>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -215,6 +216,9 @@ __global__ void __launch_bounds__(kClusterThreads) cdef_greedy_cluster_kernel(co
   uint32_t* const best32 = reinterpret_cast<uint32_t*>(best + pitch);
   uint32_t* const rows = best32 + pitch;  // the chroma rows, then the luma rows from y_first
   const uint64_t* const sse = d.sse;
+  // The first store to a peer's shared memory must find the peer started: every
+  // CTA arrives here and waits before its first step, the staging in between.
+  cg::cluster_group::arrival_token started = cluster.barrier_arrive();
   pdl_wait();
   bool large = false;  // some error too large for a lane's sum of pitch / 32 pairs of them
   const uint64_t limit = (uint64_t(1) << 31) / unsigned(pitch / 32);
@@ -232,6 +236,7 @@ __global__ void __launch_bounds__(kClusterThreads) cdef_greedy_cluster_kernel(co
     }
   }
   large = __syncthreads_or(large);
+  cluster.barrier_wait(std::move(started));
   const double nb = double(d.g->nb), lambda = d.lambda;
   int set[8];  // the pairs chosen
   int best_bits = 0;

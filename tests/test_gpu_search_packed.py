@@ -102,3 +102,14 @@ def test_block_errors_under_a_tight_cap(ctx):
     tight = G.Ctx(0, held.value - 512)
     check(search(tight, frames, 90, 20.0, False), frames, 90, 20.0, False)
     tight.close()
+
+
+@pytest.mark.parametrize("thorough", [False, True], ids=["fast", "thorough"])
+def test_batch_of_single_blocks(ctx, thorough):
+    """Many frames of one block: clusters that start apart and stage next to nothing before their first exchange."""
+    shapes = [dict(width=16 + 5 * i, height=70 - 6 * i, bit_depth=(8, 10, 12)[i % 3]) for i in range(9)]
+    frames = []
+    for i in range(45):
+        sf = A.SynthHandle(**shapes[i % 9], seed=200 + i)
+        frames.append((sf, *O.search_inputs(sf, 90 + i, amp=24)))
+    check(search(ctx, frames, 80, 9.0, thorough), frames, 80, 9.0, thorough)
