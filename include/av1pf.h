@@ -306,7 +306,16 @@ int av1pf_output_noalloc(const av1pf_frame_info* info, const av1pf_params* param
  * filtered) differs from that of the calls before it first uploads its work
  * lists, and may wait on the host for the chain queued two calls earlier.
  * The parameters are read before the call returns; the planes and maps when
- * the kernels run. */
+ * the kernels run.
+ *
+ * `stream` may be in capture (any mode; so with the stage calls above): the
+ * parameters are then those of every replay, and the call's work lists and
+ * scratch are device memory of its own, which the context holds until the
+ * graph and everything instantiated from it are destroyed (it is freed by a
+ * later call on the context). Direct calls and replays may alternate freely.
+ * Where the memory cap has no room for that scratch, the call shares the
+ * context's: its replays and the context's other calls must then be ordered
+ * (one stream, or events). No replay may run after av1pf_ctx_destroy. */
 int av1pf_chain(av1pf_ctx* ctx, const av1pf_frame_info* info,
                 const av1pf_params* params, const av1pf_maps* maps,
                 const av1pf_plane* in, av1pf_plane* ref_out,

@@ -143,9 +143,129 @@ inline void end() {}
 #endif
 }  // namespace pipe_trace
 
+// The scratch of direct calls. One that captured calls share is kept for their
+// replays when it is outgrown.
+int Ctx::ensure_scratch(size_t bytes) {
+  if (scratch.size >= bytes) return AV1PF_OK;
+  bool shared = false;
+  for (const Captured& c : captured) shared |= c.shares;
+  if (!shared) return ensure(scratch, bytes);
+  DevBuf larger;
+  const int rc = ensure(larger, bytes);
+  if (rc != AV1PF_OK) return rc;
+  retired.push_back(scratch);
+  scratch = larger;
+  return AV1PF_OK;
+}
+
+// Frees what the captured calls held whose graphs are gone, or of all of them.
+void Ctx::reap_captured(bool all) {
+  bool shared = false;
+  for (size_t k = 0; k < captured.size();) {
+    Captured& c = captured[k];
+    if (!all && !c.gone->load()) {
+      shared |= c.shares;
+      k++;
+      continue;
+    }
+    release(c.meta);
+    release(c.scratch);
+    captured.erase(captured.begin() + std::ptrdiff_t(k));
+  }
+  for (size_t k = 0; !shared && k < retired.size(); k++) release(retired[k]);
+  if (!shared) retired.clear();
+}
+
+cudaError_t Ctx::upload_stream() {
+  cudaError_t e = cudaSuccess;
+  if (!upload) {
+    e = cudaStreamCreateWithFlags(&upload, cudaStreamNonBlocking);
+    for (MetaSlot& m : metas)
+      for (cudaEvent_t* ev : {&m.uploaded, &m.done})
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  }
+  return e;
+}
+
+// A call on a stream that is being captured: planned apart, with buffers that
+// are uploaded now and belong to the graph. Its stages wait for one another
+// whole (the replays would all carry the epoch of the capture), and its grain
+// templates join the capture.
+int Ctx::capture(const FrameJob* jobs, int n, cudaStream_t s) {
+  // allocations and the upload are no part of the capture, whatever its mode
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  cudaError_t e = cudaStreamGetCaptureInfo(s, &status, &id, &graph);
+  if (e != cudaSuccess || status != cudaStreamCaptureStatusActive)
+    return cuda_status(e == cudaSuccess ? cudaErrorStreamCaptureInvalidated : e, "stream capture");
+  if ((e = upload_stream()) != cudaSuccess) return cuda_status(e, "descriptor stream");
+  Plan p;
+  std::string why;
+  int rc = build_plan(jobs, n, nullptr, p, &why);
+  if (rc != AV1PF_OK) return set_error(why), rc;
+  Captured c;
+  if ((rc = ensure(c.meta, p.meta_bytes + 256)) != AV1PF_OK) return rc;
+  if ((rc = ensure(c.scratch, p.scratch_bytes + 256)) != AV1PF_OK) {
+    cudaGetLastError();
+    c.shares = true;
+    rc = ensure_scratch(p.scratch_bytes + 256);
+  }
+  if (rc == AV1PF_OK)
+    rc = build_plan(jobs, n, static_cast<uint8_t*>(c.shares ? scratch.ptr : c.scratch.ptr), p, &why, false);
+  if (rc == AV1PF_OK) {
+    uint8_t* dmeta = static_cast<uint8_t*>(c.meta.ptr);
+    p.grain_in_meta(dmeta);
+    std::vector<uint8_t> host(p.upload_bytes);
+    pack_meta(p, host.data());
+    e = cudaMemcpyAsync(dmeta, host.data(), p.upload_bytes, cudaMemcpyHostToDevice, upload);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(upload);
+    if (e == cudaSuccess) {
+      launch_plan(p, dmeta, s, side, fork, join, nullptr, false, false, false, p.by_value);
+      e = cudaGetLastError();
+    }
+    rc = cuda_status(e, "captured call");
+  }
+  if (rc != AV1PF_OK) {
+    release(c.meta);
+    release(c.scratch);
+    return rc;
+  }
+  c.gone = std::make_shared<std::atomic<bool>>(false);
+  auto* held_by_graph = new std::shared_ptr<std::atomic<bool>>(c.gone);
+  cudaUserObject_t object = nullptr;
+  e = cudaUserObjectCreate(
+      &object, held_by_graph,
+      [](void* p) {
+        auto* gone = static_cast<std::shared_ptr<std::atomic<bool>>*>(p);
+        (*gone)->store(true);
+        delete gone;
+      },
+      1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {  // (the buffers then stay until the context goes)
+    delete held_by_graph;
+    cudaGetLastError();
+  } else if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaGetLastError();
+    c.gone = std::make_shared<std::atomic<bool>>(false);
+    cudaUserObjectRelease(object, 1);
+  }
+  captured.push_back(std::move(c));
+  return AV1PF_OK;
+}
+
 // Plans `jobs`, sizes scratch and a descriptor buffer, uploads and launches
 // on `s`.
 int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) cudaGetLastError();
+  if (status != cudaStreamCaptureStatusNone) return capture(jobs, n, s);
+  if (!captured.empty()) reap_captured(false);
   std::string why;
   int rc = AV1PF_OK;
   // Jobs with the structure of the previous call (a decoder filtering frame
@@ -171,11 +291,11 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     // memory cap the second scratch could take what another call needs.
     scratch_half = (plan.scratch_bytes + 511) / 256 * 256;
     scratch_turns = plan.flag_sync && plan.by_value && cap == 0 && plan.lff_items.size() <= size_t(kNumSMs) * 4;
-    if (scratch_turns && (rc = ensure(scratch, 2 * scratch_half)) != AV1PF_OK) {
+    if (scratch_turns && (rc = ensure_scratch(2 * scratch_half)) != AV1PF_OK) {
       cudaGetLastError();
       scratch_turns = false;
     }
-    if (!scratch_turns && (rc = ensure(scratch, plan.scratch_bytes + 256)) != AV1PF_OK) return rc;
+    if (!scratch_turns && (rc = ensure_scratch(plan.scratch_bytes + 256)) != AV1PF_OK) return rc;
     // the lists are built; with the scratch in place only the descriptors change
     rc = build_plan(jobs, n, scratch_base(), plan, &why, false);
     if (rc != AV1PF_OK) return set_error(why), rc;
@@ -186,19 +306,8 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   // it was last used for, readiness flags and film-grain scratch. A call whose
   // kernels take the descriptor as a parameter and whose buffer holds its lists
   // uploads nothing: it only launches.
-  cudaError_t e = cudaSuccess;
-  if (!upload) {
-    e = cudaStreamCreateWithFlags(&upload, cudaStreamNonBlocking);
-    for (MetaSlot& q : metas)
-      for (cudaEvent_t* ev : {&q.uploaded, &q.done})
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
-    if (e != cudaSuccess) return cuda_status(e, "descriptor stream");
-  }
-  // A capture replays its launches with the epoch they were captured with, so
-  // its stages wait for one another whole; its templates join the capture.
-  cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cap_status) != cudaSuccess) cudaGetLastError();
-  const bool capturing = cap_status != cudaStreamCaptureStatusNone;
+  cudaError_t e = upload_stream();
+  if (e != cudaSuccess) return cuda_status(e, "descriptor stream");
   if (epoch >= kEpochMax) {
     // flags and words are compared with the epoch: before it could wrap, every
     // call is done and all of them start over
@@ -209,7 +318,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
     if ((e = cudaMemset(words, 0, kWords * 4)) != cudaSuccess) return cuda_status(e, "epoch words");
     epoch = 0;
   }
-    const int turn = meta_next;
+  const int turn = meta_next;
   MetaSlot& m = metas[turn];
   meta_next ^= 1;
   if (m.dev.size < plan.meta_bytes + 256) {
@@ -220,11 +329,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   uint8_t* dmeta = static_cast<uint8_t*>(m.dev.ptr);
   // film grain: this buffer's own scratch (the previous call's output kernel
   // reads the other buffer's), so the template kernel can start at once
-  for (size_t fi = 0; fi < plan.frames.size() && fi < plan.grain_meta.size(); fi++) {
-    if (plan.grain_meta[fi].first == SIZE_MAX) continue;
-    plan.frames[fi].grain = reinterpret_cast<GrainScratch*>(dmeta + plan.off_grain_meta + plan.grain_meta[fi].first);
-    plan.frames[fi].grain_off = dmeta + plan.off_grain_meta + plan.grain_meta[fi].second;
-  }
+  plan.grain_in_meta(dmeta);
   const bool resident = m.ready && m.key == key_scratch;
   // Calls of small frames wait for the calls before them by words (SyncFlags).
   // With film grain the template kernel then runs first on the call's stream
@@ -232,11 +337,11 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   // third of a SM's registers each, so only where at most one lands on a SM (us a call,
   // against templates on the side stream and no overlap: 640x360 27.8 / 44.7,
   // 1280x720 53.9 / 52.1, 1920x1080 70.8 / 72.4, 3840x2160 235 / 233).
-  const bool chained = scratch_turns && plan.by_value && !plan.lff_items.empty() && !capturing && !prof &&
+  const bool chained = scratch_turns && plan.by_value && !plan.lff_items.empty() && !prof &&
                        (!plan.any_grain || plan.out_items.size() <= size_t(kNumSMs));
   if (plan.by_value && resident) {
     // the scratch's last readers are the launches that used this buffer before
-    if (plan.any_grain && !chained && m.used && !capturing) e = cudaStreamWaitEvent(side, m.done, 0);
+    if (plan.any_grain && !chained && m.used) e = cudaStreamWaitEvent(side, m.done, 0);
   } else {
     // the pinned staging buffer: its last upload must be done before it is
     // overwritten; the device buffer: its last readers
@@ -295,8 +400,8 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   }
   chain_run = chained ? before + 1 : 0;
   last_stream = s;
-  rc = launch_on(dmeta, s, capturing, call);
-  if (!capturing) cudaEventRecord(m.done, s);
+  rc = launch_on(dmeta, s, call);
+  cudaEventRecord(m.done, s);
   return rc;
 }
 
@@ -305,7 +410,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
 // chain without a gap at the call boundary (the first loop-filter kernel of
 // a call starts its launch while the previous call's last kernel drains);
 // profiled calls record stage events between the stages.
-int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing, const SyncFlags& call) {
+int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, const SyncFlags& call) {
   const cudaEvent_t* ev = nullptr;
   if (prof) {
     const int slot = prof_next;
@@ -316,7 +421,7 @@ int Ctx::launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing, const SyncFla
     prof_used[slot] = true;
     ev = prof_ev[slot];
   }
-  launch_plan(plan, dmeta, s, side, fork, join, ev, true, !capturing, !capturing, plan.by_value, call);
+  launch_plan(plan, dmeta, s, side, fork, join, ev, true, true, true, plan.by_value, call);
   return cuda_status(cudaGetLastError(), "kernel launch");
 }
 
@@ -431,6 +536,7 @@ int av1pf_ctx_destroy(av1pf_ctx* ctx) {
   if (!ctx) return AV1PF_OK;
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
+  ctx->reap_captured(true);
   ctx->release(ctx->scratch);
   for (Ctx::MetaSlot& m : ctx->metas) {
     ctx->release(m.dev);

@@ -4,8 +4,10 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -105,6 +107,17 @@ struct Ctx {
   // the descriptor buffers
   bool scratch_turns = false;
   size_t scratch_half = 0;
+  // A call made while its stream is captured: its replays, which the context
+  // does not see, read work lists and scratch of their own until the graph and
+  // what was instantiated from it are gone (`gone`, set by the graph's user
+  // object), so a direct call neither rewrites nor frees them.
+  struct Captured {
+    DevBuf meta, scratch;
+    bool shares = false;  // no room for a scratch of its own: it uses the context's, in stream order
+    std::shared_ptr<std::atomic<bool>> gone;
+  };
+  std::vector<Captured> captured;
+  std::vector<DevBuf> retired;  // scratches that captured calls share and the context has outgrown
   cudaStream_t upload = nullptr;  // descriptor uploads
   // the chain's stream, not the host, waits for the descriptor upload: set
   // by callers whose chains begin with a stream wait anyway (the host-buffer
@@ -137,7 +150,11 @@ struct Ctx {
   int ensure_host(HostBuf& b, size_t bytes);
   void release(DevBuf& b);
   int run(const FrameJob* jobs, int n, cudaStream_t s);
-  int launch_on(uint8_t* dmeta, cudaStream_t s, bool capturing, const SyncFlags& call);
+  int capture(const FrameJob* jobs, int n, cudaStream_t s);
+  void reap_captured(bool all);
+  int ensure_scratch(size_t bytes);
+  cudaError_t upload_stream();
+  int launch_on(uint8_t* dmeta, cudaStream_t s, const SyncFlags& call);
 };
 
 void set_error(const std::string& s);

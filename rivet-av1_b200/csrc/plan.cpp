@@ -559,6 +559,14 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
   return AV1PF_OK;
 }
 
+void Plan::grain_in_meta(uint8_t* meta) {
+  for (size_t fi = 0; fi < frames.size() && fi < grain_meta.size(); fi++) {
+    if (grain_meta[fi].first == SIZE_MAX) continue;
+    frames[fi].grain = reinterpret_cast<GrainScratch*>(meta + off_grain_meta + grain_meta[fi].first);
+    frames[fi].grain_off = meta + off_grain_meta + grain_meta[fi].second;
+  }
+}
+
 void structure_key(const FrameJob* jobs, int n, std::vector<int64_t>& key) {
   key.clear();
   key.push_back(n);

@@ -69,6 +69,8 @@ struct Plan {
   // previous call's output kernel reads.
   size_t off_grain_meta = 0;
   std::vector<std::pair<size_t, size_t>> grain_meta;
+  // points the descriptors there, in the device meta buffer `meta`
+  void grain_in_meta(uint8_t* meta);
   // one frame, all of whose kernels take its descriptor as a parameter
   bool by_value = false;
   int sr_row_max = 0;      // superres: the most source samples in a row (sr_maxx + 1)
