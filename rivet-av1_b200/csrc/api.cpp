@@ -143,6 +143,42 @@ inline void end() {}
 #endif
 }  // namespace pipe_trace
 
+namespace {
+std::pair<uintptr_t, uintptr_t> span_of(const av1pf_plane& p, int w, int h, int sb) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p.data);
+  return {at, at + uintptr_t((int64_t(h - 1) * p.stride + w) * sb)};
+}
+}  // namespace
+
+bool Written::holds_input(const FrameJob* jobs, int n) const {
+  for (int fi = 0; fi < n; fi++) {
+    const FrameJob& j = jobs[fi];
+    for (int k = 0; k < j.info->num_planes; k++)
+      for (const av1pf_plane* in : {j.in, j.cur}) {
+        if (!in) continue;
+        const auto s = span_of(in[k], in[k].width, in[k].height, j.info->sample_bytes);
+        for (const auto& w : spans)
+          if (s.first < w.second && w.first < s.second) return true;
+      }
+  }
+  return false;
+}
+
+void Written::add(const FrameJob* jobs, int n) {
+  auto put = [&](const std::pair<uintptr_t, uintptr_t>& s) {
+    if (std::find(spans.begin(), spans.end(), s) == spans.end()) spans.push_back(s);
+  };
+  for (int fi = 0; fi < n; fi++) {
+    const FrameJob& j = jobs[fi];
+    for (int k = 0; j.out && k < j.info->num_planes; k++)
+      put(span_of(j.out[k], j.out[k].width, j.out[k].height, j.info->sample_bytes));
+    if (j.frame_out) {
+      const uintptr_t at = reinterpret_cast<uintptr_t>(j.frame_out);
+      put({at, at + packed_frame_bytes(j.info)});
+    }
+  }
+}
+
 // The scratch of direct calls. One that captured calls share is kept for their
 // replays when it is outgrown.
 int Ctx::ensure_scratch(size_t bytes) {
@@ -226,7 +262,13 @@ int Ctx::capture(const FrameJob* jobs, int n, cudaStream_t s) {
     e = cudaMemcpyAsync(dmeta, host.data(), p.upload_bytes, cudaMemcpyHostToDevice, upload);
     if (e == cudaSuccess) e = cudaStreamSynchronize(upload);
     if (e == cudaSuccess) {
-      launch_plan(p, dmeta, s, side, fork, join, nullptr, false, false, false, p.by_value);
+      // (calls captured one after another overlap as direct ones do)
+      SyncFlags call;
+      if (capture_id != id) capture_written.spans.clear();
+      capture_id = id;
+      call.whole = capture_written.holds_input(jobs, n) || capture_written.spans.size() > Written::kMost;
+      capture_written.add(jobs, n);
+      launch_plan(p, dmeta, s, side, fork, join, nullptr, false, false, false, p.by_value, call);
       e = cudaGetLastError();
     }
     rc = cuda_status(e, "captured call");
@@ -337,7 +379,10 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   // third of a SM's registers each, so only where at most one lands on a SM (us a call,
   // against templates on the side stream and no overlap: 640x360 27.8 / 44.7,
   // 1280x720 53.9 / 52.1, 1920x1080 70.8 / 72.4, 3840x2160 235 / 233).
-  const bool chained = scratch_turns && plan.by_value && !plan.lff_items.empty() && !prof &&
+  // Where an input is what a call before this one writes, this one waits for it
+  // whole before it reads. (The list is of one stream's calls.)
+  const bool whole = unseen || last_stream != s || written.spans.size() > Written::kMost || written.holds_input(jobs, n);
+  const bool chained = !whole && scratch_turns && plan.by_value && !plan.lff_items.empty() && !prof &&
                        (!plan.any_grain || plan.out_items.size() <= size_t(kNumSMs));
   if (plan.by_value && resident) {
     // the scratch's last readers are the launches that used this buffer before
@@ -398,7 +443,13 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
       call.lf_wait = epoch - 2;
     }
   }
+  call.whole = whole;
   chain_run = chained ? before + 1 : 0;
+  // a call that does not run ahead lets the next begin only once the calls
+  // before it on its stream are complete
+  if (!call.ahead) written.spans.clear();
+  written.add(jobs, n);
+  unseen = false;
   last_stream = s;
   rc = launch_on(dmeta, s, call);
   cudaEventRecord(m.done, s);

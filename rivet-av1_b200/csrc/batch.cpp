@@ -75,7 +75,10 @@ void launch_groups(Batch& b, cudaStream_t s) {
     cudaStream_t gs = g ? G.stream : s;
     // the stages' readiness flags start cleared on every run
     if (G.plan.n_flags) cudaMemsetAsync(meta + G.plan.off_flags, 0, G.plan.n_flags * 4, gs);
-    launch_plan(G.plan, meta, gs, G.side, G.fork, G.join, nullptr, false, true);
+    // (a frame's input may be what a call or run before this one writes)
+    SyncFlags sync;
+    sync.whole = true;
+    launch_plan(G.plan, meta, gs, G.side, G.fork, G.join, nullptr, false, true, false, false, sync);
   }
   for (size_t g = 1; g < n; g++) {
     cudaEventRecord(b.groups[g].done, b.groups[g].stream);
@@ -232,6 +235,7 @@ int av1pf_batch_run(av1pf_batch* b, void* stream) {
     note_launch(b->kernels_per_run);
   } else {
     launch_groups(*b, s);
+    b->ctx->unseen = true;
     e = cudaGetLastError();
   }
   return cuda_status(e, "batch run");

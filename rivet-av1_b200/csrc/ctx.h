@@ -11,6 +11,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "av1pf.h"
@@ -49,6 +50,15 @@ struct CaptureScope {
   ~CaptureScope();
   uint64_t launches() const;  // launches enqueued in this scope so far
   uint64_t start;
+};
+
+// The memory that calls write whose end the next call's first kernel may not
+// wait for before it reads its inputs.
+struct Written {
+  static constexpr size_t kMost = 128;
+  std::vector<std::pair<uintptr_t, uintptr_t>> spans;  // [first, past the last)
+  bool holds_input(const FrameJob* jobs, int n) const;
+  void add(const FrameJob* jobs, int n);
 };
 
 struct Ctx {
@@ -99,6 +109,8 @@ struct Ctx {
   uint32_t epoch = 0;
   cudaStream_t last_stream = nullptr;  // of the previous call
   int chain_run = 0;                   // chained calls of one structure and stream up to the previous one
+  Written written;
+  bool unseen = false;  // launches that `written` does not cover (batches run without a graph)
   // device words (SyncFlags): [0] the last call known to be complete, [1 + turn]
   // the last call whose film-grain templates are ready in that buffer
   static constexpr int kWords = 64;
@@ -117,6 +129,8 @@ struct Ctx {
     std::shared_ptr<std::atomic<bool>> gone;
   };
   std::vector<Captured> captured;
+  unsigned long long capture_id = 0;
+  Written capture_written;  // by the captured calls of that capture
   std::vector<DevBuf> retired;  // scratches that captured calls share and the context has outgrown
   cudaStream_t upload = nullptr;  // descriptor uploads
   // the chain's stream, not the host, waits for the descriptor upload: set

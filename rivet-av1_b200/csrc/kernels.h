@@ -86,6 +86,10 @@ struct FrameSet {
 // next launch as they start, and loop restoration, which writes the caller's
 // planes, waits for the previous call.
 //
+// whole: the fused loop filter waits for the kernel before it ahead of reading
+// its inputs (which may be what that kernel, or a call before it, writes);
+// otherwise it reads them at once and waits only before it writes.
+//
 // grain: set to the epoch by the film-grain template kernel, which then runs
 // first on the call's own stream, one CTA beside the chain (so it has started
 // before the output kernel can wait for it), or null: it runs on another
@@ -96,6 +100,7 @@ struct SyncFlags {
   uint32_t* complete = nullptr;
   uint32_t lf_wait = 0;  // the loop filter waits for this in `complete` before it writes; 0: for the previous kernel
   bool ahead = false;
+  bool whole = false;
   uint32_t* grain = nullptr;
 };
 

@@ -432,6 +432,7 @@ __global__ void __launch_bounds__(256, kFusedCtas<F>) lf_fused_kernel(const __gr
   __shared__ uint32_t list_v[kFCells], list_h[kFCells];
   __shared__ uint32_t cnt[2][4], base[2][4];
   const int tid = threadIdx.x;
+  if (flags.whole) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (flags.ahead) pdl_trigger();
   FOR_EACH_ITEM(it, n_items) {
     const Item item = items[it];
@@ -570,9 +571,10 @@ __global__ void __launch_bounds__(256, kFusedCtas<F>) lf_fused_kernel(const __gr
     }
     __syncthreads();
     // Up to here the tile read only this call's inputs (the unfiltered
-    // planes, the maps, the descriptor) and worked in shared memory, so it
-    // ran while the previous call's stages drained; cur, which they read, is
-    // written only past this wait or the one above.
+    // planes, the maps, the descriptor), which no unfinished call writes
+    // (flags.whole), and worked in shared memory, so it ran while the previous
+    // call's stages drained; cur, which they read, is written only past this
+    // wait or the one above.
     if (!flags.lf_wait)
       pdl_wait();
     else if (!flags.ahead)
