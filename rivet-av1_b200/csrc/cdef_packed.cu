@@ -342,14 +342,15 @@ __device__ __forceinline__ void stage_windows(const FrameDesc& f, int sc, int y0
 
 // With readiness flags: waits (threads 0..47, one flag each) for the
 // loop-filter tiles under the CTA's windows: plane rows (y0 >> sy) - 2 ..
-// ((y0 + R) >> sy) + 1 and 8 columns past the superblock on either side.
+// ((y0 + R) >> sy) + 1 and 8 columns past the superblock on either side, in the
+// mode-info area (which all windows together cover, so every tile is waited for).
 template <int R>
 __device__ __forceinline__ void packed_wait_lf(const FrameDesc& f, const SyncFlags& flags, int sc, int y0, int tid) {
   if (tid >= 48) return;
   const int p = tid >> 4, dy = (tid >> 2) & 3, dx = tid & 3;
   if (p >= f.np || f.lf_tiles_x[p] == 0) return;
   const int sx = plane_ssx(f, p), sy = plane_ssy(f, p);
-  const int W = f.cur[p].w, H = f.cur[p].h;
+  const int W = (f.mi_cols * 4) >> sx, H = (f.mi_rows * 4) >> sy;
   const int r0 = max((y0 >> sy) - 2, 0), r1 = min(((y0 + R) >> sy) + 1, H - 1);
   const int c0 = max(((sc * 64) >> sx) - 8, 0), c1 = min(((sc * 64 + 64) >> sx) + 7, W - 1);
   const int ty = (r0 >> 6) + dy, tx = (c0 >> 6) + dx;

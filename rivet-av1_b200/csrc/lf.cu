@@ -401,8 +401,7 @@ constexpr int kFCells = kFCR * kFCC;
 constexpr int kFChunks = kFW / 8 * kFW;  // 8-sample chunks of the window (800)
 }  // namespace
 
-// Loop filter, both passes, one 64x64 tile per CTA (kind bit 0: the tile is
-// copied in -> cur; bit 1: it overlaps the mode-info area and is filtered).
+// Loop filter, both passes, one 64x64 tile of the mode-info area per CTA, in -> cur.
 // The tile and 8 samples on every side are staged once from the unfiltered
 // input. Every vertical edge that changes a staged row at the tile's columns
 // (edges at x0 .. x0 + 64) is filtered in shared memory, including the 8
@@ -443,20 +442,17 @@ __global__ void __launch_bounds__(256, kFusedCtas<F>) lf_fused_kernel(const __gr
     const int x0 = item.x0, y0 = item.y0;
     const int x1 = min(int(item.x1), src.w), y1 = min(int(item.y1), src.h);
     const int rows = y1 - y0;
-    const bool filt = (item.kind & 2) != 0;
     const int wx0 = x0 - kFH, wy0 = y0 - kFH;
     if (tid < 8) (&cnt[0][0])[tid] = 0u;  // every thread read the previous item's counts
     __syncthreads();  // the previous item's window is written out
-    // --- stage the window: a filtered tile takes all of it, a copied one its own samples ---
-    const int r_lo = filt ? 0 : kFH, r_hi = filt ? kFW : kFH + rows;
-    const int c_lo = filt ? 0 : 1, c_hi = filt ? kFW / 8 : 1 + kFT / 8;
+    // --- stage the window ---
     uint2 q8[4];
 #pragma unroll
     for (int m = 0; m < 4; m++) {
       const int k = tid + m * 256;
       const int r = k / 10, ch = k - r * 10;
       q8[m] = make_uint2(0u, 0u);
-      if (k >= kFChunks || r < r_lo || r >= r_hi || ch < c_lo || ch >= c_hi) continue;
+      if (k >= kFChunks) continue;
       const int gy = wy0 + r, gx = wx0 + ch * 8;
       uint16_t* wp = &W[r * kFS + ch * 8];
       if (gy < 0 || gy >= src.h) {
@@ -486,37 +482,35 @@ __global__ void __launch_bounds__(256, kFusedCtas<F>) lf_fused_kernel(const __gr
     // edges of the tile's 17 x 16 (postfilter.rs:107-264) ---
     int dv[2] = {0, 0}, dh[2] = {0, 0};
     const int cx0 = x0 >> 2, cy0 = (y0 >> 2) - 2;
-    if (filt) {
-      const int sx = plane_ssx(f, plane), sy = plane_ssy(f, plane);
-      const int gw = f.mi_cols >> sx, gh = f.mi_rows >> sy;
+    const int sx = plane_ssx(f, plane), sy = plane_ssy(f, plane);
+    const int gw = f.mi_cols >> sx, gh = f.mi_rows >> sy;
 #pragma unroll
-      for (int m = 0; m < 2; m++) {
-        const int k = tid + m * 256;
-        if (k >= kFCells) break;
-        const int i = k / kFCC, j = k - i * kFCC;
-        const int cx = cx0 + j, cy = cy0 + i;
-        if (cx < 0 || cy < 0 || cx >= gw || cy >= gh) continue;
-        int v = 0, h = 0;
-        lf_decide2(f, tb, plane, cx, cy, v, h);
-        // a conformant map keeps wide edges off the plane start
-        if (v && cx * 4 < ((v >> 6) == 3 ? 8 : 4)) {
-          atomicOr(&g_error_flags, ERRF_BAD_MAP);
-          v = 0;
-        }
-        if (h && cy * 4 < ((h >> 6) == 3 ? 8 : 4)) {
-          atomicOr(&g_error_flags, ERRF_BAD_MAP);
-          h = 0;
-        }
-        dv[m] = v;
-        if (i >= 2 && i <= 2 + kFT / 4 && j < kFT / 4) dh[m] = h;
+    for (int m = 0; m < 2; m++) {
+      const int k = tid + m * 256;
+      if (k >= kFCells) break;
+      const int i = k / kFCC, j = k - i * kFCC;
+      const int cx = cx0 + j, cy = cy0 + i;
+      if (cx < 0 || cy < 0 || cx >= gw || cy >= gh) continue;
+      int v = 0, h = 0;
+      lf_decide2(f, tb, plane, cx, cy, v, h);
+      // a conformant map keeps wide edges off the plane start
+      if (v && cx * 4 < ((v >> 6) == 3 ? 8 : 4)) {
+        atomicOr(&g_error_flags, ERRF_BAD_MAP);
+        v = 0;
       }
+      if (h && cy * 4 < ((h >> 6) == 3 ? 8 : 4)) {
+        atomicOr(&g_error_flags, ERRF_BAD_MAP);
+        h = 0;
+      }
+      dv[m] = v;
+      if (i >= 2 && i <= 2 + kFT / 4 && j < kFT / 4) dh[m] = h;
     }
     // u8 samples widen to the u16 window
 #pragma unroll
     for (int m = 0; m < 4; m++) {
       const int k = tid + m * 256;
       const int r = k / 10, ch = k - r * 10;
-      if (sb != 1 || k >= kFChunks || r < r_lo || r >= r_hi || ch < c_lo || ch >= c_hi) continue;
+      if (sb != 1 || k >= kFChunks) continue;
       const int gy = wy0 + r, gx = wx0 + ch * 8;
       if (gy < 0 || gy >= src.h || gx < 0 || gx + 8 > src.w) continue;
       uint16_t* wp = &W[r * kFS + ch * 8];
@@ -525,49 +519,47 @@ __global__ void __launch_bounds__(256, kFusedCtas<F>) lf_fused_kernel(const __gr
                      __byte_perm(q8[m].y, 0, 0x4140), __byte_perm(q8[m].y, 0, 0x4342));
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (filt) {
-      // --- the active edges of each pass, grouped by filter size ---
-      uint32_t iv[2], ih[2];
+    // --- the active edges of each pass, grouped by filter size ---
+    uint32_t iv[2], ih[2];
 #pragma unroll
-      for (int m = 0; m < 2; m++) {
-        iv[m] = dv[m] ? atomicAdd(&cnt[0][dv[m] >> 6], 1u) : 0u;
-        ih[m] = dh[m] ? atomicAdd(&cnt[1][dh[m] >> 6], 1u) : 0u;
+    for (int m = 0; m < 2; m++) {
+      iv[m] = dv[m] ? atomicAdd(&cnt[0][dv[m] >> 6], 1u) : 0u;
+      ih[m] = dh[m] ? atomicAdd(&cnt[1][dh[m] >> 6], 1u) : 0u;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      uint32_t run = 0;
+      for (int c = 3; c >= 1; c--) {
+        base[tid][c] = run;
+        run += cnt[tid][c];
       }
-      __syncthreads();
-      if (tid < 2) {
-        uint32_t run = 0;
-        for (int c = 3; c >= 1; c--) {
-          base[tid][c] = run;
-          run += cnt[tid][c];
-        }
-        cnt[tid][0] = run;  // the pass's edge count
-      }
-      __syncthreads();
+      cnt[tid][0] = run;  // the pass's edge count
+    }
+    __syncthreads();
 #pragma unroll
-      for (int m = 0; m < 2; m++) {
-        const int k = tid + m * 256;
-        const int i = k / kFCC, j = k - i * kFCC;
-        if (dv[m]) list_v[base[0][dv[m] >> 6] + iv[m]] = uint32_t(j) | (uint32_t(i) << 5) | (uint32_t(dv[m]) << 10);
-        if (dh[m]) list_h[base[1][dh[m] >> 6] + ih[m]] = uint32_t(j) | (uint32_t(i - 2) << 5) | (uint32_t(dh[m]) << 10);
-      }
-      __syncthreads();
-      const int bd = f.bd, sharp = f.sharpness;
-      const bool chroma = plane != 0;
-      // --- vertical edges: (edge, two rows) per thread ---
-      const int nv = int(cnt[0][0]) * 2;
-      for (int t = tid; t < nv; t += 256) {
-        const uint32_t e = list_v[t >> 1];
-        const int j = int(e & 31u), i = int((e >> 5) & 31u), d = int(e >> 10);
-        lf_pair_rows(&W[(i * 4 + (t & 1) * 2) * kFS + kFH + j * 4], kFS, d >> 6, chroma, bd, d & 63, sharp);
-      }
-      __syncthreads();
-      // --- horizontal edges: (edge, two columns) per thread ---
-      const int nh = int(cnt[1][0]) * 2;
-      for (int t = tid; t < nh; t += 256) {
-        const uint32_t e = list_h[t >> 1];
-        const int j = int(e & 31u), i = int((e >> 5) & 31u), d = int(e >> 10);
-        lf_pair_cols(&W[(kFH + i * 4) * kFS + kFH + j * 4 + (t & 1) * 2], kFS, d >> 6, chroma, bd, d & 63, sharp);
-      }
+    for (int m = 0; m < 2; m++) {
+      const int k = tid + m * 256;
+      const int i = k / kFCC, j = k - i * kFCC;
+      if (dv[m]) list_v[base[0][dv[m] >> 6] + iv[m]] = uint32_t(j) | (uint32_t(i) << 5) | (uint32_t(dv[m]) << 10);
+      if (dh[m]) list_h[base[1][dh[m] >> 6] + ih[m]] = uint32_t(j) | (uint32_t(i - 2) << 5) | (uint32_t(dh[m]) << 10);
+    }
+    __syncthreads();
+    const int bd = f.bd, sharp = f.sharpness;
+    const bool chroma = plane != 0;
+    // --- vertical edges: (edge, two rows) per thread ---
+    const int nv = int(cnt[0][0]) * 2;
+    for (int t = tid; t < nv; t += 256) {
+      const uint32_t e = list_v[t >> 1];
+      const int j = int(e & 31u), i = int((e >> 5) & 31u), d = int(e >> 10);
+      lf_pair_rows(&W[(i * 4 + (t & 1) * 2) * kFS + kFH + j * 4], kFS, d >> 6, chroma, bd, d & 63, sharp);
+    }
+    __syncthreads();
+    // --- horizontal edges: (edge, two columns) per thread ---
+    const int nh = int(cnt[1][0]) * 2;
+    for (int t = tid; t < nh; t += 256) {
+      const uint32_t e = list_h[t >> 1];
+      const int j = int(e & 31u), i = int((e >> 5) & 31u), d = int(e >> 10);
+      lf_pair_cols(&W[(kFH + i * 4) * kFS + kFH + j * 4 + (t & 1) * 2], kFS, d >> 6, chroma, bd, d & 63, sharp);
     }
     __syncthreads();
     // Up to here the tile read only this call's inputs (the unfiltered

@@ -291,26 +291,28 @@ int build_plan(const FrameJob* jobs, int n, uint8_t* scratch_base, Plan& plan, s
         d.cur[k] = d.in[k];
         continue;
       }
+      plan.any_lf = true;
+      const int sx = k ? d.ssx : 0, sy = k ? d.ssy : 0;
+      const int gw = i->mi_cols >> sx, gh = i->mi_rows >> sy;
       if (fused) {
         // one flag per 64x64 tile of the fused kernel
-        const int tx = (d.in[k].w + kTile - 1) / kTile, ty = (d.in[k].h + kTile - 1) / kTile;
+        const int tx = (gw * 4 + kTile - 1) / kTile, ty = (gh * 4 + kTile - 1) / kTile;
         d.lf_flag_base[k] = int32_t(nflags);
         d.lf_tiles_x[k] = tx;
         nflags += size_t(tx) * size_t(ty);
       } else {
         flags_fit = false;
       }
-      plan.any_lf = true;
-      const int sx = k ? d.ssx : 0, sy = k ? d.ssy : 0;
-      const int gw = i->mi_cols >> sx, gh = i->mi_rows >> sy;
       if (j.in_place_lf) {
         d.cur[k] = d.in[k];
         if (items) add_tiles(plan.lf_items, fi, k, 2, gw * 4, gh * 4, kTile, kTile);
       } else if (fused) {
-        // copy in -> cur with both passes filtered per tile
+        // copy in -> cur with both passes filtered per tile, of the mode-info
+        // area: no later stage reads beyond it, and every tile is then one that
+        // CDEF waits for (a tile that none waits for could be written after the
+        // call's last kernel)
         d.cur[k] = bump.plane(d.in[k].w, d.in[k].h, sb);
-        if (items) add_tiles(plan.lff_items, fi, k, 1, d.in[k].w, d.in[k].h, kTile, kTile, gw * 4, gh * 4,
-                             2);
+        if (items) add_tiles(plan.lff_items, fi, k, 0, gw * 4, gh * 4, kTile, kTile);
       } else if (!tiles) {
         // copy in -> cur and decide every 4x4 edge into the two edge lists
         d.cur[k] = bump.plane(d.in[k].w, d.in[k].h, sb);
