@@ -212,6 +212,13 @@ void Ctx::reap_captured(bool all) {
   if (!shared) retired.clear();
 }
 
+// Zero before anything else runs: a plain cudaMemset returns before it has run
+// and waits for the legacy stream's work, which the calls' streams need not.
+cudaError_t Ctx::clear_words(cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(words, 0, kWords * 4, s);
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 cudaError_t Ctx::upload_stream() {
   cudaError_t e = cudaSuccess;
   if (!upload) {
@@ -357,7 +364,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
       if (q.used && (e = cudaEventSynchronize(q.done)) != cudaSuccess) return cuda_status(e, "epoch wait");
       q.ready = false;
     }
-    if ((e = cudaMemset(words, 0, kWords * 4)) != cudaSuccess) return cuda_status(e, "epoch words");
+    if ((e = clear_words(upload)) != cudaSuccess) return cuda_status(e, "epoch words");
     epoch = 0;
   }
   const int turn = meta_next;
@@ -571,9 +578,9 @@ int av1pf_ctx_create(int device, uint64_t hbm_cap_bytes, av1pf_ctx** out) {
   c->device = device;
   c->cap = hbm_cap_bytes;
   if ((e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking)) != cudaSuccess ||
-      (e = cudaMalloc(&c->words, Ctx::kWords * 4)) != cudaSuccess ||
-      (e = cudaMemset(c->words, 0, Ctx::kWords * 4)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaMalloc(&c->words, Ctx::kWords * 4)) != cudaSuccess ||
+      (e = c->clear_words(c->own)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming)) != cudaSuccess) {
     delete c;

@@ -168,6 +168,7 @@ struct Ctx {
   void reap_captured(bool all);
   int ensure_scratch(size_t bytes);
   cudaError_t upload_stream();
+  cudaError_t clear_words(cudaStream_t s);
   int launch_on(uint8_t* dmeta, cudaStream_t s, const SyncFlags& call);
 };
 
