@@ -322,6 +322,11 @@ int Server::start_batch(InFlight& b, std::vector<Request*>& reqs) {
 
 void Server::run() {
   cudaSetDevice(ctx->device);
+  // This thread's queries and allocations are its own: in the default mode they
+  // fail while any other thread captures a graph in global mode, and end its
+  // capture.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   prctl(PR_SET_TIMERSLACK, 1000UL);  // this thread's waits end within 1 us of their time, not 50
   std::unique_lock<std::mutex> lk(mu);
   while (!stop) {
