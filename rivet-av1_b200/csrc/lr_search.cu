@@ -37,6 +37,7 @@ constexpr int kB = 3;            // window border (postfilter.rs:744 LRB)
 constexpr int kStrip = 64;  // columns of a strip
 constexpr int kStripPx = kStrip * kMaxH;
 constexpr int kWienerThreads = 160;  // a warp that adds and four that produce
+constexpr int kWienerWarps = kWienerThreads / 32;
 constexpr int kWienerCols = 6;  // columns a producing lane has: units reach 256 + 127 columns, two warps a row
 __constant__ int32_t kSgrParams[16][4] = AV1T_SGR_PARAMS;
 __constant__ int32_t kWienerMin[3] = AV1T_WIENER_TAPS_MIN, kWienerMax[3] = AV1T_WIENER_TAPS_MAX;
@@ -277,8 +278,20 @@ namespace {
 // banks for 16-byte loads. A chunk is two rows, of units of up to 32 columns four:
 // a column for each producing lane of a 64-column unit and of a 32-column one.
 __host__ __device__ constexpr int lr_window_stride(int wmax) { return (wmax + 2 * kB + 7) & ~7; }
+// A warp's share of a rectangle's rows, walked in fours, and the rows that the
+// warps' shares reach over, past the rectangle's last.
+__host__ __device__ constexpr int wiener_share(int h) { return ((h + kWienerWarps - 1) / kWienerWarps + 3) & ~3; }
+constexpr int wiener_reach(int h) { return (h + wiener_share(h) - 1) / wiener_share(h) * wiener_share(h); }
+__host__ __device__ constexpr int lr_window_rows(int hmax) { return ((hmax + 15) & ~15) + 2 * kB; }
+constexpr bool reach_fits() {
+  for (int hmax = 1; hmax <= kMaxH; hmax++)
+    for (int h = 1; h <= hmax; h++)
+      if (wiener_reach(h) + 2 * kB > lr_window_rows(hmax)) return false;
+  return true;
+}
+static_assert(reach_fits(), "a share's last rows are inside the window");
 __host__ __device__ constexpr size_t lr_window_bytes(int wmax, int hmax) {
-  return size_t(((hmax + 3) & ~3) + 2 * kB) * lr_window_stride(wmax) * 2;  // (rows are walked in fours)
+  return size_t(lr_window_rows(hmax)) * lr_window_stride(wmax) * 2;
 }
 __host__ __device__ constexpr int wiener_cols(int w, int step) { return (w + step - 1) / step; }
 __host__ __device__ constexpr int wiener_row(int cols) { return (cols + 7) & ~7; }
@@ -415,7 +428,7 @@ __global__ void __launch_bounds__(kWienerThreads, 4) lr_search_wiener_kernel(con
   const LrSearchFrame& F = d.frames[job.frame];
   const int p = job.plane, x0 = job.x0, w = job.w, sb = F.sb, tid = threadIdx.x, step = d.step;
   const int lane = tid & 31, warp = tid >> 5;
-  constexpr int nw = kWienerThreads / 32;
+  constexpr int nw = kWienerWarps;
   const bool unit = job.nr == 1 && w <= kStrip;  // one strip: its source and window are staged once
   const Smem sm = smem_of(lrs_smem, d);
   uint16_t* usrc = reinterpret_cast<uint16_t*>(sm.region);
@@ -428,10 +441,10 @@ __global__ void __launch_bounds__(kWienerThreads, 4) lr_search_wiener_kernel(con
     return unit ? int(usrc[i * kStrip + j]) : ld(F.src[p], sb, x0 + j, rc.y0 + i);
   };
   // Each rectangle's columns in strips of 64, two a lane, its rows a warp's share
-  // of them (a multiple of 4): run(rc, x, win, i0, per, left, cols, pair), where
+  // of them: run(rc, x, win, i0, per, left, cols, pair), where
   // pair(i) is a row's two source samples, clamped to the rectangle.
   auto strips = [&](const LrSearchRect& rc, auto run) {
-    const int per = ((rc.h + nw - 1) / nw + 3) & ~3, i0 = warp * per;
+    const int per = wiener_share(rc.h), i0 = warp * per;
     if (i0 >= rc.h) return;
     for (int x = 0; x < w; x += kStrip) {
       const int c = x + 2 * lane, cols = min(w - c, 2), left = cols > 0 ? min(rc.h - i0, per) : 0;

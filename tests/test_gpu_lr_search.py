@@ -74,3 +74,11 @@ def test_self_guided_extremes(ctx, bd, shift):
     cdef = planes(base, lambda p, a: maxv * (rng.random(a.shape) < 0.5))
     src = planes(cdef, lambda p, a: maxv - a.astype(np.int64))
     compare(ctx, sf, cdef, cdef, src, 0.0, 1)
+
+
+@pytest.mark.parametrize("height", [25, 41, 49, 52, 56])
+def test_one_stripe(ctx, height):
+    """Planes of one stripe, whose rows the warps' shares reach past, in wide units."""
+    sf = A.SynthHandle(width=330, height=height, bit_depth=10, seed=81, enable_lr=1, lr_unit_shift=2, lr_uv_shift=0)
+    cur, cdef, src = O.lr_search_inputs(sf, 82)
+    compare(ctx, sf, cur, cdef, src, 10.0, 1)
