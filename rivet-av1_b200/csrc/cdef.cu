@@ -727,8 +727,8 @@ __device__ __forceinline__ void warp_reduce_pairs(const uint32_t (&acc)[N], uint
   }
 }
 
-// The encoder's CDEF search, error tables (encoder/cdef.rs:103-190): one CTA
-// per 64x64 block, 256 threads. The block's planes are staged as in the
+// The encoder's CDEF search, error tables (encoder/cdef.rs:103-190), of a
+// launch's 12-bit frames: one CTA per 64x64 block, 256 threads. The block's planes are staged as in the
 // decoder's kernel (2-sample border, kNA outside the mode-info area) with
 // the source beside them (kNA outside the frame, so block_sse's crop,
 // encoder/cdef.rs:261-285, is a test per sample); the direction search is
@@ -739,7 +739,7 @@ __device__ __forceinline__ void warp_reduce_pairs(const uint32_t (&acc)[N], uint
 // grid covers every block of n frames: frame i's blocks start at CTA
 // ds[i].block0.
 template <bool TH>
-__global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDesc* __restrict__ ds, int n, int min_bd) {
+__global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDesc* __restrict__ ds, int n) {
   constexpr int NYP = TH ? 11 : 7, NUVP = TH ? 8 : 5, NYS = 4, NUVS = 3;
   constexpr int NY = NYP * NYS, NUV = NUVP * NUVS;
   constexpr int R = 64, top = 2, wrows = R + 2 * top;
@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDes
   __shared__ uint64_t red[8][kSearchMaxY + kSearchMaxUV];
   const CdefSearchDesc& d = ds[search_frame(ds, n, int(blockIdx.x))];
   const FrameDesc& f = *d.frame;
-  if (f.bd < min_bd) return;  // the packed kernel's
+  if (f.bd <= 10) return;  // the packed kernel's
   CdefGreedy* g = d.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int fb = int(blockIdx.x) - d.block0, nfb = d.fb_rows * d.fb_cols;
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDes
   if (tid < 16) doff[tid >> 1][tid & 1] = int16_t(c_cdef_dirs[tid >> 1][tid & 1][0] * kS + c_cdef_dirs[tid >> 1][tid & 1][1]);
   if (tid < 32) (&uvdir[0][0][0])[tid] = (&c_cdef_uv_dir[0][0][0])[tid];
   if (tid == 0) s_one = 1;
-  const int np = f.np, sb = f.sb, cs = f.bd - 8;
+  const int np = f.np, cs = f.bd - 8;
   // --- the 8x8 blocks CDEF filters (encoder/cdef.rs:106-112) ---
   if (tid < R) {
     const int by = tid >> 3, bx = tid & 7;
@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(256, 2) cdef_search_kernel(const CdefSearchDes
     for (int k = tid; k < pw * ph; k += blockDim.x) {
       const int r = k / pw, c = k - r * pw;
       const int gx = x0 + c, gy = y0 + r;
-      sp[r * kS + c] = (gx < fw && gy < fh) ? int16_t(ld_sample(d.src[p], sb, gx, gy)) : kNA;
+      sp[r * kS + c] = (gx < fw && gy < fh) ? int16_t(ld_sample(d.src[p], 2, gx, gy)) : kNA;
     }
   }
   __syncthreads();
@@ -989,9 +989,9 @@ void launch_cdef_search(const CdefSearchDesc* ds, int n, int blocks, bool thorou
   if (shallow) launch_cdef_search_packed(ds, n, blocks, thorough, s);
   if (!deep) return;
   if (thorough)
-    cdef_search_kernel<true><<<blocks, 256, kSearchSmem, s>>>(ds, n, 11);
+    cdef_search_kernel<true><<<blocks, 256, kSearchSmem, s>>>(ds, n);
   else
-    cdef_search_kernel<false><<<blocks, 256, kSearchSmem, s>>>(ds, n, 11);
+    cdef_search_kernel<false><<<blocks, 256, kSearchSmem, s>>>(ds, n);
   note_launch();
 }
 

@@ -369,7 +369,6 @@ __global__ void __launch_bounds__(4 * R, 256 / R) cdef_packed_kernel(const __gri
                                                      const Item* __restrict__ items, int n_items,
                                                                   SyncFlags flags) {
   AV1PF_TRACE_BEGIN();
-  constexpr int NT = 4 * R;
   extern __shared__ __align__(16) uint8_t packed_base[];
   uint16_t* const dwin = reinterpret_cast<uint16_t*>(packed_base);                 // [R][kDS]
   uint32_t* const lw = reinterpret_cast<uint32_t*>(packed_base + R * kDS * 2);     // [R][kPS]: rows i - 2 and i + 2

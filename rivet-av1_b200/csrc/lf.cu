@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(256, 5) lf_search_kernel(const LfSearchDesc* _
       }
       __syncthreads();
     }
-    // at most 16 samples a thread, squares below 2^24: the sum fits 32 bits
+    // at most three chunks, 24 samples a thread: 24 * 4095^2 < 2^32
     uint32_t acc = 0;
     const uint16_t* P = on ? W : W0;
 #pragma unroll

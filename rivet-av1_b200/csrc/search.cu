@@ -1,7 +1,8 @@
-// search.cu — the encoder's filter searches on the device: the greedy choice
-// of CDEF strength pairs (encoder/cdef.rs:195-250) over the error table that
-// cdef_search_kernel (cdef.cu) fills, and the plane errors of the
-// loop-filter level search (encoder/mod.rs:1494-1506).
+// search.cu — the greedy choice of the encoder's CDEF search on the device:
+// strength pairs (encoder/cdef.rs:195-250) over the error tables that
+// cdef_search_packed_kernel (cdef_packed.cu; up to 10 bits) and
+// cdef_search_kernel (cdef.cu; 12 bits) fill, and those tables turned for the
+// caller.
 //
 // The reference sums block errors into an f64 in block order
 // (`total += best as f64`). Every block error is an integer far below 2^53,
