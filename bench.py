@@ -67,9 +67,9 @@ HEADLINE_WORKLOAD = "1920x1080 10-bit 4:2:0 single-frame post-filter chain (LF+C
 # (they reach DRAM later, during the next launches). The headline frames have no film grain: the
 # loop-restoration kernel packs them and no output kernel runs.
 NCU_HEADLINE = {
-    "loop_filter": {"dram_read": 8354048, "dram_write": 0, "warp_inst": 8443133},  # lf_fused_kernel (mode 3)
-    "cdef": {"dram_read": 7251456, "dram_write": 4608, "warp_inst": 10472039},
-    "loop_restoration": {"dram_read": 6830592, "dram_write": 0, "warp_inst": 9491721},
+    "loop_filter": {"dram_read": 7911168, "dram_write": 0, "warp_inst": 7399660},  # lf_fused_kernel (mode 3)
+    "cdef": {"dram_read": 7249664, "dram_write": 3584, "warp_inst": 10478159},
+    "loop_restoration": {"dram_read": 6832384, "dram_write": 0, "warp_inst": 9491721},
 }
 B200_SMS, ISSUE_PER_SM_CLK = 148, 4  # four schedulers per SM, one warp-instruction each per clock
 

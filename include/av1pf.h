@@ -306,7 +306,10 @@ int av1pf_output_noalloc(const av1pf_frame_info* info, const av1pf_params* param
  * filtered) differs from that of the calls before it first uploads its work
  * lists, and may wait on the host for the chain queued two calls earlier.
  * The parameters are read before the call returns; the planes and maps when
- * the kernels run.
+ * the kernels run, in stream order: an input may be what a call before this
+ * one writes. (The kernels are launched with programmatic stream
+ * serialization: a kernel of the caller's that writes an input and comes right
+ * before the call must not itself let dependents launch early.)
  *
  * `stream` may be in capture (any mode; so with the stage calls above): the
  * parameters are then those of every replay, and the call's work lists and
@@ -488,7 +491,10 @@ typedef struct av1pf_serve_config {
   uint64_t hbm_cap_bytes;  /* admission cap on resident stream + batch memory */
   int32_t max_batch_frames; /* most frames one tick takes (0 = 64) */
   int32_t inflight_batches; /* batches on the device at once (0 = 2) */
-  int32_t tick_us;          /* longest wait for more work before a tick */
+  int32_t tick_us;          /* longest wait for more work before a tick (0 = 100).
+                               While batches run on the device the worker thread
+                               looks for their end every 10 us whatever this
+                               says, which takes a good part of a core */
   int32_t slots_per_stream; /* frames of one stream resident at once (0 = 2);
                                more slots let one batch take more of a
                                stream's queued frames */

@@ -15,7 +15,10 @@
 // 32-bit kernel: 36.0 -> 25.5 us (cold, under ncu), 16.2 M -> 10.0 M warp
 // instructions; the chain call 70.4 -> 64.1 us, a 4K 10-bit superres chain
 // 274 -> 243 us, a batch of 16 mixed frames 831 -> 706 us. What is left is
-// latency: loads at a CTA's start and barriers between its phases.
+// latency: loads at a CTA's start and barriers between its phases. 64 registers
+// a thread, for eight half-superblock CTAs an SM, do not hold the staging's
+// chunks and addresses or the filter's taps: 236-308 bytes a thread go to local
+// memory and come back (-Xptxas -v).
 //
 // Which samples share a word: in luma, rows r and r + 4 of an 8x8 block; in
 // chroma, the U and V samples of a position (one block's chroma planes take

@@ -126,8 +126,8 @@ __device__ __forceinline__ void pdl_wait() {
 // that a CTA of the successor holds) and waits per item for the flags of
 // the data it reads. The chain's last stage (loop restoration) waits for
 // flags that every CDEF item sets after its last read of the loop filter's
-// output, so when that stage's grid is complete no kernel of the chain
-// reads or writes the chain's buffers any more.
+// output, and CDEF for every loop-filter tile, so when that stage's grid is
+// complete no kernel of the chain reads or writes the chain's buffers any more.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Per-CTA timeline, in the AV1PF_TRACE build only (libav1pf_trace.so, read

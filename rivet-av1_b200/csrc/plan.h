@@ -58,7 +58,7 @@ struct Plan {
   // instead of on the whole previous stage: every frame runs the fused loop filter,
   // CDEF and loop restoration, without superres or the horizontal
   // loop-filter pass inside CDEF; n_flags flags at off_flags in the meta
-  // buffer, cleared before every call
+  // buffer, set to rising call numbers (batches clear them before every run)
   bool flag_sync = false;
   size_t n_flags = 0, off_flags = 0;
   // A call's own film-grain scratch (templates, scaling tables, block
