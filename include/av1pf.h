@@ -307,9 +307,9 @@ int av1pf_output_noalloc(const av1pf_frame_info* info, const av1pf_params* param
  * lists, and may wait on the host for the chain queued two calls earlier.
  * The parameters are read before the call returns; the planes and maps when
  * the kernels run, in stream order: an input may be what a call before this
- * one writes. (The kernels are launched with programmatic stream
- * serialization: a kernel of the caller's that writes an input and comes right
- * before the call must not itself let dependents launch early.)
+ * one writes, on any context. (The kernels are launched with programmatic
+ * stream serialization: a kernel of the caller's that writes an input and comes
+ * right before the call must not itself let dependents launch early.)
  *
  * `stream` may be in capture (any mode; so with the stage calls above): the
  * parameters are then those of every replay, and the call's work lists and

@@ -7,8 +7,13 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
+#include <map>
 #include <mutex>
 #include <string>
+#include <thread>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "av1pf.h"
@@ -143,41 +148,67 @@ inline void end() {}
 #endif
 }  // namespace pipe_trace
 
+namespace written {
 namespace {
-std::pair<uintptr_t, uintptr_t> span_of(const av1pf_plane& p, int w, int h, int sb) {
+using Span = std::pair<uintptr_t, uintptr_t>;  // [first, past the last)
+// (a per-thread default stream is one of each thread)
+using Key = std::tuple<int, cudaStream_t, unsigned long long, std::thread::id>;
+constexpr size_t kMostSpans = 128, kMostStreams = 64;
+std::mutex g_mu;
+std::map<Key, std::vector<Span>> g_spans;
+
+Key key_of(int device, cudaStream_t s, unsigned long long capture) {
+  return {device, s, capture, s == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id()};
+}
+Span span_of(const av1pf_plane& p, int sb) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(p.data);
-  return {at, at + uintptr_t((int64_t(h - 1) * p.stride + w) * sb)};
+  return {at, at + uintptr_t((int64_t(p.height - 1) * p.stride + p.width) * sb)};
 }
 }  // namespace
 
-bool Written::holds_input(const FrameJob* jobs, int n) const {
+bool must_wait(int device, cudaStream_t s, unsigned long long capture, const FrameJob* jobs, int n) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  const auto it = g_spans.find(key_of(device, s, capture));
+  if (it == g_spans.end() || it->second.size() > kMostSpans) return true;
   for (int fi = 0; fi < n; fi++) {
     const FrameJob& j = jobs[fi];
     for (int k = 0; k < j.info->num_planes; k++)
       for (const av1pf_plane* in : {j.in, j.cur}) {
         if (!in) continue;
-        const auto s = span_of(in[k], in[k].width, in[k].height, j.info->sample_bytes);
-        for (const auto& w : spans)
-          if (s.first < w.second && w.first < s.second) return true;
+        const Span i = span_of(in[k], j.info->sample_bytes);
+        for (const Span& w : it->second)
+          if (i.first < w.second && w.first < i.second) return true;
       }
   }
   return false;
 }
 
-void Written::add(const FrameJob* jobs, int n) {
-  auto put = [&](const std::pair<uintptr_t, uintptr_t>& s) {
-    if (std::find(spans.begin(), spans.end(), s) == spans.end()) spans.push_back(s);
+void add(int device, cudaStream_t s, unsigned long long capture, const FrameJob* jobs, int n, bool ahead) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  const Key key = key_of(device, s, capture);
+  // (streams come and go: one that is dropped here is unknown to its next call)
+  if (g_spans.size() >= kMostStreams && !g_spans.count(key)) g_spans.clear();
+  std::vector<Span>& spans = g_spans[key];
+  if (!ahead) spans.clear();
+  auto put = [&](const Span& w) {
+    if (std::find(spans.begin(), spans.end(), w) == spans.end()) spans.push_back(w);
   };
   for (int fi = 0; fi < n; fi++) {
     const FrameJob& j = jobs[fi];
-    for (int k = 0; j.out && k < j.info->num_planes; k++)
-      put(span_of(j.out[k], j.out[k].width, j.out[k].height, j.info->sample_bytes));
+    for (int k = 0; j.out && k < j.info->num_planes; k++) put(span_of(j.out[k], j.info->sample_bytes));
     if (j.frame_out) {
       const uintptr_t at = reinterpret_cast<uintptr_t>(j.frame_out);
       put({at, at + packed_frame_bytes(j.info)});
     }
   }
 }
+
+void forget(int device, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  for (auto it = g_spans.begin(); it != g_spans.end();)
+    it = std::get<0>(it->first) == device && std::get<1>(it->first) == s ? g_spans.erase(it) : std::next(it);
+}
+}  // namespace written
 
 // The scratch of direct calls. One that captured calls share is kept for their
 // replays when it is outgrown.
@@ -271,10 +302,8 @@ int Ctx::capture(const FrameJob* jobs, int n, cudaStream_t s) {
     if (e == cudaSuccess) {
       // (calls captured one after another overlap as direct ones do)
       SyncFlags call;
-      if (capture_id != id) capture_written.spans.clear();
-      capture_id = id;
-      call.whole = capture_written.holds_input(jobs, n) || capture_written.spans.size() > Written::kMost;
-      capture_written.add(jobs, n);
+      call.whole = written::must_wait(device, s, id, jobs, n);
+      written::add(device, s, id, jobs, n, false);
       launch_plan(p, dmeta, s, side, fork, join, nullptr, false, false, false, p.by_value, call);
       e = cudaGetLastError();
     }
@@ -387,8 +416,8 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   // against templates on the side stream and no overlap: 640x360 27.8 / 44.7,
   // 1280x720 53.9 / 52.1, 1920x1080 70.8 / 72.4, 3840x2160 235 / 233).
   // Where an input is what a call before this one writes, this one waits for it
-  // whole before it reads. (The list is of one stream's calls.)
-  const bool whole = unseen || last_stream != s || written.spans.size() > Written::kMost || written.holds_input(jobs, n);
+  // whole before it reads.
+  const bool whole = written::must_wait(device, s, 0, jobs, n);
   const bool chained = !whole && scratch_turns && plan.by_value && !plan.lff_items.empty() && !prof &&
                        (!plan.any_grain || plan.out_items.size() <= size_t(kNumSMs));
   if (plan.by_value && resident) {
@@ -452,11 +481,7 @@ int Ctx::run(const FrameJob* jobs, int n, cudaStream_t s) {
   }
   call.whole = whole;
   chain_run = chained ? before + 1 : 0;
-  // a call that does not run ahead lets the next begin only once the calls
-  // before it on its stream are complete
-  if (!call.ahead) written.spans.clear();
-  written.add(jobs, n);
-  unseen = false;
+  written::add(device, s, 0, jobs, n, call.ahead);
   last_stream = s;
   rc = launch_on(dmeta, s, call);
   cudaEventRecord(m.done, s);

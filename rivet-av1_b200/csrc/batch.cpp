@@ -235,7 +235,7 @@ int av1pf_batch_run(av1pf_batch* b, void* stream) {
     note_launch(b->kernels_per_run);
   } else {
     launch_groups(*b, s);
-    b->ctx->unseen = true;
+    written::forget(b->ctx->device, s);
     e = cudaGetLastError();
   }
   return cuda_status(e, "batch run");

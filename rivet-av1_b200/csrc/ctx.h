@@ -52,14 +52,19 @@ struct CaptureScope {
   uint64_t start;
 };
 
-// The memory that calls write whose end the next call's first kernel may not
-// wait for before it reads its inputs.
-struct Written {
-  static constexpr size_t kMost = 128;
-  std::vector<std::pair<uintptr_t, uintptr_t>> spans;  // [first, past the last)
-  bool holds_input(const FrameJob* jobs, int n) const;
-  void add(const FrameJob* jobs, int n);
-};
+// Per stream (of a capture, where `capture` is its id), over all contexts: the
+// memory that calls write whose end the next call's first kernel may not wait
+// for before it reads its inputs.
+namespace written {
+// Whether the call must wait for the kernel before it ahead of reading: an input
+// is in that memory, or what precedes the call is not known.
+bool must_wait(int device, cudaStream_t s, unsigned long long capture, const FrameJob* jobs, int n);
+// The call's outputs. One that does not run `ahead` lets the next begin only once
+// the calls before it are complete.
+void add(int device, cudaStream_t s, unsigned long long capture, const FrameJob* jobs, int n, bool ahead);
+// The latest launches on the stream, in a capture or not, are no such call's.
+void forget(int device, cudaStream_t s);
+}  // namespace written
 
 struct Ctx {
   int device = 0;
@@ -109,8 +114,6 @@ struct Ctx {
   uint32_t epoch = 0;
   cudaStream_t last_stream = nullptr;  // of the previous call
   int chain_run = 0;                   // chained calls of one structure and stream up to the previous one
-  Written written;
-  bool unseen = false;  // launches that `written` does not cover (batches run without a graph)
   // device words (SyncFlags): [0] the last call known to be complete, [1 + turn]
   // the last call whose film-grain templates are ready in that buffer
   static constexpr int kWords = 64;
@@ -129,8 +132,6 @@ struct Ctx {
     std::shared_ptr<std::atomic<bool>> gone;
   };
   std::vector<Captured> captured;
-  unsigned long long capture_id = 0;
-  Written capture_written;  // by the captured calls of that capture
   std::vector<DevBuf> retired;  // scratches that captured calls share and the context has outgrown
   cudaStream_t upload = nullptr;  // descriptor uploads
   // the chain's stream, not the host, waits for the descriptor upload: set

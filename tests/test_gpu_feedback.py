@@ -1,7 +1,7 @@
 """Chain calls whose input is what a call before them writes, one to three calls
 back, queued without a wait in between: stream order holds for them as for any
-other work. Also from a batch that runs without a graph, and through a captured
-pair of calls. Against the oracle, bit for bit."""
+other work. Also from a batch that runs without a graph, through a captured
+pair of calls, and between two contexts. Against the oracle, bit for bit."""
 import ctypes as C
 
 import numpy as np
@@ -123,3 +123,28 @@ def test_input_written_by_a_captured_call(name):
             fb[k].zero_()
     del g
     ctx.close()
+
+
+@pytest.mark.parametrize("back", [1, 2])
+@pytest.mark.parametrize("name", ["one_tile", "small", "small_grain", "1080p_wide"])
+def test_input_written_by_another_context(name, back):
+    """Two contexts in turn on one stream, each reading what was written one or two calls before."""
+    ctxs, n, calls = [G.Ctx(0), G.Ctx(0)], 6, 9
+    sf = A.SynthHandle(seed=54, **SHAPES[name])
+    d, host = G.DevFrame(sf), buffers(sf, n)
+    steps = walk(n, back, calls)
+    dev = [G.DevPlanes.from_host(sf.f.info, h) for h in host]
+    other, spare = G.DevPlanes.from_host(sf.f.info, host[0]), G.DevPlanes.from_host(sf.f.info, host[1])
+    fbs = [G.dev_bytes(A.frame_bytes(sf.f.info)) for _ in range(calls)]
+    want = [oracle_step(sf, host[a], host[b]) for a, b in steps]
+    for _ in range(4):
+        for k in range(8):
+            gpu_step(ctxs[k % 2], d, other, spare, fbs[0])
+        for k, ((a, b), fb) in enumerate(zip(steps, fbs)):
+            gpu_step(ctxs[k % 2], d, dev[a], dev[b], fb)
+        torch.cuda.synchronize()
+        for k, (fb, w) in enumerate(zip(fbs, want)):
+            assert np.array_equal(fb[: w.size].cpu().numpy(), w), f"call {k}"
+            fb.zero_()
+    for c in ctxs:
+        c.close()
